@@ -801,12 +801,13 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_tcgen05_kernel(const __
     const uint32_t tmem_base = bars->tmem_base;
     const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + 256;
     auto give_up = [&](int code) {
-        if (lane == 0) { atomicExch(P.err, code); *abort_flag = 1u; }
+        atomicExch(P.err, code);
+        *abort_flag = 1u;
     };
 
     if (warp == 0) {
         // ---------------- activation tiles (B operand) ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&P.xmap);
             uint32_t s = 0, ph = 1;      // parity to wait for on stage_free (1 passes on a fresh barrier)
             uint32_t cur, lim;
@@ -828,7 +829,7 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_tcgen05_kernel(const __
         }
     } else if (warp == 2) {
         // ---------------- raw weight groups ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&P.wmap);
             uint32_t r = 0, ph = 1;
             uint32_t cur, lim;
@@ -850,7 +851,7 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_tcgen05_kernel(const __
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, ph = 0, dph = 1;   // dph: parity to wait for on d_free (1 passes the first time)
             uint32_t cur, lim;
             gemm_seg_init(P, cur, lim);
@@ -1098,7 +1099,8 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
     const uint32_t tmem_base = bars->tmem_base;
     const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + 256;
     auto give_up = [&](int code) {
-        if (lane == 0) { atomicExch(P.err, code); *abort_flag = 1u; }
+        atomicExch(P.err, code);
+        *abort_flag = 1u;
     };
     // the pair's tiles: 256 weight rows (pair index wp) x 256 activation rows (xt), xt fastest
     const uint32_t pt0 = blockIdx.x >> 1, pstep = gridDim.x >> 1, plim = (P.wtiles >> 1) * P.xtiles;
@@ -1106,7 +1108,7 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
 
     if (warp == 0) {
         // ---------------- this CTA's half of the activation tile ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&P.xmap);
             uint32_t s = 0, ph = 1;
             bool ok = true;
@@ -1139,7 +1141,7 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
         }
     } else if (warp == 2) {
         // ---------------- raw weight groups of this CTA's 128 rows ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&P.wmap);
             uint32_t r = 0, ph = 1;
             bool ok = true;
@@ -1156,7 +1158,7 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: the first CTA, for both ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             uint32_t s = 0, ph = 0, dph = 1;
             bool ok = true;
             for (uint32_t pt = pt0; ok && pt < plim && !*abort_flag; pt += pstep) {

