@@ -99,46 +99,29 @@ def _torch():
     return torch
 
 
-def _stream_ptr(torch) -> int:
-    return torch.cuda.current_stream().cuda_stream
+_native = None
 
 
-def _dt(t, torch) -> int:
-    if t.dtype == torch.float32:
-        return int(DType.F32)
-    if t.dtype == torch.bfloat16:
-        return int(DType.BF16)
-    raise TypeError(f"activations must be float32 or bfloat16, got {t.dtype}")
+def _ops():
+    """The native form of the calls below (_torch_ops.so): argument checks, output and scratch allocation, the current
+    stream and the library call in one step.  Loaded with the first call, as torch is."""
+    global _native
+    if _native is None:
+        _torch()
+        from . import _torch_ops
+        _torch_ops.set_error(RlxqError)
+        _native = _torch_ops
+    return _native
 
 
 def dequant_f32(w_blocks, scheme: int, n_elems: int, out=None):
     """rlxq_dequant_f32 on a torch uint8 CUDA tensor of raw blocks."""
-    torch = _torch()
-    assert w_blocks.is_cuda and w_blocks.dtype == torch.uint8 and w_blocks.is_contiguous()
-    if out is None:
-        out = torch.empty(n_elems, dtype=torch.float32, device=w_blocks.device)
-    with torch.cuda.device(w_blocks.device):
-        check(lib.rlxq_dequant_f32(_stream_ptr(torch), int(scheme), w_blocks.data_ptr(), n_elems,
-                                   out.data_ptr()))
-    return out
+    return (_native or _ops()).dequant_f32(w_blocks, scheme, n_elems, out)
 
 
 def matmul(x, w_blocks, scheme: int, n: int, out=None, out_dtype=None, workspace=None):
     """rlxq_matmul: y[m,n] = x[m,k] . W^T for torch CUDA tensors (x f32 or bf16)."""
-    torch = _torch()
-    assert x.is_cuda and x.dim() == 2 and x.is_contiguous()
-    assert w_blocks.is_cuda and w_blocks.dtype == torch.uint8 and w_blocks.is_contiguous()
-    m, k = x.shape
-    if out is None:
-        out = torch.empty((m, n), dtype=out_dtype or torch.float32, device=x.device)
-    need = workspace_bytes(scheme, m, k, n, _dt(x, torch), _dt(out, torch))
-    if need and (workspace is None or workspace.numel() < need):
-        workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        check(lib.rlxq_matmul(_stream_ptr(torch), int(scheme), x.data_ptr(), _dt(x, torch),
-                              w_blocks.data_ptr(), out.data_ptr(), _dt(out, torch), m, k, n,
-                              workspace.data_ptr() if need else None, need))
-    return out
+    return (_native or _ops()).matmul(x, w_blocks, scheme, n, out, out_dtype, workspace)
 
 
 class ChainLayer(C.Structure):
@@ -149,27 +132,7 @@ class ChainLayer(C.Structure):
 def matmul_chain(x, layers, scheme: int, out=None, out_dtype=None, workspace=None):
     """rlxq_matmul_chain: `layers` is a list of (w_blocks, n) or (w_blocks, n, swiglu) in order; layer i takes the
     previous layer's output (or, with swiglu, the product up * silu(gate) of its [gate | up] halves).  CUDA tensors."""
-    torch = _torch()
-    assert x.is_cuda and x.dim() == 2 and x.is_contiguous()
-    m, width = x.shape
-    arr = (ChainLayer * len(layers))()
-    for i, ly in enumerate(layers):
-        w, n = ly[0], int(ly[1])
-        sw = int(bool(ly[2])) if len(ly) > 2 else 0
-        assert w.is_cuda and w.dtype == torch.uint8 and w.is_contiguous()
-        k = width // 2 if sw else width
-        arr[i] = ChainLayer(w.data_ptr(), k, n, sw)
-        width = n
-    if out is None:
-        out = torch.empty((m, width), dtype=out_dtype or torch.float32, device=x.device)
-    need = C.c_size_t()
-    check(lib.rlxq_chain_workspace_bytes(int(scheme), C.cast(arr, C.c_void_p), len(layers), m, _dt(x, torch), C.byref(need)))
-    if workspace is None or workspace.numel() < need.value:
-        workspace = torch.empty(max(need.value, 256), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        check(lib.rlxq_matmul_chain(_stream_ptr(torch), int(scheme), C.cast(arr, C.c_void_p), len(layers), x.data_ptr(),
-                                    _dt(x, torch), out.data_ptr(), _dt(out, torch), m, workspace.data_ptr(), workspace.numel()))
-    return out
+    return (_native or _ops()).matmul_chain(x, layers, scheme, out, out_dtype, workspace)
 
 
 def chain_workspace_bytes(scheme: int, layers, m: int, x_dtype: int = 0) -> int:
@@ -187,23 +150,7 @@ def grouped_matmul(x, w_blocks, expert_idx, scheme: int, n: int, num_experts: in
                    workspace=None):
     """Op::DequantGroupedMatMul: y[i] = x[i] . W_e^T with e = expert_idx[i] (f32-encoded, as the reference's
     graph input); w_blocks holds num_experts packed [n, k] slabs back to back.  CUDA tensors in and out."""
-    torch = _torch()
-    assert x.is_cuda and x.dim() == 2 and x.is_contiguous()
-    assert w_blocks.is_cuda and w_blocks.dtype == torch.uint8 and w_blocks.is_contiguous()
-    assert expert_idx.is_cuda and expert_idx.dtype == torch.float32 and expert_idx.is_contiguous()
-    m, k = x.shape
-    assert expert_idx.numel() == m
-    if out is None:
-        out = torch.empty((m, n), dtype=out_dtype or torch.float32, device=x.device)
-    need = C.c_size_t()
-    check(lib.rlxq_grouped_workspace_bytes(int(scheme), m, k, n, num_experts, C.byref(need)))
-    if workspace is None or workspace.numel() < need.value:
-        workspace = torch.empty(max(need.value, 16), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        check(lib.rlxq_grouped_matmul(_stream_ptr(torch), int(scheme), x.data_ptr(), _dt(x, torch), w_blocks.data_ptr(),
-                                      expert_idx.data_ptr(), out.data_ptr(), _dt(out, torch), m, k, n, num_experts,
-                                      workspace.data_ptr(), need.value))
-    return out
+    return (_native or _ops()).grouped_matmul(x, w_blocks, expert_idx, scheme, n, num_experts, out, out_dtype, workspace)
 
 
 # ------------------------------------------------------------------ tied LM head
@@ -222,38 +169,14 @@ def gguf_tied_lm_topk(hidden, w_bytes, n_embd: int, n_vocab: int, scheme: int, c
     (token id, logit) pairs, best first.  hidden: CUDA tensor [n_embd], f32 or bf16; w_bytes: CUDA uint8
     tensor holding the packed embedding [n_vocab, n_embd].  Returns two CUDA tensors: int32 token ids (-1 where
     fewer than cap rows could be chosen) and f32 logits."""
-    torch = _torch()
-    assert hidden.is_cuda and hidden.is_contiguous() and hidden.numel() == n_embd
-    assert w_bytes.is_cuda and w_bytes.dtype == torch.uint8 and w_bytes.is_contiguous()
-    cap = max(1, min(cap, n_vocab))          # the reference clamps the same way
-    need = lm_head_workspace_bytes(scheme, n_embd, n_vocab, _dt(hidden, torch), cap)
-    if workspace is None or workspace.numel() < need:
-        workspace = torch.empty(need, dtype=torch.uint8, device=hidden.device)
-    idx = torch.empty(cap, dtype=torch.int32, device=hidden.device)
-    val = torch.empty(cap, dtype=torch.float32, device=hidden.device)
-    with torch.cuda.device(hidden.device):
-        check(lib.rlxq_lm_head_topk(_stream_ptr(torch), int(scheme), hidden.data_ptr(), _dt(hidden, torch),
-                                    w_bytes.data_ptr(), n_embd, n_vocab, cap, 1 if exact else 0,
-                                    workspace.data_ptr(), need, idx.data_ptr(), val.data_ptr()))
-    return idx, val
+    # the reference clamps cap the same way
+    return (_native or _ops()).lm_head(hidden, w_bytes, n_embd, n_vocab, scheme, max(1, min(cap, n_vocab)), exact, workspace)
 
 
 def gguf_tied_lm_argmax(hidden, w_bytes, n_embd: int, n_vocab: int, scheme: int, exact: bool = True, workspace=None):
     """rlx_cpu::lm_head::gguf_tied_lm_argmax (rlx-cpu/src/lm_head.rs:223-251) on the GPU: (token id, logit)
     as two one-element CUDA tensors; nothing is copied to the host."""
-    torch = _torch()
-    assert hidden.is_cuda and hidden.is_contiguous() and hidden.numel() == n_embd
-    assert w_bytes.is_cuda and w_bytes.dtype == torch.uint8 and w_bytes.is_contiguous()
-    need = lm_head_workspace_bytes(scheme, n_embd, n_vocab, _dt(hidden, torch), 1)
-    if workspace is None or workspace.numel() < need:
-        workspace = torch.empty(need, dtype=torch.uint8, device=hidden.device)
-    idx = torch.empty(1, dtype=torch.int32, device=hidden.device)
-    val = torch.empty(1, dtype=torch.float32, device=hidden.device)
-    with torch.cuda.device(hidden.device):
-        check(lib.rlxq_lm_head_argmax(_stream_ptr(torch), int(scheme), hidden.data_ptr(), _dt(hidden, torch),
-                                      w_bytes.data_ptr(), n_embd, n_vocab, 1 if exact else 0,
-                                      workspace.data_ptr(), need, idx.data_ptr(), val.data_ptr()))
-    return idx, val
+    return (_native or _ops()).lm_head(hidden, w_bytes, n_embd, n_vocab, scheme, 0, exact, workspace)
 
 
 # ------------------------------------------------------------------ Graph / Session mirror

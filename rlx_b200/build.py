@@ -1,4 +1,5 @@
-"""Builds rlx_b200/librlxq.so (the C-ABI library) with nvcc for sm_100a, in-tree.
+"""Builds rlx_b200/librlxq.so (the C-ABI library) with nvcc for sm_100a, in-tree, and rlx_b200/_torch_ops.so, the
+native form of the Python calls on torch tensors, with the host compiler.
 
     python -m rlx_b200.build [--force] [--verbose]
 
@@ -13,11 +14,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(PKG, "librlxq.so")
+OPS = os.path.join(PKG, "_torch_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -56,6 +59,28 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
+def _build_ops(force: bool) -> None:
+    """csrc/python/torch_ops.cpp against this interpreter, its torch and librlxq.so beside it."""
+    src = os.path.join(CSRC, "python", "torch_ops.cpp")
+    headers = glob.glob(os.path.join(PKG, "..", "include", "*.h"))
+    newest = max(os.path.getmtime(p) for p in [src, *headers])
+    if not force and os.path.exists(OPS) and os.path.getmtime(OPS) >= newest:
+        return
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cmd = [os.environ.get("CXX") or shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"),
+           "-I", os.path.join(PKG, "..", "include"), src, "-o", OPS,
+           "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+           "-L", PKG, "-l:librlxq.so", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {src}:\n{r.stdout}\n{r.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     srcs = sources()
@@ -75,6 +100,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_ops(force)
     return LIB
 
 
