@@ -221,7 +221,8 @@ RLXQ_API uint64_t rlxq_launch_count(void);
  *                  least one tile pair per resident cluster, not Q6_K or Q3_K, no k split chosen), 1 = never, 2 = wherever
  *                  n is a multiple of 256.  Same bits as the single-CTA kernel.  "gemm_pair_clusters" (read only):
  *                  clusters the device keeps resident, 0 until the paired kernel has run
- *   "gemm_tile_x": 0 = automatic, 128 or 256 = activation rows per tile of the tcgen05 GEMM
+ *   "gemm_tile_x": 0 = automatic, a multiple of 32 up to 256 = activation rows per tile of the tcgen05 GEMM (128 at
+ *                  most with f32 activations)
  *   "gemv_inline_q": 0 = automatic, 1 = the integer GEMV always runs its activation quantiser as a
  *                  kernel of its own, 2 = the streaming kernel quantises the activations itself
  *                  whenever the shape allows it

@@ -171,7 +171,7 @@ int rlxq_set_option(const char* key, int64_t value) {
         return RLXQ_OK;
     }
     if (!strcmp(key, "gemm_tile_x")) {
-        if (value != 0 && value != 128 && value != 256) return fail(RLXQ_E_ARG, "gemm_tile_x must be 0, 128 or 256");
+        if (value < 0 || value > 256 || value % 32) return fail(RLXQ_E_ARG, "gemm_tile_x must be 0 or a multiple of 32 up to 256");
         options().gemm_tile_x = value;
         return RLXQ_OK;
     }

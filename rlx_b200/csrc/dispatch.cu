@@ -7,24 +7,44 @@
 
 namespace rlxq {
 
-// Prefill with f32 activations: the tensor-core GEMM takes bf16 operands, so x goes in as hi + lo bf16 halves
-// (twice the rows), `chunk` rows of x at a time, and the two partial results are added.  The scratch holds the
-// 2 * chunk split rows, the 2 * chunk x n f32 partial results (kept under 128 MiB) and the GEMM's own workspace.
-struct SplitPlan { bool ok; uint32_t chunk; size_t off_y2, off_gemm, bytes; };
-static SplitPlan plan_f32_split(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n) {
-    SplitPlan p{};
+// Prefill (m > 8) on the tensor-core GEMM.  Its operands are bf16: f32 activations go in as hi + lo halves, `chunk`
+// rows of x at a time (the split rows are kept under 128 MiB), multiplied by the same decoded weights.  Rows that TMA
+// cannot tile where they lie (k not a whole number of 256 weights, or of the 16-byte groups of a format's super-blocks;
+// weights that are not 16-byte aligned) are first re-laid on a padded pitch in the workspace, and the weight operand then
+// keeps hi and lo parts too, since those shapes were multiplied in f32 before they had this path.
+struct PrefillPlan { bool ok, relaid, halves; uint32_t chunk; uint64_t pitch; size_t off_w, off_y2, off_gemm, bytes; };
+static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, bool direct) {
+    PrefillPlan p{};
+    const void* aligned = (const void*)256;              // dispatch checks the real pointers
     if (m <= 8 || options().gemm_kernel.load() == 1) return p;
-    uint64_t chunk = (128ull << 20) / (8ull * n) / 128 * 128;
-    if (chunk < 128) chunk = 128;
-    if (chunk > 2048) chunk = 2048;
-    if (chunk > m) chunk = m;
-    // the GEMM's own conditions, on an aligned stand-in for the pointers (dispatch checks the real ones)
-    if (!gemm_tc_supported(scheme, 2 * (uint32_t)chunk, k, n, (const void*)256, (const void*)256, true)) return p;
+    p.relaid = !(direct && gemm_tc_supported(scheme, m, k, n, aligned, aligned));
+    if (p.relaid && !gemm_relaid_supported(scheme, m, k, n, aligned)) return p;
     auto al = [](size_t v) { return (v + 255) / 256 * 256; };
+    uint64_t chunk = m;
+    // Rows of at most 512 weights: hi and lo rows go through the GEMM as 2 m rows and their results are added behind it;
+    // the chunk keeps the two results under 128 MiB.
+    p.halves = !xbf && !p.relaid && k <= 512;
+    if (!xbf) {
+        chunk = p.halves ? (128ull << 20) / (8ull * n) / 128 * 128 : (128ull << 20) / (4ull * k) / 256 * 256;
+        const uint64_t least = p.halves ? 128 : 256;
+        if (chunk < least) chunk = least;
+        if (p.halves && chunk > 2048) chunk = 2048;
+        if (chunk > m) chunk = m;
+    }
     p.chunk = (uint32_t)chunk;
-    p.off_y2 = al((size_t)2 * chunk * k * 2);
-    p.off_gemm = p.off_y2 + al((size_t)2 * chunk * n * 4);
-    p.bytes = p.off_gemm + al(gemm_tc_workspace_bytes(2 * (uint32_t)chunk, k, n));
+    p.off_w = xbf ? 0 : al((size_t)2 * chunk * k * 2);
+    p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;
+    p.off_y2 = p.off_w + al((size_t)(p.pitch * n));
+    p.off_gemm = p.off_y2 + (p.halves ? al((size_t)2 * chunk * n * 4) : 0);
+    p.bytes = p.off_gemm;
+    if (!p.halves) {
+        size_t g = gemm_tc_workspace_bytes(scheme, (uint32_t)chunk, k, n, !xbf, p.relaid);
+        if (m % chunk) {                                 // the last, shorter chunk may be split over the SMs differently
+            const size_t g2 = gemm_tc_workspace_bytes(scheme, (uint32_t)(m % chunk), k, n, !xbf, p.relaid);
+            g = g2 > g ? g2 : g;
+        }
+        p.bytes += al(g);
+    }
     p.ok = true;
     return p;
 }
@@ -33,10 +53,6 @@ size_t matmul_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t 
                               uint32_t y_dtype) {
     (void)y_dtype;
     if (m == 0 || n == 0 || k == 0) return 0;
-    if (m > 8 && x_dtype == RLXQ_F32) {
-        const SplitPlan sp = plan_f32_split(scheme, m, k, n);
-        return sp.ok ? sp.bytes : 0;
-    }
     if (m <= 8) {
         // large enough for whichever GEMV kernel the dispatcher (or a forced option) picks
         const size_t a = staged_workspace_bytes(scheme, m, k, n);
@@ -48,7 +64,8 @@ size_t matmul_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t 
         const size_t ab = a > b ? a : b, cd = c > d ? c : d;
         return ab > cd ? ab : cd;
     }
-    return gemm_tc_workspace_bytes(m, k, n);      // partial tiles of the stream-K split, when the shape wants it
+    const PrefillPlan p = plan_prefill(scheme, m, k, n, x_dtype == RLXQ_BF16, true);
+    return p.ok ? p.bytes : 0;
 }
 
 int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y,
@@ -105,31 +122,48 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
         }
         return launch_matmul_generic(stream, scheme, x, xbf, w, y, ybf, m, k, n);
     }
-    // m > 8: tensor-memory GEMM for bf16 activations; for f32 activations the same GEMM on their hi + lo bf16
-    // halves when the caller's workspace holds them; the tiled generic kernel otherwise
+    // m > 8: the tensor-memory GEMM; without the workspace it needs, the tiled generic kernel
     const int64_t gforce = options().gemm_kernel.load();
-    if (!xbf && gforce != 1 && !((uintptr_t)w & 15u) && !((uintptr_t)ws & 255u)) {
-        const SplitPlan sp = plan_f32_split(scheme, m, k, n);
-        if (sp.ok && ws && ws_bytes >= sp.bytes) {
-            uint8_t* base = static_cast<uint8_t*>(ws);
-            for (uint32_t r0 = 0; r0 < m; r0 += sp.chunk) {
-                const uint32_t rows = m - r0 < sp.chunk ? m - r0 : sp.chunk;
-                int rc = launch_split_hi_lo(stream, static_cast<const float*>(x) + (size_t)r0 * k, base, rows, k);
-                if (rc) return rc;
-                rc = launch_gemm_tc(stream, scheme, base, w, base + sp.off_y2, false, 2 * rows, k, n, base + sp.off_gemm,
-                                    sp.bytes - sp.off_gemm);
-                if (rc) return rc;
-                rc = launch_add_halves(stream, reinterpret_cast<const float*>(base + sp.off_y2),
-                                       static_cast<uint8_t*>(y) + (size_t)r0 * n * (ybf ? 2 : 4), ybf, rows, n);
-                if (rc) return rc;
-            }
-            return RLXQ_OK;
-        }
-    }
-    const bool can = gemm_tc_supported(scheme, m, k, n, w, x, xbf);
-    if (gforce == 2 && !can)
+    const bool direct = gemm_tc_supported(scheme, m, k, n, w, x);
+    if (gforce == 2 && (!direct || !xbf))
         return fail(RLXQ_E_SHAPE, "the tcgen05 GEMM needs bf16 activations, k %% 256 == 0 (2048 for Q6_K), one of Q4_0/Q8_0/Q4_K/Q5_K/Q6_K and 16-byte alignment");
-    if (can && gforce != 1) return launch_gemm_tc(stream, scheme, x, w, y, ybf, m, k, n, ws, ws_bytes);
+    const PrefillPlan p = plan_prefill(scheme, m, k, n, xbf, direct);
+    const bool fits = ws && ws_bytes >= p.bytes && !((uintptr_t)ws & 255u);
+    if (p.ok && (fits || (xbf && direct))) {
+        uint8_t* base = static_cast<uint8_t*>(ws);
+        GemmCall c{};
+        c.w = w; c.w_pitch = p.pitch; c.precise = p.relaid; c.k = k; c.n = n;
+        if (p.relaid) {
+            Geometry g;
+            geometry(scheme, &g);
+            int rc = launch_relay_rows(stream, w, (uint64_t)k / g.elems * g.bytes, n, base + p.off_w, p.pitch);
+            if (rc) return rc;
+            c.w = base + p.off_w;
+        }
+        for (uint32_t r0 = 0; r0 < m; r0 += p.chunk) {
+            const uint32_t rows = m - r0 < p.chunk ? m - r0 : p.chunk;
+            void* const out = static_cast<uint8_t*>(y) + (size_t)r0 * n * (ybf ? 2 : 4);
+            c.x = static_cast<const uint8_t*>(x) + (size_t)r0 * k * (xbf ? 2 : 4);
+            if (!xbf) {
+                int rc = launch_split_hi_lo(stream, static_cast<const float*>(c.x), base, rows, k);
+                if (rc) return rc;
+                c.x = base;
+            }
+            int rc;
+            if (p.halves) {
+                float* y2 = reinterpret_cast<float*>(base + p.off_y2);
+                c.x_rows = 2 * rows; c.y = y2;
+                rc = launch_gemm(stream, scheme, c, nullptr, 0);
+                if (!rc) rc = launch_add_slices(stream, y2, 2, (uint64_t)rows * n, out, ybf, (uint64_t)rows * n);
+            } else {
+                c.x_rows = rows; c.f32 = !xbf; c.y = out; c.ybf = ybf;
+                // (bf16 activations: a workspace too small for the k split runs whole tiles)
+                rc = launch_gemm(stream, scheme, c, fits ? base + p.off_gemm : nullptr, fits ? ws_bytes - p.off_gemm : 0);
+            }
+            if (rc) return rc;
+        }
+        return RLXQ_OK;
+    }
     return launch_matmul_generic(stream, scheme, x, xbf, w, y, ybf, m, k, n);
 }
 

@@ -59,10 +59,13 @@ int launch_copy_bytes(cudaStream_t stream, void* dst, const void* src, uint64_t 
 
 // f32 activations for the tensor-core GEMM, whose operands are bf16: x = hi + lo with hi = bf16(x) and
 // lo = bf16(x - hi), which leaves 2^-17 of x behind.  Rows [row0, row0 + rows) of x become rows [0, rows)
-// (hi) and [rows, 2 rows) (lo) of `out`; the GEMM multiplies all 2 rows and add_halves_kernel adds the pairs.
+// (hi) and [rows, 2 rows) (lo) of `out`; the GEMM multiplies both by the same decoded weights.  One pass of 8 bytes a
+// value, a few microseconds; the GEMM behind it is resident meanwhile and fetches its first weights.
 __global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restrict__ x, uint16_t* __restrict__ out,
                                                           uint64_t rows, uint64_t k) {
     const uint64_t total = rows * k / 4, stride = (uint64_t)gridDim.x * blockDim.x;     // k % 4 == 0
+    griddep_launch_dependents();
+    griddep_wait();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const float4 v = reinterpret_cast<const float4*>(x)[i];
         const float f[4] = {v.x, v.y, v.z, v.w};
@@ -78,34 +81,142 @@ __global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restric
     }
 }
 
-__global__ void __launch_bounds__(256) add_halves_kernel(const float* __restrict__ y2, void* __restrict__ y, uint32_t y_bf16,
-                                                         uint64_t rows, uint64_t n) {
-    const uint64_t total = rows * n, stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const float v = y2[i] + y2[total + i];
-        if (y_bf16) reinterpret_cast<uint16_t*>(y)[i] = (uint16_t)f32_to_bf16_bits(v);
-        else reinterpret_cast<float*>(y)[i] = v;
-    }
-}
-
 int launch_split_hi_lo(cudaStream_t stream, const float* x, void* out, uint64_t rows, uint64_t k) {
     if (rows == 0 || k == 0) return RLXQ_OK;
     uint64_t blocks = (rows * k / 4 + 255) / 256;
     const uint64_t cap = (uint64_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    split_hi_lo_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, reinterpret_cast<uint16_t*>(out), rows, k);
+    int rc = launch_pdl(split_hi_lo_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, x, reinterpret_cast<uint16_t*>(out), rows, k);
+    if (rc) return rc;
     count_launch();
     return check_launch("split_hi_lo_kernel");
 }
 
-int launch_add_halves(cudaStream_t stream, const float* y2, void* y, bool ybf, uint64_t rows, uint64_t n) {
-    if (rows == 0 || n == 0) return RLXQ_OK;
-    uint64_t blocks = (rows * n + 255) / 256;
+// y[i] = the sum over s, in order, of part[s * stride + i]: the k slices of a GEMM with few tiles, or (two "slices") the
+// hi and lo results of f32 activations.  Every slice's value is loaded before the first is added; out of L2.
+template <bool VEC>
+__global__ void __launch_bounds__(256) add_slices_kernel(const float* __restrict__ part, uint32_t slices, uint64_t stride,
+                                                         void* __restrict__ y, uint32_t y_bf16, uint64_t total) {
+    constexpr uint32_t W = VEC ? 4 : 1, kAtOnce = 8;
+    griddep_launch_dependents();
+    griddep_wait();
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total / W; i += step) {
+        float acc[W];
+#pragma unroll
+        for (uint32_t q = 0; q < W; ++q) acc[q] = 0.f;
+        for (uint32_t s0 = 0; s0 < slices; s0 += kAtOnce) {
+            float v[kAtOnce][W];
+#pragma unroll
+            for (uint32_t s = 0; s < kAtOnce; ++s) {
+                if (s0 + s >= slices) continue;
+                const float* p = part + (s0 + s) * stride + i * W;
+                if constexpr (VEC) {
+                    const float4 t = __ldcg(reinterpret_cast<const float4*>(p));
+                    v[s][0] = t.x; v[s][1] = t.y; v[s][2] = t.z; v[s][3] = t.w;
+                } else {
+                    v[s][0] = __ldcg(p);
+                }
+            }
+#pragma unroll
+            for (uint32_t s = 0; s < kAtOnce; ++s)
+                if (s0 + s < slices)
+#pragma unroll
+                    for (uint32_t q = 0; q < W; ++q) acc[q] = s0 + s == 0 ? v[s][q] : acc[q] + v[s][q];
+        }
+        if (y_bf16) {
+            uint32_t b[W];
+#pragma unroll
+            for (uint32_t q = 0; q < W; ++q) b[q] = f32_to_bf16_bits(acc[q]) & 0xFFFFu;
+            if constexpr (VEC) reinterpret_cast<uint2*>(y)[i] = make_uint2(b[0] | (b[1] << 16), b[2] | (b[3] << 16));
+            else reinterpret_cast<uint16_t*>(y)[i] = (uint16_t)b[0];
+        } else {
+            if constexpr (VEC) reinterpret_cast<float4*>(y)[i] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            else reinterpret_cast<float*>(y)[i] = acc[0];
+        }
+    }
+}
+
+int launch_add_slices(cudaStream_t stream, const float* part, uint32_t slices, uint64_t stride, void* y, bool ybf, uint64_t total) {
+    if (total == 0) return RLXQ_OK;
+    const bool vec = total % 4 == 0 && stride % 4 == 0 && !(((uintptr_t)y | (uintptr_t)part) & 15u);
+    uint64_t blocks = (total / (vec ? 4 : 1) + 255) / 256;
     const uint64_t cap = (uint64_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    add_halves_kernel<<<(unsigned)blocks, 256, 0, stream>>>(y2, y, ybf ? 1u : 0u, rows, n);
+    int rc = launch_pdl(vec ? add_slices_kernel<true> : add_slices_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, stream, part, slices,
+                        stride, y, ybf ? 1u : 0u, total);
+    if (rc) return rc;
     count_launch();
-    return check_launch("add_halves_kernel");
+    return check_launch("add_slices_kernel");
+}
+
+// Packed weight rows of any (even) length on a pitch that TMA can tile: row r moves from byte r * row_bytes to byte
+// r * pitch, zeros behind it (a zero block decodes to zeros).  Rows start on any even byte, so a 4-byte word of the
+// result is two halves of neighbouring source words; a warp reads its 1 KB piece of a row in eight coalesced loads,
+// all in flight together, and takes the neighbour's word by shuffle.  HBM-bound: one read and one write of the weights
+// (the write mostly stays in L2 for the GEMM behind it).
+// used (expert stacks; may be null): slab s of slab_rows rows is skipped when used[s + 1] == used[s].
+__global__ void __launch_bounds__(256) relay_rows_kernel(const uint8_t* __restrict__ w, uint64_t row_bytes, uint64_t n,
+                                                         uint8_t* __restrict__ out, uint64_t pitch,
+                                                         const uint32_t* __restrict__ used, uint32_t slab_rows) {
+    constexpr uint32_t kSeg = 1024;
+    griddep_launch_dependents();
+    griddep_wait();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t segs = (uint32_t)((pitch + kSeg - 1) / kSeg);
+    const uint64_t items = (uint64_t)segs * n, total = row_bytes * n;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    const uintptr_t base = reinterpret_cast<uintptr_t>(w), end = base + total;
+    // the 32-bit word at aligned address a: halves outside the weights read as zero
+    auto word = [&](uintptr_t a) -> uint32_t {
+        if (a >= base && a + 4 <= end) return __ldg(reinterpret_cast<const uint32_t*>(a));
+        uint32_t v = 0u;
+        if (a >= base && a + 2 <= end) v = __ldg(reinterpret_cast<const uint16_t*>(a));
+        if (a + 2 >= base && a + 4 <= end) v |= (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(a + 2)) << 16;
+        return v;
+    };
+    for (uint64_t it = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += warps) {
+        const uint64_t r = items <= 0xFFFFFFFFull ? (uint32_t)it / segs : it / segs;
+        const uint64_t o0 = (it - r * segs) * kSeg;                        // byte offset of the piece inside its row
+        if (used) {
+            const uint32_t slab = (uint32_t)(r / slab_rows);
+            if (used[slab + 1] == used[slab]) continue;
+        }
+        const uintptr_t src = base + r * row_bytes + o0, a_first = src & ~(uintptr_t)3, a0 = a_first + 4 * lane;
+        const uint32_t sh = (uint32_t)(src & 2u) * 8u;
+        uint32_t v[9];
+        if (a_first >= base && a_first + kSeg + 4 <= end) {                // (what lies behind the row is masked below)
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) v[i] = __ldg(reinterpret_cast<const uint32_t*>(a0 + 128 * i));
+            v[8] = lane == 0 ? __ldg(reinterpret_cast<const uint32_t*>(a0 + kSeg)) : 0u;
+        } else {
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) v[i] = word(a0 + 128 * i);
+            v[8] = lane == 0 ? word(a0 + kSeg) : 0u;
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+            const uint32_t up = __shfl_down_sync(0xFFFFFFFFu, v[i], 1), wrap = __shfl_sync(0xFFFFFFFFu, v[i + 1], 0);
+            uint32_t q = __funnelshift_r(v[i], lane == 31u ? wrap : up, sh);
+            const uint64_t o = o0 + 128 * i + 4 * lane;
+            if (o + 4 > row_bytes) q = o + 2 <= row_bytes ? q & 0xFFFFu : 0u;
+            if (o < pitch) *reinterpret_cast<uint32_t*>(out + r * pitch + o) = q;
+        }
+    }
+}
+
+int launch_relay_rows(cudaStream_t stream, const uint8_t* w, uint64_t row_bytes, uint64_t n, uint8_t* out, uint64_t pitch,
+                      const uint32_t* used, uint32_t slab_rows) {
+    if (n == 0 || pitch == 0) return RLXQ_OK;
+    if (((uintptr_t)w & 1u) || ((uintptr_t)out & 15u) || pitch % 16 || row_bytes % 2 || row_bytes > pitch)
+        return fail(RLXQ_E_ALIGN, "relay_rows: bad alignment");
+    uint64_t blocks = ((pitch + 1023) / 1024 * n + 7) / 8;
+    const uint64_t cap = (uint64_t)sm_count() * 8;
+    if (blocks > cap) blocks = cap;
+    int rc = launch_pdl(relay_rows_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, w, row_bytes, n, out, pitch, used, slab_rows);
+    if (rc) return rc;
+    count_launch();
+    return check_launch("relay_rows_kernel");
 }
 
 }  // namespace rlxq

@@ -25,6 +25,9 @@
 // dimension for n > 1.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <chrono>
+
 #include "common.cuh"
 #include "decode.cuh"
 #include "kernels.h"
@@ -35,15 +38,10 @@
 namespace rlxq {
 
 constexpr uint32_t kGemmTileW = 128;    // weight rows per tile (MMA M, tensor-memory lanes)
-// activation rows per tile (MMA N): a template parameter, 256, or 128 when that fills more SMs
 constexpr uint32_t kGemmBK = 64;        // k per pipeline stage (one 128-byte swizzled row of bf16)
-constexpr uint32_t kGemmMaxStages = 6;  // B shared-memory stages == A tensor-memory stages (4 or 5, by format)
-constexpr uint32_t kGemmRawStages = 2;  // raw weight boxes (256 weights of 128 rows each)
-
-// Instruction descriptor: f32 accumulator, bf16 A and B, both K-major, M = 128, N = 256.
-template <uint32_t TX> struct GemmIdesc {
-    static constexpr uint32_t value = (1u << 4) | (1u << 7) | (1u << 10) | ((TX >> 3) << 17) | ((kGemmTileW >> 4) << 24);
-};
+constexpr uint32_t kGemmMaxStages = 8;  // B shared-memory stages == A tensor-memory stages (8 x 32 columns)
+constexpr uint32_t kGemmMaxRaw = 8;     // raw weight boxes (256 weights of 128 rows each): what shared memory is left for
+constexpr uint32_t kGemmRawStages = 2;  // the paired kernel's
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);       // .x (low half) = lo
@@ -56,26 +54,26 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 template <uint32_t SCHEME> struct GemmRaw;
 // GROUPS: decode warp groups (four warps each).  Two keep pace with the MMA for the cheap decoders (more only
 // add contention: measured 917 against 950 TFLOP/s for Q8_0); Q6_K's decoder is the slow one and gains 10 % from three.
-template <> struct GemmRaw<RLXQ_Q4_0> { static constexpr uint32_t ROW = 144, STAGES = 5, GROUPS = 2; };
-template <> struct GemmRaw<RLXQ_Q8_0> { static constexpr uint32_t ROW = 272, STAGES = 4, GROUPS = 2; };
-template <> struct GemmRaw<RLXQ_Q4_K> { static constexpr uint32_t ROW = 144, STAGES = 5, GROUPS = 2; };
-template <> struct GemmRaw<RLXQ_Q5_K> { static constexpr uint32_t ROW = 176, STAGES = 4, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q4_0> { static constexpr uint32_t ROW = 144, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q8_0> { static constexpr uint32_t ROW = 272, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q4_K> { static constexpr uint32_t ROW = 144, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q5_K> { static constexpr uint32_t ROW = 176, GROUPS = 2; };
 // Q6_K super-blocks are 210 bytes: group g of a row starts at byte 210 g, which is only 2-byte aligned.
 // The box starts at the 16-byte boundary below it and is 240 bytes wide (15 chunks: conflict-free, and
 // 14 + 210 <= 240); the decoder is compiled for each of the eight possible offsets 2 (g mod 8).
-template <> struct GemmRaw<RLXQ_Q6_K> { static constexpr uint32_t ROW = 240, STAGES = 4, GROUPS = 3; };
+template <> struct GemmRaw<RLXQ_Q6_K> { static constexpr uint32_t ROW = 240, GROUPS = 3; };
 // Q2_K super-blocks are 84 bytes (group g starts 4 (g mod 4) bytes past a 16-byte boundary: a 112-byte box covers
 // 12 + 84), Q3_K's 110 bytes (2-byte aligned only, like Q6_K: a 144-byte box covers 14 + 110).
-template <> struct GemmRaw<RLXQ_Q2_K> { static constexpr uint32_t ROW = 112, STAGES = 5, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q2_K> { static constexpr uint32_t ROW = 112, GROUPS = 2; };
 // The 32-weight container types: Q4_1 (20-byte blocks: 160 bytes per 256 weights, fetched as 176 so that a row of the
 // box is an odd number of 16-byte chunks), Q5_0 (22: 176), Q5_1 (24: 192, fetched as 208).
-template <> struct GemmRaw<RLXQ_Q4_1> { static constexpr uint32_t ROW = 176, STAGES = 5, GROUPS = 2; };
-template <> struct GemmRaw<RLXQ_Q5_0> { static constexpr uint32_t ROW = 176, STAGES = 4, GROUPS = 2; };
-template <> struct GemmRaw<RLXQ_Q5_1> { static constexpr uint32_t ROW = 208, STAGES = 4, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q4_1> { static constexpr uint32_t ROW = 176, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q5_0> { static constexpr uint32_t ROW = 176, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q5_1> { static constexpr uint32_t ROW = 208, GROUPS = 2; };
 // Q8_K: 292 bytes (f32 d, 256 int8, 16 int16 block sums that the decoder does not read); 4 (g mod 4) bytes past a
 // boundary, a 304-byte box (19 chunks) covers 12 + 292.
-template <> struct GemmRaw<RLXQ_Q8_K> { static constexpr uint32_t ROW = 304, STAGES = 4, GROUPS = 2; };
-template <> struct GemmRaw<RLXQ_Q3_K> { static constexpr uint32_t ROW = 144, STAGES = 5, GROUPS = 3; };
+template <> struct GemmRaw<RLXQ_Q8_K> { static constexpr uint32_t ROW = 304, GROUPS = 2; };
+template <> struct GemmRaw<RLXQ_Q3_K> { static constexpr uint32_t ROW = 144, GROUPS = 3; };
 template <uint32_t SCHEME> __device__ __forceinline__ uint32_t gemm_raw_x(uint32_t g) {   // box start, 8-byte elements
     if (SCHEME == RLXQ_Q6_K) return ((210u * g) & ~15u) / 8u;
     if (SCHEME == RLXQ_Q2_K) return ((84u * g) & ~15u) / 8u;
@@ -128,15 +126,33 @@ __device__ __forceinline__ uint32_t bf16x2_of(uint64_t v) {
 template <int H> __device__ __forceinline__ uint64_t magic_pair(uint32_t u) {
     return f32x2(__byte_perm(u, 0x4B000000u, 0x7440 + 2 * H), __byte_perm(u, 0x4B000000u, 0x7441 + 2 * H));
 }
-// (byte - OFF) * scale for bytes 2 H, 2 H + 1 of u, as a bf16 pair
-template <int H> __device__ __forceinline__ uint32_t scaled_pair(uint32_t u, uint64_t neg_off, uint64_t scale) {
-    return bf16x2_of(mul_f32x2(add_f32x2(magic_pair<H>(u), neg_off), scale));
+// (byte - OFF) * scale for bytes 2 H, 2 H + 1 of u
+template <int H> __device__ __forceinline__ uint64_t scaled_pair(uint32_t u, uint64_t neg_off, uint64_t scale) {
+    return mul_f32x2(add_f32x2(magic_pair<H>(u), neg_off), scale);
 }
+// Where a decoder puts its 64 weights, two f32 at a time: rounded to bf16 pairs, or as bf16 hi and lo parts.
+template <bool PRECISE> struct GemmOut {
+    uint32_t hi[32];
+    __device__ __forceinline__ void put(int i, uint64_t pair) { hi[i] = bf16x2_of(pair); }
+};
+// hi is the upper half of the f32 bits (one byte-permute per pair; a conversion instruction would pace the decoder), lo
+// the upper half of what that leaves behind, which is exact in f32: together the first 16 bits of the weight.
+template <> struct GemmOut<true> {
+    uint32_t hi[32], lo[32];
+    __device__ __forceinline__ void put(int i, uint64_t pair) {
+        uint32_t a, b;
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(pair));
+        hi[i] = __byte_perm(a, b, 0x7632);
+        const uint64_t rest = add_f32x2(pair, f32x2((a & 0xFFFF0000u) ^ 0x80000000u, (b & 0xFFFF0000u) ^ 0x80000000u));
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(rest));
+        lo[i] = __byte_perm(a, b, 0x7632);
+    }
+};
 
 template <uint32_t SCHEME, int S> struct Decode64;
 
 template <int S> struct Decode64<RLXQ_Q4_0, S> {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         // blocks 2S and 2S+1 = bytes [36 S, 36 S + 36): read the 16-byte chunks that cover them
         constexpr int B0 = 36 * S, C0 = B0 / 16, C1 = (B0 + 36 + 15) / 16, W0 = B0 / 4 - 4 * C0;
         uint32_t w[4 * (C1 - C0) + 1];
@@ -162,17 +178,17 @@ template <int S> struct Decode64<RLXQ_Q4_0, S> {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {   // weights 4i..4i+3: low nibbles of bytes 4i..; weights 16+4i..: high nibbles
                 const uint32_t lo = qs[i] & 0x0F0F0F0Fu, hi = (qs[i] >> 4) & 0x0F0F0F0Fu;
-                v[16 * blk + 2 * i] = scaled_pair<0>(lo, off, d2);
-                v[16 * blk + 2 * i + 1] = scaled_pair<1>(lo, off, d2);
-                v[16 * blk + 8 + 2 * i] = scaled_pair<0>(hi, off, d2);
-                v[16 * blk + 8 + 2 * i + 1] = scaled_pair<1>(hi, off, d2);
+                v.put(16 * blk + 2 * i, scaled_pair<0>(lo, off, d2));
+                v.put(16 * blk + 2 * i + 1, scaled_pair<1>(lo, off, d2));
+                v.put(16 * blk + 8 + 2 * i, scaled_pair<0>(hi, off, d2));
+                v.put(16 * blk + 8 + 2 * i + 1, scaled_pair<1>(hi, off, d2));
             }
         }
     }
 };
 
 template <int S> struct Decode64<RLXQ_Q8_0, S> {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         // blocks 2S and 2S+1 = bytes [68 S, 68 S + 68)
         constexpr int B0 = 68 * S, C0 = B0 / 16, C1 = (B0 + 68 + 15) / 16, W0 = B0 / 4 - 4 * C0;
         uint32_t w[4 * (C1 - C0) + 1];
@@ -198,15 +214,15 @@ template <int S> struct Decode64<RLXQ_Q8_0, S> {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {   // int8 -> (q + 128) unsigned -> float, minus 128
                 const uint32_t u = q[i] ^ 0x80808080u;
-                v[16 * blk + 2 * i] = scaled_pair<0>(u, off, d2);
-                v[16 * blk + 2 * i + 1] = scaled_pair<1>(u, off, d2);
+                v.put(16 * blk + 2 * i, scaled_pair<0>(u, off, d2));
+                v.put(16 * blk + 2 * i + 1, scaled_pair<1>(u, off, d2));
             }
         }
     }
 };
 
 template <int S> struct Decode64<RLXQ_Q4_K, S> {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         const uint4 hd = *reinterpret_cast<const uint4*>(row);   // d, dmin, 12 scale bytes
         const float d = f16_bits_to_f32(hd.x & 0xFFFFu), dmin = f16_bits_to_f32(hd.x >> 16);
         // sub-blocks 2S (low nibbles) and 2S+1 (high nibbles) of bytes [16 + 32 S, +32)
@@ -232,10 +248,10 @@ template <int S> struct Decode64<RLXQ_Q4_K, S> {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {       // scale * nibble - min, rounded after each step as the dequantiser does
             const uint32_t lo = qs[i] & 0x0F0F0F0Fu, hi = (qs[i] >> 4) & 0x0F0F0F0Fu;
-            v[2 * i] = bf16x2_of(add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(lo), off)), ml2));
-            v[2 * i + 1] = bf16x2_of(add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(lo), off)), ml2));
-            v[16 + 2 * i] = bf16x2_of(add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<0>(hi), off)), mh2));
-            v[16 + 2 * i + 1] = bf16x2_of(add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<1>(hi), off)), mh2));
+            v.put(2 * i, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(lo), off)), ml2));
+            v.put(2 * i + 1, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(lo), off)), ml2));
+            v.put(16 + 2 * i, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<0>(hi), off)), mh2));
+            v.put(16 + 2 * i + 1, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<1>(hi), off)), mh2));
         }
     }
 };
@@ -243,7 +259,7 @@ template <int S> struct Decode64<RLXQ_Q4_K, S> {
 // Q5_K: d | dmin | 12 scale bytes | qh[32] | qs[128] (rlx-gguf/src/lib.rs:1019-1068): Q4_K with bit j of
 // qh[l] adding 16 to weight l of sub-block j.
 template <int S> struct Decode64<RLXQ_Q5_K, S> {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         const uint4 hd = *reinterpret_cast<const uint4*>(row);
         const float d = f16_bits_to_f32(hd.x & 0xFFFFu), dmin = f16_bits_to_f32(hd.x >> 16);
         uint32_t sc[2], mn[2];
@@ -271,10 +287,10 @@ template <int S> struct Decode64<RLXQ_Q5_K, S> {
         for (int i = 0; i < 8; ++i) {
             const uint32_t lo = (qs[i] & 0x0F0F0F0Fu) | (((qh[i] >> (2 * S)) & 0x01010101u) << 4);
             const uint32_t hi = ((qs[i] >> 4) & 0x0F0F0F0Fu) | (((qh[i] >> (2 * S + 1)) & 0x01010101u) << 4);
-            v[2 * i] = bf16x2_of(add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(lo), off)), ml2));
-            v[2 * i + 1] = bf16x2_of(add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(lo), off)), ml2));
-            v[16 + 2 * i] = bf16x2_of(add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<0>(hi), off)), mh2));
-            v[16 + 2 * i + 1] = bf16x2_of(add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<1>(hi), off)), mh2));
+            v.put(2 * i, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(lo), off)), ml2));
+            v.put(2 * i + 1, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(lo), off)), ml2));
+            v.put(16 + 2 * i, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<0>(hi), off)), mh2));
+            v.put(16 + 2 * i + 1, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<1>(hi), off)), mh2));
         }
     }
 };
@@ -302,7 +318,7 @@ template <int B0, int LEN> struct Span {
 // S = which 64 of the 256 weights, O = byte offset of the super-block inside the 240-byte row buffer.
 // Layout ql[128] | qh[64] | sc[16] (i8) | d (f16) and element order as rlx-gguf/src/lib.rs:1070-1114.
 template <int S, int O> struct Decode64Q6 {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         constexpr int h = S / 2;
         Span<O + 64 * h, 64> ql;
         Span<O + 128 + 32 * h, 32> qh;
@@ -325,8 +341,8 @@ template <int S, int O> struct Decode64Q6 {
                 const uint32_t mw = lo | hi;
                 const uint64_t ds = f32x2_splat(gsel == 0 ? (i < 4 ? s00 : s01) : (i < 4 ? s10 : s11));
                 const uint64_t off = f32x2_splat(-(8388608.0f + 32.0f));
-                v[16 * gsel + 2 * i] = scaled_pair<0>(mw, off, ds);
-                v[16 * gsel + 2 * i + 1] = scaled_pair<1>(mw, off, ds);
+                v.put(16 * gsel + 2 * i, scaled_pair<0>(mw, off, ds));
+                v.put(16 * gsel + 2 * i + 1, scaled_pair<1>(mw, off, ds));
             }
         }
     }
@@ -356,7 +372,7 @@ template <int S, int O> struct Decode64Q6 {
 // 32 quant bytes of half S / 2, sixteen weights per scale byte: w = (d * sc) * q - dmin * mn, product and
 // difference rounded separately.  O = byte offset of the super-block in the row buffer (a multiple of 4).
 template <int S, int O> struct Decode64Q2 {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         constexpr int h = S / 2;
         Span<O, 4> hd;
         Span<O + 4 + 8 * h + 4 * (S % 2), 4> sc;
@@ -374,8 +390,8 @@ template <int S, int O> struct Decode64Q2 {
                 const uint32_t sb = (scw >> (16 * pl + 8 * (i >> 2))) & 0xFFu;
                 const uint64_t dl2 = f32x2_splat(d * (float)(sb & 0xFu)), ml2 = f32x2_splat(-(dmin * (float)(sb >> 4)));
                 const uint32_t q = (word_at(qs, i) >> shift) & 0x03030303u;
-                v[16 * pl + 2 * i] = bf16x2_of(add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(q), off)), ml2));
-                v[16 * pl + 2 * i + 1] = bf16x2_of(add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(q), off)), ml2));
+                v.put(16 * pl + 2 * i, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(q), off)), ml2));
+                v.put(16 * pl + 2 * i + 1, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(q), off)), ml2));
             }
         }
     }
@@ -389,8 +405,8 @@ template <int S, int O> struct Decode64Q2 {
         }
     }
 };
-template <int S>
-__device__ __forceinline__ void decode64_q2(const uint8_t* row, uint32_t g, uint32_t (&v)[32]) {
+template <int S, typename Out>
+__device__ __forceinline__ void decode64_q2(const uint8_t* row, uint32_t g, Out& v) {
     switch (g & 3u) {      // 84 g mod 16 = 4 (g mod 4)
         case 0: Decode64Q2<S, 0>::run(row, v); break;   case 1: Decode64Q2<S, 4>::run(row, v); break;
         case 2: Decode64Q2<S, 8>::run(row, v); break;   default: Decode64Q2<S, 12>::run(row, v); break;
@@ -408,7 +424,7 @@ __device__ __forceinline__ uint32_t spread4(uint32_t x) { return ((x & 0xFu) * 0
 // bytes; low nibbles are weights 0..15, high nibbles 16..31, bit j (j + 16) of qh the fifth bit of weight j (16 + j).
 // Q4_1, Q5_1: d * q + m (product and sum rounded separately); Q5_0: d * (q - 16).
 template <int S, int BB, bool HAS_M, bool HAS_H> struct Decode64Blk32 {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         constexpr int B0 = 2 * BB * S;
         Span<B0, 2 * BB> sp;
         sp.load(row);
@@ -428,15 +444,15 @@ template <int S, int BB, bool HAS_M, bool HAS_H> struct Decode64Blk32 {
                 uint32_t lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;
                 if (HAS_H) { lo |= spread4(qh >> (4 * i)) << 4; hi |= spread4(qh >> (16 + 4 * i)) << 4; }
                 if (HAS_M) {
-                    v[16 * blk + 2 * i] = bf16x2_of(add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<0>(lo), off)), m2));
-                    v[16 * blk + 2 * i + 1] = bf16x2_of(add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<1>(lo), off)), m2));
-                    v[16 * blk + 8 + 2 * i] = bf16x2_of(add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<0>(hi), off)), m2));
-                    v[16 * blk + 8 + 2 * i + 1] = bf16x2_of(add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<1>(hi), off)), m2));
+                    v.put(16 * blk + 2 * i, add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<0>(lo), off)), m2));
+                    v.put(16 * blk + 2 * i + 1, add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<1>(lo), off)), m2));
+                    v.put(16 * blk + 8 + 2 * i, add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<0>(hi), off)), m2));
+                    v.put(16 * blk + 8 + 2 * i + 1, add_f32x2(mul_f32x2(d2, add_f32x2(magic_pair<1>(hi), off)), m2));
                 } else {
-                    v[16 * blk + 2 * i] = scaled_pair<0>(lo, off, d2);
-                    v[16 * blk + 2 * i + 1] = scaled_pair<1>(lo, off, d2);
-                    v[16 * blk + 8 + 2 * i] = scaled_pair<0>(hi, off, d2);
-                    v[16 * blk + 8 + 2 * i + 1] = scaled_pair<1>(hi, off, d2);
+                    v.put(16 * blk + 2 * i, scaled_pair<0>(lo, off, d2));
+                    v.put(16 * blk + 2 * i + 1, scaled_pair<1>(lo, off, d2));
+                    v.put(16 * blk + 8 + 2 * i, scaled_pair<0>(hi, off, d2));
+                    v.put(16 * blk + 8 + 2 * i + 1, scaled_pair<1>(hi, off, d2));
                 }
             }
         }
@@ -448,7 +464,7 @@ template <int S> struct Decode64<RLXQ_Q5_1, S> : Decode64Blk32<S, 24, true, true
 
 // Q8_K (rlx-gguf/src/lib.rs:848-854, 1121-1140): w = d * q with an f32 d.
 template <int S, int O> struct Decode64Q8K {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         Span<O, 4> hd;
         Span<O + 4 + 64 * S, 64> qs;
         hd.load(row); qs.load(row);
@@ -456,13 +472,13 @@ template <int S, int O> struct Decode64Q8K {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const uint32_t u = qs.w[(O + 4 + 64 * S) / 4 - 4 * Span<O + 4 + 64 * S, 64>::C0 + i] ^ 0x80808080u;   // int8 -> q + 128
-            v[2 * i] = scaled_pair<0>(u, off, d2);
-            v[2 * i + 1] = scaled_pair<1>(u, off, d2);
+            v.put(2 * i, scaled_pair<0>(u, off, d2));
+            v.put(2 * i + 1, scaled_pair<1>(u, off, d2));
         }
     }
 };
-template <int S>
-__device__ __forceinline__ void decode64_q8k(const uint8_t* row, uint32_t g, uint32_t (&v)[32]) {
+template <int S, typename Out>
+__device__ __forceinline__ void decode64_q8k(const uint8_t* row, uint32_t g, Out& v) {
     switch (g & 3u) {      // 292 g mod 16 = 4 (g mod 4)
         case 0: Decode64Q8K<S, 0>::run(row, v); break;   case 1: Decode64Q8K<S, 4>::run(row, v); break;
         case 2: Decode64Q8K<S, 8>::run(row, v); break;   default: Decode64Q8K<S, 12>::run(row, v); break;
@@ -474,7 +490,7 @@ __device__ __forceinline__ void decode64_q8k(const uint8_t* row, uint32_t g, uin
 // half S / 2; weight = (d * (scale - 32)) * (q - (mask bit ? 0 : 4)), mask bit 4 (S / 2) + plane of the weight's
 // mask byte.  The four scales of the group are the bytes of word S of the unpacked scale words.
 template <int S, int O> struct Decode64Q3 {
-    __device__ static __forceinline__ void run(const uint8_t* row, uint32_t (&v)[32]) {
+    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
         constexpr int h = S / 2;
         Span<O, 14> hd;
         Span<O + 14, 32> hm;
@@ -498,8 +514,8 @@ template <int S, int O> struct Decode64Q3 {
                 const uint32_t q = (word_q(qs, i) >> (2 * plane)) & 0x03030303u;
                 const uint32_t hb = (word_h(hm, i) >> (4 * h + plane)) & 0x01010101u;
                 const uint32_t u = q | (hb << 2);                 // q + 4 where the mask bit is set: weight = u - 4
-                v[16 * pl + 2 * i] = scaled_pair<0>(u, off, dl2);
-                v[16 * pl + 2 * i + 1] = scaled_pair<1>(u, off, dl2);
+                v.put(16 * pl + 2 * i, scaled_pair<0>(u, off, dl2));
+                v.put(16 * pl + 2 * i + 1, scaled_pair<1>(u, off, dl2));
             }
         }
     }
@@ -522,8 +538,8 @@ template <int S, int O> struct Decode64Q3 {
         }
     }
 };
-template <int S>
-__device__ __forceinline__ void decode64_q3(const uint8_t* row, uint32_t g, uint32_t (&v)[32]) {
+template <int S, typename Out>
+__device__ __forceinline__ void decode64_q3(const uint8_t* row, uint32_t g, Out& v) {
     switch (g & 7u) {      // 110 g mod 16 = (16 - 2 (g mod 8)) mod 16
         case 0: Decode64Q3<S, 0>::run(row, v); break;   case 1: Decode64Q3<S, 14>::run(row, v); break;
         case 2: Decode64Q3<S, 12>::run(row, v); break;  case 3: Decode64Q3<S, 10>::run(row, v); break;
@@ -533,8 +549,8 @@ __device__ __forceinline__ void decode64_q3(const uint8_t* row, uint32_t g, uint
 }
 
 // Dispatch on the (warp-uniform) offset of group g inside its row buffer.
-template <int S>
-__device__ __forceinline__ void decode64_q6(const uint8_t* row, uint32_t g, uint32_t (&v)[32]) {
+template <int S, typename Out>
+__device__ __forceinline__ void decode64_q6(const uint8_t* row, uint32_t g, Out& v) {
     switch (g & 7u) {
         case 0: Decode64Q6<S, 0>::run(row, v); break;   case 1: Decode64Q6<S, 2>::run(row, v); break;
         case 2: Decode64Q6<S, 4>::run(row, v); break;   case 3: Decode64Q6<S, 6>::run(row, v); break;
@@ -543,8 +559,8 @@ __device__ __forceinline__ void decode64_q6(const uint8_t* row, uint32_t g, uint
     }
 }
 
-template <uint32_t SCHEME, int S>
-__device__ __forceinline__ void decode64(const uint8_t* row, uint32_t g, uint32_t (&v)[32]) {
+template <uint32_t SCHEME, int S, typename Out>
+__device__ __forceinline__ void decode64(const uint8_t* row, uint32_t g, Out& v) {
     if constexpr (SCHEME == RLXQ_Q6_K) decode64_q6<S>(row, g, v);
     else if constexpr (SCHEME == RLXQ_Q2_K) decode64_q2<S>(row, g, v);
     else if constexpr (SCHEME == RLXQ_Q8_K) decode64_q8k<S>(row, g, v);
@@ -557,47 +573,62 @@ constexpr uint32_t kGemmMaxDecodeGroups = 3;
 constexpr uint32_t kGemmMaxBlock = (4 + 4 * kGemmMaxDecodeGroups + 4) * 32;   // B TMA, MMA, raw TMA, spare | decode | epilogue
 // warp roles: 0 = activation (B) TMA producer, 1 = MMA issuer and tensor-memory owner,
 // 2 = raw weight TMA producer, 3 = idle, then GROUPS x 4 decode warps (tensor-memory lane quarter =
-// warp % 4; group (warp - 4) / 4 takes the 64-wide k blocks whose running index is its number modulo
-// GROUPS), then 4 epilogue warps (lane quarter = warp % 4).
+// warp % 4), then 4 epilogue warps (lane quarter = warp % 4).
 
 struct GemmParams {
-    CUtensorMap xmap;      // x[m, k] bf16, box 256 rows x 64 columns, 128-byte swizzle
+    CUtensorMap xmap;      // x[rows, k] bf16, box tx rows x 64 columns, 128-byte swizzle
     CUtensorMap wmap;      // W[n, row_bytes / 8] eight-byte elements, box 128 rows x one 256-weight group
     void* y;
     int* err;
     uint32_t m, n, k, y_bf16, y_vec;      // y_vec: y rows can be written in aligned 16-byte pieces
     uint32_t wtiles, xtiles;
+    uint32_t tx;           // activation rows per tile: a multiple of 32, at most 256
+    // f32 activations (lo_row != 0): x holds bf16(x) in rows [0, lo_row) and bf16(x - bf16(x)) in the same number of
+    // rows behind them; a stage carries both boxes and both are multiplied by the same decoded weights into the same
+    // accumulator, so a weight is decoded once for the two halves.
+    uint32_t lo_row;
+    uint32_t nstages, nraw;               // depth of the operand ring (B in shared memory, A in tensor memory) and of the raw ring
+    uint32_t b_bytes;                     // bytes of a B stage: tx * 128, twice that with lo_row
+    uint32_t w_late;       // the weights are written by a kernel in front (re-laid rows): read them after the dependency wait
     // Work split.  streamk == 0: CTA c takes whole tiles c, c + grid, ...  streamk == 1: the units
     // (tile, 256-weight k group), tile-major, are dealt as contiguous ranges of units_q units (the first
     // units_r CTAs one more), so every SM gets the same work however many tiles there are; a tile cut
     // by range boundaries is completed by the last of its contributors to arrive (partial tiles in
-    // `partial`, one slot per CTA and end of its range; arrival counters in `counters`, zeroed by the host).
-    uint32_t streamk, kgroups, units_q, units_r;
+    // `partial`, one slot per CTA and end of its range).  Arrivals are counted in `counters` under the call's tag
+    // ((tag << 32) | count; any other upper half reads as zero), so the words need no zeroing before the call; the
+    // last arrival clears its word for a replay of the same launch.
+    // slices > 1 (never with streamk): unit (tile, slice) covers an equal part of the tile's k groups and stores its
+    // sums to slice `slice` of an f32 array of y's shape (y points at it, slice_elems apart); a kernel behind this one
+    // adds the slices in order.
+    uint32_t streamk, kgroups, units_q, units_r, slices;
+    size_t slice_elems;
     float* partial;
-    uint32_t* counters;
+    unsigned long long* counters;
+    uint32_t tag;
     // Grouped mode (MoE expert stacks; null = one dense matrix): W is a stack of [n, k] slabs and activation
-    // tile xt is described by groups[xt] = {first row in x, rows (0 = no such tile), expert, -}: the tile
-    // multiplies those rows by slab `expert`.  The table is written on the device by the kernel in front, and
-    // xtiles is only an upper bound of the tiles in use.  Never combined with the k split.
+    // tile xt is described by groups[1 + xt] = {first row in x, rows, expert, -}: the tile multiplies those rows by slab
+    // `expert`.  groups[0].x is the number of tiles.  The table is written on the device by the kernels in front.  Never
+    // combined with a k split.  row_map[r]: the row of y that row r of x belongs to.
     const uint4* groups;
+    const uint32_t* row_map;
 };
 
 // Where tile `tile` reads and writes: activation rows [xrow0, xlim), weight rows from wrow0 (in the stack).
-struct GemmTileRows { uint32_t xrow0, xlim, wrow0; };
-template <uint32_t TX>
-__device__ __forceinline__ bool gemm_tile_rows(const GemmParams& P, uint32_t tile, GemmTileRows& t) {
-    const uint32_t wt = tile / P.xtiles, xt = tile % P.xtiles;
+struct GemmTileRows { uint32_t wt, xrow0, xlim, wrow0; };
+__device__ __forceinline__ GemmTileRows gemm_tile_rows(const GemmParams& P, uint32_t xtiles, uint32_t tile) {
+    GemmTileRows t;
+    t.wt = tile / xtiles;
+    const uint32_t xt = tile - t.wt * xtiles;
     if (P.groups) {
-        const uint4 g = __ldg(&P.groups[xt]);
-        t.xrow0 = g.x; t.xlim = g.x + g.y; t.wrow0 = g.z * P.n + wt * kGemmTileW;
-        return g.y != 0u;
+        const uint4 g = __ldg(&P.groups[1 + xt]);
+        t.xrow0 = g.x; t.xlim = g.x + g.y; t.wrow0 = g.z * P.n + t.wt * kGemmTileW;
+    } else {
+        t.xrow0 = xt * P.tx; t.xlim = min(P.m, t.xrow0 + P.tx); t.wrow0 = t.wt * kGemmTileW;
     }
-    t.xrow0 = xt * TX; t.xlim = P.m; t.wrow0 = wt * kGemmTileW;
-    return true;
+    return t;
 }
 
-
-struct GemmSeg { uint32_t tile, g0, g1; };     // k groups [g0, g1) of one tile
+struct GemmSeg { uint32_t tile, g0, g1, slice; };     // k groups [g0, g1) of one tile
 
 __device__ __forceinline__ uint32_t gemm_range_start(const GemmParams& P, uint32_t c) {
     return c * P.units_q + min(c, P.units_r);
@@ -608,12 +639,13 @@ __device__ __forceinline__ uint32_t gemm_owner(const GemmParams& P, uint32_t u) 
     return u < big ? u / (P.units_q + 1) : P.units_r + (u - big) / P.units_q;
 }
 // Iteration over this CTA's segments, in the order every warp role walks them.
-__device__ __forceinline__ void gemm_seg_init(const GemmParams& P, uint32_t& cur, uint32_t& lim) {
+__device__ __forceinline__ void gemm_seg_init(const GemmParams& P, uint32_t xtiles, uint32_t& cur, uint32_t& lim) {
     if (P.streamk) { cur = gemm_range_start(P, blockIdx.x); lim = gemm_range_start(P, blockIdx.x + 1); }
-    else { cur = blockIdx.x; lim = P.wtiles * P.xtiles; }
+    else { cur = blockIdx.x; lim = P.wtiles * xtiles * P.slices; }
 }
 __device__ __forceinline__ bool gemm_seg_next(const GemmParams& P, uint32_t& cur, uint32_t lim, GemmSeg& sg) {
     if (cur >= lim) return false;
+    sg.slice = 0;
     if (P.streamk) {
         sg.tile = cur / P.kgroups;
         sg.g0 = cur - sg.tile * P.kgroups;
@@ -621,9 +653,33 @@ __device__ __forceinline__ bool gemm_seg_next(const GemmParams& P, uint32_t& cur
         cur += sg.g1 - sg.g0;
     } else {
         sg.tile = cur; sg.g0 = 0; sg.g1 = P.kgroups;
+        if (P.slices > 1) {
+            sg.tile = cur / P.slices;
+            sg.slice = cur - sg.tile * P.slices;
+            sg.g0 = sg.slice * P.kgroups / P.slices;
+            sg.g1 = (sg.slice + 1) * P.kgroups / P.slices;
+        }
         cur += gridDim.x;
     }
     return true;
+}
+// Counts one contributor in and returns how many came before it.  Only the first arrival finds another call's (or
+// anybody's) bits in the word and has to install the tag.
+__device__ __forceinline__ uint32_t gemm_arrive(unsigned long long* word, uint32_t tag) {
+    unsigned long long old = *reinterpret_cast<volatile unsigned long long*>(word);
+    for (;;) {
+        if ((uint32_t)(old >> 32) == tag) return (uint32_t)atomicAdd(word, 1ull);
+        const unsigned long long prev = atomicCAS(word, old, ((unsigned long long)tag << 32) | 1ull);
+        if (prev == old) return 0u;
+        old = prev;
+    }
+}
+// Barrier of the four epilogue warps that tells all of them whether any thread passed true.
+__device__ __forceinline__ bool epilogue_any(bool v) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)v) : "memory");
+    return r != 0u;
 }
 
 // Where an epilogue pass writes: y (bf16 or f32, row pitch n) or a partial tile (f32, row pitch 128).
@@ -631,6 +687,7 @@ struct GemmDst {
     uint8_t* base;
     size_t ld;                        // elements per activation row
     uint32_t m0, mlim, n0, nlim;      // first row / column of the tile in the destination, and its extents
+    const uint32_t* map;              // the destination row of activation row r is map[r] (null: r)
 };
 constexpr uint32_t kGemmEpiStage = 2 * 8192;   // two 8 KB transposition buffers
 
@@ -667,7 +724,7 @@ __device__ __forceinline__ void gemm_store_vec(uint8_t* stage, uint32_t epi_tid,
             const uint32_t mi = d.m0 + 32u * c + h * CP + j, ni = d.n0 + pc * (16u / ES);
             if (mi < d.mlim && ni < d.nlim) {
                 const uint4 t = *reinterpret_cast<const uint4*>(buf + j * (kGemmTileW * ES) + pc * 16u);
-                *reinterpret_cast<uint4*>(d.base + ((size_t)mi * d.ld + ni) * ES) = t;
+                *reinterpret_cast<uint4*>(d.base + ((size_t)(d.map ? __ldg(d.map + mi) : mi) * d.ld + ni) * ES) = t;
             }
         }
     }
@@ -753,45 +810,114 @@ __device__ __noinline__ void gemm_reduce_parts(const GemmParams& P, uint32_t til
 
 struct GemmBars {
     uint64_t b_full[kGemmMaxStages], a_full[kGemmMaxStages], stage_free[kGemmMaxStages];
-    uint64_t raw_full[kGemmRawStages], raw_empty[kGemmRawStages];
-    uint64_t d_full, d_free;
+    uint64_t raw_full[kGemmMaxRaw], raw_empty[kGemmMaxRaw];
+    uint64_t d_full[2], d_free[2];
     uint32_t tmem_base, abort_flag, epi_prev, epi_prev1;   // epi_prev, epi_prev1: arrival counts of alternate segments
 };
 
-template <uint32_t SCHEME, uint32_t kGemmTileX>
+// One decode warp: raw blocks -> bf16 rows in tensor memory.  The 64-weight parts of the groups are dealt to the decode
+// warp groups in turn.  With two of them group GRP takes parts GRP and GRP + 2 of every group, known when the code is
+// compiled (a Q4_K block in 680 cycles, 885 with the turn kept in a register); with three (the slow decoders of Q6_K and
+// Q3_K, whose code is eight variants per part long: separate copies per group cost more in instruction fetch than they
+// save) the turn is counted.
+template <uint32_t SCHEME, bool PRECISE, uint32_t GRP>
+__device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* bars, const uint8_t* raw_stage, uint32_t tmem_a,
+                                                 uint32_t xtiles, uint32_t warp, uint32_t lane) {
+    constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW, GROUPS = GemmRaw<SCHEME>::GROUPS;
+    constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128, A_COLS = PRECISE ? 64 : 32;
+    constexpr bool STATIC = GROUPS == 2;
+    volatile uint32_t* abort_flag = &bars->abort_flag;
+    auto give_up = [&](int code) {
+        atomicExch(P.err, code);
+        *abort_flag = 1u;
+    };
+    const uint32_t quarter = warp & 3u, grp = (warp - 4) >> 2, NS = P.nstages, NR = P.nraw;
+    const uint32_t row = quarter * 32 + lane;                       // weight row of the tile == tensor-memory lane
+    const uint32_t lane_addr = (quarter * 32) << 16;
+    uint32_t r = 0, rph = 0, turn = 0;   // turn (three groups): whose part comes next
+    uint32_t s = 0, fph = 1;             // operand stage of the next part, and the parity that says it is free
+    uint32_t cur, lim;
+    gemm_seg_init(P, xtiles, cur, lim);
+    GemmSeg sg;
+    while (!*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
+        for (uint32_t g = sg.g0; g < sg.g1; ++g) {
+            if (*abort_flag || !mbar_wait(smem_u32(&bars->raw_full[r]), rph)) { give_up(15); return; }
+            const uint8_t* rp = raw_stage + r * RAW_STRIDE + row * RAW_ROW;
+#pragma unroll
+            for (uint32_t sub = 0; sub < 4; ++sub) {
+                const uint32_t st = s, sph = fph;
+                if (++s == NS) { s = 0; fph ^= 1u; }
+                if constexpr (STATIC) {
+                    if (sub % GROUPS != GRP) continue;
+                } else {
+                    const bool mine = turn == grp;
+                    if (++turn == GROUPS) turn = 0;
+                    if (!mine) continue;
+                }
+                // decode into registers first: only the store needs the stage's tensor-memory columns,
+                // so the arithmetic stays off the free -> store -> MMA chain
+                const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);    // answered while decoding
+                GemmOut<PRECISE> v;
+                if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
+                else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
+                else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
+                else decode64<SCHEME, 3>(rp, g, v);
+                if (!__all_sync(0xFFFFFFFFu, ready) && (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[st]), sph))) { give_up(16); return; }
+                tc_fence_after();
+                tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
+                if constexpr (PRECISE) tmem_st32(tmem_a + lane_addr + A_COLS * st + 32, v.lo);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&bars->a_full[st]));
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[r]));
+            if (++r == NR) { r = 0; rph ^= 1u; }
+        }
+    }
+}
+
+// PRECISE: the weight operand keeps 16 significand bits, as bf16 hi and lo parts in two sets of tensor-memory columns,
+// and every activation box is multiplied by both (the lo half of f32 activations by the hi part only: what is left out
+// is below 2^-16 of a product).  It serves the shapes whose other kernel multiplies f32 weights.
+template <uint32_t SCHEME, bool PRECISE>
 __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
-    constexpr uint32_t kGemmStages = GemmRaw<SCHEME>::STAGES;   // shared memory left after the raw boxes decides
     constexpr uint32_t kGemmDecodeGroups = GemmRaw<SCHEME>::GROUPS;
     constexpr uint32_t RAW_BYTES = kGemmTileW * RAW_ROW;
-    constexpr uint32_t B_BYTES = kGemmTileX * kGemmBK * 2;           // 32 KB
+    constexpr uint32_t RAW_STRIDE = (RAW_BYTES + 127) / 128 * 128;
+    constexpr uint32_t A_COLS = PRECISE ? 64 : 32;                    // tensor-memory columns of a weight stage
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* b_stage = smem;                                          // kGemmStages x 32 KB, 1024-aligned
-    uint8_t* raw_stage = smem + kGemmStages * B_BYTES;                // kGemmRawStages x RAW_BYTES (128-aligned)
-    GemmBars* bars = reinterpret_cast<GemmBars*>(raw_stage + kGemmRawStages * ((RAW_BYTES + 127) / 128 * 128));
-    constexpr uint32_t RAW_STRIDE = (RAW_BYTES + 127) / 128 * 128;
+    const uint32_t NS = P.nstages, NR = P.nraw, B_BYTES = P.b_bytes;
+    uint8_t* b_stage = smem;                                          // NS x B_BYTES, 1024-aligned
+    uint8_t* raw_stage = smem + NS * B_BYTES;                         // NR x RAW_BYTES (128-aligned)
+    GemmBars* bars = reinterpret_cast<GemmBars*>(raw_stage + NR * RAW_STRIDE);
     uint8_t* epi_stage = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(bars + 1) + 15) & ~(uintptr_t)15);
 
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     volatile uint32_t* abort_flag = &bars->abort_flag;
+    griddep_launch_dependents();
 
     if (tid == 0) {
-        for (uint32_t s = 0; s < kGemmStages; ++s) {
+        for (uint32_t s = 0; s < NS; ++s) {
             mbar_init(smem_u32(&bars->b_full[s]), 1);
             mbar_init(smem_u32(&bars->a_full[s]), 4);
             mbar_init(smem_u32(&bars->stage_free[s]), 1);
         }
-        for (uint32_t r = 0; r < kGemmRawStages; ++r) {
+        for (uint32_t r = 0; r < NR; ++r) {
             mbar_init(smem_u32(&bars->raw_full[r]), 1);
             mbar_init(smem_u32(&bars->raw_empty[r]), 4 * kGemmDecodeGroups);
         }
-        mbar_init(smem_u32(&bars->d_full), 1);
-        mbar_init(smem_u32(&bars->d_free), 4);
+        for (uint32_t b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&bars->d_full[b]), 1);
+            mbar_init(smem_u32(&bars->d_free[b]), 4);
+        }
         bars->abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {               // the whole warp allocates all 512 columns: 256 accumulator + up to 8 x 32 weight stages
+    if (warp == 1) {               // the whole warp allocates all 512 columns: 256 of accumulators, 256 of weight stages
         tmem_alloc(smem_u32(&bars->tmem_base), 512);
         tmem_relinquish();
     }
@@ -800,145 +926,129 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_tcgen05_kernel(const __
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
     const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + 256;
+    // up to 128 activation rows there are two accumulators: a tile's epilogue runs under the next tile's MMAs
+    const uint32_t nacc = P.tx <= 128 ? 2u : 1u;
     auto give_up = [&](int code) {
         atomicExch(P.err, code);
         *abort_flag = 1u;
     };
+    // The weights may be requested while the kernel in front still runs; all else that is read from global memory
+    // (or written) comes after the dependency wait.  In grouped mode the tile table does, too.
+    if (P.groups) griddep_wait();
+    const uint32_t xtiles = P.groups ? __ldg(&P.groups[0]).x : P.xtiles;
 
     if (warp == 0) {
         // ---------------- activation tiles (B operand) ----------------
         if (elect_one()) {
             tma_prefetch_desc(&P.xmap);
+            griddep_wait();
             uint32_t s = 0, ph = 1;      // parity to wait for on stage_free (1 passes on a fresh barrier)
             uint32_t cur, lim;
-            gemm_seg_init(P, cur, lim);
+            gemm_seg_init(P, xtiles, cur, lim);
             GemmSeg sg;
-            while (!*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
-                GemmTileRows tr;
-                if (!gemm_tile_rows<kGemmTileX>(P, sg.tile, tr)) continue;
-                bool ok = true;
+            bool ok = true;
+            while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
+                const GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
                 for (uint32_t kb = 4 * sg.g0; kb < 4 * sg.g1; ++kb) {
                     if (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[s]), ph)) { give_up(11); ok = false; break; }
-                    const uint32_t full = smem_u32(&bars->b_full[s]);
+                    const uint32_t full = smem_u32(&bars->b_full[s]), dst = smem_u32(b_stage + s * B_BYTES);
                     mbar_arrive_expect_tx(full, B_BYTES);
-                    tma_load_2d(smem_u32(b_stage + s * B_BYTES), &P.xmap, (int32_t)(kb * kGemmBK), (int32_t)tr.xrow0, full);
-                    if (++s == kGemmStages) { s = 0; ph ^= 1u; }
+                    tma_load_2d(dst, &P.xmap, (int32_t)(kb * kGemmBK), (int32_t)tr.xrow0, full);
+                    if (P.lo_row) tma_load_2d(dst + P.tx * 128u, &P.xmap, (int32_t)(kb * kGemmBK), (int32_t)(P.lo_row + tr.xrow0), full);
+                    if (++s == NS) { s = 0; ph ^= 1u; }
                 }
-                if (!ok) break;
             }
         }
     } else if (warp == 2) {
         // ---------------- raw weight groups ----------------
         if (elect_one()) {
             tma_prefetch_desc(&P.wmap);
+            if (P.w_late) griddep_wait();
             uint32_t r = 0, ph = 1;
             uint32_t cur, lim;
-            gemm_seg_init(P, cur, lim);
+            gemm_seg_init(P, xtiles, cur, lim);
             GemmSeg sg;
-            while (!*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
-                GemmTileRows tr;
-                if (!gemm_tile_rows<kGemmTileX>(P, sg.tile, tr)) continue;
-                bool ok = true;
+            bool ok = true;
+            while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
+                const GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
                 for (uint32_t g = sg.g0; g < sg.g1; ++g) {
                     if (*abort_flag || !mbar_wait(smem_u32(&bars->raw_empty[r]), ph)) { give_up(12); ok = false; break; }
                     const uint32_t full = smem_u32(&bars->raw_full[r]);
                     mbar_arrive_expect_tx(full, RAW_BYTES);
                     tma_load_2d(smem_u32(raw_stage + r * RAW_STRIDE), &P.wmap, (int32_t)gemm_raw_x<SCHEME>(g), (int32_t)tr.wrow0, full);
-                    if (++r == kGemmRawStages) { r = 0; ph ^= 1u; }
+                    if (++r == NR) { r = 0; ph ^= 1u; }
                 }
-                if (!ok) break;
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (elect_one()) {
-            uint32_t s = 0, ph = 0, dph = 1;   // dph: parity to wait for on d_free (1 passes the first time)
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((P.tx >> 3) << 17) | ((kGemmTileW >> 4) << 24);
+            uint32_t s = 0, ph = 0, d = 0, dph = 1;   // dph: parity to wait for on d_free (1 passes the first time)
             uint32_t cur, lim;
-            gemm_seg_init(P, cur, lim);
+            gemm_seg_init(P, xtiles, cur, lim);
             GemmSeg sg;
-            while (!*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
-                { GemmTileRows tr; if (!gemm_tile_rows<kGemmTileX>(P, sg.tile, tr)) continue; }
-                if (!mbar_wait(smem_u32(&bars->d_free), dph)) { give_up(13); break; }
-                dph ^= 1u;
+            bool ok = true;
+            while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
+                if (!mbar_wait(smem_u32(&bars->d_free[d]), dph)) { give_up(13); break; }
                 tc_fence_after();
-                bool ok = true;
+                const uint32_t acc = tmem_d + 128u * d;
+                uint32_t rb = mbar_test(smem_u32(&bars->b_full[s]), ph), ra = mbar_test(smem_u32(&bars->a_full[s]), ph);
                 for (uint32_t kb = 0; kb < 4 * (sg.g1 - sg.g0); ++kb) {    // the first MMA of a segment overwrites the accumulator
-                    if (*abort_flag || !mbar_wait(smem_u32(&bars->b_full[s]), ph) ||
-                        !mbar_wait(smem_u32(&bars->a_full[s]), ph)) { give_up(14); ok = false; break; }
+                    if ((!rb && (*abort_flag || !mbar_wait(smem_u32(&bars->b_full[s]), ph))) ||
+                        (!ra && (*abort_flag || !mbar_wait(smem_u32(&bars->a_full[s]), ph)))) { give_up(14); ok = false; break; }
                     tc_fence_after();
+                    // look at the next stage now: the answer arrives while this stage's MMAs are issued
+                    const uint32_t sn = s + 1 == NS ? 0u : s + 1, phn = s + 1 == NS ? ph ^ 1u : ph;
+                    rb = mbar_test(smem_u32(&bars->b_full[sn]), phn);
+                    ra = mbar_test(smem_u32(&bars->a_full[sn]), phn);
                     const uint64_t bdesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES));
+                    const uint32_t a = tmem_a + A_COLS * s;
 #pragma unroll
                     for (uint32_t j = 0; j < kGemmBK / 16; ++j)
-                        tc_mma_ts(tmem_d, tmem_a + 32 * s + 8 * j, bdesc + 2 * j, GemmIdesc<kGemmTileX>::value, (kb | j) ? 1u : 0u);
+                        tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, (kb | j) ? 1u : 0u);
+                    if (PRECISE) {
+#pragma unroll
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 32 + 8 * j, bdesc + 2 * j, idesc, 1u);
+                    }
+                    if (P.lo_row) {
+                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + P.tx * 128u));
+#pragma unroll
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
+                    }
                     tc_commit(smem_u32(&bars->stage_free[s]));     // frees the B stage and the A columns when the MMAs retire
-                    if (++s == kGemmStages) { s = 0; ph ^= 1u; }
+                    s = sn;
+                    ph = phn;
                 }
                 if (!ok) break;
-                tc_commit(smem_u32(&bars->d_full));
+                tc_commit(smem_u32(&bars->d_full[d]));
+                if (++d == nacc) { d = 0; dph ^= 1u; }
             }
         }
     } else if (warp >= 4 && warp < 4 + 4 * kGemmDecodeGroups) {
-        // ---------------- decode: raw blocks -> bf16 rows in tensor memory ----------------
-        // Group grp takes the k blocks whose running index is grp modulo the number of groups, so the
-        // groups alternate whatever the number of 64-wide blocks per raw group (4) is.
-        const uint32_t quarter = warp & 3u, grp = (warp - 4) >> 2;
-        const uint32_t row = quarter * 32 + lane;                       // weight row of the tile == tensor-memory lane
-        const uint32_t lane_addr = (quarter * 32) << 16;
-        uint32_t r = 0, rph = 0, kbg0 = 0;   // kbg0: k blocks this CTA has gone through before the current group
-        bool ok = true;
-        uint32_t cur, lim;
-        gemm_seg_init(P, cur, lim);
-        GemmSeg sg;
-        while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
-            { GemmTileRows tr; if (!gemm_tile_rows<kGemmTileX>(P, sg.tile, tr)) continue; }
-            for (uint32_t g = sg.g0; g < sg.g1 && ok; ++g, kbg0 += 4) {
-                if (*abort_flag || !mbar_wait(smem_u32(&bars->raw_full[r]), rph)) { give_up(15); ok = false; break; }
-                const uint8_t* rp = raw_stage + r * RAW_STRIDE + row * RAW_ROW;
-#pragma unroll
-                for (uint32_t sub = 0; sub < 4; ++sub) {                 // which 64 weights of the group
-                    const uint32_t kbg = kbg0 + sub;                     // running k-block index -> owner, ring slot, phase
-                    if (kbg % kGemmDecodeGroups != grp) continue;
-                    const uint32_t s = kbg % kGemmStages, fph = ((kbg / kGemmStages) & 1u) ^ 1u;
-                    // decode into registers first: only the store needs the stage's tensor-memory columns,
-                    // so the arithmetic stays off the free -> store -> MMA chain
-                    uint32_t v[32];
-                    if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
-                    else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
-                    else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
-                    else decode64<SCHEME, 3>(rp, g, v);
-                    if (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[s]), fph)) { give_up(16); ok = false; break; }
-                    tc_fence_after();
-                    tmem_st32(tmem_a + lane_addr + 32 * s, v);
-                    tmem_st_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&bars->a_full[s]));
-                }
-                if (!ok) break;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[r]));
-                if (++r == kGemmRawStages) { r = 0; rph ^= 1u; }
-            }
-        }
+        // ---------------- decode ----------------
+        if (kGemmDecodeGroups != 2 || warp < 8) gemm_decode_role<SCHEME, PRECISE, 0>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
+        else gemm_decode_role<SCHEME, PRECISE, 1>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
     } else if (warp >= 4 + 4 * kGemmDecodeGroups) {
         // ---------------- epilogue: accumulator -> y (or -> a partial tile, completed by the last contributor) ----------------
         const uint32_t quarter = warp & 3u;
         const uint32_t lane_addr = (quarter * 32) << 16;
         const uint32_t row = quarter * 32 + lane;
         const uint32_t epi_tid = (warp - (4 + 4 * kGemmDecodeGroups)) * 32 + lane;
-        uint32_t dph = 0, nseg = 0;
+        uint32_t d = 0, dph = 0, nseg = 0;
         uint32_t cur, lim;
-        gemm_seg_init(P, cur, lim);
+        gemm_seg_init(P, xtiles, cur, lim);
         GemmSeg sg;
-        while (!*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
-            const uint32_t wt = sg.tile / P.xtiles, xt = sg.tile % P.xtiles;
-            GemmTileRows tr;
-            if (!gemm_tile_rows<kGemmTileX>(P, sg.tile, tr)) continue;
-            if (!mbar_wait(smem_u32(&bars->d_full), dph)) { give_up(17); break; }
-            dph ^= 1u;
+        griddep_wait();                      // y and the workspace may still be in use by the kernel in front
+        bool stop = false;                   // the four warps leave together: they share a named barrier
+        while (!stop && gemm_seg_next(P, cur, lim, sg)) {
+            const GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
+            if (!mbar_wait(smem_u32(&bars->d_full[d]), dph)) { give_up(17); break; }
             tc_fence_after();
-            const uint32_t n_idx = wt * kGemmTileW + row;
-            const bool whole = sg.g0 == 0 && sg.g1 == P.kgroups;
+            const uint32_t n0 = tr.wt * kGemmTileW, n_idx = n0 + row;
+            const bool whole = !P.streamk || (sg.g0 == 0 && sg.g1 == P.kgroups);
+            uint8_t* const out = static_cast<uint8_t*>(P.y) + sg.slice * P.slice_elems * 4;
+            const uint32_t ncols = (tr.xlim - tr.xrow0 + 31u) / 32u;       // groups of 32 accumulator columns in use
             // a cut tile: this CTA's part goes to its head slot when its range begins inside the tile
             // (only a first segment can), to its tail slot otherwise; layout [activation row][weight row]
             const uint32_t u0 = sg.tile * P.kgroups;
@@ -946,69 +1056,77 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_tcgen05_kernel(const __
             float* slot = nullptr;
             const float* other = nullptr;     // two contributors and the other one has already published
             if (!whole) {
-                slot = P.partial + (size_t)(2 * blockIdx.x + ((nseg == 0 && sg.g0 != 0) ? 0u : 1u)) * (kGemmTileW * kGemmTileX);
+                slot = P.partial + (size_t)(2 * blockIdx.x + ((nseg == 0 && sg.g0 != 0) ? 0u : 1u)) * (kGemmTileW * P.tx);
                 c_first = gemm_owner(P, u0);
                 c_last = gemm_owner(P, u0 + P.kgroups - 1);
                 if (c_last - c_first == 1u) {
                     // a + b == b + a: with two parts the sum does not depend on who adds, so the second one
                     // to arrive adds the published part to its own registers and never publishes
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (epi_tid == 0) (&bars->epi_prev)[nseg & 1u] = *reinterpret_cast<volatile uint32_t*>(&P.counters[sg.tile]);
+                    if (epi_tid == 0) {
+                        const unsigned long long word = *reinterpret_cast<volatile unsigned long long*>(&P.counters[sg.tile]);
+                        (&bars->epi_prev)[nseg & 1u] = word == (((unsigned long long)P.tag << 32) | 1ull) ? 1u : 0u;
+                    }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (reinterpret_cast<volatile uint32_t*>(&bars->epi_prev)[nseg & 1u] == 1u) {
                         __threadfence();
                         const uint32_t oc = blockIdx.x == c_first ? c_last : c_first;
                         const uint32_t sid = 2 * oc + (gemm_range_start(P, oc) > u0 ? 0u : 1u);
-                        other = P.partial + (size_t)sid * (kGemmTileW * kGemmTileX);
+                        other = P.partial + (size_t)sid * (kGemmTileW * P.tx);
                     }
                 }
             }
 #pragma unroll 1
-            for (uint32_t c = 0; c < kGemmTileX / 32; ++c) {
+            for (uint32_t c = 0; c < ncols; ++c) {
                 uint32_t v[32];
-                tmem_ld32(tmem_d + lane_addr + 32 * c, v);
+                tmem_ld32(tmem_d + 128u * d + lane_addr + 32 * c, v);
                 tmem_ld_wait();
-                if (c == kGemmTileX / 32 - 1) {      // everything is in registers: the accumulator may be overwritten
+                if (c == ncols - 1) {      // everything is in registers: the accumulator may be overwritten
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&bars->d_free));
+                    if (lane == 0) mbar_arrive(smem_u32(&bars->d_free[d]));
                 }
                 if (other) {
                     gemm_add_store(epi_stage, epi_tid, row, v, reinterpret_cast<const uint4*>(other + (size_t)(32 * c) * kGemmTileW),
-                                   P, xt * kGemmTileX + 32 * c, wt * kGemmTileW);
+                                   P, tr.xrow0 + 32 * c, n0);
                 } else if (!whole) {
-                    const GemmDst d{reinterpret_cast<uint8_t*>(slot), kGemmTileW, 0u, kGemmTileX, 0u, kGemmTileW};
-                    gemm_store_vec<true>(epi_stage, epi_tid, row, v, d, c);
+                    const GemmDst dst{reinterpret_cast<uint8_t*>(slot), kGemmTileW, 0u, 32u * ncols, 0u, kGemmTileW, nullptr};
+                    gemm_store_vec<true>(epi_stage, epi_tid, row, v, dst, c);
                 } else if (P.y_vec) {
-                    const GemmDst d{reinterpret_cast<uint8_t*>(P.y), P.n, tr.xrow0, tr.xlim, wt * kGemmTileW, P.n};
-                    if (P.y_bf16) gemm_store_vec<false>(epi_stage, epi_tid, row, v, d, c);
-                    else gemm_store_vec<true>(epi_stage, epi_tid, row, v, d, c);
+                    const GemmDst dst{out, P.n, tr.xrow0, tr.xlim, n0, P.n, P.row_map};
+                    if (P.y_bf16) gemm_store_vec<false>(epi_stage, epi_tid, row, v, dst, c);
+                    else gemm_store_vec<true>(epi_stage, epi_tid, row, v, dst, c);
                 } else if (n_idx < P.n) {
 #pragma unroll
                     for (uint32_t j = 0; j < 32; ++j) {
                         const uint32_t m_idx = tr.xrow0 + 32 * c + j;
                         if (m_idx < tr.xlim) {
-                            const size_t o = (size_t)m_idx * P.n + n_idx;
-                            if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[o] = (uint16_t)bf16x2_of(f32x2(v[j], 0u));
-                            else reinterpret_cast<float*>(P.y)[o] = __uint_as_float(v[j]);
+                            const size_t o = (size_t)(P.row_map ? __ldg(&P.row_map[m_idx]) : m_idx) * P.n + n_idx;
+                            if (P.y_bf16) reinterpret_cast<uint16_t*>(out)[o] = (uint16_t)bf16x2_of(f32x2(v[j], 0u));
+                            else reinterpret_cast<float*>(out)[o] = __uint_as_float(v[j]);
                         }
                     }
                 }
             }
-            if (!whole && !other) {
+            if (other) {
+                if (epi_tid == 0) P.counters[sg.tile] = 0ull;          // both contributors are through with the word
+            } else if (!whole) {
                 // publish, count, and let the last contributor add all parts in contributor order (its own
                 // included, re-read from memory: the sum then never depends on who came last)
                 __threadfence();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (epi_tid == 0) (&bars->epi_prev)[nseg & 1u] = atomicAdd(&P.counters[sg.tile], 1u);
+                if (epi_tid == 0) (&bars->epi_prev)[nseg & 1u] = gemm_arrive(&P.counters[sg.tile], P.tag);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 const uint32_t prev = reinterpret_cast<volatile uint32_t*>(&bars->epi_prev)[nseg & 1u];
                 if (prev == c_last - c_first) {
                     __threadfence();
-                    gemm_reduce_parts(P, kGemmTileX, c_first, c_last, u0, xt * kGemmTileX, wt * kGemmTileW, epi_tid);
+                    if (epi_tid == 0) P.counters[sg.tile] = 0ull;
+                    gemm_reduce_parts(P, P.tx, c_first, c_last, u0, tr.xrow0, n0, epi_tid);
                 }
             }
+            stop = epilogue_any(*abort_flag != 0u);    // and the next segment starts on the first transposition buffer again
             ++nseg;
+            if (++d == nacc) { d = 0; dph ^= 1u; }
         }
     }
     // everybody meets here, also after a timeout, so the tensor memory is always returned
@@ -1071,12 +1189,14 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t rank = cluster_cta_rank();            // 0 issues the MMAs
     volatile uint32_t* abort_flag = &bars->abort_flag;
+    const bool dual = P.lo_row != 0;     // a round is 128 wide in k, or, for f32 activations, 64 wide with a hi and a lo box
+    griddep_launch_dependents();
 
     if (tid == 0) {
         for (uint32_t s = 0; s < kPairStages; ++s) {
             mbar_init(smem_u32(&bars->b_full[s]), 2);        // own TMA (with its bytes) + the other CTA's, forwarded
             mbar_init(smem_u32(&bars->b_own[s]), 1);
-            mbar_init(smem_u32(&bars->a_full[s]), 8 * kPairRound);   // per 64-wide block four decode warps, of each CTA
+            mbar_init(smem_u32(&bars->a_full[s]), dual ? 8 : 8 * kPairRound);   // per 64-wide block four decode warps, of each CTA
             mbar_init(smem_u32(&bars->stage_free[s]), 1);
         }
         for (uint32_t r = 0; r < kGemmRawStages; ++r) {
@@ -1104,12 +1224,13 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
     };
     // the pair's tiles: 256 weight rows (pair index wp) x 256 activation rows (xt), xt fastest
     const uint32_t pt0 = blockIdx.x >> 1, pstep = gridDim.x >> 1, plim = (P.wtiles >> 1) * P.xtiles;
-    const uint32_t rounds = 4 * P.kgroups / kPairRound;  // rounds of a tile
+    const uint32_t rounds = dual ? 4 * P.kgroups : 4 * P.kgroups / kPairRound;  // rounds of a tile
 
     if (warp == 0) {
         // ---------------- this CTA's half of the activation tile ----------------
         if (elect_one()) {
             tma_prefetch_desc(&P.xmap);
+            griddep_wait();
             uint32_t s = 0, ph = 1;
             bool ok = true;
             for (uint32_t pt = pt0; ok && pt < plim && !*abort_flag; pt += pstep) {
@@ -1121,7 +1242,8 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
 #pragma unroll
                     for (uint32_t q = 0; q < kPairRound; ++q)
                         tma_load_2d(smem_u32(b_stage + s * kPairBBytes + q * kPairSubBytes), &P.xmap,
-                                    (int32_t)((kb * kPairRound + q) * kGemmBK), (int32_t)xrow, full);
+                                    (int32_t)((dual ? kb : kb * kPairRound + q) * kGemmBK),
+                                    (int32_t)(dual && q ? P.lo_row + xrow : xrow), full);
                     if (++s == kPairStages) { s = 0; ph ^= 1u; }
                 }
             }
@@ -1165,17 +1287,22 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
                 if (!mbar_wait(smem_u32(&bars->d_free), dph)) { give_up(24); break; }
                 dph ^= 1u;
                 tc_fence_after();
+                uint32_t rb = mbar_test(smem_u32(&bars->b_full[s]), ph), ra = mbar_test(smem_u32(&bars->a_full[s]), ph);
                 for (uint32_t kb = 0; kb < rounds; ++kb) {
-                    if (*abort_flag || !mbar_wait(smem_u32(&bars->b_full[s]), ph) ||
-                        !mbar_wait(smem_u32(&bars->a_full[s]), ph)) { give_up(25); ok = false; break; }
+                    if ((!rb && (*abort_flag || !mbar_wait(smem_u32(&bars->b_full[s]), ph))) ||
+                        (!ra && (*abort_flag || !mbar_wait(smem_u32(&bars->a_full[s]), ph)))) { give_up(25); ok = false; break; }
                     tc_fence_after();
+                    const uint32_t sn = s + 1 == kPairStages ? 0u : s + 1, phn = s + 1 == kPairStages ? ph ^ 1u : ph;
+                    rb = mbar_test(smem_u32(&bars->b_full[sn]), phn);
+                    ra = mbar_test(smem_u32(&bars->a_full[sn]), phn);
 #pragma unroll
                     for (uint32_t j = 0; j < kPairRound * kGemmBK / 16; ++j) {
                         const uint64_t bdesc = kmajor_sw128_desc(smem_u32(b_stage + s * kPairBBytes + (j >> 2) * kPairSubBytes));
-                        tc_mma_ts_pair(tmem_d, tmem_a + 32 * kPairRound * s + 8 * j, bdesc + 2 * (j & 3u), kPairIdesc, (kb | j) ? 1u : 0u);
+                        tc_mma_ts_pair(tmem_d, tmem_a + 32 * kPairRound * s + 8 * (dual ? j & 3u : j), bdesc + 2 * (j & 3u), kPairIdesc, (kb | j) ? 1u : 0u);
                     }
                     tc_commit_pair_both(smem_u32(&bars->stage_free[s]), 3);     // frees the stage in both CTAs
-                    if (++s == kPairStages) { s = 0; ph ^= 1u; }
+                    s = sn;
+                    ph = phn;
                 }
                 if (!ok) break;
                 tc_commit_pair_both(smem_u32(&bars->d_full), 3);
@@ -1197,15 +1324,17 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
                     const uint32_t kbg = kbg0 + sub;
                     if (kbg % kGemmDecodeGroups != grp) continue;
                     // 64-wide block kbg is part kbg % kPairRound of round kbg / kPairRound
-                    const uint32_t rd = kbg / kPairRound, s = rd % kPairStages, fph = ((rd / kPairStages) & 1u) ^ 1u;
-                    uint32_t v[32];
+                    const uint32_t rd = dual ? kbg : kbg / kPairRound, s = rd % kPairStages, fph = ((rd / kPairStages) & 1u) ^ 1u;
+                    const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[s]), fph);     // answered while decoding
+                    GemmOut<false> v;
                     if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
                     else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
                     else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
                     else decode64<SCHEME, 3>(rp, g, v);
-                    if (*abort_flag || !pair_wait<SCHEME>(smem_u32(&bars->stage_free[s]), fph, lane)) { give_up(27); ok = false; break; }
+                    if (!__all_sync(0xFFFFFFFFu, ready) &&
+                        (*abort_flag || !pair_wait<SCHEME>(smem_u32(&bars->stage_free[s]), fph, lane))) { give_up(27); ok = false; break; }
                     tc_fence_after();
-                    tmem_st32(tmem_a + lane_addr + 32 * (kPairRound * s + kbg % kPairRound), v);
+                    tmem_st32(tmem_a + lane_addr + 32 * (kPairRound * s + (dual ? 0u : kbg % kPairRound)), v.hi);
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
@@ -1227,6 +1356,7 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
         const uint32_t row = quarter * 32 + lane;
         const uint32_t epi_tid = (warp - (4 + 4 * kGemmDecodeGroups)) * 32 + lane;
         uint32_t dph = 0;
+        griddep_wait();                      // y may still be in use by the kernel in front
         for (uint32_t pt = pt0; pt < plim && !*abort_flag; pt += pstep) {
             const uint32_t wt = 2 * (pt / P.xtiles) + rank, xrow0 = (pt % P.xtiles) * TX;
             if (!mbar_wait_warp(smem_u32(&bars->d_full), dph, lane)) { give_up(28); break; }
@@ -1247,7 +1377,7 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
                     }
                 }
                 if (P.y_vec) {
-                    const GemmDst d{reinterpret_cast<uint8_t*>(P.y), P.n, xrow0, P.m, wt * kGemmTileW, P.n};
+                    const GemmDst d{reinterpret_cast<uint8_t*>(P.y), P.n, xrow0, P.m, wt * kGemmTileW, P.n, nullptr};
                     if (P.y_bf16) gemm_store_vec<false>(epi_stage, epi_tid, row, v, d, c);
                     else gemm_store_vec<true>(epi_stage, epi_tid, row, v, d, c);
                 } else if (n_idx < P.n) {
@@ -1272,138 +1402,211 @@ __global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __gri
 }
 
 // ---- host side --------------------------------------------------------------------------------
-bool gemm_tc_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* w, const void* x, bool xbf) {
-    if (!xbf || m == 0 || n == 0 || k == 0 || k % 256) return false;
-    if (scheme != RLXQ_Q4_0 && scheme != RLXQ_Q8_0 && scheme != RLXQ_Q4_K && scheme != RLXQ_Q6_K && scheme != RLXQ_Q5_K &&
-        scheme != RLXQ_Q2_K && scheme != RLXQ_Q3_K && scheme != RLXQ_Q8_K && scheme != RLXQ_Q4_1 && scheme != RLXQ_Q5_0 &&
-        scheme != RLXQ_Q5_1) return false;
+static bool gemm_tc_format(uint32_t scheme) {
+    switch (scheme) {
+        case RLXQ_Q4_0: case RLXQ_Q8_0: case RLXQ_Q4_K: case RLXQ_Q6_K: case RLXQ_Q5_K: case RLXQ_Q2_K: case RLXQ_Q3_K:
+        case RLXQ_Q8_K: case RLXQ_Q4_1: case RLXQ_Q5_0: case RLXQ_Q5_1: return true;
+        default: return false;
+    }
+}
+// The GEMM on the weights where they lie: rows of whole 256-weight groups that start on 16-byte boundaries.
+bool gemm_tc_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* w, const void* x) {
+    if (m == 0 || n == 0 || k == 0 || k % 256 || !gemm_tc_format(scheme)) return false;
     if ((scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K) && k % 2048) return false;   // rows must stay 16-byte aligned
     if ((scheme == RLXQ_Q2_K || scheme == RLXQ_Q8_K) && k % 1024) return false;
     if (((uintptr_t)w & 15u) || ((uintptr_t)x & 15u)) return false;
     return true;
 }
-
-// The k split ("stream-K") evens the work out over the SMs, at the price of exchanging partial tiles through
-// memory, which costs about as much as 36 steps of one 256-wide k group.  It is chosen when it saves at
-// least that many steps on the busiest SM against whole tiles (of the width they would be given): few
-// tiles and a long k, e.g. the down projection of a tensor-parallel shard at a small batch.
-static bool gemm_wants_streamk(uint32_t m, uint32_t k, uint32_t n) {
-    const int64_t opt = options().gemm_streamk.load();
-    if (opt == 1) return false;
-    if (opt == 2) return true;
-    const uint64_t sms = (uint64_t)sm_count(), wt = (n + kGemmTileW - 1) / kGemmTileW, kgroups = k / 256;
-    const uint64_t ntiles256 = wt * ((m + 255) / 256), ntiles128 = wt * ((m + 127) / 128);
-    const uint64_t whole_tiles = ntiles256 * 4 < sms * 3 ? ntiles128 : ntiles256;
-    const uint64_t steps_whole = (whole_tiles + sms - 1) / sms * kgroups;
-    const uint64_t steps_split = (ntiles256 * kgroups + sms - 1) / sms;
-    return steps_whole >= steps_split + 36;
+// Every other row length (and alignment of the weights): rows re-laid on a pitch TMA can tile, then the PRECISE form.
+bool gemm_relaid_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* x) {
+    return m != 0 && n != 0 && k != 0 && k % 32 == 0 && gemm_tc_format(scheme) && !((uintptr_t)x & 15u);
 }
-static size_t gemm_streamk_bytes(uint32_t ntiles, size_t* off_partial) {
-    const size_t counters = ((size_t)ntiles * 4 + 255) / 256 * 256;
+// Bytes from one re-laid row to the next: whole 256-weight groups (zero blocks past k), a multiple of 16.
+uint64_t gemm_relaid_pitch(uint32_t scheme, uint32_t k) {
+    Geometry g;
+    geometry(scheme, &g);
+    return ((uint64_t)((k + 255) / 256) * (256 / g.elems) * g.bytes + 15) / 16 * 16;
+}
+
+struct GemmShape { uint32_t tx, xtiles, slices; bool streamk, pair; };
+
+// Activation rows per tile, work split and kernel for a shape, by estimated time in cycles.  A 64-wide k block of a tile
+// costs the larger of its MMAs (2 cycles per activation row and product plus the hand-over; `products`: bf16 activations
+// 1, f32 2, one more with PRECISE weights) and its decode, whatever part of the tile's rows is padding (measured slopes
+// over k at n = 14336); so few rows get a narrow tile, and rows are split evenly over the fewest tiles that leave no SM
+// idle.
+static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t products, bool precise) {
+    const uint32_t mma = 2 * tx * products + 225;
+    uint32_t dec = (scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K) ? 1130 : scheme == RLXQ_Q8_0 ? 520 : 680;
+    if (precise) dec += 350;
+    return mma > dec ? mma : dec;
+}
+static GemmShape gemm_shape(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise, bool can_split) {
+    const uint64_t sms = (uint64_t)sm_count(), wt = (n + kGemmTileW - 1) / kGemmTileW, groups = (k + 255) / 256, blocks = 4 * groups;
+    const uint32_t products = 1 + (f32 ? 1 : 0) + (precise ? 1 : 0);
+    const uint32_t most = f32 ? 128 : 256;               // a stage holds 256 box rows
+    const int64_t fx = options().gemm_tile_x.load(), fs = can_split ? options().gemm_streamk.load() : 1;
+    GemmShape best{};
+    uint64_t best_cost = ~0ull;
+    auto take = [&](uint64_t cost, const GemmShape& sh) { if (cost < best_cost) { best_cost = cost; best = sh; } };
+    const uint32_t least_tiles = (m + most - 1) / most;
+    for (uint32_t xt = least_tiles; xt <= least_tiles + 8; ++xt) {
+        uint32_t tx = ((m + xt - 1) / xt + 31) / 32 * 32;
+        if (fx) tx = (uint32_t)fx < most ? (uint32_t)fx : most;
+        const uint32_t tiles_x = (m + tx - 1) / tx;
+        if (tiles_x != xt && !fx) continue;              // the same width as one tile fewer
+        const uint64_t ntiles = wt * tiles_x, cyc = gemm_block_cycles(scheme, tx, products, precise);
+        const uint64_t epi = 24 * tx;                    // the last tile's epilogue, and with one accumulator every tile's
+        if (fs != 2) take((ntiles + sms - 1) / sms * (blocks * cyc + (tx > 128 ? epi : 0)) + epi, GemmShape{tx, tiles_x, 1, false, false});
+        // k split over the SMs (stream-K): every SM gets the same blocks, and exchanges up to two parts of 128 x tx values
+        if (fs != 1 && (fs == 2 || ntiles % sms))
+            take((ntiles * blocks + sms - 1) / sms * cyc + epi + 8000 + 100 * tx, GemmShape{tx, tiles_x, 1, true, false});
+        // few tiles: every SM takes a slice of some tile's k, and a kernel behind this one adds the slices
+        if (fs == 0 && 2 * ntiles <= sms) {
+            const uint64_t fit = sms / ntiles, sl = groups < fit ? groups : fit;
+            if (sl > 1) take((groups + sl - 1) / sl * 4 * cyc + epi + 3200 + sl * m * n / 600, GemmShape{tx, tiles_x, (uint32_t)sl, false, false});
+        }
+        if (fx) break;
+    }
+    return best;
+}
+static bool gemm_pair_fits(uint32_t n, bool precise) { return n % 256 == 0 && !precise; }
+// Two CTAs per MMA: chosen where it measured faster, with at least one 256 x 256 tile pair per resident cluster and a
+// format whose decoder keeps pace with two groups of decode warps (Q6_K and Q3_K, with three groups, lose 5-12 % in the
+// paired form on large shapes).
+static bool gemm_wants_pair(uint32_t scheme, uint32_t m, uint32_t n, bool precise) {
+    const int64_t opt = options().gemm_pair.load();
+    if (opt == 1 || !gemm_pair_fits(n, precise)) return false;
+    if (opt == 2) return true;
+    if (scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K || options().gemm_tile_x.load() || options().gemm_streamk.load() == 2) return false;
+    return (uint64_t)(n / 256) * ((m + 255) / 256) >= (uint64_t)sm_count() / 2;
+}
+static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise, bool can_split) {
+    if (gemm_wants_pair(scheme, m, n, precise)) return GemmShape{256, (m + 255) / 256, 1, false, true};
+    return gemm_shape(scheme, m, k, n, f32, precise, can_split);
+}
+static size_t gemm_streamk_bytes(uint64_t ntiles, uint32_t tx, size_t* off_partial) {
+    const size_t counters = ((size_t)ntiles * 8 + 255) / 256 * 256;
     if (off_partial) *off_partial = counters;
-    return counters + 2 * (size_t)sm_count() * kGemmTileW * 256 * 4;     // two partial tiles per CTA
+    return counters + 2 * (size_t)sm_count() * kGemmTileW * tx * 4;     // two partial tiles per CTA
+}
+static size_t gemm_slice_elems(uint32_t m, uint32_t n) { return ((size_t)m * n + 3) / 4 * 4; }
+static size_t gemm_shape_bytes(const GemmShape& sh, uint32_t m, uint32_t n) {
+    if (sh.slices > 1) return sh.slices * gemm_slice_elems(m, n) * 4;
+    return sh.streamk ? gemm_streamk_bytes((uint64_t)((n + kGemmTileW - 1) / kGemmTileW) * sh.xtiles, sh.tx, nullptr) : 0;
 }
 
 // Scratch the GEMM would use for this shape (0 when whole tiles fill the SMs well enough).
-size_t gemm_tc_workspace_bytes(uint32_t m, uint32_t k, uint32_t n) {
-    if (m <= 8 || k == 0 || k % 256) return 0;
-    const uint32_t ntiles = ((n + kGemmTileW - 1) / kGemmTileW) * ((m + 255) / 256);
-    return gemm_wants_streamk(m, k, n) ? gemm_streamk_bytes(ntiles, nullptr) : 0;
+size_t gemm_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise) {
+    if (m == 0 || k == 0 || n == 0) return 0;
+    return gemm_shape_bytes(gemm_choose(scheme, m, k, n, f32, precise, true), m, n);
 }
 
-template <uint32_t SCHEME, uint32_t TX>
-static int launch_gemm_t(cudaStream_t stream, const void* x, const uint8_t* w, void* y, bool ybf, uint32_t m,
-                         uint32_t k, uint32_t n, void* ws, bool streamk, const uint4* groups = nullptr,
-                         uint32_t group_tiles = 0, uint32_t num_slabs = 1) {
+// Odd 32-bit tags, a different one for each of the calls that may be in flight together.
+static uint32_t next_gemm_tag() {
+    static std::atomic<uint32_t> epoch{(uint32_t)std::chrono::steady_clock::now().time_since_epoch().count() * 0x9E3779B9u};
+    return (epoch.fetch_add(1) << 1) | 1u;
+}
+
+template <uint32_t SCHEME, bool PRECISE>
+static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape& sh, void* ws) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
     constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128;
     Geometry g;
     geometry(SCHEME, &g);
     GemmParams P{};
-    int rc = encode_bf16_kmajor_map(&P.xmap, x, m, k, TX);
+    P.tx = sh.tx;
+    P.lo_row = c.f32 ? c.x_rows : 0u;
+    int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * (c.f32 ? 2 : 1), c.k, P.tx);
     if (rc) return rc;
-    rc = encode_weight_map(&P.wmap, w, (uint64_t)n * num_slabs, (uint64_t)k / g.elems * g.bytes, RAW_ROW / 8, kGemmTileW);
+    rc = encode_weight_map(&P.wmap, c.w, (uint64_t)c.n * c.num_slabs, c.w_pitch ? c.w_pitch : (uint64_t)c.k / g.elems * g.bytes,
+                           RAW_ROW / 8, kGemmTileW);
     if (rc) return rc;
-    P.y = y; P.m = m; P.n = n; P.k = k; P.y_bf16 = ybf;
-    P.groups = groups;
-    P.y_vec = (((uintptr_t)y & 15u) == 0 && n % (ybf ? 8u : 4u) == 0) ? 1u : 0u;
-    P.wtiles = (n + kGemmTileW - 1) / kGemmTileW;
-    P.xtiles = groups ? group_tiles : (m + TX - 1) / TX;
-    P.kgroups = k / 256;
+    P.y = c.y; P.m = c.x_rows; P.n = c.n; P.k = c.k; P.y_bf16 = c.ybf;
+    P.slices = sh.slices;
+    if (sh.slices > 1) {
+        P.y = ws; P.y_bf16 = 0;
+        P.slice_elems = gemm_slice_elems(c.x_rows, c.n);
+    }
+    P.groups = static_cast<const uint4*>(c.groups);
+    P.row_map = c.row_map;
+    P.w_late = c.w_pitch ? 1u : 0u;
+    P.y_vec = (((uintptr_t)P.y & 15u) == 0 && c.n % (P.y_bf16 ? 8u : 4u) == 0) ? 1u : 0u;
+    P.wtiles = (c.n + kGemmTileW - 1) / kGemmTileW;
+    P.xtiles = sh.xtiles;
+    P.kgroups = (c.k + 255) / 256;
     P.err = device_error_word();
     if (!P.err) return fail(RLXQ_E_CUDA, "device error word unavailable");
-    const size_t smem = 1024 + (size_t)GemmRaw<SCHEME>::STAGES * TX * kGemmBK * 2 + (size_t)kGemmRawStages * RAW_STRIDE +
-                        sizeof(GemmBars) + 64 + kGemmEpiStage;
+    // as many operand stages as tensor memory and shared memory hold beside two raw boxes, then raw boxes
+    P.b_bytes = P.tx * kGemmBK * 2 * (c.f32 ? 2 : 1);
+    const uint32_t smem = 227 * 1024;   // all of it: one CTA per SM, so that none waits for another's tensor memory
+    const uint32_t budget = smem - (1024 + sizeof(GemmBars) + 64 + kGemmEpiStage);
+    P.nstages = std::min<uint32_t>(PRECISE ? 4 : kGemmMaxStages, (budget - kGemmRawStages * RAW_STRIDE) / P.b_bytes);
+    P.nraw = std::min<uint32_t>(kGemmMaxRaw, (budget - P.nstages * P.b_bytes) / RAW_STRIDE);
     static std::atomic<uint32_t> attr_set[64];
     int dev = 0;
     RLXQ_CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && attr_set[dev].load() == 0) {
-        RLXQ_CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<SCHEME, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RLXQ_CUDA_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<SCHEME, PRECISE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set[dev].store(1);
     }
     uint32_t grid = (uint32_t)sm_count();
-    const uint32_t ntiles = P.wtiles * P.xtiles;
-    if (streamk) {
-        const uint64_t units = (uint64_t)ntiles * P.kgroups;
-        if (units > 0xFFFFFFFFull) return fail(RLXQ_E_LIMIT, "GEMM too large for the stream-K split");
+    const uint64_t ntiles = (uint64_t)P.wtiles * P.xtiles * P.slices;
+    if (ntiles * P.kgroups > 0xFFFFFFFFull) return fail(RLXQ_E_LIMIT, "GEMM too large");
+    if (sh.streamk) {
+        const uint64_t units = ntiles * P.kgroups;
         if (grid > units) grid = (uint32_t)units;
         size_t off_partial = 0;
-        gemm_streamk_bytes(ntiles, &off_partial);
+        gemm_streamk_bytes(ntiles, P.tx, &off_partial);
         P.streamk = 1;
         P.units_q = (uint32_t)(units / grid);
         P.units_r = (uint32_t)(units % grid);
-        P.counters = reinterpret_cast<uint32_t*>(ws);
-        P.partial = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + off_partial);
-        RLXQ_CUDA_TRY(cudaMemsetAsync(P.counters, 0, (size_t)ntiles * 4, stream));
-    } else if (grid > ntiles) {
-        grid = ntiles;
+        P.counters = static_cast<unsigned long long*>(ws);
+        P.partial = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + off_partial);
+        P.tag = next_gemm_tag();
+    } else if (grid > ntiles && !c.groups) {
+        grid = (uint32_t)ntiles;
     }
-    gemm_tcgen05_kernel<SCHEME, TX><<<grid, (4 + 4 * GemmRaw<SCHEME>::GROUPS + 4) * 32, smem, stream>>>(P);
+    rc = launch_pdl(gemm_tcgen05_kernel<SCHEME, PRECISE>, dim3(grid), dim3((4 + 4 * GemmRaw<SCHEME>::GROUPS + 4) * 32), smem, stream, P);
+    if (rc) return rc;
     count_launch();
+    if (P.slices > 1) return launch_add_slices(stream, static_cast<const float*>(ws), P.slices, P.slice_elems, c.y, c.ybf, (uint64_t)c.x_rows * c.n);
     return check_launch("gemm_tcgen05_kernel");
+}
+template <uint32_t SCHEME>
+static int launch_gemm_t_any(cudaStream_t stream, const GemmCall& c, const GemmShape& sh, void* ws) {
+    return c.precise ? launch_gemm_t<SCHEME, true>(stream, c, sh, ws) : launch_gemm_t<SCHEME, false>(stream, c, sh, ws);
 }
 
 // The two-CTA form: whole 256 x 256 tile pairs dealt round-robin to as many clusters as are resident at once.
-static bool gemm_pair_fits(uint32_t m, uint32_t k, uint32_t n) {
-    return n % 256 == 0 && m >= 1 && k % 256 == 0;
-}
-// Chosen by itself where it measured faster: at least one 256 x 256 tile pair per resident cluster, and a format
-// whose decoder keeps pace with two groups of decode warps (Q6_K and Q3_K, with three groups, lose 5-12 % in the
-// paired form on large shapes).
 template <uint32_t SCHEME>
-static bool gemm_wants_pair(uint32_t m, uint32_t k, uint32_t n) {
-    const int64_t opt = options().gemm_pair.load();
-    if (opt == 1 || !gemm_pair_fits(m, k, n)) return false;
-    if (opt == 2) return true;
-    if (SCHEME == RLXQ_Q6_K || SCHEME == RLXQ_Q3_K) return false;
-    return (uint64_t)(n / 256) * ((m + 255) / 256) >= (uint64_t)sm_count() / 2;
-}
-template <uint32_t SCHEME>
-static int launch_gemm_pair_t(cudaStream_t stream, const void* x, const uint8_t* w, void* y, bool ybf, uint32_t m,
-                              uint32_t k, uint32_t n) {
+static int launch_gemm_pair_t(cudaStream_t stream, const GemmCall& c) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
     constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128;
     Geometry g;
     geometry(SCHEME, &g);
     GemmParams P{};
-    int rc = encode_bf16_kmajor_map(&P.xmap, x, m, k, kPairHalf);
+    P.lo_row = c.f32 ? c.x_rows : 0u;
+    int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * (c.f32 ? 2 : 1), c.k, kPairHalf);
     if (rc) return rc;
-    rc = encode_weight_map(&P.wmap, w, n, (uint64_t)k / g.elems * g.bytes, RAW_ROW / 8, kGemmTileW);
+    rc = encode_weight_map(&P.wmap, c.w, c.n, (uint64_t)c.k / g.elems * g.bytes, RAW_ROW / 8, kGemmTileW);
     if (rc) return rc;
-    P.y = y; P.m = m; P.n = n; P.k = k; P.y_bf16 = ybf;
-    P.y_vec = (((uintptr_t)y & 15u) == 0 && n % (ybf ? 8u : 4u) == 0) ? 1u : 0u;
-    P.wtiles = n / kGemmTileW;
-    P.xtiles = (m + 255) / 256;
-    P.kgroups = k / 256;
+    P.y = c.y; P.m = c.x_rows; P.n = c.n; P.k = c.k; P.y_bf16 = c.ybf;
+    P.y_vec = (((uintptr_t)c.y & 15u) == 0 && c.n % (c.ybf ? 8u : 4u) == 0) ? 1u : 0u;
+    P.wtiles = c.n / kGemmTileW;
+    P.xtiles = (c.x_rows + 255) / 256;
+    P.kgroups = c.k / 256;
     P.err = device_error_word();
     if (!P.err) return fail(RLXQ_E_CUDA, "device error word unavailable");
     const size_t smem = 1024 + (size_t)kPairStages * kPairBBytes + (size_t)kGemmRawStages * RAW_STRIDE + sizeof(PairBars) + 64 +
                         kGemmEpiStage;
     const uint32_t threads = (4 + 4 * GemmRaw<SCHEME>::GROUPS + 4) * 32;
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = options().pdl.load() ? 1 : 0;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -1426,77 +1629,36 @@ static int launch_gemm_pair_t(cudaStream_t stream, const void* x, const uint8_t*
     if (pairs > (uint32_t)sm_count() / 2) pairs = (uint32_t)sm_count() / 2;
     if (pairs > ptiles) pairs = ptiles;
     cfg.gridDim = dim3(2 * pairs);
+    cfg.numAttrs = 2;
     RLXQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<SCHEME>, P));
     count_launch();
     return check_launch("gemm_pair_kernel");
 }
 
-// 256-row activation tiles halve the activation traffic per FLOP.  When whole tiles would fill the SMs
-// badly the k dimension is split as well (stream-K, needs the workspace); without a workspace, 128-row
-// tiles are used when the wider ones would leave more than a quarter of the SMs without a tile.
 template <uint32_t SCHEME>
-static int launch_gemm_s(cudaStream_t stream, const void* x, const uint8_t* w, void* y, bool ybf, uint32_t m,
-                         uint32_t k, uint32_t n, void* ws, size_t ws_bytes) {
-    const uint32_t wt = (n + kGemmTileW - 1) / kGemmTileW, sms = (uint32_t)sm_count();
-    const int64_t force = options().gemm_tile_x.load();
-    const uint32_t ntiles256 = wt * ((m + 255) / 256);
-    if (options().gemm_pair.load() == 2 && gemm_pair_fits(m, k, n))               // forced: two CTAs per MMA
-        return launch_gemm_pair_t<SCHEME>(stream, x, w, y, ybf, m, k, n);
-    if (force != 128 && gemm_wants_streamk(m, k, n) && ws && !((uintptr_t)ws & 15u) &&
-        ws_bytes >= gemm_streamk_bytes(ntiles256, nullptr))
-        return launch_gemm_t<SCHEME, 256>(stream, x, w, y, ybf, m, k, n, ws, true);
-    const bool narrow = force ? force == 128 : (ntiles256 * 4 < sms * 3);
-    if (narrow) return launch_gemm_t<SCHEME, 128>(stream, x, w, y, ybf, m, k, n, nullptr, false);
-    if (force == 0 && gemm_wants_pair<SCHEME>(m, k, n)) return launch_gemm_pair_t<SCHEME>(stream, x, w, y, ybf, m, k, n);
-    return launch_gemm_t<SCHEME, 256>(stream, x, w, y, ybf, m, k, n, nullptr, false);
+static int launch_gemm_s(cudaStream_t stream, const GemmCall& c, void* ws, size_t ws_bytes) {
+    if (c.groups) return launch_gemm_t_any<SCHEME>(stream, c, GemmShape{c.tile_rows, c.group_tiles, 1, false, false}, nullptr);
+    GemmShape sh = gemm_choose(SCHEME, c.x_rows, c.k, c.n, c.f32, c.precise, true);
+    if ((sh.streamk || sh.slices > 1) && (!ws || ((uintptr_t)ws & 15u) || ws_bytes < gemm_shape_bytes(sh, c.x_rows, c.n)))
+        sh = gemm_choose(SCHEME, c.x_rows, c.k, c.n, c.f32, c.precise, false);
+    if (sh.pair) return launch_gemm_pair_t<SCHEME>(stream, c);
+    return launch_gemm_t_any<SCHEME>(stream, c, sh, ws);
 }
 
-// Grouped form for MoE expert stacks: x holds x_rows gathered bf16 activation rows, w a stack of num_slabs
-// [n, k] slabs, groups[0 .. group_tiles) the device-side table of activation tiles of tile_rows (128 or 256) rows
-// (GemmParams::groups), y2 the f32 result rows in the order of x.
-template <uint32_t SCHEME>
-static int launch_gemm_grouped_s(cudaStream_t stream, const void* x, uint32_t x_rows, const uint8_t* w, uint32_t num_slabs,
-                                 float* y2, uint32_t k, uint32_t n, const uint4* gt, uint32_t group_tiles, uint32_t tile_rows) {
-    if (tile_rows == 256) return launch_gemm_t<SCHEME, 256>(stream, x, w, y2, false, x_rows, k, n, nullptr, false, gt, group_tiles, num_slabs);
-    return launch_gemm_t<SCHEME, 128>(stream, x, w, y2, false, x_rows, k, n, nullptr, false, gt, group_tiles, num_slabs);
-}
-
-int launch_gemm_grouped(cudaStream_t stream, uint32_t scheme, const void* x, uint32_t x_rows, const uint8_t* w,
-                        uint32_t num_slabs, float* y2, uint32_t k, uint32_t n, const void* groups, uint32_t group_tiles,
-                        uint32_t tile_rows) {
-    const uint4* gt = static_cast<const uint4*>(groups);
-    if ((uint64_t)n * num_slabs > 0x7FFFFFFFull) return fail(RLXQ_E_LIMIT, "expert stack too tall for a tensor map");
-    if (tile_rows != 128 && tile_rows != 256) return fail(RLXQ_E_ARG, "activation tiles are 128 or 256 rows");
+int launch_gemm(cudaStream_t stream, uint32_t scheme, const GemmCall& c, void* ws, size_t ws_bytes) {
+    if ((uint64_t)c.n * c.num_slabs > 0x7FFFFFFFull) return fail(RLXQ_E_LIMIT, "weights too tall for a tensor map");
     switch (scheme) {
-        case RLXQ_Q4_0: return launch_gemm_grouped_s<RLXQ_Q4_0>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q8_0: return launch_gemm_grouped_s<RLXQ_Q8_0>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q4_K: return launch_gemm_grouped_s<RLXQ_Q4_K>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q5_K: return launch_gemm_grouped_s<RLXQ_Q5_K>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q2_K: return launch_gemm_grouped_s<RLXQ_Q2_K>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q8_K: return launch_gemm_grouped_s<RLXQ_Q8_K>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q4_1: return launch_gemm_grouped_s<RLXQ_Q4_1>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q5_0: return launch_gemm_grouped_s<RLXQ_Q5_0>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q5_1: return launch_gemm_grouped_s<RLXQ_Q5_1>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q3_K: return launch_gemm_grouped_s<RLXQ_Q3_K>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        case RLXQ_Q6_K: return launch_gemm_grouped_s<RLXQ_Q6_K>(stream, x, x_rows, w, num_slabs, y2, k, n, gt, group_tiles, tile_rows);
-        default: return fail(RLXQ_E_SCHEME, "unknown scheme");
-    }
-}
-
-int launch_gemm_tc(cudaStream_t stream, uint32_t scheme, const void* x, const uint8_t* w, void* y, bool ybf,
-                   uint32_t m, uint32_t k, uint32_t n, void* ws, size_t ws_bytes) {
-    switch (scheme) {
-        case RLXQ_Q4_0: return launch_gemm_s<RLXQ_Q4_0>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q8_0: return launch_gemm_s<RLXQ_Q8_0>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q4_K: return launch_gemm_s<RLXQ_Q4_K>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q5_K: return launch_gemm_s<RLXQ_Q5_K>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q2_K: return launch_gemm_s<RLXQ_Q2_K>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q8_K: return launch_gemm_s<RLXQ_Q8_K>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q4_1: return launch_gemm_s<RLXQ_Q4_1>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q5_0: return launch_gemm_s<RLXQ_Q5_0>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q5_1: return launch_gemm_s<RLXQ_Q5_1>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q3_K: return launch_gemm_s<RLXQ_Q3_K>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
-        case RLXQ_Q6_K: return launch_gemm_s<RLXQ_Q6_K>(stream, x, w, y, ybf, m, k, n, ws, ws_bytes);
+        case RLXQ_Q4_0: return launch_gemm_s<RLXQ_Q4_0>(stream, c, ws, ws_bytes);
+        case RLXQ_Q8_0: return launch_gemm_s<RLXQ_Q8_0>(stream, c, ws, ws_bytes);
+        case RLXQ_Q4_K: return launch_gemm_s<RLXQ_Q4_K>(stream, c, ws, ws_bytes);
+        case RLXQ_Q5_K: return launch_gemm_s<RLXQ_Q5_K>(stream, c, ws, ws_bytes);
+        case RLXQ_Q2_K: return launch_gemm_s<RLXQ_Q2_K>(stream, c, ws, ws_bytes);
+        case RLXQ_Q8_K: return launch_gemm_s<RLXQ_Q8_K>(stream, c, ws, ws_bytes);
+        case RLXQ_Q4_1: return launch_gemm_s<RLXQ_Q4_1>(stream, c, ws, ws_bytes);
+        case RLXQ_Q5_0: return launch_gemm_s<RLXQ_Q5_0>(stream, c, ws, ws_bytes);
+        case RLXQ_Q5_1: return launch_gemm_s<RLXQ_Q5_1>(stream, c, ws, ws_bytes);
+        case RLXQ_Q3_K: return launch_gemm_s<RLXQ_Q3_K>(stream, c, ws, ws_bytes);
+        case RLXQ_Q6_K: return launch_gemm_s<RLXQ_Q6_K>(stream, c, ws, ws_bytes);
         default: return fail(RLXQ_E_SCHEME, "unknown scheme");
     }
 }

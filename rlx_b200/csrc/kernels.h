@@ -25,7 +25,7 @@ int launch_gemv_int(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
 
 // tcgen05 / tensor-memory GEMV (m <= 8): weights decoded to fp16 in tensor memory, activations as bf16 high / low rows.
 int launch_split_hi_lo(cudaStream_t stream, const float* x, void* out, uint64_t rows, uint64_t k);
-int launch_add_halves(cudaStream_t stream, const float* y2, void* y, bool ybf, uint64_t rows, uint64_t n);
+int launch_add_slices(cudaStream_t stream, const float* part, uint32_t slices, uint64_t stride, void* y, bool ybf, uint64_t total);
 int launch_swiglu_pair(cudaStream_t stream, const float* gu, void* h, uint32_t m, uint32_t f);
 // A chain of dependent batch-1/2 GEMVs in one cooperative launch (gemv_int.cu, gemv_chain_kernel).
 struct ChainLayer { const uint8_t* w; uint32_t k, n, swiglu; };
@@ -43,14 +43,33 @@ size_t gemv_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t
 int launch_gemv_tc(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf,
                    uint32_t m, uint32_t k, uint32_t n, void* ws, size_t ws_bytes);
 
-// tcgen05 / tensor-memory GEMM (m > 8, bf16 activations).
-bool gemm_tc_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* w, const void* x, bool xbf);
-size_t gemm_tc_workspace_bytes(uint32_t m, uint32_t k, uint32_t n);
-int launch_gemm_grouped(cudaStream_t stream, uint32_t scheme, const void* x, uint32_t x_rows, const uint8_t* w,
-                        uint32_t num_slabs, float* y2, uint32_t k, uint32_t n, const void* groups, uint32_t group_tiles,
-                        uint32_t tile_rows);
-int launch_gemm_tc(cudaStream_t stream, uint32_t scheme, const void* x, const uint8_t* w, void* y, bool ybf,
-                   uint32_t m, uint32_t k, uint32_t n, void* ws, size_t ws_bytes);
+// tcgen05 / tensor-memory GEMM (m > 8).
+struct GemmCall {
+    const void* x;             // bf16 [x_rows, k]; with f32 set, bf16(x) followed by bf16(x - bf16(x)), x_rows rows each
+    uint32_t x_rows;
+    bool f32;
+    const uint8_t* w;
+    uint64_t w_pitch;          // bytes between weight rows that a kernel in front has re-laid (0: packed, and constant)
+    bool precise;              // weights as bf16 hi + lo instead of rounded to bf16
+    void* y;
+    bool ybf;
+    uint32_t k, n;
+    // expert stacks: num_slabs [n, k] slabs, groups = the device-side tile table (GemmParams::groups) of tiles of tile_rows
+    // rows, at most group_tiles of them, and the row of y every gathered row of x belongs to
+    uint32_t num_slabs = 1;
+    const void* groups = nullptr;
+    uint32_t group_tiles = 0, tile_rows = 0;
+    const uint32_t* row_map = nullptr;
+};
+bool gemm_tc_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* w, const void* x);
+bool gemm_relaid_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* x);
+uint64_t gemm_relaid_pitch(uint32_t scheme, uint32_t k);
+size_t gemm_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise);
+int launch_gemm(cudaStream_t stream, uint32_t scheme, const GemmCall& c, void* ws, size_t ws_bytes);
+// n rows of row_bytes bytes -> rows of pitch bytes (a multiple of 16), zero behind the row.  With `used` (the exclusive
+// scan of an expert stack's row counts) slabs of slab_rows rows that nobody is routed to are left out.
+int launch_relay_rows(cudaStream_t stream, const uint8_t* w, uint64_t row_bytes, uint64_t n, uint8_t* out, uint64_t pitch,
+                      const uint32_t* used = nullptr, uint32_t slab_rows = 1);
 
 // One MoE decode row: the slab of the weight stack is chosen by *expert_sel on the device.
 bool int_expert_supported(uint32_t scheme, uint32_t k, uint32_t n, const void* w, const void* x);

@@ -2,8 +2,8 @@
 //
 // Replaces the reference's host-sorted lowering (rlx-cuda/src/gguf_gpu.rs:142-280): D2H of x and the
 // expert ids, counting sort on the CPU, per-expert dequantise + sgemm, H2D of the result.  Here:
-//   moe_sort_kernel     one CTA: rows per expert (shared-memory atomics), exclusive scan, row
-//                       permutation grouped by expert -- grouped_moe_sort_plan
+//   moe_count_kernel    one CTA: rows per expert (shared-memory atomics), exclusive scan
+//   moe_place_kernel    the row permutation grouped by expert -- grouped_moe_sort_plan
 //                       (rlx-cpu/src/gguf_matmul.rs:178-205) without the copy of x: the matmul
 //                       kernel reads the rows through the permutation instead
 //   moe_grouped_kernel  grid (weight-row tiles, experts): a warp owns one weight row of one expert,
@@ -13,56 +13,108 @@
 //                       grouped_moe_unpermute_out, gguf_matmul.rs:207-218, is the store address)
 // Accumulation is f32 in a different order from the CPU loop; same tolerance as the general kernel.
 //
-// Prefill-sized batches (32 rows and more, the tensor-core GEMM's formats and shapes) go through the tcgen05
-// GEMM in its grouped form instead of moe_grouped_kernel:
-//   moe_tiles_kernel    the table of 128- or 256-row activation tiles, one list per expert, from the sorted offsets
+// More than eight rows (and eight or fewer of a shape the streaming GEMV does not take) go through the tcgen05 GEMM in
+// its grouped form instead of moe_grouped_kernel, which only runs when the workspace is too small for it:
+//   moe_tiles_kernel    the table of activation tiles, one list per expert, from the sorted offsets
+//   relay_rows_kernel   (rows TMA cannot tile) the slabs of the experts in use on a padded pitch
 //   moe_gather_kernel   the rows of every expert, gathered next to each other as bf16 (f32 activations as
-//                       bf16 hi rows followed by the expert's lo rows, so nothing of x is lost)
-//   gemm_tcgen05_kernel every tile against its expert's slab of the stack (gemm_tcgen05.cu, GemmParams::groups)
-//   moe_scatter_kernel  results (hi + lo) to the rows' original positions
-// The weight operand is bf16(d * q) there, as in the dense GEMM: same tolerance as that kernel.
+//                       bf16 hi rows and, m rows further on, lo rows, so nothing of x is lost)
+//   gemm_tcgen05_kernel every tile against its expert's slab of the stack (gemm_tcgen05.cu, GemmParams::groups), results
+//                       stored at the rows' original positions
+// The weight operand is bf16(d * q) there, as in the dense GEMM; for fewer than 32 rows, and rows of those other lengths,
+// it keeps 16 bits (hi + lo).
+// All of them are launched as programmatic dependents.  1024 rows over 8 experts of 4096 -> 14336 Q4_K: 230 us; 331 us
+// with fixed 128-row tiles, an f32 result array and a scatter kernel behind the GEMM.
 //
 // Decode (m <= 8 rows, Q4_0 / Q8_0 / Q4_K / Q6_K, k a multiple of 256 up to 12288) skips both kernels:
 // every row is one launch of the streaming integer GEMV over the whole stack seen as an
 // [experts * n, k] matrix, with the slab picked on the device from expert_idx[i] (gemv_int.cu,
 // expert-indirect mode), so a routed expert's weights come through the TMA ring at GEMV speed.
+#include <cmath>
+
 #include "common.cuh"
 #include "decode.cuh"
 #include "kernels.h"
 #include "rlxq_moe.h"
+#include "staged_common.cuh"
 
 namespace rlxq {
 
 constexpr uint32_t kMoeInvalid = 0xFFFFFFFFu;
 
-// offsets[0..E] (exclusive scan of the counts), perm[sorted position] = original row.
-__global__ void __launch_bounds__(1024) moe_sort_kernel(const float* __restrict__ expert_idx, uint32_t m, uint32_t E,
-                                                        uint32_t* __restrict__ offsets, uint32_t* __restrict__ cursor,
-                                                        uint32_t* __restrict__ perm) {
-    extern __shared__ uint32_t cnt[];          // [E]
-    for (uint32_t e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0u;
+constexpr uint32_t kMoeScanThreads = 1024;
+// Inclusive block-wide running sum over kMoeScanThreads threads.
+__device__ __forceinline__ uint32_t moe_block_scan(uint32_t v, uint32_t (&wsum)[32]) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += u;
+    }
+    __syncthreads();                           // the previous call's sums have been read
+    if (lane == 31) wsum[warp] = v;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+    uint32_t before = 0u;
+    for (uint32_t w = 0; w < warp; ++w) before += wsum[w];
+    return v + before;
+}
+
+// One CTA: offsets[0..E] = exclusive scan of the rows per expert, cursor[0..E] the same (where the next row of an expert
+// goes; [E]: the rows no expert takes, behind all others).
+__global__ void __launch_bounds__(kMoeScanThreads) moe_count_kernel(const float* __restrict__ expert_idx, uint32_t m, uint32_t E,
+                                                                    uint32_t* __restrict__ offsets, uint32_t* __restrict__ cursor) {
+    extern __shared__ uint32_t cnt[];          // [E]
+    __shared__ uint32_t wsum[32], total;
+    griddep_launch_dependents();
+    for (uint32_t e = threadIdx.x; e < E; e += kMoeScanThreads) cnt[e] = 0u;
+    griddep_wait();
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < m; i += kMoeScanThreads) {
         uint32_t e;
         if (expert_of_row(expert_idx[i], E, &e)) atomicAdd(&cnt[e], 1u);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {                    // E is small (tens to hundreds): a serial scan is enough
-        uint32_t run = 0;
-        for (uint32_t e = 0; e < E; ++e) {
-            offsets[e] = run;
-            cursor[e] = run;
-            run += cnt[e];
-        }
-        offsets[E] = run;
+    uint32_t carry = 0u;
+    for (uint32_t e0 = 0; e0 < E; e0 += kMoeScanThreads) {
+        const uint32_t e = e0 + threadIdx.x, c = e < E ? cnt[e] : 0u, incl = carry + moe_block_scan(c, wsum);
+        if (e < E) { offsets[e] = incl - c; cursor[e] = incl - c; }
+        if (threadIdx.x == kMoeScanThreads - 1) total = incl;
+        __syncthreads();
+        carry = total;
     }
-    __syncthreads();
-    __threadfence_block();
-    // cursor lives in global memory (this CTA is its only user); atomics hand out the slots
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-        uint32_t e;
-        if (expert_of_row(expert_idx[i], E, &e)) perm[atomicAdd(&cursor[e], 1u)] = i;
+    if (threadIdx.x == 0) { offsets[E] = carry; cursor[E] = carry; }
+}
+
+// perm[sorted position] = original row.
+__global__ void __launch_bounds__(256) moe_place_kernel(const float* __restrict__ expert_idx, uint32_t m, uint32_t E,
+                                                        uint32_t* __restrict__ cursor, uint32_t* __restrict__ perm) {
+    griddep_launch_dependents();
+    griddep_wait();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    uint32_t e;
+    if (!expert_of_row(expert_idx[i], E, &e)) e = E;
+    perm[atomicAdd(&cursor[e], 1u)] = i;
+}
+
+// The GEMM's tile table: table[0] = {tiles, routed rows}, table[1 + t] = {first sorted position, rows, expert, 0}, tiles of
+// tile_rows rows, expert by expert.
+__global__ void __launch_bounds__(kMoeScanThreads) moe_tiles_kernel(const uint32_t* __restrict__ offsets, uint32_t E,
+                                                                    uint4* __restrict__ table, uint32_t tile_rows) {
+    __shared__ uint32_t wsum[32], total;
+    griddep_launch_dependents();
+    griddep_wait();
+    uint32_t carry = 0u;
+    for (uint32_t e0 = 0; e0 < E; e0 += kMoeScanThreads) {
+        const uint32_t e = e0 + threadIdx.x, r0 = e < E ? offsets[e] : 0u, c = e < E ? offsets[e + 1] - r0 : 0u;
+        const uint32_t t = (c + tile_rows - 1) / tile_rows, incl = carry + moe_block_scan(t, wsum);
+        for (uint32_t q = 0; q < t; ++q)
+            table[1 + incl - t + q] = make_uint4(r0 + q * tile_rows, min(tile_rows, c - q * tile_rows), e, 0u);
+        if (threadIdx.x == kMoeScanThreads - 1) total = incl;
+        __syncthreads();
+        carry = total;
     }
+    if (threadIdx.x == 0) table[0] = make_uint4(carry, offsets[E], 0u, 0u);
 }
 
 template <bool XBF16>
@@ -142,48 +194,41 @@ static void launch_grouped_s(cudaStream_t s, dim3 grid, bool xbf, bool ybf, cons
 
 constexpr uint32_t kMoeDecodeRows = 8;      // up to this many rows go row by row through the streaming GEMV
 
-// ---- prefill-sized batches on the tensor-core GEMM ------------------------------------------------------------
+// ---- the tensor-core GEMM in its grouped form ------------------------------------------------------------------
 
-// activation rows per GEMM tile in grouped mode: 256 when the experts get about that many gathered rows each
-// (a weight tile is then decoded once for all of them), else 128
-static uint32_t moe_tile_rows(uint32_t gathered_rows, uint32_t E) { return gathered_rows / E >= 160u ? 256u : 128u; }
-constexpr uint32_t kMoeTcMinRows = 32;      // smaller batches stay on moe_grouped_kernel
+constexpr uint32_t kMoeBf16Rows = 32;       // batches of this size and more multiply bf16-rounded weights (where TMA can
+                                            // tile them); smaller ones keep 16 bits of the weights (GemmCall::precise)
 
-// table[t] = {first gathered row, rows, expert, 0} for the tiles in use, {0, 0, 0, 0} up to `bound`.
-// mult = gathered rows per activation row (2 for f32 activations: hi and lo halves).
-__global__ void moe_tiles_kernel(const uint32_t* __restrict__ offsets, uint32_t E, uint32_t mult, uint4* __restrict__ table,
-                                 uint32_t bound, uint32_t tile_rows) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        uint32_t t = 0;
-        for (uint32_t e = 0; e < E; ++e) {
-            const uint32_t base = mult * offsets[e], rows = mult * (offsets[e + 1] - offsets[e]);
-            for (uint32_t r = 0; r < rows && t < bound; r += tile_rows, ++t)
-                table[t] = make_uint4(base + r, min(tile_rows, rows - r), e, 0u);
-        }
-        for (; t < bound; ++t) table[t] = make_uint4(0u, 0u, 0u, 0u);
-    }
+// Activation rows per GEMM tile: what one expert's share of the rows needs, with room for an uneven routing (2.5 standard
+// deviations of an even one), so that a slab is hardly ever decoded twice; f32 activations take two boxes per tile.
+static uint32_t moe_tile_rows(uint32_t m, uint32_t E, bool xbf) {
+    const float share = (float)m / (float)E;
+    const uint32_t want = ((uint32_t)(share + 2.5f * sqrtf(share)) + 31u) / 32u * 32u, most = xbf ? 256u : 128u;
+    return want < 32u ? 32u : (want > most ? most : want);
 }
 
-// One CTA per sorted position i: row perm[i] of x goes to row mult * offsets[e] + j of xg (j = position inside
-// the expert's group), and for f32 activations its lo half to row mult * offsets[e] + count_e + j.
+// One CTA per sorted position i: row perm[i] of x becomes row i of xg, as bf16 hi and, for f32 activations, lo part (m
+// rows further on).  The rows no expert takes come last; their outputs are set to zero here.
 template <bool XBF16>
-__global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict__ x, const float* __restrict__ expert_idx,
-                                                         const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ perm,
-                                                         uint32_t E, uint32_t k, uint16_t* __restrict__ xg) {
-    const uint32_t i = blockIdx.x;
-    if (i >= offsets[E]) return;
-    const uint32_t src = perm[i];
-    uint32_t e = 0;
-    expert_of_row(expert_idx[src], E, &e);
-    const uint32_t j = i - offsets[e], cnt = offsets[e + 1] - offsets[e];
+__global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict__ x, const uint32_t* __restrict__ perm,
+                                                         const uint4* __restrict__ table, uint32_t m, uint32_t k,
+                                                         uint16_t* __restrict__ xg, uint8_t* __restrict__ y, uint64_t y_row_bytes) {
+    griddep_launch_dependents();
+    griddep_wait();
+    const uint32_t i = blockIdx.x, src = perm[i];
+    if (i >= table[0].y) {
+        uint8_t* row = y + (size_t)src * y_row_bytes;
+        for (uint64_t b = 2 * threadIdx.x; b < y_row_bytes; b += 2 * blockDim.x) *reinterpret_cast<uint16_t*>(row + b) = 0;
+        return;
+    }
     if constexpr (XBF16) {
-        const uint2* in = reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(x) + (size_t)src * k);
-        uint2* out = reinterpret_cast<uint2*>(xg + (size_t)(offsets[e] + j) * k);
-        for (uint32_t c = threadIdx.x; c < k / 4; c += blockDim.x) out[c] = in[c];
+        const uint4* in = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + (size_t)src * k);
+        uint4* out = reinterpret_cast<uint4*>(xg + (size_t)i * k);
+        for (uint32_t c = threadIdx.x; c < k / 8; c += blockDim.x) out[c] = in[c];
     } else {
         const float4* in = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + (size_t)src * k);
-        uint2* hi = reinterpret_cast<uint2*>(xg + (size_t)(2 * offsets[e] + j) * k);
-        uint2* lo = reinterpret_cast<uint2*>(xg + (size_t)(2 * offsets[e] + cnt + j) * k);
+        uint2* hi = reinterpret_cast<uint2*>(xg + (size_t)i * k);
+        uint2* lo = reinterpret_cast<uint2*>(xg + (size_t)(m + i) * k);
         for (uint32_t c = threadIdx.x; c < k / 4; c += blockDim.x) {
             const float4 v = in[c];
             const float f[4] = {v.x, v.y, v.z, v.w};
@@ -200,57 +245,38 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict_
     }
 }
 
-// One CTA per sorted position: y[perm[i]] = y2[hi row] (+ y2[lo row]).
-template <bool YBF16>
-__global__ void __launch_bounds__(256) moe_scatter_kernel(const float* __restrict__ y2, const float* __restrict__ expert_idx,
-                                                          const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ perm,
-                                                          uint32_t E, uint32_t n, uint32_t mult, void* __restrict__ y) {
-    const uint32_t i = blockIdx.x;
-    if (i >= offsets[E]) return;
-    const uint32_t dst = perm[i];
-    uint32_t e = 0;
-    expert_of_row(expert_idx[dst], E, &e);
-    const uint32_t j = i - offsets[e], cnt = offsets[e + 1] - offsets[e];
-    const float* a = y2 + (size_t)(mult * offsets[e] + j) * n;
-    const float* b = a + (size_t)cnt * n;
-    for (uint32_t c = threadIdx.x; c < n; c += blockDim.x) {
-        const float v = mult == 2 ? a[c] + b[c] : a[c];
-        if constexpr (YBF16) reinterpret_cast<uint16_t*>(y)[(size_t)dst * n + c] = (uint16_t)f32_to_bf16_bits(v);
-        else reinterpret_cast<float*>(y)[(size_t)dst * n + c] = v;
-    }
-}
+struct MoeTcPlan { bool ok, relaid; uint32_t tiles, tile_rows; uint64_t pitch; size_t off_table, off_xg, off_w, bytes; };
 
-struct MoeTcPlan { bool ok; uint32_t mult, rows, tiles, tile_rows; size_t off_table, off_xg, off_y2, bytes; };
-
-// The scratch of the tensor-core path behind the sort's arrays (which end at `base`): tile table, gathered
-// activations, result rows.  Not taken (ok = false) for small batches, other formats or shapes, or when it would
-// need more than 4 GiB.
-static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, size_t base) {
+// The scratch of the tensor-core path behind the sort's arrays (which end at `base`): tile table, gathered activations
+// and, for rows TMA cannot tile where they lie, the re-laid slabs.  Not taken (ok = false) for other formats or when it
+// would need more than 4 GiB.
+static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, bool w_aligned, size_t base) {
     MoeTcPlan p{};
-    if (m < kMoeTcMinRows || options().gemm_kernel.load() == 1) return p;
-    if (!gemm_tc_supported(scheme, m, k, n, (const void*)256, (const void*)256, true)) return p;
+    const void* aligned = (const void*)256;
+    if (options().gemm_kernel.load() == 1) return p;
+    p.relaid = !(w_aligned && gemm_tc_supported(scheme, m, k, n, aligned, aligned));
+    if (p.relaid && !gemm_relaid_supported(scheme, m, k, n, aligned)) return p;
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-    p.mult = xbf ? 1u : 2u;
-    p.rows = p.mult * m;
-    p.tile_rows = moe_tile_rows(p.rows, E);
-    p.tiles = (p.rows + 127) / 128 + E;      // enough for either tile size
+    p.tile_rows = moe_tile_rows(m, E, xbf);
+    p.tiles = m / p.tile_rows + (E < m ? E : m);
+    p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;
     p.off_table = up(base);
-    p.off_xg = p.off_table + up((size_t)p.tiles * 16);
-    p.off_y2 = p.off_xg + up((size_t)p.rows * k * 2);
-    p.bytes = p.off_y2 + up((size_t)p.rows * n * 4);
+    p.off_xg = p.off_table + up((size_t)(p.tiles + 1) * 16);
+    p.off_w = p.off_xg + up((size_t)(xbf ? 1 : 2) * m * k * 2);
+    p.bytes = p.off_w + up((size_t)p.pitch * n * E);
     p.ok = p.bytes <= (4ull << 30) && (uint64_t)n * E <= 0x7FFFFFFFull;
     return p;
 }
 
-static size_t grouped_ws(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, size_t* off_cursor,
-                         size_t* off_perm, MoeTcPlan* tc) {
+static size_t grouped_ws(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, bool w_aligned,
+                         size_t* off_cursor, size_t* off_perm, MoeTcPlan* tc) {
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
     size_t off = up(((size_t)E + 1) * 4);
     if (off_cursor) *off_cursor = off;
-    off += up((size_t)E * 4);
+    off += up(((size_t)E + 1) * 4);
     if (off_perm) *off_perm = off;
     off += up((size_t)m * 4);
-    const MoeTcPlan p = plan_moe_tc(scheme, m, k, n, E, xbf, off);
+    const MoeTcPlan p = plan_moe_tc(scheme, m, k, n, E, xbf, w_aligned, off);
     if (tc) *tc = p;
     if (p.ok) off = p.bytes;
     const size_t gemv = m <= kMoeDecodeRows ? up(int_workspace_bytes(scheme, 1, k, n)) : 0;   // the decode path's scratch
@@ -268,8 +294,10 @@ extern "C" int rlxq_grouped_workspace_bytes(uint32_t scheme, uint32_t m, uint32_
     if (!geometry(scheme, &g)) return fail(RLXQ_E_SCHEME, "unknown scheme %u", scheme);
     if (k == 0 || k % g.elems) return fail(RLXQ_E_SHAPE, "k=%u is not a positive multiple of the block size %u", k, g.elems);
     if (num_experts == 0 || num_experts > 8192) return fail(RLXQ_E_LIMIT, "num_experts=%u must be in [1, 8192]", num_experts);
-    // sized for f32 activations (two gathered rows per row); bf16 activations need less of it
-    *bytes = grouped_ws(scheme, m, k, n, num_experts, false, nullptr, nullptr, nullptr);
+    // f32 activations gather twice the rows, bf16 ones may need another tile table
+    *bytes = grouped_ws(scheme, m, k, n, num_experts, false, true, nullptr, nullptr, nullptr);
+    const size_t bf = grouped_ws(scheme, m, k, n, num_experts, true, true, nullptr, nullptr, nullptr);
+    if (bf > *bytes) *bytes = bf;
     return RLXQ_OK;
 }
 
@@ -289,10 +317,12 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     if ((uintptr_t)y & (y_dtype == RLXQ_BF16 ? 1u : 3u)) return fail(RLXQ_E_ALIGN, "y must be aligned to its element size");
     size_t off_cursor = 0, off_perm = 0;
     const bool xbf = x_dtype == RLXQ_BF16, ybf = y_dtype == RLXQ_BF16;
+    const uint8_t* wst = (const uint8_t*)w_blocks;
+    const size_t xes = xbf ? 2 : 4, yes = ybf ? 2 : 4;
     MoeTcPlan tc{};
-    size_t need = grouped_ws(scheme, m, k, n, num_experts, xbf, &off_cursor, &off_perm, &tc);
+    size_t need = grouped_ws(scheme, m, k, n, num_experts, xbf, !((uintptr_t)wst & 15u), &off_cursor, &off_perm, &tc);
     // the tensor-core path is taken when the workspace holds its arrays; a smaller one still runs the general kernel
-    if (tc.ok && (workspace_bytes < tc.bytes || ((uintptr_t)workspace & 255u) || ((uintptr_t)w_blocks & 15u))) {
+    if (tc.ok && (workspace_bytes < tc.bytes || ((uintptr_t)workspace & 255u) || (m <= kMoeDecodeRows && options().gemv_kernel.load() == 1))) {
         tc.ok = false;
         need = off_perm + ((size_t)m * 4 + 255) / 256 * 256;
     }
@@ -302,12 +332,11 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     uint32_t* offsets = reinterpret_cast<uint32_t*>(ws);
     uint32_t* cursor = reinterpret_cast<uint32_t*>(ws + off_cursor);
     uint32_t* perm = reinterpret_cast<uint32_t*>(ws + off_perm);
-    // rows with an id of num_experts or more are in no group: their outputs stay zero
-    RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * (ybf ? 2 : 4), s));
-    const uint8_t* wst = (const uint8_t*)w_blocks;
-    const size_t xes = xbf ? 2 : 4, yes = ybf ? 2 : 4;
-    if (m <= kMoeDecodeRows && options().gemv_kernel.load() != 1 && ((size_t)k * xes) % 16 == 0 &&
-        (uint64_t)n * num_experts <= 0x7FFFFFFFull && int_expert_supported(scheme, k, n, wst, x)) {
+    const bool decode = m <= kMoeDecodeRows && options().gemv_kernel.load() != 1 && ((size_t)k * xes) % 16 == 0 &&
+                        (uint64_t)n * num_experts <= 0x7FFFFFFFull && int_expert_supported(scheme, k, n, wst, x);
+    // rows with an id of num_experts or more are in no group: their outputs are zero (the gather kernel sees to it)
+    if (decode || !tc.ok) RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * yes, s));
+    if (decode) {
         for (uint32_t i = 0; i < m; ++i) {
             int rc = launch_gemv_int_expert(s, scheme, (const uint8_t*)x + (size_t)i * k * xes, xbf, wst,
                                             (uint8_t*)y + (size_t)i * n * yes, ybf, k, n, num_experts, expert_idx + i,
@@ -316,25 +345,34 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
         }
         return RLXQ_OK;
     }
-    moe_sort_kernel<<<1, 1024, num_experts * sizeof(uint32_t), s>>>(expert_idx, m, num_experts, offsets, cursor, perm);
+    int rc = launch_pdl(moe_count_kernel, dim3(1), dim3(kMoeScanThreads), num_experts * sizeof(uint32_t), s, expert_idx, m, num_experts,
+                        offsets, cursor);
+    if (rc) return rc;
+    count_launch();
+    rc = launch_pdl(moe_place_kernel, dim3((m + 255) / 256), dim3(256), 0, s, expert_idx, m, num_experts, cursor, perm);
+    if (rc) return rc;
     count_launch();
     if (tc.ok) {
-        uint4* table = reinterpret_cast<uint4*>(ws + tc.off_table);
         uint16_t* xg = reinterpret_cast<uint16_t*>(ws + tc.off_xg);
-        float* y2 = reinterpret_cast<float*>(ws + tc.off_y2);
-        moe_tiles_kernel<<<1, 32, 0, s>>>(offsets, num_experts, tc.mult, table, tc.tiles, tc.tile_rows);
-        count_launch();
-        if (xbf) moe_gather_kernel<true><<<m, 256, 0, s>>>(x, expert_idx, offsets, perm, num_experts, k, xg);
-        else moe_gather_kernel<false><<<m, 256, 0, s>>>(x, expert_idx, offsets, perm, num_experts, k, xg);
-        count_launch();
-        int rc = check_launch("moe_gather_kernel");
+        uint4* table = reinterpret_cast<uint4*>(ws + tc.off_table);
+        rc = launch_pdl(moe_tiles_kernel, dim3(1), dim3(kMoeScanThreads), 0, s, (const uint32_t*)offsets, num_experts, table, tc.tile_rows);
         if (rc) return rc;
-        rc = launch_gemm_grouped(s, scheme, xg, tc.rows, wst, num_experts, y2, k, n, table, tc.tiles, tc.tile_rows);
-        if (rc) return rc;
-        if (ybf) moe_scatter_kernel<true><<<m, 256, 0, s>>>(y2, expert_idx, offsets, perm, num_experts, n, tc.mult, y);
-        else moe_scatter_kernel<false><<<m, 256, 0, s>>>(y2, expert_idx, offsets, perm, num_experts, n, tc.mult, y);
         count_launch();
-        return check_launch("moe_scatter_kernel");
+        GemmCall c{};
+        c.w = wst;
+        if (tc.relaid) {
+            rc = launch_relay_rows(s, wst, (uint64_t)k / g.elems * g.bytes, (uint64_t)n * num_experts, ws + tc.off_w, tc.pitch, offsets, n);
+            if (rc) return rc;
+            c.w = ws + tc.off_w;
+        }
+        rc = launch_pdl(xbf ? moe_gather_kernel<true> : moe_gather_kernel<false>, dim3(m), dim3(256), 0, s, x, (const uint32_t*)perm,
+                        (const uint4*)table, m, k, xg, (uint8_t*)y, (uint64_t)n * yes);
+        if (rc) return rc;
+        count_launch();
+        c.x = xg; c.x_rows = m; c.f32 = !xbf; c.w_pitch = tc.pitch; c.precise = tc.relaid || m < kMoeBf16Rows;
+        c.y = y; c.ybf = ybf; c.k = k; c.n = n;
+        c.num_slabs = num_experts; c.groups = table; c.group_tiles = tc.tiles; c.tile_rows = tc.tile_rows; c.row_map = perm;
+        return launch_gemm(s, scheme, c, nullptr, 0);
     }
     const uint32_t wpc = 8;
     unsigned gx = (n + wpc - 1) / wpc;
