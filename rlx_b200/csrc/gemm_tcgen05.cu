@@ -4,7 +4,7 @@
 // y[m,n] = x[m,k] . W^T is computed transposed, tile by tile: D[128 weight rows, 256 activation
 // rows] += A[128, 64] . B[256, 64]^T per 64-wide k block.
 //   * A (weights) never exists in memory.  The raw GGUF blocks of 128 rows x 256 weights arrive in
-//     shared memory through one 2-D TMA box; eight decode warps, twelve for Q6_K (one thread per weight row, which
+//     shared memory through one 2-D TMA box; eight decode warps, twelve for Q3_K (one thread per weight row, which
 //     is also that thread's tensor-memory lane) turn 64 weights at a time into bf16(d * q) in
 //     registers and store them to tensor memory with tcgen05.st.  d * q is formed in f32 exactly as
 //     the reference decoder does (rlx-gguf/src/lib.rs:574-597, 974-1013) and rounded once to bf16.
@@ -53,15 +53,15 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // chunks, so one-row-per-lane 128-bit reads do not conflict).  `S` = which 64 of the 256.
 template <uint32_t SCHEME> struct GemmRaw;
 // GROUPS: decode warp groups (four warps each).  Two keep pace with the MMA for the cheap decoders (more only
-// add contention: measured 917 against 950 TFLOP/s for Q8_0); Q6_K's decoder is the slow one and gains 10 % from three.
+// add contention: measured 917 against 950 TFLOP/s for Q8_0); Q3_K's decoder is the slow one and gains from three.
 template <> struct GemmRaw<RLXQ_Q4_0> { static constexpr uint32_t ROW = 144, GROUPS = 2; };
 template <> struct GemmRaw<RLXQ_Q8_0> { static constexpr uint32_t ROW = 272, GROUPS = 2; };
 template <> struct GemmRaw<RLXQ_Q4_K> { static constexpr uint32_t ROW = 144, GROUPS = 2; };
 template <> struct GemmRaw<RLXQ_Q5_K> { static constexpr uint32_t ROW = 176, GROUPS = 2; };
 // Q6_K super-blocks are 210 bytes: group g of a row starts at byte 210 g, which is only 2-byte aligned.
 // The box starts at the 16-byte boundary below it and is 240 bytes wide (15 chunks: conflict-free, and
-// 14 + 210 <= 240); the decoder is compiled for each of the eight possible offsets 2 (g mod 8).
-template <> struct GemmRaw<RLXQ_Q6_K> { static constexpr uint32_t ROW = 240, GROUPS = 3; };
+// 14 + 210 <= 240); the decoder moves the words by the offset.
+template <> struct GemmRaw<RLXQ_Q6_K> { static constexpr uint32_t ROW = 240, GROUPS = 2; };
 // Q2_K super-blocks are 84 bytes (group g starts 4 (g mod 4) bytes past a 16-byte boundary: a 112-byte box covers
 // 12 + 84), Q3_K's 110 bytes (2-byte aligned only, like Q6_K: a 144-byte box covers 14 + 110).
 template <> struct GemmRaw<RLXQ_Q2_K> { static constexpr uint32_t ROW = 112, GROUPS = 2; };
@@ -315,57 +315,64 @@ template <int B0, int LEN> struct Span {
     }
 };
 
-// S = which 64 of the 256 weights, O = byte offset of the super-block inside the 240-byte row buffer.
-// Layout ql[128] | qh[64] | sc[16] (i8) | d (f16) and element order as rlx-gguf/src/lib.rs:1070-1114.
-template <int S, int O> struct Decode64Q6 {
-    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
-        constexpr int h = S / 2;
-        Span<O + 64 * h, 64> ql;
-        Span<O + 128 + 32 * h, 32> qh;
-        Span<O + 192 + 8 * h + 4 * (S % 2), 4> sc;
-        Span<O + 208, 2> dd;
-        ql.load(row); qh.load(row); sc.load(row); dd.load(row);
-        const float d = f16_bits_to_f32(dd.template word<O + 208>() & 0xFFFFu);
-        const uint32_t scw = sc.template word<O + 192 + 8 * h + 4 * (S % 2)>();   // scales 2 g4, 2 g4 + 1 of both groups
-        const float s00 = d * (float)(int8_t)(scw & 0xFFu), s01 = d * (float)(int8_t)((scw >> 8) & 0xFFu);
-        const float s10 = d * (float)(int8_t)((scw >> 16) & 0xFFu), s11 = d * (float)(int8_t)(scw >> 24);
+// Words [0, N) behind byte `off` (even, below 16) of the 16-byte aligned row piece p: the chunks that cover them, moved by
+// whole words where bits 2 and 3 of off say so and by half a word where bit 1 does.  The offset stays a run-time value: one
+// copy of the decoder instead of one per offset, whose eight copies did not stay in the instruction cache.
+template <int N> __device__ __forceinline__ void words_at(const uint8_t* p, uint32_t off, uint32_t (&q)[N]) {
+    constexpr int C = (4 * N + 14 + 15) / 16;
+    uint32_t w[4 * C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * c);
+        w[4 * c] = t.x; w[4 * c + 1] = t.y; w[4 * c + 2] = t.z; w[4 * c + 3] = t.w;
+    }
+    const bool one = off & 4u, two = off & 8u;
+    const uint32_t sh = (off & 2u) * 8u;
+#pragma unroll
+    for (int i = 0; i + 1 < 4 * C; ++i) w[i] = one ? w[i + 1] : w[i];
+#pragma unroll
+    for (int i = 0; i + 2 < 4 * C; ++i) w[i] = two ? w[i + 2] : w[i];
+#pragma unroll
+    for (int i = 0; i < N; ++i) q[i] = __funnelshift_r(w[i], w[i + 1], sh);
+}
+
+// Q6_K: ql[128] | qh[64] | sc[16] (i8) | d (f16), element order as rlx-gguf/src/lib.rs:1070-1114.  Half h (128 weights)
+// reads 64 bytes of ql and 32 of qh; its part p takes the low (p = 0) or high nibbles and two bits of qh for two
+// interleaved 32-weight groups, so both parts come from the same words.  Group g of a row starts at byte 210 g, `off` =
+// 210 g mod 16 behind the start of the row's 240-byte buffer.
+struct Q6Half {
+    uint32_t ql[16], qh[8], sc[2];
+    float d;
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t off, uint32_t h) {
+        words_at<16>(row + 64 * h, off, ql);
+        words_at<8>(row + 128 + 32 * h, off, qh);
+        uint32_t tail[5];                                                 // sc[16], d
+        words_at<5>(row + 192, off, tail);
+        sc[0] = h ? tail[2] : tail[0];
+        sc[1] = h ? tail[3] : tail[1];
+        d = f16_bits_to_f32(tail[4] & 0xFFFFu);
+    }
+    template <int PART, typename Out> __device__ __forceinline__ void decode(Out& v) const {
+        const uint64_t off = f32x2_splat(-(8388608.0f + 32.0f));
 #pragma unroll
         for (int gsel = 0; gsel < 2; ++gsel) {
-            const int g4 = 2 * (S % 2) + gsel;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const uint32_t qlw = gsel == 0 ? word_ql<0>(ql, i) : word_ql<1>(ql, i);
-                const uint32_t qhw = word_qh(qh, i);
-                const uint32_t lo = (qlw >> (4 * (g4 >> 1))) & 0x0F0F0F0Fu;
-                const uint32_t hi = (g4 < 2 ? (qhw << (4 - 2 * g4)) : (qhw >> (2 * g4 - 4))) & 0x30303030u;
-                const uint32_t mw = lo | hi;
-                const uint64_t ds = f32x2_splat(gsel == 0 ? (i < 4 ? s00 : s01) : (i < 4 ? s10 : s11));
-                const uint64_t off = f32x2_splat(-(8388608.0f + 32.0f));
-                v.put(16 * gsel + 2 * i, scaled_pair<0>(mw, off, ds));
-                v.put(16 * gsel + 2 * i + 1, scaled_pair<1>(mw, off, ds));
+                const uint64_t ds = f32x2_splat(d * (float)(int8_t)((sc[PART] >> (16 * gsel + 8 * (i >> 2))) & 0xFFu));
+                const uint32_t lo = (ql[8 * gsel + i] >> (4 * PART)) & 0x0F0F0F0Fu;
+                const uint32_t hi = (PART == 0 ? qh[i] << (4 - 2 * gsel) : qh[i] >> (2 * gsel)) & 0x30303030u;
+                v.put(16 * gsel + 2 * i, scaled_pair<0>(lo | hi, off, ds));
+                v.put(16 * gsel + 2 * i + 1, scaled_pair<1>(lo | hi, off, ds));
             }
         }
     }
-    // word i (0..7) of the 32 ql bytes of group (g4 & 1) = GSEL (within this half) / of the 32 qh bytes
-    template <int GSEL> __device__ static __forceinline__ uint32_t word_ql(const Span<O + 64 * (S / 2), 64>& ql, int i) {
-        constexpr int base = O + 64 * (S / 2) + 32 * GSEL;
-        switch (i) {
-            case 0: return ql.template word<base>();      case 1: return ql.template word<base + 4>();
-            case 2: return ql.template word<base + 8>();  case 3: return ql.template word<base + 12>();
-            case 4: return ql.template word<base + 16>(); case 5: return ql.template word<base + 20>();
-            case 6: return ql.template word<base + 24>(); default: return ql.template word<base + 28>();
-        }
-    }
-    __device__ static __forceinline__ uint32_t word_qh(const Span<O + 128 + 32 * (S / 2), 32>& qh, int i) {
-        constexpr int base = O + 128 + 32 * (S / 2);
-        switch (i) {
-            case 0: return qh.template word<base>();      case 1: return qh.template word<base + 4>();
-            case 2: return qh.template word<base + 8>();  case 3: return qh.template word<base + 12>();
-            case 4: return qh.template word<base + 16>(); case 5: return qh.template word<base + 20>();
-            case 6: return qh.template word<base + 24>(); default: return qh.template word<base + 28>();
-        }
-    }
 };
+template <int S, typename Out>
+__device__ __forceinline__ void decode64_q6(const uint8_t* row, uint32_t g, Out& v) {
+    Q6Half hf;
+    hf.load(row, (210u * g) & 15u, S / 2);
+    hf.template decode<S % 2>(v);
+}
 
 // Q2_K as the reference reads it (rlx-gguf/src/lib.rs:857-886): d, dmin (f16) | 16 scale bytes (low nibble scale,
 // high nibble min) | 64 quant bytes.  Weights [64 S, 64 S + 64) are two 2-bit planes (shift 4 (S % 2), + 2) of the
@@ -548,17 +555,6 @@ __device__ __forceinline__ void decode64_q3(const uint8_t* row, uint32_t g, Out&
     }
 }
 
-// Dispatch on the (warp-uniform) offset of group g inside its row buffer.
-template <int S, typename Out>
-__device__ __forceinline__ void decode64_q6(const uint8_t* row, uint32_t g, Out& v) {
-    switch (g & 7u) {
-        case 0: Decode64Q6<S, 0>::run(row, v); break;   case 1: Decode64Q6<S, 2>::run(row, v); break;
-        case 2: Decode64Q6<S, 4>::run(row, v); break;   case 3: Decode64Q6<S, 6>::run(row, v); break;
-        case 4: Decode64Q6<S, 8>::run(row, v); break;   case 5: Decode64Q6<S, 10>::run(row, v); break;
-        case 6: Decode64Q6<S, 12>::run(row, v); break;  default: Decode64Q6<S, 14>::run(row, v); break;
-    }
-}
-
 template <uint32_t SCHEME, int S, typename Out>
 __device__ __forceinline__ void decode64(const uint8_t* row, uint32_t g, Out& v) {
     if constexpr (SCHEME == RLXQ_Q6_K) decode64_q6<S>(row, g, v);
@@ -569,8 +565,9 @@ __device__ __forceinline__ void decode64(const uint8_t* row, uint32_t g, Out& v)
 }
 
 // ---- kernel -----------------------------------------------------------------------------------
-constexpr uint32_t kGemmMaxDecodeGroups = 3;
-constexpr uint32_t kGemmMaxBlock = (4 + 4 * kGemmMaxDecodeGroups + 4) * 32;   // B TMA, MMA, raw TMA, spare | decode | epilogue
+// B TMA, MMA, raw TMA, spare | decode | epilogue.  The block's real size goes into the launch bounds: with two decode
+// groups a thread may then use 128 registers, and the decoders keep a row's loads and 32 (PRECISE: 64) results in flight.
+constexpr uint32_t gemm_threads(uint32_t groups) { return (4 + 4 * groups + 4) * 32; }
 // warp roles: 0 = activation (B) TMA producer, 1 = MMA issuer and tensor-memory owner,
 // 2 = raw weight TMA producer, 3 = idle, then GROUPS x 4 decode warps (tensor-memory lane quarter =
 // warp % 4), then 4 epilogue warps (lane quarter = warp % 4).
@@ -816,16 +813,16 @@ struct GemmBars {
 };
 
 // One decode warp: raw blocks -> bf16 rows in tensor memory.  The 64-weight parts of the groups are dealt to the decode
-// warp groups in turn.  With two of them group GRP takes parts GRP and GRP + 2 of every group, known when the code is
-// compiled (a Q4_K block in 680 cycles, 885 with the turn kept in a register); with three (the slow decoders of Q6_K and
-// Q3_K, whose code is eight variants per part long: separate copies per group cost more in instruction fetch than they
-// save) the turn is counted.
+// warp groups.  With two of them group GRP takes parts GRP and GRP + 2 of every group (Q6_K, whose halves share their
+// bytes: 2 GRP and 2 GRP + 1), known when the code is compiled (a Q4_K block in 650 cycles, 885 with the turn kept in a
+// register); with three (Q3_K, whose decoder is eight variants per part long: separate copies per group cost more in
+// instruction fetch than they save) the turn is counted.
 template <uint32_t SCHEME, bool PRECISE, uint32_t GRP>
 __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* bars, const uint8_t* raw_stage, uint32_t tmem_a,
                                                  uint32_t xtiles, uint32_t warp, uint32_t lane) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW, GROUPS = GemmRaw<SCHEME>::GROUPS;
     constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128, A_COLS = PRECISE ? 64 : 32;
-    constexpr bool STATIC = GROUPS == 2;
+    constexpr bool STATIC = GROUPS == 2, HALVES = STATIC && SCHEME == RLXQ_Q6_K;
     volatile uint32_t* abort_flag = &bars->abort_flag;
     auto give_up = [&](int code) {
         atomicExch(P.err, code);
@@ -843,25 +840,32 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
         for (uint32_t g = sg.g0; g < sg.g1; ++g) {
             if (*abort_flag || !mbar_wait(smem_u32(&bars->raw_full[r]), rph)) { give_up(15); return; }
             const uint8_t* rp = raw_stage + r * RAW_STRIDE + row * RAW_ROW;
+            // Decoded into registers first: only the store needs the stage's tensor-memory columns, so the arithmetic stays
+            // off the free -> store -> MMA chain.
+            Q6Half hf;
+            if constexpr (HALVES) hf.load(rp, (210u * g) & 15u, GRP);
 #pragma unroll
             for (uint32_t sub = 0; sub < 4; ++sub) {
                 const uint32_t st = s, sph = fph;
                 if (++s == NS) { s = 0; fph ^= 1u; }
                 if constexpr (STATIC) {
-                    if (sub % GROUPS != GRP) continue;
+                    if ((HALVES ? sub / 2 : sub % 2) != GRP) continue;
                 } else {
                     const bool mine = turn == grp;
                     if (++turn == GROUPS) turn = 0;
                     if (!mine) continue;
                 }
-                // decode into registers first: only the store needs the stage's tensor-memory columns,
-                // so the arithmetic stays off the free -> store -> MMA chain
                 const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);    // answered while decoding
                 GemmOut<PRECISE> v;
-                if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
-                else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
-                else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
-                else decode64<SCHEME, 3>(rp, g, v);
+                if constexpr (HALVES) {
+                    if (sub % 2 == 0) hf.template decode<0>(v);
+                    else hf.template decode<1>(v);
+                } else {
+                    if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
+                    else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
+                    else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
+                    else decode64<SCHEME, 3>(rp, g, v);
+                }
                 if (!__all_sync(0xFFFFFFFFu, ready) && (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[st]), sph))) { give_up(16); return; }
                 tc_fence_after();
                 tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
@@ -882,7 +886,7 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
 // and every activation box is multiplied by both (the lo half of f32 activations by the hi part only: what is left out
 // is below 2^-16 of a product).  It serves the shapes whose other kernel multiplies f32 weights.
 template <uint32_t SCHEME, bool PRECISE>
-__global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P) {
+__global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
     constexpr uint32_t kGemmDecodeGroups = GemmRaw<SCHEME>::GROUPS;
     constexpr uint32_t RAW_BYTES = kGemmTileW * RAW_ROW;
@@ -1173,7 +1177,7 @@ __device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, uint32_
 }
 
 template <uint32_t SCHEME>
-__global__ void __launch_bounds__(kGemmMaxBlock, 1) gemm_pair_kernel(const __grid_constant__ GemmParams P) {
+__global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm_pair_kernel(const __grid_constant__ GemmParams P) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
     constexpr uint32_t kGemmDecodeGroups = GemmRaw<SCHEME>::GROUPS;
     constexpr uint32_t RAW_BYTES = kGemmTileW * RAW_ROW;
@@ -1567,7 +1571,7 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     } else if (grid > ntiles && !c.groups) {
         grid = (uint32_t)ntiles;
     }
-    rc = launch_pdl(gemm_tcgen05_kernel<SCHEME, PRECISE>, dim3(grid), dim3((4 + 4 * GemmRaw<SCHEME>::GROUPS + 4) * 32), smem, stream, P);
+    rc = launch_pdl(gemm_tcgen05_kernel<SCHEME, PRECISE>, dim3(grid), dim3(gemm_threads(GemmRaw<SCHEME>::GROUPS)), smem, stream, P);
     if (rc) return rc;
     count_launch();
     if (P.slices > 1) return launch_add_slices(stream, static_cast<const float*>(ws), P.slices, P.slice_elems, c.y, c.ybf, (uint64_t)c.x_rows * c.n);
@@ -1600,7 +1604,7 @@ static int launch_gemm_pair_t(cudaStream_t stream, const GemmCall& c) {
     if (!P.err) return fail(RLXQ_E_CUDA, "device error word unavailable");
     const size_t smem = 1024 + (size_t)kPairStages * kPairBBytes + (size_t)kGemmRawStages * RAW_STRIDE + sizeof(PairBars) + 64 +
                         kGemmEpiStage;
-    const uint32_t threads = (4 + 4 * GemmRaw<SCHEME>::GROUPS + 4) * 32;
+    const uint32_t threads = gemm_threads(GemmRaw<SCHEME>::GROUPS);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
