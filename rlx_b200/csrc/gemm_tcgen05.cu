@@ -151,150 +151,6 @@ template <> struct GemmOut<true> {
 
 template <uint32_t SCHEME, int S> struct Decode64;
 
-template <int S> struct Decode64<RLXQ_Q4_0, S> {
-    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
-        // blocks 2S and 2S+1 = bytes [36 S, 36 S + 36): read the 16-byte chunks that cover them
-        constexpr int B0 = 36 * S, C0 = B0 / 16, C1 = (B0 + 36 + 15) / 16, W0 = B0 / 4 - 4 * C0;
-        uint32_t w[4 * (C1 - C0) + 1];
-#pragma unroll
-        for (int c = C0; c < C1; ++c) {
-            const uint4 t = *reinterpret_cast<const uint4*>(row + 16 * c);
-            w[4 * (c - C0)] = t.x; w[4 * (c - C0) + 1] = t.y; w[4 * (c - C0) + 2] = t.z; w[4 * (c - C0) + 3] = t.w;
-        }
-        w[4 * (C1 - C0)] = 0;
-#pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-            uint32_t qs[4], dbits;
-            if (blk == 0) {   // starts on word W0: d in the low half, quants shifted by two bytes
-                dbits = w[W0] & 0xFFFFu;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) qs[i] = __funnelshift_r(w[W0 + i], w[W0 + i + 1], 16);
-            } else {          // starts two bytes into word W0 + 4
-                dbits = w[W0 + 4] >> 16;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) qs[i] = w[W0 + 5 + i];
-            }
-            const uint64_t d2 = f32x2_splat(f16_bits_to_f32(dbits)), off = f32x2_splat(-(8388608.0f + 8.0f));
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {   // weights 4i..4i+3: low nibbles of bytes 4i..; weights 16+4i..: high nibbles
-                const uint32_t lo = qs[i] & 0x0F0F0F0Fu, hi = (qs[i] >> 4) & 0x0F0F0F0Fu;
-                v.put(16 * blk + 2 * i, scaled_pair<0>(lo, off, d2));
-                v.put(16 * blk + 2 * i + 1, scaled_pair<1>(lo, off, d2));
-                v.put(16 * blk + 8 + 2 * i, scaled_pair<0>(hi, off, d2));
-                v.put(16 * blk + 8 + 2 * i + 1, scaled_pair<1>(hi, off, d2));
-            }
-        }
-    }
-};
-
-template <int S> struct Decode64<RLXQ_Q8_0, S> {
-    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
-        // blocks 2S and 2S+1 = bytes [68 S, 68 S + 68)
-        constexpr int B0 = 68 * S, C0 = B0 / 16, C1 = (B0 + 68 + 15) / 16, W0 = B0 / 4 - 4 * C0;
-        uint32_t w[4 * (C1 - C0) + 1];
-#pragma unroll
-        for (int c = C0; c < C1; ++c) {
-            const uint4 t = *reinterpret_cast<const uint4*>(row + 16 * c);
-            w[4 * (c - C0)] = t.x; w[4 * (c - C0) + 1] = t.y; w[4 * (c - C0) + 2] = t.z; w[4 * (c - C0) + 3] = t.w;
-        }
-        w[4 * (C1 - C0)] = 0;
-#pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-            uint32_t q[8], dbits;
-            if (blk == 0) {
-                dbits = w[W0] & 0xFFFFu;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) q[i] = __funnelshift_r(w[W0 + i], w[W0 + i + 1], 16);
-            } else {
-                dbits = w[W0 + 8] >> 16;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) q[i] = w[W0 + 9 + i];
-            }
-            const uint64_t d2 = f32x2_splat(f16_bits_to_f32(dbits)), off = f32x2_splat(-(8388608.0f + 128.0f));
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {   // int8 -> (q + 128) unsigned -> float, minus 128
-                const uint32_t u = q[i] ^ 0x80808080u;
-                v.put(16 * blk + 2 * i, scaled_pair<0>(u, off, d2));
-                v.put(16 * blk + 2 * i + 1, scaled_pair<1>(u, off, d2));
-            }
-        }
-    }
-};
-
-template <int S> struct Decode64<RLXQ_Q4_K, S> {
-    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
-        const uint4 hd = *reinterpret_cast<const uint4*>(row);   // d, dmin, 12 scale bytes
-        const float d = f16_bits_to_f32(hd.x & 0xFFFFu), dmin = f16_bits_to_f32(hd.x >> 16);
-        // sub-blocks 2S (low nibbles) and 2S+1 (high nibbles) of bytes [16 + 32 S, +32)
-        uint32_t sc[2], mn[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int j = 2 * S + i;
-            if (j < 4) {
-                sc[i] = (hd.y >> (8 * j)) & 63u;
-                mn[i] = (hd.z >> (8 * j)) & 63u;
-            } else {
-                sc[i] = ((hd.w >> (8 * (j - 4))) & 0x0Fu) | (((hd.y >> (8 * (j - 4) + 6)) & 3u) << 4);
-                mn[i] = ((hd.w >> (8 * (j - 4) + 4)) & 0x0Fu) | (((hd.z >> (8 * (j - 4) + 6)) & 3u) << 4);
-            }
-        }
-        const float dl = d * (float)sc[0], ml = dmin * (float)mn[0];
-        const float dh = d * (float)sc[1], mh = dmin * (float)mn[1];
-        const uint4 a = *reinterpret_cast<const uint4*>(row + 16 + 32 * S);
-        const uint4 b = *reinterpret_cast<const uint4*>(row + 32 + 32 * S);
-        const uint32_t qs[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        const uint64_t off = f32x2_splat(-8388608.0f);
-        const uint64_t dl2 = f32x2_splat(dl), ml2 = f32x2_splat(-ml), dh2 = f32x2_splat(dh), mh2 = f32x2_splat(-mh);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {       // scale * nibble - min, rounded after each step as the dequantiser does
-            const uint32_t lo = qs[i] & 0x0F0F0F0Fu, hi = (qs[i] >> 4) & 0x0F0F0F0Fu;
-            v.put(2 * i, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(lo), off)), ml2));
-            v.put(2 * i + 1, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(lo), off)), ml2));
-            v.put(16 + 2 * i, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<0>(hi), off)), mh2));
-            v.put(16 + 2 * i + 1, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<1>(hi), off)), mh2));
-        }
-    }
-};
-
-// Q5_K: d | dmin | 12 scale bytes | qh[32] | qs[128] (rlx-gguf/src/lib.rs:1019-1068): Q4_K with bit j of
-// qh[l] adding 16 to weight l of sub-block j.
-template <int S> struct Decode64<RLXQ_Q5_K, S> {
-    template <typename Out> __device__ static __forceinline__ void run(const uint8_t* row, Out& v) {
-        const uint4 hd = *reinterpret_cast<const uint4*>(row);
-        const float d = f16_bits_to_f32(hd.x & 0xFFFFu), dmin = f16_bits_to_f32(hd.x >> 16);
-        uint32_t sc[2], mn[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int j = 2 * S + i;
-            if (j < 4) {
-                sc[i] = (hd.y >> (8 * j)) & 63u;
-                mn[i] = (hd.z >> (8 * j)) & 63u;
-            } else {
-                sc[i] = ((hd.w >> (8 * (j - 4))) & 0x0Fu) | (((hd.y >> (8 * (j - 4) + 6)) & 3u) << 4);
-                mn[i] = ((hd.w >> (8 * (j - 4) + 4)) & 0x0Fu) | (((hd.z >> (8 * (j - 4) + 6)) & 3u) << 4);
-            }
-        }
-        const float dl = d * (float)sc[0], ml = dmin * (float)mn[0];
-        const float dh = d * (float)sc[1], mh = dmin * (float)mn[1];
-        const uint4 ha = *reinterpret_cast<const uint4*>(row + 16), hb = *reinterpret_cast<const uint4*>(row + 32);
-        const uint4 a = *reinterpret_cast<const uint4*>(row + 48 + 32 * S);
-        const uint4 b = *reinterpret_cast<const uint4*>(row + 64 + 32 * S);
-        const uint32_t qs[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        const uint32_t qh[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
-        const uint64_t off = f32x2_splat(-8388608.0f);
-        const uint64_t dl2 = f32x2_splat(dl), ml2 = f32x2_splat(-ml), dh2 = f32x2_splat(dh), mh2 = f32x2_splat(-mh);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t lo = (qs[i] & 0x0F0F0F0Fu) | (((qh[i] >> (2 * S)) & 0x01010101u) << 4);
-            const uint32_t hi = ((qs[i] >> 4) & 0x0F0F0F0Fu) | (((qh[i] >> (2 * S + 1)) & 0x01010101u) << 4);
-            v.put(2 * i, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(lo), off)), ml2));
-            v.put(2 * i + 1, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(lo), off)), ml2));
-            v.put(16 + 2 * i, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<0>(hi), off)), mh2));
-            v.put(16 + 2 * i + 1, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<1>(hi), off)), mh2));
-        }
-    }
-};
-
 // Words of a row buffer at compile-time byte offsets: loads the 16-byte chunks covering [B0, B0 + LEN)
 // and hands out the 32-bit little-endian word at any even byte offset inside.
 template <int B0, int LEN> struct Span {
@@ -352,28 +208,24 @@ struct Q6Half {
         sc[1] = h ? tail[3] : tail[1];
         d = f16_bits_to_f32(tail[4] & 0xFFFFu);
     }
-    template <int PART, typename Out> __device__ __forceinline__ void decode(Out& v) const {
+    template <typename Out> __device__ __forceinline__ void decode(uint32_t part, Out& v) const {
         const uint64_t off = f32x2_splat(-(8388608.0f + 32.0f));
+        const uint32_t scw = part ? sc[1] : sc[0];
 #pragma unroll
         for (int gsel = 0; gsel < 2; ++gsel) {
+            // int8 -> (s + 128) unsigned -> float, minus 128
+            const float s0 = d * u8_minus<128>(((scw >> (16 * gsel)) & 0xFFu) ^ 0x80u), s1 = d * u8_minus<128>(((scw >> (16 * gsel + 8)) & 0xFFu) ^ 0x80u);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const uint64_t ds = f32x2_splat(d * (float)(int8_t)((sc[PART] >> (16 * gsel + 8 * (i >> 2))) & 0xFFu));
-                const uint32_t lo = (ql[8 * gsel + i] >> (4 * PART)) & 0x0F0F0F0Fu;
-                const uint32_t hi = (PART == 0 ? qh[i] << (4 - 2 * gsel) : qh[i] >> (2 * gsel)) & 0x30303030u;
+                const uint64_t ds = f32x2_splat(i < 4 ? s0 : s1);
+                const uint32_t lo = (ql[8 * gsel + i] >> (4 * part)) & 0x0F0F0F0Fu;
+                const uint32_t hi = ((qh[i] >> (4 * part)) << (4 - 2 * gsel)) & 0x30303030u;
                 v.put(16 * gsel + 2 * i, scaled_pair<0>(lo | hi, off, ds));
                 v.put(16 * gsel + 2 * i + 1, scaled_pair<1>(lo | hi, off, ds));
             }
         }
     }
 };
-template <int S, typename Out>
-__device__ __forceinline__ void decode64_q6(const uint8_t* row, uint32_t g, Out& v) {
-    Q6Half hf;
-    hf.load(row, (210u * g) & 15u, S / 2);
-    hf.template decode<S % 2>(v);
-}
-
 // Q2_K as the reference reads it (rlx-gguf/src/lib.rs:857-886): d, dmin (f16) | 16 scale bytes (low nibble scale,
 // high nibble min) | 64 quant bytes.  Weights [64 S, 64 S + 64) are two 2-bit planes (shift 4 (S % 2), + 2) of the
 // 32 quant bytes of half S / 2, sixteen weights per scale byte: w = (d * sc) * q - dmin * mn, product and
@@ -557,11 +409,97 @@ __device__ __forceinline__ void decode64_q3(const uint8_t* row, uint32_t g, Out&
 
 template <uint32_t SCHEME, int S, typename Out>
 __device__ __forceinline__ void decode64(const uint8_t* row, uint32_t g, Out& v) {
-    if constexpr (SCHEME == RLXQ_Q6_K) decode64_q6<S>(row, g, v);
-    else if constexpr (SCHEME == RLXQ_Q2_K) decode64_q2<S>(row, g, v);
+    if constexpr (SCHEME == RLXQ_Q2_K) decode64_q2<S>(row, g, v);
     else if constexpr (SCHEME == RLXQ_Q8_K) decode64_q8k<S>(row, g, v);
     else if constexpr (SCHEME == RLXQ_Q3_K) decode64_q3<S>(row, g, v);
     else Decode64<SCHEME, S>::run(row, v);
+}
+
+// ---- one 64-weight part, its number known at run time -------------------------------------------
+// The decode warps run a loop over parts whose body exists once (Q4_K, Q5_K, Q6_K) or once per warp group (the 32-weight
+// formats, whose odd parts start one word later): four unrolled copies of 250 instructions left a quarter of the decode
+// warps' time to instruction fetch.  The other formats keep unrolled copies (Decode64).
+constexpr bool gemm_part_loop(uint32_t scheme) {
+    return scheme == RLXQ_Q4_0 || scheme == RLXQ_Q8_0 || scheme == RLXQ_Q4_K || scheme == RLXQ_Q5_K || scheme == RLXQ_Q6_K;
+}
+// Words [0, N) from word GRP + 2 * high on of the chunks at p.
+template <int N, uint32_t GRP> __device__ __forceinline__ void words_from(const uint8_t* p, bool high, uint32_t (&q)[N]) {
+    constexpr int C = (N + 3 + 3) / 4;
+    uint32_t w[4 * C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * c);
+        w[4 * c] = t.x; w[4 * c + 1] = t.y; w[4 * c + 2] = t.z; w[4 * c + 3] = t.w;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) q[i] = high ? w[i + GRP + 2] : w[i + GRP];
+}
+// Q4_0 and Q8_0: part S = GRP + 2 p, blocks 2 S and 2 S + 1.  The first starts on a word (d, quants two bytes on), the second
+// two bytes into one (d in its upper half, quants aligned behind it).
+template <uint32_t SCHEME, uint32_t GRP, typename Out>
+__device__ __forceinline__ void decode_blocks32(const uint8_t* row, uint32_t p, Out& v) {
+    constexpr int QW = SCHEME == RLXQ_Q4_0 ? 4 : 8, N = 2 * QW + 1;
+    constexpr uint32_t STEP = SCHEME == RLXQ_Q4_0 ? 32 : 64;              // 36 S or 68 S, less the S words
+    uint32_t w[N];
+    words_from<N, GRP>(row + STEP * (GRP + 2 * p), p != 0, w);
+#pragma unroll
+    for (int blk = 0; blk < 2; ++blk) {
+        const uint32_t dbits = blk == 0 ? w[0] & 0xFFFFu : w[QW] >> 16;
+        const uint64_t d2 = f32x2_splat(f16_bits_to_f32(dbits));
+        const uint64_t off = f32x2_splat(-(8388608.0f + (SCHEME == RLXQ_Q4_0 ? 8.0f : 128.0f)));
+#pragma unroll
+        for (int i = 0; i < QW; ++i) {
+            const uint32_t q = blk == 0 ? __funnelshift_r(w[i], w[i + 1], 16) : w[QW + 1 + i];
+            if (SCHEME == RLXQ_Q4_0) {       // weights 4i..: low nibbles; 16 + 4i..: high nibbles
+                const uint32_t lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;
+                v.put(16 * blk + 2 * i, scaled_pair<0>(lo, off, d2));
+                v.put(16 * blk + 2 * i + 1, scaled_pair<1>(lo, off, d2));
+                v.put(16 * blk + 8 + 2 * i, scaled_pair<0>(hi, off, d2));
+                v.put(16 * blk + 8 + 2 * i + 1, scaled_pair<1>(hi, off, d2));
+            } else {                         // int8 -> (q + 128) unsigned -> float, minus 128
+                const uint32_t u = q ^ 0x80808080u;
+                v.put(16 * blk + 2 * i, scaled_pair<0>(u, off, d2));
+                v.put(16 * blk + 2 * i + 1, scaled_pair<1>(u, off, d2));
+            }
+        }
+    }
+}
+// Q4_K and Q5_K: part S, sub-blocks 2 S (low nibbles) and 2 S + 1 (high nibbles) of 32 bytes; bit j of qh[l] adds 16 to
+// weight l of sub-block j (Q5_K).
+template <uint32_t SCHEME, typename Out>
+__device__ __forceinline__ void decode_k45(const uint8_t* row, uint32_t S, Out& v) {
+    constexpr bool FIVE = SCHEME == RLXQ_Q5_K;
+    const uint4 hd = *reinterpret_cast<const uint4*>(row);   // d, dmin, 12 scale bytes
+    const uint8_t* qp = row + (FIVE ? 48 : 16) + 32 * S;
+    const uint4 a = *reinterpret_cast<const uint4*>(qp), b = *reinterpret_cast<const uint4*>(qp + 16);
+    const uint32_t qs[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t qh[8];
+    if (FIVE) {
+        const uint4 ha = *reinterpret_cast<const uint4*>(row + 16), hb = *reinterpret_cast<const uint4*>(row + 32);
+        qh[0] = ha.x; qh[1] = ha.y; qh[2] = ha.z; qh[3] = ha.w; qh[4] = hb.x; qh[5] = hb.y; qh[6] = hb.z; qh[7] = hb.w;
+    }
+    const bool upper = S >= 2;
+    const uint32_t scb = upper ? (hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u) : hd.y & 0x3F3F3F3Fu;
+    const uint32_t mnb = upper ? ((hd.w >> 4) & 0x0F0F0F0Fu) | ((hd.z >> 2) & 0x30303030u) : hd.z & 0x3F3F3F3Fu;
+    const uint32_t sc = scb >> (16 * (S & 1u)), mn = mnb >> (16 * (S & 1u));
+    const float d = f16_bits_to_f32(hd.x & 0xFFFFu), dmin = f16_bits_to_f32(hd.x >> 16);
+    const float dl = d * u8_to_f32(sc & 0xFFu), ml = dmin * u8_to_f32(mn & 0xFFu);
+    const float dh = d * u8_to_f32((sc >> 8) & 0xFFu), mh = dmin * u8_to_f32((mn >> 8) & 0xFFu);
+    const uint64_t off = f32x2_splat(-8388608.0f);
+    const uint64_t dl2 = f32x2_splat(dl), ml2 = f32x2_splat(-ml), dh2 = f32x2_splat(dh), mh2 = f32x2_splat(-mh);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {       // scale * quant - min, rounded after each step as the dequantiser does
+        uint32_t lo = qs[i] & 0x0F0F0F0Fu, hi = (qs[i] >> 4) & 0x0F0F0F0Fu;
+        if (FIVE) {
+            const uint32_t t = qh[i] >> (2 * S);
+            lo |= (t << 4) & 0x10101010u;
+            hi |= (t << 3) & 0x10101010u;
+        }
+        v.put(2 * i, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<0>(lo), off)), ml2));
+        v.put(2 * i + 1, add_f32x2(mul_f32x2(dl2, add_f32x2(magic_pair<1>(lo), off)), ml2));
+        v.put(16 + 2 * i, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<0>(hi), off)), mh2));
+        v.put(16 + 2 * i + 1, add_f32x2(mul_f32x2(dh2, add_f32x2(magic_pair<1>(hi), off)), mh2));
+    }
 }
 
 // ---- kernel -----------------------------------------------------------------------------------
@@ -813,16 +751,13 @@ struct GemmBars {
 };
 
 // One decode warp: raw blocks -> bf16 rows in tensor memory.  The 64-weight parts of the groups are dealt to the decode
-// warp groups.  With two of them group GRP takes parts GRP and GRP + 2 of every group (Q6_K, whose halves share their
-// bytes: 2 GRP and 2 GRP + 1), known when the code is compiled (a Q4_K block in 650 cycles, 885 with the turn kept in a
-// register); with three (Q3_K, whose decoder is eight variants per part long: separate copies per group cost more in
-// instruction fetch than they save) the turn is counted.
+// warp groups: of two, group grp takes parts grp and grp + 2 (Q6_K, whose halves share their bytes: 2 grp and 2 grp + 1);
+// of three (Q3_K) whoever's turn it is.  GRP = grp where a group has code of its own.
 template <uint32_t SCHEME, bool PRECISE, uint32_t GRP>
 __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* bars, const uint8_t* raw_stage, uint32_t tmem_a,
                                                  uint32_t xtiles, uint32_t warp, uint32_t lane) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW, GROUPS = GemmRaw<SCHEME>::GROUPS;
     constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128, A_COLS = PRECISE ? 64 : 32;
-    constexpr bool STATIC = GROUPS == 2, HALVES = STATIC && SCHEME == RLXQ_Q6_K;
     volatile uint32_t* abort_flag = &bars->abort_flag;
     auto give_up = [&](int code) {
         atomicExch(P.err, code);
@@ -833,53 +768,89 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
     const uint32_t lane_addr = (quarter * 32) << 16;
     uint32_t r = 0, rph = 0, turn = 0;   // turn (three groups): whose part comes next
     uint32_t s = 0, fph = 1;             // operand stage of the next part, and the parity that says it is free
+    // A part's tensor-memory store is announced when the next one is ready to be stored: its few hundred cycles pass
+    // under the next part's arithmetic.
+    uint32_t pending = 0;                // the barrier to announce it on (0: nothing stored since)
+    auto announce = [&]() {
+        if (!pending) return;
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(pending);
+        pending = 0;
+    };
     uint32_t cur, lim;
     gemm_seg_init(P, xtiles, cur, lim);
     GemmSeg sg;
+    uint32_t raw_ready = 0;              // whether the next raw box had arrived when this group's last part was decoded
     while (!*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
         for (uint32_t g = sg.g0; g < sg.g1; ++g) {
-            if (*abort_flag || !mbar_wait(smem_u32(&bars->raw_full[r]), rph)) { give_up(15); return; }
+            if (!__all_sync(0xFFFFFFFFu, raw_ready)) {
+                announce();
+                if (*abort_flag || !mbar_wait(smem_u32(&bars->raw_full[r]), rph)) { give_up(15); return; }
+            }
             const uint8_t* rp = raw_stage + r * RAW_STRIDE + row * RAW_ROW;
             // Decoded into registers first: only the store needs the stage's tensor-memory columns, so the arithmetic stays
             // off the free -> store -> MMA chain.
-            Q6Half hf;
-            if constexpr (HALVES) hf.load(rp, (210u * g) & 15u, GRP);
-#pragma unroll
-            for (uint32_t sub = 0; sub < 4; ++sub) {
-                const uint32_t st = s, sph = fph;
-                if (++s == NS) { s = 0; fph ^= 1u; }
-                if constexpr (STATIC) {
-                    if ((HALVES ? sub / 2 : sub % 2) != GRP) continue;
-                } else {
-                    const bool mine = turn == grp;
-                    if (++turn == GROUPS) turn = 0;
-                    if (!mine) continue;
+            const uint32_t s0 = s, ph0 = fph;
+            s += 4;
+            if (s >= NS) { s -= NS; fph ^= 1u; }
+            auto stage_of = [&](uint32_t sub, uint32_t& st, uint32_t& sph) {
+                st = s0 + sub;
+                sph = ph0;
+                if (st >= NS) { st -= NS; sph ^= 1u; }
+            };
+            auto store = [&](uint32_t st, uint32_t sph, uint32_t ready, const GemmOut<PRECISE>& v) -> bool {
+                announce();
+                if (!__all_sync(0xFFFFFFFFu, ready) && (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[st]), sph))) { give_up(16); return false; }
+                tc_fence_after();
+                tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
+                if constexpr (PRECISE) tmem_st32(tmem_a + lane_addr + A_COLS * st + 32, v.lo);
+                pending = smem_u32(&bars->a_full[st]);
+                return true;
+            };
+            uint32_t st, sph;
+            if constexpr (gemm_part_loop(SCHEME)) {
+                Q6Half hf;
+                if constexpr (SCHEME == RLXQ_Q6_K) hf.load(rp, (210u * g) & 15u, grp);
+#pragma unroll 1
+                for (uint32_t p = 0; p < 2; ++p) {
+                    const uint32_t sub = SCHEME == RLXQ_Q6_K ? 2 * grp + p : grp + 2 * p;
+                    stage_of(sub, st, sph);
+                    const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);    // answered while decoding
+                    GemmOut<PRECISE> v;
+                    if constexpr (SCHEME == RLXQ_Q6_K) hf.decode(p, v);
+                    else if constexpr (SCHEME == RLXQ_Q4_K || SCHEME == RLXQ_Q5_K) decode_k45<SCHEME>(rp, sub, v);
+                    else decode_blocks32<SCHEME, GRP>(rp, p, v);
+                    if (!store(st, sph, ready, v)) return;
                 }
-                const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);    // answered while decoding
-                GemmOut<PRECISE> v;
-                if constexpr (HALVES) {
-                    if (sub % 2 == 0) hf.template decode<0>(v);
-                    else hf.template decode<1>(v);
-                } else {
+            } else {
+#pragma unroll
+                for (uint32_t sub = 0; sub < 4; ++sub) {
+                    if constexpr (GROUPS == 2) {
+                        if (sub % 2 != GRP) continue;
+                    } else {
+                        const bool mine = turn == grp;
+                        if (++turn == GROUPS) turn = 0;
+                        if (!mine) continue;
+                    }
+                    stage_of(sub, st, sph);
+                    const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);
+                    GemmOut<PRECISE> v;
                     if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
                     else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
                     else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
                     else decode64<SCHEME, 3>(rp, g, v);
+                    if (!store(st, sph, ready, v)) return;
                 }
-                if (!__all_sync(0xFFFFFFFFu, ready) && (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[st]), sph))) { give_up(16); return; }
-                tc_fence_after();
-                tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
-                if constexpr (PRECISE) tmem_st32(tmem_a + lane_addr + A_COLS * st + 32, v.lo);
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->a_full[st]));
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[r]));
             if (++r == NR) { r = 0; rph ^= 1u; }
+            raw_ready = mbar_test(smem_u32(&bars->raw_full[r]), rph);
         }
     }
+    announce();
 }
 
 // PRECISE: the weight operand keeps 16 significand bits, as bf16 hi and lo parts in two sets of tensor-memory columns,
@@ -1031,8 +1002,10 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
         }
     } else if (warp >= 4 && warp < 4 + 4 * kGemmDecodeGroups) {
         // ---------------- decode ----------------
-        if (kGemmDecodeGroups != 2 || warp < 8) gemm_decode_role<SCHEME, PRECISE, 0>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
+        constexpr bool ONE = kGemmDecodeGroups != 2 || SCHEME == RLXQ_Q4_K || SCHEME == RLXQ_Q5_K || SCHEME == RLXQ_Q6_K;
+        if (ONE || warp < 8) gemm_decode_role<SCHEME, PRECISE, 0>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
         else gemm_decode_role<SCHEME, PRECISE, 1>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
+        tmem_st_wait();                      // (after a timeout a store may still be on its way)
     } else if (warp >= 4 + 4 * kGemmDecodeGroups) {
         // ---------------- epilogue: accumulator -> y (or -> a partial tile, completed by the last contributor) ----------------
         const uint32_t quarter = warp & 3u;
@@ -1319,38 +1292,69 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
         const uint32_t lane_addr = (quarter * 32) << 16;
         uint32_t r = 0, rph = 0, kbg0 = 0;
         bool ok = true;
+        uint32_t raw_ready = 0;
         for (uint32_t pt = pt0; ok && pt < plim && !*abort_flag; pt += pstep) {
             for (uint32_t g = 0; g < P.kgroups && ok; ++g, kbg0 += 4) {
-                if (*abort_flag || !pair_wait<SCHEME>(smem_u32(&bars->raw_full[r]), rph, lane)) { give_up(26); ok = false; break; }
+                if (!__all_sync(0xFFFFFFFFu, raw_ready) &&
+                    (*abort_flag || !pair_wait<SCHEME>(smem_u32(&bars->raw_full[r]), rph, lane))) { give_up(26); ok = false; break; }
                 const uint8_t* rp = raw_stage + r * RAW_STRIDE + row * RAW_ROW;
-#pragma unroll
-                for (uint32_t sub = 0; sub < 4; ++sub) {
-                    const uint32_t kbg = kbg0 + sub;
-                    if (kbg % kGemmDecodeGroups != grp) continue;
-                    // 64-wide block kbg is part kbg % kPairRound of round kbg / kPairRound
-                    const uint32_t rd = dual ? kbg : kbg / kPairRound, s = rd % kPairStages, fph = ((rd / kPairStages) & 1u) ^ 1u;
-                    const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[s]), fph);     // answered while decoding
-                    GemmOut<false> v;
-                    if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
-                    else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
-                    else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
-                    else decode64<SCHEME, 3>(rp, g, v);
+                // 64-wide block kbg is part kbg % kPairRound of round kbg / kPairRound
+                auto stage_of = [&](uint32_t sub, uint32_t& st, uint32_t& sph, uint32_t& col) {
+                    const uint32_t kbg = kbg0 + sub, rd = dual ? kbg : kbg / kPairRound;
+                    st = rd % kPairStages;
+                    sph = ((rd / kPairStages) & 1u) ^ 1u;
+                    col = 32 * (kPairRound * st + (dual ? 0u : kbg % kPairRound));
+                };
+                auto store = [&](uint32_t st, uint32_t sph, uint32_t col, uint32_t ready, const GemmOut<false>& v) -> bool {
                     if (!__all_sync(0xFFFFFFFFu, ready) &&
-                        (*abort_flag || !pair_wait<SCHEME>(smem_u32(&bars->stage_free[s]), fph, lane))) { give_up(27); ok = false; break; }
+                        (*abort_flag || !pair_wait<SCHEME>(smem_u32(&bars->stage_free[st]), sph, lane))) { give_up(27); return false; }
                     tc_fence_after();
-                    tmem_st32(tmem_a + lane_addr + 32 * (kPairRound * s + (dual ? 0u : kbg % kPairRound)), v.hi);
+                    tmem_st32(tmem_a + lane_addr + col, v.hi);
+                    // announced at once (the single-CTA kernel's delay costs 4 % here: a round waits for sixteen of these)
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        if (rank == 0) mbar_arrive(smem_u32(&bars->a_full[s]));
-                        else mbar_arrive_cluster(cluster_map(smem_u32(&bars->a_full[s]), 0));
+                        if (rank == 0) mbar_arrive(smem_u32(&bars->a_full[st]));
+                        else mbar_arrive_cluster(cluster_map(smem_u32(&bars->a_full[st]), 0));
+                    }
+                    return true;
+                };
+                uint32_t st, sph, col;
+                if constexpr (gemm_part_loop(SCHEME)) {
+                    Q6Half hf;
+                    if constexpr (SCHEME == RLXQ_Q6_K) hf.load(rp, (210u * g) & 15u, grp);
+#pragma unroll 1
+                    for (uint32_t p = 0; p < 2 && ok; ++p) {
+                        const uint32_t sub = SCHEME == RLXQ_Q6_K ? 2 * grp + p : grp + 2 * p;
+                        stage_of(sub, st, sph, col);
+                        const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);     // answered while decoding
+                        GemmOut<false> v;
+                        if constexpr (SCHEME == RLXQ_Q6_K) hf.decode(p, v);
+                        else if constexpr (SCHEME == RLXQ_Q4_K || SCHEME == RLXQ_Q5_K) decode_k45<SCHEME>(rp, sub, v);
+                        else if (grp == 0) decode_blocks32<SCHEME, 0>(rp, p, v);
+                        else decode_blocks32<SCHEME, 1>(rp, p, v);
+                        ok = store(st, sph, col, ready, v);
+                    }
+                } else {
+#pragma unroll
+                    for (uint32_t sub = 0; sub < 4; ++sub) {
+                        if (!ok || (kbg0 + sub) % kGemmDecodeGroups != grp) continue;
+                        stage_of(sub, st, sph, col);
+                        const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);
+                        GemmOut<false> v;
+                        if (sub == 0) decode64<SCHEME, 0>(rp, g, v);
+                        else if (sub == 1) decode64<SCHEME, 1>(rp, g, v);
+                        else if (sub == 2) decode64<SCHEME, 2>(rp, g, v);
+                        else decode64<SCHEME, 3>(rp, g, v);
+                        ok = store(st, sph, col, ready, v);
                     }
                 }
                 if (!ok) break;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[r]));
                 if (++r == kGemmRawStages) { r = 0; rph ^= 1u; }
+                raw_ready = mbar_test(smem_u32(&bars->raw_full[r]), rph);
             }
         }
     } else if (warp >= 4 + 4 * kGemmDecodeGroups) {
