@@ -120,6 +120,8 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
                                        static_cast<uint8_t*>(y) + 4 * yrow, ybf, m - 4, k, n, ws, ws_bytes);
             }
         }
+        // rows that TMA cannot tile: f32 arithmetic like the general kernel's, at streaming speed
+        if (force == 0 && gemv_f32_supported(scheme, m, k, x)) return launch_gemv_f32(stream, scheme, x, xbf, w, y, ybf, m, k, n);
         return launch_matmul_generic(stream, scheme, x, xbf, w, y, ybf, m, k, n);
     }
     // m > 8: the tensor-memory GEMM; without the workspace it needs, the tiled generic kernel

@@ -1,0 +1,385 @@
+// Streaming decode GEMV for weight rows of any length (batch 1-8; Q4_0, Q8_0, Q6_K): the rows that TMA cannot tile, because
+// they are no multiple of 16 bytes (Q6_K with k not a multiple of 2048, the 32-weight formats with k not a multiple of 256)
+// or the weights do not start on a 16-byte boundary.
+//
+// Activations stay f32, in registers.  A CTA's warps stand side by side over the columns: warp c owns columns
+// [c * 32 * LW, (c + 1) * 32 * LW), a lane LW of them, and keeps its activations of MR batch rows for the whole kernel, while
+// the CTA's weight rows stream by.  Each warp fetches its own piece of every row into a ring of its own, in 16-byte
+// asynchronous copies from the boundary below the piece, so a row may start on any even byte and no warp waits for another;
+// the ring's depth keeps about 100 KB per SM in flight.  A lane decodes its LW weights (one byte-permute each, packed
+// two-float arithmetic from there on), multiplies, and applies the block scale once per block; the warp's sum goes to
+// shared memory, where the warps' sums meet once per 32 rows.
+//
+// Bound: HBM for one or two batch rows, where a weight costs about 3.5 (Q8_0) to 4.5 (Q6_K) lane instructions of the 4.5 to
+// 6 that the stream leaves time for; instruction issue above that.  The kernel this replaces on these shapes read four
+// weights per lane at a time through 2-byte loads (gemv_generic.cu).
+#include "common.cuh"
+#include "decode.cuh"
+#include "kernels.h"
+#include "staged_common.cuh"
+
+namespace rlxq {
+
+constexpr uint32_t kF32Batch = 32;        // weight rows between two meetings of the warps
+constexpr uint32_t kF32MaxWarps = 16;
+
+struct F32Params {
+    const void* x;
+    const uint8_t* w;
+    void* y;
+    uint32_t x_bf16, y_bf16, m, k, n;
+    uint64_t row_bytes;
+    uint32_t passes;                      // column passes: more than kF32MaxWarps pieces are taken one set after the other
+    uint32_t tiles, groups;               // CTA b: tile b / groups of the weight rows, batch rows MR * (b % groups) ..
+    // Expert stacks: w holds num_experts slabs of n rows, groups = m, and CTA b multiplies batch row b % groups by the slab
+    // that expert_idx names for it (none: the row of y is zero).
+    const float* expert_idx;
+    uint32_t num_experts;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ uint32_t s32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+// N consecutive words / the 16 bits at an even shared-memory byte address.
+template <int N> __device__ __forceinline__ void s32_even(uint32_t a, uint32_t (&w)[N]) {
+    const uint32_t b = a & ~3u, sh = (a & 2u) * 8u;
+    uint32_t prev = s32(b);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const uint32_t next = s32(b + 4 * i + 4);
+        w[i] = __funnelshift_r(prev, next, sh);
+        prev = next;
+    }
+}
+__device__ __forceinline__ uint32_t s16_even(uint32_t a) { return (s32(a & ~3u) >> ((a & 2u) * 8u)) & 0xFFFFu; }
+
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ float sum2(uint64_t v) {
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+    return __uint_as_float(lo) + __uint_as_float(hi);
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// The four bytes of u, less OFF, times x pairs xi, xi + 1 of every batch row.
+template <int OFF, int MR, int NX>
+__device__ __forceinline__ void mul_word(uint32_t u, const uint64_t (&x)[MR][NX], int xi, uint64_t (&acc)[MR]) {
+    const uint32_t o = __float_as_uint(-(8388608.0f + (float)OFF));
+    const uint64_t off = pack2(o, o);
+    const uint64_t a = add2(pack2(__byte_perm(u, 0x4B000000u, 0x7440), __byte_perm(u, 0x4B000000u, 0x7441)), off);
+    const uint64_t b = add2(pack2(__byte_perm(u, 0x4B000000u, 0x7442), __byte_perm(u, 0x4B000000u, 0x7443)), off);
+#pragma unroll
+    for (int r = 0; r < MR; ++r) {
+        acc[r] = fma2(a, x[r][xi], acc[r]);
+        acc[r] = fma2(b, x[r][xi + 1], acc[r]);
+    }
+}
+
+// One lane's LW weights of a row piece whose first block lies at shared-memory address p (even), added to sum[].
+template <uint32_t SCHEME, int MR, int LW> struct F32Lane;
+
+template <int MR, int LW> struct F32Lane<RLXQ_Q8_0, MR, LW> {
+    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], float (&sum)[MR]) {
+        const uint32_t blk = p + 34u * (lane * LW / 32);
+        uint32_t q[LW / 4];
+        s32_even<LW / 4>(blk + 2 + (lane * LW) % 32, q);
+        const float d = f16_bits_to_f32(s16_even(blk));
+        uint64_t acc[MR];
+#pragma unroll
+        for (int r = 0; r < MR; ++r) acc[r] = 0ull;
+#pragma unroll
+        for (int i = 0; i < LW / 4; ++i) mul_word<128>(q[i] ^ 0x80808080u, x, 2 * i, acc);
+#pragma unroll
+        for (int r = 0; r < MR; ++r) sum[r] = d * sum2(acc[r]);
+    }
+};
+
+template <int MR, int LW> struct F32Lane<RLXQ_Q4_0, MR, LW> {
+    // low nibbles: weights 0..15 of the block, high nibbles: 16..31
+    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], float (&sum)[MR]) {
+        const uint32_t blk = p + 18u * (lane * LW / 32);
+        uint64_t acc[MR];
+#pragma unroll
+        for (int r = 0; r < MR; ++r) acc[r] = 0ull;
+        uint32_t q[4];
+        s32_even<4>(blk + 2, q);
+        if constexpr (LW == 32) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                mul_word<8>(q[i] & 0x0F0F0F0Fu, x, 2 * i, acc);
+                mul_word<8>((q[i] >> 4) & 0x0F0F0F0Fu, x, 8 + 2 * i, acc);
+            }
+        } else {
+            static_assert(LW == 16, "half a block");
+            const uint32_t sh = 4u * (lane & 1u);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mul_word<8>((q[i] >> sh) & 0x0F0F0F0Fu, x, 2 * i, acc);
+        }
+        const float d = f16_bits_to_f32(s16_even(blk));
+#pragma unroll
+        for (int r = 0; r < MR; ++r) sum[r] = d * sum2(acc[r]);
+    }
+};
+
+// Q6_K (ql[128] | qh[64] | sc[16] i8 | d f16, order as rlx-gguf/src/lib.rs:1070-1114): weights 128 h + 32 g + 16 i .. of the
+// super-block are nibble g >> 1 of ql bytes 64 h + 32 (g & 1) + 16 i .. and bits 2 g, 2 g + 1 of qh bytes 32 h + 16 i ..
+template <int MR, int LW> struct F32Lane<RLXQ_Q6_K, MR, LW> {
+    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], float (&sum)[MR]) {
+        constexpr uint32_t PER = 256 / LW;                 // lanes per super-block
+        const uint32_t sb = p + 210u * (lane / PER), j = lane % PER;
+        const uint32_t e = j * LW, h = e >> 7, g = (e >> 5) & 3u, i0 = (e >> 4) & 1u;
+        uint32_t ql[LW / 4], qh[LW / 4];
+        s32_even<LW / 4>(sb + 64 * h + 32 * (g & 1u) + 16 * i0, ql);
+        s32_even<LW / 4>(sb + 128 + 32 * h + 16 * i0, qh);
+        const uint32_t sc = s16_even(sb + 192 + ((8 * h + 2 * g + i0) & ~1u)) >> (LW == 16 ? 8 * i0 : 0);
+        const float d = f16_bits_to_f32(s16_even(sb + 208));
+        const uint32_t nib = 4u * (g >> 1), hs = 2u * g;
+#pragma unroll
+        for (int r = 0; r < MR; ++r) sum[r] = 0.f;
+#pragma unroll
+        for (int s = 0; s < LW / 16; ++s) {
+            uint64_t acc[MR];
+#pragma unroll
+            for (int r = 0; r < MR; ++r) acc[r] = 0ull;
+#pragma unroll
+            for (int i = 4 * s; i < 4 * s + 4; ++i)
+                mul_word<32>(((ql[i] >> nib) & 0x0F0F0F0Fu) | (((qh[i] >> hs) << 4) & 0x30303030u), x, 2 * i, acc);
+            const float ds = d * (float)(int8_t)((sc >> (8 * s)) & 0xFFu);
+#pragma unroll
+            for (int r = 0; r < MR; ++r) sum[r] = fmaf(ds, sum2(acc[r]), sum[r]);
+        }
+    }
+};
+
+template <int MR> constexpr int f32_lane_weights() { return MR <= 2 ? 32 : 16; }
+// bytes of a ring stage: a piece of 32 * LW weights, from the 16-byte boundary below it to the one above
+template <uint32_t SCHEME, int LW> constexpr uint32_t f32_piece_bytes() {
+    return 32u * LW / SchemeTraits<SCHEME>::kElems * SchemeTraits<SCHEME>::kBytes;
+}
+template <uint32_t SCHEME, int LW> constexpr uint32_t f32_stage_bytes() { return (f32_piece_bytes<SCHEME, LW>() + 30) / 16 * 16 + 16; }
+template <uint32_t SCHEME, int LW> constexpr int f32_depth() {
+    constexpr int d = 6400 / (int)f32_stage_bytes<SCHEME, LW>();      // about 100 KB over sixteen warps
+    return d < 3 ? 3 : d > 12 ? 12 : d;
+}
+
+template <uint32_t SCHEME, int MR>
+__global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __grid_constant__ F32Params P) {
+    constexpr int LW = f32_lane_weights<MR>(), D = f32_depth<SCHEME, LW>();
+    constexpr uint32_t COLS = 32 * LW, PIECE = f32_piece_bytes<SCHEME, LW>(), STAGE = f32_stage_bytes<SCHEME, LW>();
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    float* red = reinterpret_cast<float*>(smem);                                   // [2][kF32Batch][nwarps][MR]
+    const uint32_t ring = smem_u32(smem) + 2 * kF32Batch * nwarps * MR * 4 + warp * (D * STAGE);
+    griddep_launch_dependents();
+
+    const uint32_t tile = blockIdx.x / P.groups, m0 = (blockIdx.x - tile * P.groups) * MR;
+    const uint32_t r0 = (uint32_t)((uint64_t)tile * P.n / P.tiles), r1 = (uint32_t)((uint64_t)(tile + 1) * P.n / P.tiles);
+    const uint32_t rows = r1 - r0;
+    const uint8_t* w = P.w;
+    bool none = false;
+    if (P.expert_idx) {                   // which slab is known only after the kernel in front
+        griddep_wait();
+        uint32_t e = 0;
+        none = !expert_of_row(P.expert_idx[m0], P.num_experts, &e);
+        w += (uint64_t)e * P.n * P.row_bytes;
+    }
+    // Steps: (batch of up to kF32Batch rows, column pass, row).  A step's piece of the weights for this warp:
+    auto fetch = [&](uint32_t b, uint32_t pass, uint32_t i, uint32_t slot) {
+        const uint64_t off = (uint64_t)(pass * nwarps + warp) * PIECE;
+        if (off < P.row_bytes && !none) {
+            const uint8_t* src = w + (uint64_t)(r0 + b * kF32Batch + i) * P.row_bytes + off;
+            const uint32_t lead = (uint32_t)((uintptr_t)src & 15u);
+            const uint32_t len = (uint32_t)min((uint64_t)PIECE, P.row_bytes - off);
+            const uint32_t chunks = (lead + len + 15u) / 16u;
+            const uint8_t* from = src - lead;
+            for (uint32_t c = lane; c < chunks; c += 32u) cp_async16(ring + slot * STAGE + 16 * c, from + 16 * c);
+        }
+        cp_async_commit();
+    };
+    struct Pos { uint32_t b, pass, i; };
+    auto batch_rows = [&](uint32_t b) { return min(kF32Batch, rows - b * kF32Batch); };
+    const uint32_t batches = (rows + kF32Batch - 1) / kF32Batch;
+    auto advance = [&](Pos& p) {
+        if (++p.i == batch_rows(p.b)) {
+            p.i = 0;
+            if (++p.pass == P.passes) { p.pass = 0; ++p.b; }
+        }
+    };
+    Pos next{0, 0, 0};
+    uint32_t slot_in = 0, slot = 0;
+#pragma unroll 1
+    for (int s = 0; s < D - 1; ++s) {
+        if (next.b < batches) { fetch(next.b, next.pass, next.i, slot_in); advance(next); }
+        else cp_async_commit();
+        if (++slot_in == (uint32_t)D) slot_in = 0;
+    }
+    if (!P.expert_idx) griddep_wait();    // the weights are on their way; x and y belong to the kernel in front until here
+
+    uint64_t x[MR][LW / 2];
+    uint32_t loaded = 0xFFFFFFFFu;        // the column pass whose activations are in x
+    for (uint32_t b = 0; b < batches; ++b) {
+        const uint32_t nb = batch_rows(b);
+        float* rb = red + (b & 1u) * (kF32Batch * nwarps * MR);
+        for (uint32_t pass = 0; pass < P.passes; ++pass) {
+            const uint32_t c0 = (pass * nwarps + warp) * COLS + lane * LW;
+            const bool in = c0 < P.k && !none;
+            if (loaded != pass) {
+                loaded = pass;
+#pragma unroll
+                for (int r = 0; r < MR; ++r) {
+                    const bool have = in && m0 + r < P.m;
+                    if (P.x_bf16) {
+                        const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(P.x) + (size_t)(m0 + r) * P.k + c0);
+#pragma unroll
+                        for (int t = 0; t < LW / 8; ++t) {
+                            const uint4 v = have ? src[t] : make_uint4(0u, 0u, 0u, 0u);
+                            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) x[r][4 * t + q] = pack2(u[q] << 16, u[q] & 0xFFFF0000u);
+                        }
+                    } else {
+                        const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(P.x) + (size_t)(m0 + r) * P.k + c0);
+#pragma unroll
+                        for (int t = 0; t < LW / 4; ++t) {
+                            const uint4 v = have ? src[t] : make_uint4(0u, 0u, 0u, 0u);
+                            x[r][2 * t] = pack2(v.x, v.y);
+                            x[r][2 * t + 1] = pack2(v.z, v.w);
+                        }
+                    }
+                }
+            }
+            const uint64_t poff = (uint64_t)(pass * nwarps + warp) * PIECE;
+#pragma unroll 1
+            for (uint32_t i = 0; i < nb; ++i) {
+                cp_async_wait<D - 2>();
+                __syncwarp();             // every lane's copies of this step have landed, and the slot refilled below is read
+                float sum[MR];
+#pragma unroll
+                for (int r = 0; r < MR; ++r) sum[r] = 0.f;
+                if (in) {
+                    const uint32_t lead = (uint32_t)((uintptr_t)(w + (uint64_t)(r0 + b * kF32Batch + i) * P.row_bytes + poff) & 15u);
+                    F32Lane<SCHEME, MR, LW>::run(ring + slot * STAGE + lead, lane, x, sum);
+                }
+                if (next.b < batches) { fetch(next.b, next.pass, next.i, slot_in); advance(next); }
+                else cp_async_commit();
+                if (++slot_in == (uint32_t)D) slot_in = 0;
+                if (++slot == (uint32_t)D) slot = 0;
+                // the warp's sum of every batch row: lanes exchange halves of the rows first, then the rest
+                if constexpr (MR == 4) {
+                    const bool up = lane & 16u, up2 = lane & 8u;
+                    float a = up ? sum[2] : sum[0], c = up ? sum[3] : sum[1];
+                    a += __shfl_xor_sync(0xFFFFFFFFu, up ? sum[0] : sum[2], 16);
+                    c += __shfl_xor_sync(0xFFFFFFFFu, up ? sum[1] : sum[3], 16);
+                    float v = (up2 ? c : a) + __shfl_xor_sync(0xFFFFFFFFu, up2 ? a : c, 8);
+                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 4);
+                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+                    if ((lane & 7u) == 0) {
+                        float* dst = rb + (i * nwarps + warp) * MR + (lane >> 3);
+                        *dst = pass ? *dst + v : v;
+                    }
+                } else {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                        for (int r = 0; r < MR; ++r) sum[r] += __shfl_xor_sync(0xFFFFFFFFu, sum[r], o);
+                    if (lane == 0) {
+#pragma unroll
+                        for (int r = 0; r < MR; ++r) {
+                            float* dst = rb + (i * nwarps + warp) * MR + r;
+                            *dst = pass ? *dst + sum[r] : sum[r];
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();                  // (the buffers alternate: the next batch writes the other one)
+        for (uint32_t o = tid; o < nb * MR; o += blockDim.x) {
+            const uint32_t i = o / MR, r = o - i * MR;
+            float v = 0.f;
+            for (uint32_t c = 0; c < nwarps; ++c) v += rb[(i * nwarps + c) * MR + r];
+            if (m0 + r < P.m) {
+                const size_t at = (size_t)(m0 + r) * P.n + r0 + b * kF32Batch + i;
+                if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[at] = (uint16_t)f32_to_bf16_bits(v);
+                else reinterpret_cast<float*>(P.y)[at] = v;
+            }
+        }
+    }
+}
+
+template <uint32_t SCHEME, int MR>
+static int launch_f32_t(cudaStream_t stream, F32Params P) {
+    constexpr int LW = f32_lane_weights<MR>(), D = f32_depth<SCHEME, LW>();
+    constexpr uint32_t COLS = 32 * LW, STAGE = f32_stage_bytes<SCHEME, LW>();
+    const uint32_t pieces = (P.k + COLS - 1) / COLS;
+    P.passes = (pieces + kF32MaxWarps - 1) / kF32MaxWarps;
+    const uint32_t warps = (pieces + P.passes - 1) / P.passes;
+    if (!P.groups) P.groups = (P.m + MR - 1) / MR;
+    // sixteen warps per SM, all of them resident at once
+    const uint32_t per_sm = kF32MaxWarps / warps, ctas = (uint32_t)sm_count() * per_sm;
+    P.tiles = ctas / P.groups;
+    if (P.tiles < 1) P.tiles = 1;
+    if (P.tiles > P.n) P.tiles = P.n;
+    const uint32_t smem = 2 * kF32Batch * warps * MR * 4 + warps * D * STAGE;
+    static std::atomic<uint32_t> attr_set[64];
+    int dev = 0;
+    RLXQ_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && attr_set[dev].load() == 0) {
+        RLXQ_CUDA_TRY(cudaFuncSetAttribute(gemv_f32_kernel<SCHEME, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        attr_set[dev].store(1);
+    }
+    int rc = launch_pdl(gemv_f32_kernel<SCHEME, MR>, dim3(P.tiles * P.groups), dim3(warps * 32), smem, stream, P);
+    if (rc) return rc;
+    count_launch();
+    return check_launch("gemv_f32_kernel");
+}
+
+template <uint32_t SCHEME>
+static int launch_f32_s(cudaStream_t stream, const F32Params& P) {
+    if (P.expert_idx || P.m == 1) return launch_f32_t<SCHEME, 1>(stream, P);
+    if (P.m == 2) return launch_f32_t<SCHEME, 2>(stream, P);
+    return launch_f32_t<SCHEME, 4>(stream, P);
+}
+
+bool gemv_f32_supported(uint32_t scheme, uint32_t m, uint32_t k, const void* x) {
+    return (scheme == RLXQ_Q4_0 || scheme == RLXQ_Q8_0 || scheme == RLXQ_Q6_K) && m >= 1 && m <= 8 && !((uintptr_t)x & 15u) && k % 32 == 0;
+}
+
+int launch_gemv_f32(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf, uint32_t m,
+                    uint32_t k, uint32_t n, const float* expert_idx, uint32_t num_experts) {
+    Geometry g;
+    if (!geometry(scheme, &g)) return fail(RLXQ_E_SCHEME, "unknown scheme %u", scheme);
+    F32Params P{};
+    P.x = x; P.w = w; P.y = y; P.x_bf16 = xbf; P.y_bf16 = ybf; P.m = m; P.k = k; P.n = n;
+    P.row_bytes = (uint64_t)k / g.elems * g.bytes;
+    P.expert_idx = expert_idx; P.num_experts = num_experts;
+    P.groups = expert_idx ? m : 0u;
+    switch (scheme) {
+        case RLXQ_Q4_0: return launch_f32_s<RLXQ_Q4_0>(stream, P);
+        case RLXQ_Q8_0: return launch_f32_s<RLXQ_Q8_0>(stream, P);
+        case RLXQ_Q6_K: return launch_f32_s<RLXQ_Q6_K>(stream, P);
+        default: return fail(RLXQ_E_SCHEME, "no f32 streaming GEMV for scheme %u", scheme);
+    }
+}
+
+}  // namespace rlxq

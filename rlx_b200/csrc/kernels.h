@@ -71,6 +71,11 @@ int launch_gemm(cudaStream_t stream, uint32_t scheme, const GemmCall& c, void* w
 int launch_relay_rows(cudaStream_t stream, const uint8_t* w, uint64_t row_bytes, uint64_t n, uint8_t* out, uint64_t pitch,
                       const uint32_t* used = nullptr, uint32_t slab_rows = 1);
 
+// f32 streaming GEMV (m <= 8) for rows of any length; with expert_idx, row i of x by the slab it names, all rows in one launch.
+bool gemv_f32_supported(uint32_t scheme, uint32_t m, uint32_t k, const void* x);
+int launch_gemv_f32(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf, uint32_t m,
+                    uint32_t k, uint32_t n, const float* expert_idx = nullptr, uint32_t num_experts = 0);
+
 // One MoE decode row: the slab of the weight stack is chosen by *expert_sel on the device.
 bool int_expert_supported(uint32_t scheme, uint32_t k, uint32_t n, const void* w, const void* x);
 int launch_gemv_int_expert(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w_stack, void* y,

@@ -334,6 +334,10 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     uint32_t* perm = reinterpret_cast<uint32_t*>(ws + off_perm);
     const bool decode = m <= kMoeDecodeRows && options().gemv_kernel.load() != 1 && ((size_t)k * xes) % 16 == 0 &&
                         (uint64_t)n * num_experts <= 0x7FFFFFFFull && int_expert_supported(scheme, k, n, wst, x);
+    // a few rows of a length TMA cannot tile: one launch of the f32 streaming GEMV for all of them (an id out of range
+    // leaves zeros there, too)
+    if (!decode && m <= kMoeDecodeRows && options().gemv_kernel.load() == 0 && gemv_f32_supported(scheme, m, k, x))
+        return launch_gemv_f32(s, scheme, x, xbf, wst, y, ybf, m, k, n, expert_idx, num_experts);
     // rows with an id of num_experts or more are in no group: their outputs are zero (the gather kernel sees to it)
     if (decode || !tc.ok) RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * yes, s));
     if (decode) {
