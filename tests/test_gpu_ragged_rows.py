@@ -1,0 +1,109 @@
+"""Weight rows of lengths TMA cannot tile: the streaming f32 GEMV (batch 1-8) and, above it, the tensor-core GEMM on rows
+re-laid on a padded pitch with 16-bit weights; and the tensor-core GEMM's tile widths and k slices."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests.helpers import assert_within_tolerance
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(sch, m, k, n, x_bf16, seed):
+    import torch
+    s = O.SCHEMES[sch]
+    w = O.fill_weights(s, seed, k, n)
+    x = O.fill_normal(seed + 1, m * k).reshape(m, k)
+    xd = torch.from_numpy(x).cuda()
+    if x_bf16:
+        xd = xd.to(torch.bfloat16)
+        x = xd.float().cpu().numpy()
+    return s, w, x, xd
+
+
+def _bound(s, w, x, k, n):
+    return np.sqrt((x.astype(np.float64) ** 2).sum(1))[:, None] * O.row_norms(s, w, k, n)[None, :]
+
+
+# one block, one block more or less than a lane group / a warp's piece / sixteen pieces, two column passes, one row, odd widths
+@pytest.mark.parametrize("sch,k", [("q8_0", 32), ("q8_0", 992), ("q8_0", 1056), ("q4_0", 480), ("q4_0", 2080), ("q8_0", 16416),
+                                   ("q6_k", 256), ("q6_k", 1280), ("q6_k", 11008), ("q6_k", 16640)])
+@pytest.mark.parametrize("m,n,x_bf16", [(1, 1, False), (1, 5003, True), (2, 333, False), (3, 150, True), (5, 1021, False), (8, 64, False)])
+def test_streaming_f32_gemv(sch, k, m, n, x_bf16):
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, k + m)
+    wd = torch.from_numpy(w).cuda()
+    before = R.launch_count()
+    y = R.matmul(xd, wd, s, n)
+    yb = R.matmul(xd, wd, s, n, out_dtype=torch.bfloat16)
+    assert R.launch_count() - before == 2
+    ref = O.matmul_bt_mt(x, w, m, k, n, s)
+    assert_within_tolerance(y.cpu().numpy(), ref, _bound(s, w, x, k, n), tol=2e-6, what=f"f32 gemv {sch} {m}x{k}x{n}")
+    assert torch.equal(yb, y.to(torch.bfloat16))
+
+
+def test_streaming_f32_gemv_on_weights_at_an_odd_address():
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs("q6_k", 2, 2048, 70, False, 9)
+    buf = torch.zeros(w.size + 64, dtype=torch.uint8, device="cuda")
+    ref = O.matmul_bt_mt(x, w, 2, 2048, 70, s)
+    for shift in (2, 6, 14):
+        wd = buf[shift:shift + w.size]
+        wd.copy_(torch.from_numpy(w))
+        assert_within_tolerance(R.matmul(xd, wd, s, 70).cpu().numpy(), ref, _bound(s, w, x, 2048, 70), tol=2e-6, what=f"shift {shift}")
+
+
+@pytest.mark.parametrize("sch,m,k,n,E", [("q6_k", 2, 2304, 200, 5), ("q8_0", 8, 288, 77, 3), ("q4_0", 5, 4128, 130, 4)])
+def test_expert_rows_of_odd_lengths_in_one_launch(sch, m, k, n, E):
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n * E, False, 70 + m)
+    idx = ((np.arange(m) * 2 + 1) % E).astype(np.float32)
+    idx[m - 1] = E                                             # in no group: a zero row
+    before = R.launch_count()
+    y = R.grouped_matmul(xd, torch.from_numpy(w).cuda(), torch.from_numpy(idx).cuda(), s, n, E).cpu().numpy()
+    assert R.launch_count() - before == 1
+    ref = O.grouped_matmul_bt(x, w, idx, m, k, n, E, s)
+    assert np.all(y[m - 1] == 0)
+    assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("sch,m,k,n,x_bf16", [("q6_k", 9, 256, 130, False), ("q6_k", 300, 2304, 128, True), ("q8_0", 33, 288, 77, True),
+                                              ("q4_0", 40, 4128, 257, False), ("q8_0", 130, 1056, 64, False), ("q5_0", 20, 96, 40, True),
+                                              ("q2_k", 17, 768, 40, False), ("q3_k", 12, 512, 136, True)])
+def test_gemm_on_relaid_rows(sch, m, k, n, x_bf16):
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, 300 + m)
+    before = R.launch_count()
+    y = R.matmul(xd, torch.from_numpy(w).cuda(), s, n).cpu().numpy()
+    assert R.launch_count() - before <= 4                      # rows, (halves,) GEMM, (slices): never a pass per eight rows
+    ref = O.matmul_bt_mt(x, w, m, k, n, s)
+    assert_within_tolerance(y, ref, _bound(s, w, x, k, n), tol=2e-5, what=f"relaid {sch} {m}x{k}x{n}")
+
+
+@pytest.mark.parametrize("sch", ["q4_0", "q8_0", "q4_k", "q5_k", "q6_k"])
+@pytest.mark.parametrize("m,n,x_bf16", [(32, 128, True), (33, 200, False), (97, 2000, True), (224, 136, True), (257, 264, False)])
+def test_gemm_tile_widths_and_slices(sch, m, n, x_bf16):
+    """The automatic choice of tile width and k slices, and whole tiles of every width."""
+    import torch
+    import rlx_b200 as R
+    k = 4096
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, 500 + m)
+    wd = torch.from_numpy(w).cuda()
+    ref, bnd = O.matmul_bt_mt(x, w, m, k, n, s), _bound(s, w, x, k, n)
+    tol = 12e-3 / np.sqrt(k)                                   # weights rounded once to bf16
+    y = R.matmul(xd, wd, s, n)
+    assert torch.equal(y, R.matmul(xd, wd, s, n))
+    assert_within_tolerance(y.cpu().numpy(), ref, bnd, tol=tol, what="automatic")
+    try:
+        R.set_option("gemm_streamk", 1)
+        for width in (32, 96, 160, 256):
+            R.set_option("gemm_tile_x", width)
+            assert_within_tolerance(R.matmul(xd, wd, s, n).cpu().numpy(), ref, bnd, tol=tol, what=f"width {width}")
+    finally:
+        R.set_option("gemm_tile_x", 0)
+        R.set_option("gemm_streamk", 0)
+    R.device_status()
