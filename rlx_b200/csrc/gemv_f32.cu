@@ -4,15 +4,17 @@
 //
 // Activations stay f32, in registers.  A CTA's warps stand side by side over the columns: warp c owns columns
 // [c * 32 * LW, (c + 1) * 32 * LW), a lane LW of them, and keeps its activations of MR batch rows for the whole kernel, while
-// the CTA's weight rows stream by.  Each warp fetches its own piece of every row into a ring of its own, in 16-byte
-// asynchronous copies from the boundary below the piece, so a row may start on any even byte and no warp waits for another;
-// the ring's depth keeps about 100 KB per SM in flight.  A lane decodes its LW weights (one byte-permute each, packed
-// two-float arithmetic from there on), multiplies, and applies the block scale once per block; the warp's sum goes to
-// shared memory, where the warps' sums meet once per 32 rows.
+// the CTA's weight rows stream by, RS rows a step.  Each warp fetches its own pieces of the rows into a ring of its own, in
+// 16-byte asynchronous copies from the boundary below the piece, so a row may start on any even byte and no warp waits for
+// another; the ring's depth keeps about 100 KB per SM in flight.  A lane decodes its LW weights (one byte-permute each,
+// packed two-float arithmetic from there on), multiplies, and applies the block scale once per block; the warp's sums of a
+// step's rows are reduced together and go to shared memory, where the warps' sums meet once per 32 rows.
 //
-// Bound: HBM for one or two batch rows, where a weight costs about 3.5 (Q8_0) to 4.5 (Q6_K) lane instructions of the 4.5 to
-// 6 that the stream leaves time for; instruction issue above that.  The kernel this replaces on these shapes read four
-// weights per lane at a time through 2-byte loads (gemv_generic.cu).
+// Bound: instruction issue (a weight costs 3.5 lane instructions in Q8_0, 4.5 in Q6_K, 2 of them the multiplication).  Row
+// by row (RS = 1) as much again went into ring positions, copy addresses and the reduction, in a chain that left half of
+// the issue slots empty; RS rows a step share that and overlap.  Batch 1, 5888 or 5920 -> 28672, RS = 1 against now: Q6_K
+// 79 -> 53 us, Q8_0 63 -> 42 us (4.3 TB/s), Q4_0 61 -> 37 us; batch 4: 112 -> 92, 123 -> 79, 101 -> 78 us.  More warps per SM
+// (18 for 16) and half as many weights a lane did not help.
 #include "common.cuh"
 #include "decode.cuh"
 #include "kernels.h"
@@ -95,7 +97,7 @@ __device__ __forceinline__ void mul_word(uint32_t u, const uint64_t (&x)[MR][NX]
     }
 }
 
-// One lane's LW weights of a row piece whose first block lies at shared-memory address p (even), added to sum[].
+// One lane's LW weights of a row piece whose first block lies at shared-memory address p (even), in sum[].
 template <uint32_t SCHEME, int MR, int LW> struct F32Lane;
 
 template <int MR, int LW> struct F32Lane<RLXQ_Q8_0, MR, LW> {
@@ -172,24 +174,47 @@ template <int MR, int LW> struct F32Lane<RLXQ_Q6_K, MR, LW> {
 };
 
 template <int MR> constexpr int f32_lane_weights() { return MR <= 2 ? 32 : 16; }
-// bytes of a ring stage: a piece of 32 * LW weights, from the 16-byte boundary below it to the one above
+// bytes of a row's piece (32 * LW weights), and of its slot: from the 16-byte boundary below it to the one above
 template <uint32_t SCHEME, int LW> constexpr uint32_t f32_piece_bytes() {
     return 32u * LW / SchemeTraits<SCHEME>::kElems * SchemeTraits<SCHEME>::kBytes;
 }
-template <uint32_t SCHEME, int LW> constexpr uint32_t f32_stage_bytes() { return (f32_piece_bytes<SCHEME, LW>() + 30) / 16 * 16 + 16; }
-template <uint32_t SCHEME, int LW> constexpr int f32_depth() {
-    constexpr int d = 6400 / (int)f32_stage_bytes<SCHEME, LW>();      // about 100 KB over sixteen warps
-    return d < 3 ? 3 : d > 12 ? 12 : d;
+template <uint32_t SCHEME, int LW> constexpr uint32_t f32_slot_bytes() { return (f32_piece_bytes<SCHEME, LW>() + 30) / 16 * 16 + 16; }
+// RS, rows per step: 4 or 8 sums meet in one reduction; three steps of sixteen warps have to fit in shared memory
+template <uint32_t SCHEME, int MR> constexpr int f32_step_rows() {
+    return MR >= 2 || f32_slot_bytes<SCHEME, f32_lane_weights<MR>()>() > 1000 ? 2 : 4;
+}
+template <uint32_t SCHEME, int MR, int RS> constexpr int f32_depth() {             // about 128 KB over sixteen warps, 3 to 8 steps
+    constexpr int d = 8192 / (int)(f32_slot_bytes<SCHEME, f32_lane_weights<MR>()>() * RS);
+    return d < 3 ? 3 : d > 8 ? 8 : d;
+}
+// Adds OUT values over the lanes of a warp: lanes exchange halves of the values first (OUT / 2, OUT / 4, .. shuffles), then
+// the rest.  Value v ends in the lanes whose upper bits spell v.
+template <int OUT> __device__ __forceinline__ float warp_sums(float (&v)[OUT], uint32_t lane) {
+#pragma unroll
+    for (int w = OUT / 2, bit = 16; w >= 1; w /= 2, bit /= 2) {
+        const bool up = lane & (uint32_t)bit;
+#pragma unroll
+        for (int q = 0; q < w; ++q) {
+            const float mine = up ? v[q + w] : v[q], theirs = up ? v[q] : v[q + w];
+            v[q] = mine + __shfl_xor_sync(0xFFFFFFFFu, theirs, bit);
+        }
+    }
+    float r = v[0];
+#pragma unroll
+    for (int o = 16 / OUT; o >= 1; o /= 2) r += __shfl_xor_sync(0xFFFFFFFFu, r, o);
+    return r;
 }
 
-template <uint32_t SCHEME, int MR>
+template <uint32_t SCHEME, int MR, int RS>
 __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __grid_constant__ F32Params P) {
-    constexpr int LW = f32_lane_weights<MR>(), D = f32_depth<SCHEME, LW>();
-    constexpr uint32_t COLS = 32 * LW, PIECE = f32_piece_bytes<SCHEME, LW>(), STAGE = f32_stage_bytes<SCHEME, LW>();
+    constexpr int LW = f32_lane_weights<MR>(), D = f32_depth<SCHEME, MR, RS>(), OUT = RS * MR;
+    constexpr uint32_t COLS = 32 * LW, PIECE = f32_piece_bytes<SCHEME, LW>(), SLOT = f32_slot_bytes<SCHEME, LW>();
+    constexpr uint32_t LPR = 32 / RS;                      // lanes that copy one row of a step
+    constexpr int COPIES = (int)((PIECE + 14 + 15) / 16 + LPR - 1) / (int)LPR;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarps = blockDim.x >> 5;
     float* red = reinterpret_cast<float*>(smem);                                   // [2][kF32Batch][nwarps][MR]
-    const uint32_t ring = smem_u32(smem) + 2 * kF32Batch * nwarps * MR * 4 + warp * (D * STAGE);
+    const uint32_t ring = smem_u32(smem) + 2 * kF32Batch * nwarps * MR * 4 + warp * (D * RS * SLOT);
     griddep_launch_dependents();
 
     const uint32_t tile = blockIdx.x / P.groups, m0 = (blockIdx.x - tile * P.groups) * MR;
@@ -203,24 +228,29 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
         none = !expert_of_row(P.expert_idx[m0], P.num_experts, &e);
         w += (uint64_t)e * P.n * P.row_bytes;
     }
-    // Steps: (batch of up to kF32Batch rows, column pass, row).  A step's piece of the weights for this warp:
-    auto fetch = [&](uint32_t b, uint32_t pass, uint32_t i, uint32_t slot) {
-        const uint64_t off = (uint64_t)(pass * nwarps + warp) * PIECE;
+    // A step: RS rows of a batch of up to kF32Batch rows, in one column pass.  Rows past the last are the last row again.
+    const uint32_t batches = (rows + kF32Batch - 1) / kF32Batch;
+    struct Pos { uint32_t b, pass, i; };
+    auto batch_rows = [&](uint32_t b) { return min(kF32Batch, rows - b * kF32Batch); };
+    const uint32_t crow = lane / LPR, cchunk = lane % LPR;                         // this lane's share of the copies
+    auto fetch = [&](const Pos& p, uint32_t slot) {
+        const uint64_t off = (uint64_t)(p.pass * nwarps + warp) * PIECE;
         if (off < P.row_bytes && !none) {
-            const uint8_t* src = w + (uint64_t)(r0 + b * kF32Batch + i) * P.row_bytes + off;
+            const uint32_t row = min(p.b * kF32Batch + p.i + crow, rows - 1);
+            const uint8_t* src = w + (uint64_t)(r0 + row) * P.row_bytes + off;
             const uint32_t lead = (uint32_t)((uintptr_t)src & 15u);
-            const uint32_t len = (uint32_t)min((uint64_t)PIECE, P.row_bytes - off);
-            const uint32_t chunks = (lead + len + 15u) / 16u;
-            const uint8_t* from = src - lead;
-            for (uint32_t c = lane; c < chunks; c += 32u) cp_async16(ring + slot * STAGE + 16 * c, from + 16 * c);
+            const uint32_t chunks = (lead + (uint32_t)min((uint64_t)PIECE, P.row_bytes - off) + 15u) / 16u;
+            const uint8_t* from = src - lead + 16 * cchunk;
+            const uint32_t to = ring + (slot * RS + crow) * SLOT + 16 * cchunk;
+#pragma unroll
+            for (int c = 0; c < COPIES; ++c)
+                if (cchunk + c * LPR < chunks) cp_async16(to + 16 * LPR * c, from + 16 * LPR * c);
         }
         cp_async_commit();
     };
-    struct Pos { uint32_t b, pass, i; };
-    auto batch_rows = [&](uint32_t b) { return min(kF32Batch, rows - b * kF32Batch); };
-    const uint32_t batches = (rows + kF32Batch - 1) / kF32Batch;
     auto advance = [&](Pos& p) {
-        if (++p.i == batch_rows(p.b)) {
+        p.i += RS;
+        if (p.i >= batch_rows(p.b)) {
             p.i = 0;
             if (++p.pass == P.passes) { p.pass = 0; ++p.b; }
         }
@@ -229,7 +259,7 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
     uint32_t slot_in = 0, slot = 0;
 #pragma unroll 1
     for (int s = 0; s < D - 1; ++s) {
-        if (next.b < batches) { fetch(next.b, next.pass, next.i, slot_in); advance(next); }
+        if (next.b < batches) { fetch(next, slot_in); advance(next); }
         else cp_async_commit();
         if (++slot_in == (uint32_t)D) slot_in = 0;
     }
@@ -268,48 +298,36 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
                     }
                 }
             }
-            const uint64_t poff = (uint64_t)(pass * nwarps + warp) * PIECE;
+            uint32_t at = (uint32_t)(uintptr_t)w + (r0 + b * kF32Batch) * (uint32_t)P.row_bytes + (pass * nwarps + warp) * PIECE;
 #pragma unroll 1
-            for (uint32_t i = 0; i < nb; ++i) {
+            for (uint32_t i = 0; i < nb; i += RS) {
                 cp_async_wait<D - 2>();
                 __syncwarp();             // every lane's copies of this step have landed, and the slot refilled below is read
-                float sum[MR];
+                float v[OUT];
 #pragma unroll
-                for (int r = 0; r < MR; ++r) sum[r] = 0.f;
+                for (int o = 0; o < OUT; ++o) v[o] = 0.f;
                 if (in) {
-                    const uint32_t lead = (uint32_t)((uintptr_t)(w + (uint64_t)(r0 + b * kF32Batch + i) * P.row_bytes + poff) & 15u);
-                    F32Lane<SCHEME, MR, LW>::run(ring + slot * STAGE + lead, lane, x, sum);
+#pragma unroll
+                    for (int q = 0; q < RS; ++q) {
+                        // (a row past the batch's last holds the last row's bytes; its sums are not stored)
+                        const uint32_t lead = (at + min((uint32_t)q, nb - 1 - i) * (uint32_t)P.row_bytes) & 15u;
+                        float sum[MR];
+                        F32Lane<SCHEME, MR, LW>::run(ring + (slot * RS + q) * SLOT + lead, lane, x, sum);
+#pragma unroll
+                        for (int r = 0; r < MR; ++r) v[q * MR + r] = sum[r];
+                    }
                 }
-                if (next.b < batches) { fetch(next.b, next.pass, next.i, slot_in); advance(next); }
+                at += RS * (uint32_t)P.row_bytes;
+                if (next.b < batches) { fetch(next, slot_in); advance(next); }
                 else cp_async_commit();
                 if (++slot_in == (uint32_t)D) slot_in = 0;
                 if (++slot == (uint32_t)D) slot = 0;
-                // the warp's sum of every batch row: lanes exchange halves of the rows first, then the rest
-                if constexpr (MR == 4) {
-                    const bool up = lane & 16u, up2 = lane & 8u;
-                    float a = up ? sum[2] : sum[0], c = up ? sum[3] : sum[1];
-                    a += __shfl_xor_sync(0xFFFFFFFFu, up ? sum[0] : sum[2], 16);
-                    c += __shfl_xor_sync(0xFFFFFFFFu, up ? sum[1] : sum[3], 16);
-                    float v = (up2 ? c : a) + __shfl_xor_sync(0xFFFFFFFFu, up2 ? a : c, 8);
-                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 4);
-                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
-                    if ((lane & 7u) == 0) {
-                        float* dst = rb + (i * nwarps + warp) * MR + (lane >> 3);
-                        *dst = pass ? *dst + v : v;
-                    }
-                } else {
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                        for (int r = 0; r < MR; ++r) sum[r] += __shfl_xor_sync(0xFFFFFFFFu, sum[r], o);
-                    if (lane == 0) {
-#pragma unroll
-                        for (int r = 0; r < MR; ++r) {
-                            float* dst = rb + (i * nwarps + warp) * MR + r;
-                            *dst = pass ? *dst + sum[r] : sum[r];
-                        }
-                    }
+                const float t = warp_sums<OUT>(v, lane);
+                constexpr uint32_t SP = 32 / OUT;
+                const uint32_t o = lane / SP, q = o / MR;
+                if (lane % SP == 0 && i + q < nb) {
+                    float* dst = rb + ((i + q) * nwarps + warp) * MR + o % MR;
+                    *dst = pass ? *dst + t : t;
                 }
             }
         }
@@ -319,36 +337,37 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
             float v = 0.f;
             for (uint32_t c = 0; c < nwarps; ++c) v += rb[(i * nwarps + c) * MR + r];
             if (m0 + r < P.m) {
-                const size_t at = (size_t)(m0 + r) * P.n + r0 + b * kF32Batch + i;
-                if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[at] = (uint16_t)f32_to_bf16_bits(v);
-                else reinterpret_cast<float*>(P.y)[at] = v;
+                const size_t out = (size_t)(m0 + r) * P.n + r0 + b * kF32Batch + i;
+                if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[out] = (uint16_t)f32_to_bf16_bits(v);
+                else reinterpret_cast<float*>(P.y)[out] = v;
             }
         }
     }
 }
 
-template <uint32_t SCHEME, int MR>
+template <uint32_t SCHEME, int MR, int RS>
 static int launch_f32_t(cudaStream_t stream, F32Params P) {
-    constexpr int LW = f32_lane_weights<MR>(), D = f32_depth<SCHEME, LW>();
-    constexpr uint32_t COLS = 32 * LW, STAGE = f32_stage_bytes<SCHEME, LW>();
+    constexpr int LW = f32_lane_weights<MR>(), D = f32_depth<SCHEME, MR, RS>();
+    constexpr uint32_t COLS = 32 * LW, SLOT = f32_slot_bytes<SCHEME, LW>();
     const uint32_t pieces = (P.k + COLS - 1) / COLS;
     P.passes = (pieces + kF32MaxWarps - 1) / kF32MaxWarps;
     const uint32_t warps = (pieces + P.passes - 1) / P.passes;
-    if (!P.groups) P.groups = (P.m + MR - 1) / MR;
     // sixteen warps per SM, all of them resident at once
     const uint32_t per_sm = kF32MaxWarps / warps, ctas = (uint32_t)sm_count() * per_sm;
     P.tiles = ctas / P.groups;
     if (P.tiles < 1) P.tiles = 1;
     if (P.tiles > P.n) P.tiles = P.n;
-    const uint32_t smem = 2 * kF32Batch * warps * MR * 4 + warps * D * STAGE;
+    if constexpr (RS > 1)                 // tiles of fewer rows than a step takes would multiply rows they do not have
+        if (P.n / P.tiles < (uint32_t)RS) return launch_f32_t<SCHEME, MR, 1>(stream, P);
+    const uint32_t smem = 2 * kF32Batch * warps * MR * 4 + warps * D * RS * SLOT;
     static std::atomic<uint32_t> attr_set[64];
     int dev = 0;
     RLXQ_CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && attr_set[dev].load() == 0) {
-        RLXQ_CUDA_TRY(cudaFuncSetAttribute(gemv_f32_kernel<SCHEME, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        RLXQ_CUDA_TRY(cudaFuncSetAttribute(gemv_f32_kernel<SCHEME, MR, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set[dev].store(1);
     }
-    int rc = launch_pdl(gemv_f32_kernel<SCHEME, MR>, dim3(P.tiles * P.groups), dim3(warps * 32), smem, stream, P);
+    int rc = launch_pdl(gemv_f32_kernel<SCHEME, MR, RS>, dim3(P.tiles * P.groups), dim3(warps * 32), smem, stream, P);
     if (rc) return rc;
     count_launch();
     return check_launch("gemv_f32_kernel");
@@ -356,9 +375,9 @@ static int launch_f32_t(cudaStream_t stream, F32Params P) {
 
 template <uint32_t SCHEME>
 static int launch_f32_s(cudaStream_t stream, const F32Params& P) {
-    if (P.expert_idx || P.m == 1) return launch_f32_t<SCHEME, 1>(stream, P);
-    if (P.m == 2) return launch_f32_t<SCHEME, 2>(stream, P);
-    return launch_f32_t<SCHEME, 4>(stream, P);
+    if (P.expert_idx || P.m == 1) return launch_f32_t<SCHEME, 1, f32_step_rows<SCHEME, 1>()>(stream, P);
+    if (P.m == 2) return launch_f32_t<SCHEME, 2, f32_step_rows<SCHEME, 2>()>(stream, P);
+    return launch_f32_t<SCHEME, 4, f32_step_rows<SCHEME, 4>()>(stream, P);
 }
 
 bool gemv_f32_supported(uint32_t scheme, uint32_t m, uint32_t k, const void* x) {
@@ -373,7 +392,7 @@ int launch_gemv_f32(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
     P.x = x; P.w = w; P.y = y; P.x_bf16 = xbf; P.y_bf16 = ybf; P.m = m; P.k = k; P.n = n;
     P.row_bytes = (uint64_t)k / g.elems * g.bytes;
     P.expert_idx = expert_idx; P.num_experts = num_experts;
-    P.groups = expert_idx ? m : 0u;
+    P.groups = expert_idx ? m : m <= 2 ? 1u : (m + 3) / 4;
     switch (scheme) {
         case RLXQ_Q4_0: return launch_f32_s<RLXQ_Q4_0>(stream, P);
         case RLXQ_Q8_0: return launch_f32_s<RLXQ_Q8_0>(stream, P);
