@@ -1440,35 +1440,48 @@ struct GemmShape { uint32_t tx, xtiles, slices; bool streamk, pair; };
 
 // Activation rows per tile, work split and kernel for a shape, by estimated time in cycles.  A 64-wide k block of a tile
 // costs the larger of its MMAs (2 cycles per activation row and product plus the hand-over; `products`: bf16 activations
-// 1, f32 2, one more with PRECISE weights) and its decode, whatever part of the tile's rows is padding (measured slopes
-// over k at n = 14336); so few rows get a narrow tile, and rows are split evenly over the fewest tiles that leave no SM
-// idle.
-static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t products, bool precise) {
-    const uint32_t mma = 2 * tx * products + 225;
-    uint32_t dec = (scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K) ? 1130 : scheme == RLXQ_Q8_0 ? 520 : 680;
+// 1, f32 2, one more with PRECISE weights) and its decode, whatever part of the tile's rows is padding; so few rows get a
+// narrow tile, and rows are split evenly over the fewest tiles that leave no SM idle.  The constants are fits to 45 shapes
+// (five formats, 16 to 1526 rows, k 2048 to 14336), each timed at every tile width, split and kernel: the choice made here
+// takes 1 % longer than the best one in the geometric mean, up to 10 % at worst.
+static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t products, bool precise, bool pair) {
+    const bool heavy = scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K;
+    if (pair) return heavy && products == 1 ? 925 : 750 * products;        // 256 activation rows, both CTAs at once
+    uint32_t mma = 2 * tx * products + 265 + (products > 1 ? 65 : 0);
+    if (products == 2 && tx >= 96 && mma < 800) mma = 800;
+    if (heavy) mma += 90;
+    uint32_t dec = scheme == RLXQ_Q3_K ? 1130 : heavy ? 740 : scheme == RLXQ_Q8_0 || scheme == RLXQ_Q4_0 || scheme == RLXQ_Q4_K ? 570 : 620;
     if (precise) dec += 350;
     return mma > dec ? mma : dec;
 }
-static GemmShape gemm_shape(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise, bool can_split) {
+// Two CTAs per MMA; PRECISE weights are not built in that form.
+static bool gemm_pair_fits(uint32_t n, bool precise) { return n % 256 == 0 && !precise; }
+static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise, bool can_split) {
     const uint64_t sms = (uint64_t)sm_count(), wt = (n + kGemmTileW - 1) / kGemmTileW, groups = (k + 255) / 256, blocks = 4 * groups;
     const uint32_t products = 1 + (f32 ? 1 : 0) + (precise ? 1 : 0);
     const uint32_t most = f32 ? 128 : 256;               // a stage holds 256 box rows
-    const int64_t fx = options().gemm_tile_x.load(), fs = can_split ? options().gemm_streamk.load() : 1;
+    const int64_t fx = options().gemm_tile_x.load(), fs = can_split ? options().gemm_streamk.load() : 1, fp = options().gemm_pair.load();
+    const GemmShape pair{256, (m + 255) / 256, 1, false, true};
+    if (fp == 2 && gemm_pair_fits(n, precise)) return pair;
     GemmShape best{};
     uint64_t best_cost = ~0ull;
     auto take = [&](uint64_t cost, const GemmShape& sh) { if (cost < best_cost) { best_cost = cost; best = sh; } };
+    if (fp != 1 && !fx && fs != 2 && gemm_pair_fits(n, precise)) {
+        const uint64_t ptiles = (uint64_t)(n / 256) * pair.xtiles, pairs = sms / 2;
+        take((ptiles + pairs - 1) / pairs * blocks * gemm_block_cycles(scheme, 256, products, precise, true) + 24 * 256, pair);
+    }
     const uint32_t least_tiles = (m + most - 1) / most;
     for (uint32_t xt = least_tiles; xt <= least_tiles + 8; ++xt) {
         uint32_t tx = ((m + xt - 1) / xt + 31) / 32 * 32;
         if (fx) tx = (uint32_t)fx < most ? (uint32_t)fx : most;
         const uint32_t tiles_x = (m + tx - 1) / tx;
         if (tiles_x != xt && !fx) continue;              // the same width as one tile fewer
-        const uint64_t ntiles = wt * tiles_x, cyc = gemm_block_cycles(scheme, tx, products, precise);
+        const uint64_t ntiles = wt * tiles_x, cyc = gemm_block_cycles(scheme, tx, products, precise, false);
         const uint64_t epi = 24 * tx;                    // the last tile's epilogue, and with one accumulator every tile's
         if (fs != 2) take((ntiles + sms - 1) / sms * (blocks * cyc + (tx > 128 ? epi : 0)) + epi, GemmShape{tx, tiles_x, 1, false, false});
         // k split over the SMs (stream-K): every SM gets the same blocks, and exchanges up to two parts of 128 x tx values
         if (fs != 1 && (fs == 2 || ntiles % sms))
-            take((ntiles * blocks + sms - 1) / sms * cyc + epi + 8000 + 100 * tx, GemmShape{tx, tiles_x, 1, true, false});
+            take((ntiles * blocks + sms - 1) / sms * cyc + epi + 6000 + 200 * tx, GemmShape{tx, tiles_x, 1, true, false});
         // few tiles: every SM takes a slice of some tile's k, and a kernel behind this one adds the slices
         if (fs == 0 && 2 * ntiles <= sms) {
             const uint64_t fit = sms / ntiles, sl = groups < fit ? groups : fit;
@@ -1477,21 +1490,6 @@ static GemmShape gemm_shape(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n,
         if (fx) break;
     }
     return best;
-}
-static bool gemm_pair_fits(uint32_t n, bool precise) { return n % 256 == 0 && !precise; }
-// Two CTAs per MMA: chosen where it measured faster, with at least one 256 x 256 tile pair per resident cluster and a
-// format whose decoder keeps pace with two groups of decode warps (Q6_K and Q3_K, with three groups, lose 5-12 % in the
-// paired form on large shapes).
-static bool gemm_wants_pair(uint32_t scheme, uint32_t m, uint32_t n, bool precise) {
-    const int64_t opt = options().gemm_pair.load();
-    if (opt == 1 || !gemm_pair_fits(n, precise)) return false;
-    if (opt == 2) return true;
-    if (scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K || options().gemm_tile_x.load() || options().gemm_streamk.load() == 2) return false;
-    return (uint64_t)(n / 256) * ((m + 255) / 256) >= (uint64_t)sm_count() / 2;
-}
-static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise, bool can_split) {
-    if (gemm_wants_pair(scheme, m, n, precise)) return GemmShape{256, (m + 255) / 256, 1, false, true};
-    return gemm_shape(scheme, m, k, n, f32, precise, can_split);
 }
 static size_t gemm_streamk_bytes(uint64_t ntiles, uint32_t tx, size_t* off_partial) {
     const size_t counters = ((size_t)ntiles * 8 + 255) / 256 * 256;
