@@ -220,6 +220,18 @@ class Graph:
         check(lib.rlxq_graph_set_output(self._h, nodes[0]))
 
 
+_session_native = None
+
+
+def _load_session_native():
+    """The native form of CompiledGraph.run (_session_ops.so)."""
+    global _session_native
+    from . import _session_ops
+    _session_ops.setup(RlxqError, lambda a: np.ascontiguousarray(a, np.float32))
+    _session_native = _session_ops
+    return _session_native
+
+
 class CompiledGraph:
     def __init__(self, handle: int):
         self._h = handle
@@ -238,13 +250,8 @@ class CompiledGraph:
 
     def run(self, inputs: Sequence[tuple[str, np.ndarray]], out_shape: tuple[int, int]) -> np.ndarray:
         """run(&[("x", &[f32])]) -> f32 output [m, n]."""
-        n = len(inputs)
-        names = (C.c_char_p * n)(*[nm.encode() for nm, _ in inputs])
-        arrs = [np.ascontiguousarray(a, np.float32) for _, a in inputs]
-        ptrs = (C.c_void_p * n)(*[a.ctypes.data for a in arrs])
-        elems = (C.c_uint64 * n)(*[a.size for a in arrs])
         out = np.empty(out_shape, np.float32)
-        check(lib.rlxq_compiled_run(self._h, n, names, ptrs, elems, out.ctypes.data, out.size))
+        (_session_native or _load_session_native()).run(self._h, inputs, out)
         return out
 
     def run_typed(self, inputs: Sequence[tuple[str, np.ndarray, DType]], out_shape: tuple[int, int],

@@ -21,6 +21,7 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(PKG, "librlxq.so")
 OPS = os.path.join(PKG, "_torch_ops.so")
+SESSION_OPS = os.path.join(PKG, "_session_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -59,26 +60,30 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
-def _build_ops(force: bool) -> None:
-    """csrc/python/torch_ops.cpp against this interpreter, its torch and librlxq.so beside it."""
-    src = os.path.join(CSRC, "python", "torch_ops.cpp")
+def _build_ext(name: str, out: str, flags, force: bool) -> None:
+    """csrc/python/<name> against this interpreter and librlxq.so beside it; flags() -> what else it needs."""
+    src = os.path.join(CSRC, "python", name)
     headers = glob.glob(os.path.join(PKG, "..", "include", "*.h"))
     newest = max(os.path.getmtime(p) for p in [src, *headers])
-    if not force and os.path.exists(OPS) and os.path.getmtime(OPS) >= newest:
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
         return
-    import torch
-    root = os.path.dirname(torch.__file__)
-    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    compile_flags, link_flags = flags()
     cmd = [os.environ.get("CXX") or shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
-           "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"),
-           "-I", os.path.join(PKG, "..", "include"), src, "-o", OPS,
-           "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
-           "-L", PKG, "-l:librlxq.so", "-Wl,-rpath,$ORIGIN"]
+           *compile_flags, "-isystem", sysconfig.get_paths()["include"], "-I", os.path.join(PKG, "..", "include"), src, "-o", out,
+           *link_flags, "-L", PKG, "-l:librlxq.so", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"{cmd[0]} failed for {src}:\n{r.stdout}\n{r.stderr}")
+
+
+def _torch_flags():
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    return ([f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+             "-isystem", os.path.join(cuda, "include")],
+            ["-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -100,7 +105,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    _build_ops(force)
+    _build_ext("torch_ops.cpp", OPS, _torch_flags, force)
+    _build_ext("session_ops.cpp", SESSION_OPS, lambda: ([], []), force)
     return LIB
 
 
