@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(kLmThreads) lm_rank_kernel(const __grid_consta
     __shared__ float fv[RLXQ_LM_MAX_CAP];
     __shared__ uint32_t fi[RLXQ_LM_MAX_CAP];
     const uint32_t t = threadIdx.x;
+    griddep_launch_dependents();
     griddep_wait();
     for (uint32_t q = t; q < P.nslices; q += kLmThreads) peaks[q] = P.peaks[q];
     if (t == 0) { nsel = 0; ncand = 0; mine = 0ull; }
@@ -248,7 +249,6 @@ __global__ void __launch_bounds__(kLmThreads) lm_rank_kernel(const __grid_consta
         if (rank == blockIdx.x) mine = key;
     }
     __syncthreads();
-    griddep_launch_dependents();          // the chain of additions leaves the SMs to the next kernel's first weights
     const uint32_t row = mine ? ~(uint32_t)mine : kLmNone;
     float v = row != kLmNone ? ord_to_float((uint32_t)(mine >> 32)) : -CUDART_INF_F;
     if (P.exact && row != kLmNone) v = lm_exact_logit<SCHEME>(P.hidden, P.h_bf16, P.w, P.k, row, prod);
