@@ -1,6 +1,7 @@
-// Streaming decode GEMV for weight rows of any length (batch 1-8; Q4_0, Q8_0, Q6_K): the rows that TMA cannot tile, because
-// they are no multiple of 16 bytes (Q6_K with k not a multiple of 2048, the 32-weight formats with k not a multiple of 256)
-// or the weights do not start on a 16-byte boundary.
+// Streaming decode GEMV for weight rows of any length (batch 1-8; Q4_0, Q8_0, Q4_K, Q5_K, Q6_K): the rows that TMA cannot
+// tile, because they are no multiple of 16 bytes (Q6_K with k not a multiple of 2048, the 32-weight formats with k not a
+// multiple of 256) or the weights do not start on a 16-byte boundary; and, in one launch, the rows of an expert batch that
+// has too few of them for the GEMM (moe.cu).
 //
 // Activations stay f32, in registers.  A CTA's warps stand side by side over the columns: warp c owns columns
 // [c * 32 * LW, (c + 1) * 32 * LW), a lane LW of them, and keeps its activations of MR batch rows for the whole kernel, while
@@ -97,11 +98,13 @@ __device__ __forceinline__ void mul_word(uint32_t u, const uint64_t (&x)[MR][NX]
     }
 }
 
-// One lane's LW weights of a row piece whose first block lies at shared-memory address p (even), in sum[].
+// One lane's LW weights of a row piece whose first block lies at shared-memory address p (even), in sum[].  xs: the sums of
+// the lane's activations (NEEDS_SUM: formats with a minimum).
 template <uint32_t SCHEME, int MR, int LW> struct F32Lane;
 
 template <int MR, int LW> struct F32Lane<RLXQ_Q8_0, MR, LW> {
-    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], float (&sum)[MR]) {
+    static constexpr bool NEEDS_SUM = false;
+    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], const float (&)[MR], float (&sum)[MR]) {
         const uint32_t blk = p + 34u * (lane * LW / 32);
         uint32_t q[LW / 4];
         s32_even<LW / 4>(blk + 2 + (lane * LW) % 32, q);
@@ -117,8 +120,9 @@ template <int MR, int LW> struct F32Lane<RLXQ_Q8_0, MR, LW> {
 };
 
 template <int MR, int LW> struct F32Lane<RLXQ_Q4_0, MR, LW> {
+    static constexpr bool NEEDS_SUM = false;
     // low nibbles: weights 0..15 of the block, high nibbles: 16..31
-    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], float (&sum)[MR]) {
+    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], const float (&)[MR], float (&sum)[MR]) {
         const uint32_t blk = p + 18u * (lane * LW / 32);
         uint64_t acc[MR];
 #pragma unroll
@@ -146,7 +150,8 @@ template <int MR, int LW> struct F32Lane<RLXQ_Q4_0, MR, LW> {
 // Q6_K (ql[128] | qh[64] | sc[16] i8 | d f16, order as rlx-gguf/src/lib.rs:1070-1114): weights 128 h + 32 g + 16 i .. of the
 // super-block are nibble g >> 1 of ql bytes 64 h + 32 (g & 1) + 16 i .. and bits 2 g, 2 g + 1 of qh bytes 32 h + 16 i ..
 template <int MR, int LW> struct F32Lane<RLXQ_Q6_K, MR, LW> {
-    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], float (&sum)[MR]) {
+    static constexpr bool NEEDS_SUM = false;
+    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], const float (&)[MR], float (&sum)[MR]) {
         constexpr uint32_t PER = 256 / LW;                 // lanes per super-block
         const uint32_t sb = p + 210u * (lane / PER), j = lane % PER;
         const uint32_t e = j * LW, h = e >> 7, g = (e >> 5) & 3u, i0 = (e >> 4) & 1u;
@@ -172,6 +177,39 @@ template <int MR, int LW> struct F32Lane<RLXQ_Q6_K, MR, LW> {
         }
     }
 };
+
+// Q4_K, Q5_K (d f16 | dmin f16 | 12 bytes of 6-bit scales and minima | Q5_K: qh[32] | qs[128], order as
+// rlx-gguf/src/lib.rs:988-1068): weights 32 s .. of the super-block are nibble s & 1 of qs bytes 32 (s >> 1) .., plus bit s of
+// qh[0..32) as 16; the value is d * scale * q - dmin * minimum.
+template <uint32_t SCHEME, int MR, int LW> struct F32LaneK45 {
+    static constexpr bool NEEDS_SUM = true;
+    __device__ static __forceinline__ void run(uint32_t p, uint32_t lane, const uint64_t (&x)[MR][LW / 2], const float (&xs)[MR], float (&sum)[MR]) {
+        constexpr bool K5 = SCHEME == RLXQ_Q5_K;
+        constexpr uint32_t PER = 256 / LW;                 // lanes per super-block
+        const uint32_t sb = p + (K5 ? 176u : 144u) * (lane / PER), e = (lane % PER) * LW, s = e >> 5, i0 = e & 16u;
+        uint32_t h[4], q[LW / 4], qh[LW / 4];
+        s32_even<4>(sb, h);
+        s32_even<LW / 4>(sb + (K5 ? 48 : 16) + 32 * (s >> 1) + i0, q);
+        if constexpr (K5) s32_even<LW / 4>(sb + 16 + i0, qh);
+        const uint32_t nib = 4u * (s & 1u), j = 8u * (s & 3u);
+        const uint32_t a = (h[1] >> j) & 0xFFu, b = (h[2] >> j) & 0xFFu, c = (h[3] >> j) & 0xFFu;
+        const uint32_t sc = s < 4 ? a & 63u : (c & 15u) | ((a >> 6) << 4), mn = s < 4 ? b & 63u : (c >> 4) | ((b >> 6) << 4);
+        uint64_t acc[MR];
+#pragma unroll
+        for (int r = 0; r < MR; ++r) acc[r] = 0ull;
+#pragma unroll
+        for (int i = 0; i < LW / 4; ++i) {
+            uint32_t u = (q[i] >> nib) & 0x0F0F0F0Fu;
+            if constexpr (K5) u |= ((qh[i] >> s) & 0x01010101u) << 4;
+            mul_word<0>(u, x, 2 * i, acc);
+        }
+        const float d = f16_bits_to_f32(h[0] & 0xFFFFu) * (float)sc, dm = f16_bits_to_f32(h[0] >> 16) * (float)mn;
+#pragma unroll
+        for (int r = 0; r < MR; ++r) sum[r] = fmaf(d, sum2(acc[r]), -dm * xs[r]);
+    }
+};
+template <int MR, int LW> struct F32Lane<RLXQ_Q4_K, MR, LW> : F32LaneK45<RLXQ_Q4_K, MR, LW> {};
+template <int MR, int LW> struct F32Lane<RLXQ_Q5_K, MR, LW> : F32LaneK45<RLXQ_Q5_K, MR, LW> {};
 
 template <int MR> constexpr int f32_lane_weights() { return MR <= 2 ? 32 : 16; }
 // bytes of a row's piece (32 * LW weights), and of its slot: from the 16-byte boundary below it to the one above
@@ -266,6 +304,7 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
     if (!P.expert_idx) griddep_wait();    // the weights are on their way; x and y belong to the kernel in front until here
 
     uint64_t x[MR][LW / 2];
+    float xs[MR] = {};
     uint32_t loaded = 0xFFFFFFFFu;        // the column pass whose activations are in x
     for (uint32_t b = 0; b < batches; ++b) {
         const uint32_t nb = batch_rows(b);
@@ -298,6 +337,15 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
                     }
                 }
             }
+            if constexpr (F32Lane<SCHEME, MR, LW>::NEEDS_SUM) {
+#pragma unroll
+                for (int r = 0; r < MR; ++r) {
+                    uint64_t t = 0ull;
+#pragma unroll
+                    for (int q = 0; q < LW / 2; ++q) t = add2(t, x[r][q]);
+                    xs[r] = sum2(t);
+                }
+            }
             uint32_t at = (uint32_t)(uintptr_t)w + (r0 + b * kF32Batch) * (uint32_t)P.row_bytes + (pass * nwarps + warp) * PIECE;
 #pragma unroll 1
             for (uint32_t i = 0; i < nb; i += RS) {
@@ -312,7 +360,7 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
                         // (a row past the batch's last holds the last row's bytes; its sums are not stored)
                         const uint32_t lead = (at + min((uint32_t)q, nb - 1 - i) * (uint32_t)P.row_bytes) & 15u;
                         float sum[MR];
-                        F32Lane<SCHEME, MR, LW>::run(ring + (slot * RS + q) * SLOT + lead, lane, x, sum);
+                        F32Lane<SCHEME, MR, LW>::run(ring + (slot * RS + q) * SLOT + lead, lane, x, xs, sum);
 #pragma unroll
                         for (int r = 0; r < MR; ++r) v[q * MR + r] = sum[r];
                     }
@@ -381,7 +429,8 @@ static int launch_f32_s(cudaStream_t stream, const F32Params& P) {
 }
 
 bool gemv_f32_supported(uint32_t scheme, uint32_t m, uint32_t k, const void* x) {
-    return (scheme == RLXQ_Q4_0 || scheme == RLXQ_Q8_0 || scheme == RLXQ_Q6_K) && m >= 1 && m <= 8 && !((uintptr_t)x & 15u) && k % 32 == 0;
+    const bool known = scheme == RLXQ_Q4_0 || scheme == RLXQ_Q8_0 || scheme == RLXQ_Q6_K || scheme == RLXQ_Q4_K || scheme == RLXQ_Q5_K;
+    return known && m >= 1 && m <= 8 && !((uintptr_t)x & 15u) && k % 32 == 0;
 }
 
 int launch_gemv_f32(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf, uint32_t m,
@@ -397,6 +446,8 @@ int launch_gemv_f32(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
         case RLXQ_Q4_0: return launch_f32_s<RLXQ_Q4_0>(stream, P);
         case RLXQ_Q8_0: return launch_f32_s<RLXQ_Q8_0>(stream, P);
         case RLXQ_Q6_K: return launch_f32_s<RLXQ_Q6_K>(stream, P);
+        case RLXQ_Q4_K: return launch_f32_s<RLXQ_Q4_K>(stream, P);
+        case RLXQ_Q5_K: return launch_f32_s<RLXQ_Q5_K>(stream, P);
         default: return fail(RLXQ_E_SCHEME, "no f32 streaming GEMV for scheme %u", scheme);
     }
 }

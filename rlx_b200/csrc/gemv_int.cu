@@ -127,7 +127,7 @@ struct IntParams {
     uint32_t early;              // single-kernel mode: stages requested before the dependency wait
     // Expert-indirect mode (MoE decode): W is a stack of [n, k] slabs and this launch multiplies by slab
     // *expert_sel read as the reference's `as usize` cast does (expert_of_row), on the device after the
-    // dependency wait; an id of num_experts or more makes the kernel return at once (the caller has zeroed y).
+    // dependency wait; an id of num_experts or more makes the kernel write zeros and return at once.
     const float* expert_sel;
     uint32_t num_experts;
 };
@@ -1452,7 +1452,17 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
 
     if (warp == CW + 1) {
         // ---------------- finisher warp ----------------
-        { uint32_t ro; if (!resolve_expert(ro)) return; }
+        {
+            uint32_t ro;
+            if (!resolve_expert(ro)) {    // no such expert: this CTA's share of the row is zero
+                const uint32_t e1 = (uint32_t)((uint64_t)(me + 1) * P.n / G);
+                for (uint32_t j = (uint32_t)((uint64_t)me * P.n / G) + lane; j < e1; j += 32) {
+                    if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[j] = 0;
+                    else reinterpret_cast<float*>(P.y)[j] = 0.f;
+                }
+                return;
+            }
+        }
         // Adds the 16 partials of every output (2 halves x 8 warps, fixed order) and writes the tile,
         // or, for a tile shared with other CTAs, runs the publish / count / re-read sequence.  That
         // sequence is a chain of three global round trips; here it delays nobody, because the

@@ -207,6 +207,20 @@ static uint32_t moe_tile_rows(uint32_t m, uint32_t E, bool xbf) {
     return want < 32u ? 32u : (want > most ? most : want);
 }
 
+// Whether m rows are cheaper row by row (the f32 GEMV: every row reads its expert's slab, about 0.25 us per million weights,
+// and nothing goes in front of it) than as a GEMM (sort, gather and PRECISE weights: 14 us, and 0.5 us for each 64 columns of
+// each wave of 128-row weight tiles of the experts in use).  GEMV and GEMM measured: 4 x 7424 x 640 Q5_K E16 F1 and 72 us,
+// 12 x 1792 x 8320 Q5_K E16 F2 and 76 us, 10 x 3072 x 576 Q4_K E16 F3 and 33 us, 20 x 2816 x 6720 Q8_0 E16 F4 and 117 us.
+// Batches that the GEMM multiplies in bf16 (kMoeBf16Rows and more) stay with it.
+static bool moe_rows_stream(uint32_t m, uint32_t k, uint32_t n, uint32_t E) {
+    if (m <= kMoeDecodeRows) return true;
+    if (m >= kMoeBf16Rows) return false;
+    const float stream_us = 4.0f + 0.25e-6f * (float)m * (float)k * (float)n;
+    const float used = (float)E * (1.0f - powf(1.0f - 1.0f / (float)E, (float)m));
+    const float waves = ceilf(ceilf((float)n / 128.0f) * used / (float)sm_count());
+    return stream_us < 14.0f + waves * (float)(k / 64) * 0.5f;
+}
+
 // One CTA per sorted position i: row perm[i] of x becomes row i of xg, as bf16 hi and, for f32 activations, lo part (m
 // rows further on).  The rows no expert takes come last; their outputs are set to zero here.
 template <bool XBF16>
@@ -334,12 +348,14 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     uint32_t* perm = reinterpret_cast<uint32_t*>(ws + off_perm);
     const bool decode = m <= kMoeDecodeRows && options().gemv_kernel.load() != 1 && ((size_t)k * xes) % 16 == 0 &&
                         (uint64_t)n * num_experts <= 0x7FFFFFFFull && int_expert_supported(scheme, k, n, wst, x);
-    // a few rows of a length TMA cannot tile: one launch of the f32 streaming GEMV for all of them (an id out of range
-    // leaves zeros there, too)
-    if (!decode && m <= kMoeDecodeRows && options().gemv_kernel.load() == 0 && gemv_f32_supported(scheme, m, k, x))
+    // a few rows that the integer GEMV does not take: one launch of the f32 streaming GEMV for all of them (an id out of
+    // range leaves zeros there, too)
+    if (!decode && options().gemv_kernel.load() == 0 && options().gemm_kernel.load() == 0 && gemv_f32_supported(scheme, 1, k, x) &&
+        moe_rows_stream(m, k, n, num_experts))
         return launch_gemv_f32(s, scheme, x, xbf, wst, y, ybf, m, k, n, expert_idx, num_experts);
-    // rows with an id of num_experts or more are in no group: their outputs are zero (the gather kernel sees to it)
-    if (decode || !tc.ok) RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * yes, s));
+    // rows with an id of num_experts or more are in no group: their outputs are zero (the gather kernel and the decode kernel
+    // see to it)
+    if (!decode && !tc.ok) RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * yes, s));
     if (decode) {
         for (uint32_t i = 0; i < m; ++i) {
             int rc = launch_gemv_int_expert(s, scheme, (const uint8_t*)x + (size_t)i * k * xes, xbf, wst,

@@ -55,7 +55,8 @@ def test_streaming_f32_gemv_on_weights_at_an_odd_address():
         assert_within_tolerance(R.matmul(xd, wd, s, 70).cpu().numpy(), ref, _bound(s, w, x, 2048, 70), tol=2e-6, what=f"shift {shift}")
 
 
-@pytest.mark.parametrize("sch,m,k,n,E", [("q6_k", 2, 2304, 200, 5), ("q8_0", 8, 288, 77, 3), ("q4_0", 5, 4128, 130, 4)])
+@pytest.mark.parametrize("sch,m,k,n,E", [("q6_k", 2, 2304, 200, 5), ("q8_0", 8, 288, 77, 3), ("q4_0", 5, 4128, 130, 4),
+                                         ("q4_k", 10, 3072, 576, 16), ("q5_k", 12, 1792, 330, 5), ("q6_k", 31, 768, 40, 9)])
 def test_expert_rows_of_odd_lengths_in_one_launch(sch, m, k, n, E):
     import torch
     import rlx_b200 as R
