@@ -13,8 +13,9 @@
 //                       grouped_moe_unpermute_out, gguf_matmul.rs:207-218, is the store address)
 // Accumulation is f32 in a different order from the CPU loop; same tolerance as the general kernel.
 //
-// More than eight rows (and eight or fewer of a shape the streaming GEMV does not take) go through the tcgen05 GEMM in
-// its grouped form instead of moe_grouped_kernel, which only runs when the workspace is too small for it:
+// More than eight rows go through the tcgen05 GEMM in its grouped form instead of moe_grouped_kernel, which only runs when
+// the workspace is too small for it (fewer than 32 rows of little work, moe_rows_stream, and eight or fewer of a shape the
+// integer GEMV does not take: one launch of the f32 streaming GEMV, gemv_f32.cu):
 //   moe_tiles_kernel    the table of activation tiles, one list per expert, from the sorted offsets
 //   relay_rows_kernel   (rows TMA cannot tile) the slabs of the experts in use on a padded pitch
 //   moe_gather_kernel   the rows of every expert, gathered next to each other as bf16 (f32 activations as
@@ -23,10 +24,10 @@
 //                       stored at the rows' original positions
 // The weight operand is bf16(d * q) there, as in the dense GEMM; for fewer than 32 rows, and rows of those other lengths,
 // it keeps 16 bits (hi + lo).
-// All of them are launched as programmatic dependents.  1024 rows over 8 experts of 4096 -> 14336 Q4_K: 230 us; 331 us
+// All of them are launched as programmatic dependents.  1024 rows over 8 experts of 4096 -> 14336 Q4_K: 190 us; 331 us
 // with fixed 128-row tiles, an f32 result array and a scatter kernel behind the GEMM.
 //
-// Decode (m <= 8 rows, Q4_0 / Q8_0 / Q4_K / Q6_K, k a multiple of 256 up to 12288) skips both kernels:
+// Decode (m <= 8 rows, Q4_0 / Q8_0 / Q4_K / Q5_K / Q6_K, k a multiple of 256 up to 12288) skips both kernels:
 // every row is one launch of the streaming integer GEMV over the whole stack seen as an
 // [experts * n, k] matrix, with the slab picked on the device from expert_idx[i] (gemv_int.cu,
 // expert-indirect mode), so a routed expert's weights come through the TMA ring at GEMV speed.
@@ -209,8 +210,8 @@ static uint32_t moe_tile_rows(uint32_t m, uint32_t E, bool xbf) {
 
 // Whether m rows are cheaper row by row (the f32 GEMV: every row reads its expert's slab, about 0.25 us per million weights,
 // and nothing goes in front of it) than as a GEMM (sort, gather and PRECISE weights: 14 us, and 0.5 us for each 64 columns of
-// each wave of 128-row weight tiles of the experts in use).  GEMV and GEMM measured: 4 x 7424 x 640 Q5_K E16 F1 and 72 us,
-// 12 x 1792 x 8320 Q5_K E16 F2 and 76 us, 10 x 3072 x 576 Q4_K E16 F3 and 33 us, 20 x 2816 x 6720 Q8_0 E16 F4 and 117 us.
+// each wave of 128-row weight tiles of the experts in use).  GEMV and GEMM measured: 4 x 7424 x 640 Q5_K E16 11 and 73 us,
+// 12 x 1792 x 8320 Q5_K E16 63 and 76 us, 10 x 3072 x 576 Q4_K E16 8 and 34 us, 20 x 2816 x 6720 Q8_0 E16 96 and 118 us.
 // Batches that the GEMM multiplies in bf16 (kMoeBf16Rows and more) stay with it.
 static bool moe_rows_stream(uint32_t m, uint32_t k, uint32_t n, uint32_t E) {
     if (m <= kMoeDecodeRows) return true;
