@@ -1320,7 +1320,9 @@ static __device__ __noinline__ void tp_wait_and_sum(const TpPush& tp, unsigned l
 // ---------------------------------------------------------------------------------------------
 // Kernel 2: the streaming kernel
 // ---------------------------------------------------------------------------------------------
-template <uint32_t SCHEME, int MM, bool MMA = false, bool TP = false>
+// EXPERT (one activation row): the expert-indirect mode, an instance of its own, because the code for an id out of range in
+// the dense kernel cost that one 1-2 %.
+template <uint32_t SCHEME, int MM, bool MMA = false, bool TP = false, bool EXPERT = false>
 __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gemv_int_kernel(const __grid_constant__ IntParams P) {
     constexpr uint32_t CW = int_warps(MMA), WPU = CW / kIntCU, RL = int_red_lanes(MMA);
     using T = StagedTraits<SCHEME>;
@@ -1370,11 +1372,12 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
     // before it) and leaves at once when the id is out of range
     auto resolve_expert = [&](uint32_t& row_off) -> bool {
         row_off = 0u;
-        if (!P.expert_sel) return true;
-        griddep_wait();
-        uint32_t e;
-        if (!expert_of_row(*P.expert_sel, P.num_experts, &e)) return false;
-        row_off = e * P.n;
+        if constexpr (EXPERT) {
+            griddep_wait();
+            uint32_t e;
+            if (!expert_of_row(*P.expert_sel, P.num_experts, &e)) return false;
+            row_off = e * P.n;
+        }
         return true;
     };
 
@@ -2207,7 +2210,7 @@ static unsigned long long next_call_token() {
     return (epoch.fetch_add(1) << 2) | 1ull;
 }
 
-template <uint32_t SCHEME, int MM, bool MMA = false, bool TP = false>
+template <uint32_t SCHEME, int MM, bool MMA = false, bool TP = false, bool EXPERT = false>
 static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf,
                         uint32_t k, uint32_t n, void* ws, size_t ws_bytes, const IntPlan& pl, int* err_word, bool pair,
                         const float* expert_sel = nullptr, uint32_t num_experts = 0, uint32_t m_real = (uint32_t)MM,
@@ -2263,7 +2266,7 @@ static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint
     int dev = 0;
     RLXQ_CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && attr_set[dev].load() == 0) {
-        RLXQ_CUDA_TRY(cudaFuncSetAttribute(gemv_int_kernel<SCHEME, MM, MMA, TP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        RLXQ_CUDA_TRY(cudaFuncSetAttribute(gemv_int_kernel<SCHEME, MM, MMA, TP, EXPERT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         attr_set[dev].store(1);
     }
     const uint32_t groups = (k / 8) * m_real;
@@ -2275,7 +2278,7 @@ static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint
                         (pair ? 1u : 0u), tp ? reinterpret_cast<unsigned long long*>(tp->buf[tp->rank]) : nullptr, tp ? pl.grid : 0u);
     if (rc) return rc;
     if (!P.inline_q) count_launch();
-    rc = launch_pdl(gemv_int_kernel<SCHEME, MM, MMA, TP>, dim3(pl.grid), dim3(int_threads(MMA)), pl.smem_bytes, stream, P);
+    rc = launch_pdl(gemv_int_kernel<SCHEME, MM, MMA, TP, EXPERT>, dim3(pl.grid), dim3(int_threads(MMA)), pl.smem_bytes, stream, P);
     if (rc) return rc;
     count_launch();
     return check_launch("gemv_int_kernel");
@@ -2313,7 +2316,9 @@ static int launch_int_s(cudaStream_t stream, const void* x, bool xbf, const uint
             }
             return fail(RLXQ_E_SHAPE, "no pushing dp4a GEMV for scheme %u at m=%u", (unsigned)SCHEME, m);
         }
-        if (m == 1) return launch_int_t<SCHEME, 1>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, expert_sel, num_experts, 1);
+        if (m == 1 && expert_sel)
+            return launch_int_t<SCHEME, 1, false, false, true>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, expert_sel, num_experts, 1);
+        if (m == 1) return launch_int_t<SCHEME, 1>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair);
         if (m == 2) return launch_int_t<SCHEME, 2>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, nullptr, 0, 2);
         return launch_int_t<SCHEME, 4>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, nullptr, 0, m);
     } else {
