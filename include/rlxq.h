@@ -90,11 +90,11 @@ RLXQ_API int rlxq_packed_bytes(uint32_t scheme, uint64_t k, uint64_t n, uint64_t
 /* Replaces dequant_gguf_scratch_bytes (rlx-cuda/src/gguf_gpu.rs:35-59) at plan time: the
  * scratch rlxq_matmul needs for this shape.  For m <= 8 that is the converted activations
  * (a few bytes per element of x), the partial output tiles of CTAs that share a row tile and
- * their counters: tens to hundreds of KiB (up to 4.9 MB while the option gemv_kernel is 4).  The tensor-core GEMM needs none for most shapes; for few
- * output tiles and a long k it asks for two partial 128 x 256 f32 tiles per SM (39 MB on a 148-SM
- * part) for its stream-K split; without them it runs whole tiles.  With f32 activations and m > 8 the GEMM runs
- * on their bf16 hi + lo halves, a chunk of rows at a time: the split rows and the two partial results need up to
- * about 150 MB (256-byte aligned); without that workspace such a call runs the tiled generic kernel, some 40 times
+ * their counters: tens to hundreds of KiB (up to 4.9 MB while the option gemv_kernel is 4).  The tensor-core GEMM needs
+ * none for most shapes; for few output tiles it asks for k slices of the result or two partial tiles per SM (tens of MB);
+ * without them it runs whole tiles.  With f32 activations and m > 8 it needs their bf16 hi + lo parts (4 bytes a value), and
+ * for rows that are no multiple of 16 bytes a copy of the weights on a padded pitch (256-byte aligned); without that
+ * workspace such a call runs the tiled generic kernel, some 40 times
  * slower.  The reference reserves k*n*4 bytes. */
 RLXQ_API int rlxq_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n,
                          uint32_t x_dtype, uint32_t y_dtype, size_t* bytes);
@@ -213,14 +213,13 @@ RLXQ_API uint64_t rlxq_launch_count(void);
  *   "gemv_chain": 1 = rlxq_matmul_chain runs a chain as one cooperative kernel where it can, 0 (default) = always
  *                  layer by layer
  *   "gemm_kernel": 0 = automatic, 1 = force the tiled generic kernel, 2 = force the tcgen05 GEMM
- *   "gemm_streamk": 0 = automatic (split the k dimension across SMs when that saves at least 36
- *                  256-wide k steps on the busiest SM and a workspace is given), 1 = never,
- *                  2 = whenever a workspace is given
+ *   "gemm_streamk": 0 = automatic (split the k dimension across SMs where the estimated time is less and a workspace is
+ *                  given), 1 = never, 2 = whenever a workspace is given
  *   "gemm_pair": the tcgen05 GEMM with two CTAs per MMA (a cluster of two SMs on 256 weight rows x 256 activation
- *                  rows, each CTA loading half of the activation tile): 0 = automatic (n a multiple of 256, at
- *                  least one tile pair per resident cluster, not Q6_K or Q3_K, no k split chosen), 1 = never, 2 = wherever
- *                  n is a multiple of 256.  Same bits as the single-CTA kernel.  "gemm_pair_clusters" (read only):
- *                  clusters the device keeps resident, 0 until the paired kernel has run
+ *                  rows, each CTA loading half of the activation tile): 0 = automatic (n a multiple of 256 and the
+ *                  estimated time is less), 1 = never, 2 = wherever n is a multiple of 256.  Same bits as the single-CTA
+ *                  kernel.  "gemm_pair_clusters" (read only): clusters the device keeps resident, 0 until the paired
+ *                  kernel has run
  *   "gemm_tile_x": 0 = automatic, a multiple of 32 up to 256 = activation rows per tile of the tcgen05 GEMM (128 at
  *                  most with f32 activations)
  *   "gemv_inline_q": 0 = automatic, 1 = the integer GEMV always runs its activation quantiser as a

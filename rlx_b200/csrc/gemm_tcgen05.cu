@@ -1,8 +1,8 @@
-// Prefill GEMM (m >= 128 activation rows) on the 5th-generation tensor cores: tcgen05.mma with
+// Prefill GEMM (m > 8 activation rows) on the 5th-generation tensor cores: tcgen05.mma with
 // the accumulator AND the dequantised weight operand in tensor memory, activations by TMA.
 //
-// y[m,n] = x[m,k] . W^T is computed transposed, tile by tile: D[128 weight rows, 256 activation
-// rows] += A[128, 64] . B[256, 64]^T per 64-wide k block.
+// y[m,n] = x[m,k] . W^T is computed transposed, tile by tile: D[128 weight rows, 32 to 256 activation
+// rows] += A[128, 64] . B[rows, 64]^T per 64-wide k block.
 //   * A (weights) never exists in memory.  The raw GGUF blocks of 128 rows x 256 weights arrive in
 //     shared memory through one 2-D TMA box; eight decode warps, twelve for Q3_K (one thread per weight row, which
 //     is also that thread's tensor-memory lane) turn 64 weights at a time into bf16(d * q) in
