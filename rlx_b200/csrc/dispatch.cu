@@ -10,8 +10,8 @@ namespace rlxq {
 // Prefill (m > 8) on the tensor-core GEMM.  Its operands are bf16: f32 activations go in as hi + lo halves, `chunk`
 // rows of x at a time (the split rows are kept under 128 MiB), multiplied by the same decoded weights.  Rows that TMA
 // cannot tile where they lie (k not a whole number of 256 weights, or of the 16-byte groups of a format's super-blocks;
-// weights that are not 16-byte aligned) are first re-laid on a padded pitch in the workspace, and the weight operand then
-// keeps hi and lo parts too, since those shapes were multiplied in f32 before they had this path.
+// weights that are not 16-byte aligned) are first re-laid on a padded pitch in the workspace, and weights and activations
+// then keep all of their 24 bits (PRECISE), since those shapes were multiplied in f32 before they had this path.
 struct PrefillPlan { bool ok, relaid, halves; uint32_t chunk; uint64_t pitch; size_t off_w, off_y2, off_gemm, bytes; };
 static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, bool direct) {
     PrefillPlan p{};
@@ -25,14 +25,19 @@ static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_
     // the chunk keeps the two results under 128 MiB.
     p.halves = !xbf && !p.relaid && k <= 512;
     if (!xbf) {
-        chunk = p.halves ? (128ull << 20) / (8ull * n) / 128 * 128 : (128ull << 20) / (4ull * k) / 256 * 256;
+        chunk = p.halves ? (128ull << 20) / (8ull * n) / 128 * 128 : (128ull << 20) / (4ull * k) / 256 * 256;      // (PRECISE: 192 MiB)
         const uint64_t least = p.halves ? 128 : 256;
         if (chunk < least) chunk = least;
         if (p.halves && chunk > 2048) chunk = 2048;
         if (chunk > m) chunk = m;
     }
+    // PRECISE: a slice of the result for each 1024 columns, 192 MiB of them at once (but no fewer than 192 rows)
+    if (p.relaid) {
+        const uint64_t rows = (192ull << 20) / (4ull * n * ((k + 1023) / 1024)) / 192 * 192;
+        if (chunk > rows) chunk = rows < 192 ? (m < 192 ? m : 192) : rows;
+    }
     p.chunk = (uint32_t)chunk;
-    p.off_w = xbf ? 0 : al((size_t)2 * chunk * k * 2);
+    p.off_w = xbf ? 0 : al((size_t)gemm_x_parts(true, p.relaid) * chunk * k * 2);
     p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;
     p.off_y2 = p.off_w + al((size_t)(p.pitch * n));
     p.off_gemm = p.off_y2 + (p.halves ? al((size_t)2 * chunk * n * 4) : 0);
@@ -147,7 +152,7 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
             void* const out = static_cast<uint8_t*>(y) + (size_t)r0 * n * (ybf ? 2 : 4);
             c.x = static_cast<const uint8_t*>(x) + (size_t)r0 * k * (xbf ? 2 : 4);
             if (!xbf) {
-                int rc = launch_split_hi_lo(stream, static_cast<const float*>(c.x), base, rows, k);
+                int rc = launch_split_hi_lo(stream, static_cast<const float*>(c.x), base, rows, k, gemm_x_parts(true, p.relaid));
                 if (rc) return rc;
                 c.x = base;
             }

@@ -58,35 +58,37 @@ int launch_copy_bytes(cudaStream_t stream, void* dst, const void* src, uint64_t 
 }
 
 // f32 activations for the tensor-core GEMM, whose operands are bf16: x = hi + lo with hi = bf16(x) and
-// lo = bf16(x - hi), which leaves 2^-17 of x behind.  Rows [row0, row0 + rows) of x become rows [0, rows)
-// (hi) and [rows, 2 rows) (lo) of `out`; the GEMM multiplies both by the same decoded weights.  One pass of 8 bytes a
+// lo = bf16(x - hi), which leaves 2^-17 of x behind, or (parts = 3) x = hi + mid + lo, which leaves nothing.  Rows [row0,
+// row0 + rows) of x become rows [0, rows) (hi), [rows, 2 rows) and, if asked for, [2 rows, 3 rows) of `out`; the GEMM multiplies both by the same decoded weights.  One pass of 8 bytes a
 // value, a few microseconds; the GEMM behind it is resident meanwhile and fetches its first weights.
 __global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restrict__ x, uint16_t* __restrict__ out,
-                                                          uint64_t rows, uint64_t k) {
+                                                          uint64_t rows, uint64_t k, uint32_t parts) {
     const uint64_t total = rows * k / 4, stride = (uint64_t)gridDim.x * blockDim.x;     // k % 4 == 0
     griddep_launch_dependents();
     griddep_wait();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const float4 v = reinterpret_cast<const float4*>(x)[i];
         const float f[4] = {v.x, v.y, v.z, v.w};
-        uint16_t h[4], l[4];
+        uint16_t h[4], l[4], e[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             h[j] = (uint16_t)f32_to_bf16_bits(f[j]);
-            const float rest = f[j] - __uint_as_float((uint32_t)h[j] << 16);     // exact; inf - inf = NaN stays NaN in y
-            l[j] = (uint16_t)f32_to_bf16_bits(isfinite(f[j]) ? rest : 0.f);
+            const float rest = isfinite(f[j]) ? f[j] - __uint_as_float((uint32_t)h[j] << 16) : 0.f;     // exact
+            l[j] = (uint16_t)f32_to_bf16_bits(rest);
+            e[j] = (uint16_t)f32_to_bf16_bits(rest - __uint_as_float((uint32_t)l[j] << 16));
         }
         reinterpret_cast<uint2*>(out)[i] = make_uint2(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16));
         reinterpret_cast<uint2*>(out + rows * k)[i] = make_uint2(l[0] | ((uint32_t)l[1] << 16), l[2] | ((uint32_t)l[3] << 16));
+        if (parts == 3) reinterpret_cast<uint2*>(out + 2 * rows * k)[i] = make_uint2(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16));
     }
 }
 
-int launch_split_hi_lo(cudaStream_t stream, const float* x, void* out, uint64_t rows, uint64_t k) {
+int launch_split_hi_lo(cudaStream_t stream, const float* x, void* out, uint64_t rows, uint64_t k, uint32_t parts) {
     if (rows == 0 || k == 0) return RLXQ_OK;
     uint64_t blocks = (rows * k / 4 + 255) / 256;
     const uint64_t cap = (uint64_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    int rc = launch_pdl(split_hi_lo_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, x, reinterpret_cast<uint16_t*>(out), rows, k);
+    int rc = launch_pdl(split_hi_lo_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, x, reinterpret_cast<uint16_t*>(out), rows, k, parts);
     if (rc) return rc;
     count_launch();
     return check_launch("split_hi_lo_kernel");

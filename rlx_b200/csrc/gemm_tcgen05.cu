@@ -130,22 +130,24 @@ template <int H> __device__ __forceinline__ uint64_t magic_pair(uint32_t u) {
 template <int H> __device__ __forceinline__ uint64_t scaled_pair(uint32_t u, uint64_t neg_off, uint64_t scale) {
     return mul_f32x2(add_f32x2(magic_pair<H>(u), neg_off), scale);
 }
-// Where a decoder puts its 64 weights, two f32 at a time: rounded to bf16 pairs, or as bf16 hi and lo parts.
+// Where a decoder puts its 64 weights, two f32 at a time: rounded to bf16 pairs, or kept as they are (PRECISE).
 template <bool PRECISE> struct GemmOut {
     uint32_t hi[32];
     __device__ __forceinline__ void put(int i, uint64_t pair) { hi[i] = bf16x2_of(pair); }
 };
-// hi is the upper half of the f32 bits (one byte-permute per pair; a conversion instruction would pace the decoder), lo
-// the upper half of what that leaves behind, which is exact in f32: together the first 16 bits of the weight.
+// An f32 weight is the sum of three bf16 values: the upper half of its bits, of what that leaves behind, and of what is
+// left then, all of it exact (one byte-permute per pair and part; a conversion instruction would pace the decoder).
 template <> struct GemmOut<true> {
-    uint32_t hi[32], lo[32];
-    __device__ __forceinline__ void put(int i, uint64_t pair) {
-        uint32_t a, b;
-        asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(pair));
-        hi[i] = __byte_perm(a, b, 0x7632);
-        const uint64_t rest = add_f32x2(pair, f32x2((a & 0xFFFF0000u) ^ 0x80000000u, (b & 0xFFFF0000u) ^ 0x80000000u));
-        asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(rest));
-        lo[i] = __byte_perm(a, b, 0x7632);
+    uint64_t f[32];
+    __device__ __forceinline__ void put(int i, uint64_t pair) { f[i] = pair; }
+    __device__ __forceinline__ void part(uint32_t (&p)[32]) {          // the next part
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            uint32_t a, b;
+            asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(f[i]));
+            p[i] = __byte_perm(a, b, 0x7632);
+            f[i] = add_f32x2(f[i], f32x2((a & 0xFFFF0000u) ^ 0x80000000u, (b & 0xFFFF0000u) ^ 0x80000000u));
+        }
     }
 };
 
@@ -521,7 +523,7 @@ struct GemmParams {
     // f32 activations (lo_row != 0): x holds bf16(x) in rows [0, lo_row) and bf16(x - bf16(x)) in the same number of
     // rows behind them; a stage carries both boxes and both are multiplied by the same decoded weights into the same
     // accumulator, so a weight is decoded once for the two halves.
-    uint32_t lo_row;
+    uint32_t lo_row, xparts;
     uint32_t nstages, nraw;               // depth of the operand ring (B in shared memory, A in tensor memory) and of the raw ring
     uint32_t b_bytes;                     // bytes of a B stage: tx * 128, twice that with lo_row
     uint32_t w_late;       // the weights are written by a kernel in front (re-laid rows): read them after the dependency wait
@@ -757,7 +759,7 @@ template <uint32_t SCHEME, bool PRECISE, uint32_t GRP>
 __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* bars, const uint8_t* raw_stage, uint32_t tmem_a,
                                                  uint32_t xtiles, uint32_t warp, uint32_t lane) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW, GROUPS = GemmRaw<SCHEME>::GROUPS;
-    constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128, A_COLS = PRECISE ? 64 : 32;
+    constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128, A_COLS = PRECISE ? 96 : 32;
     volatile uint32_t* abort_flag = &bars->abort_flag;
     auto give_up = [&](int code) {
         atomicExch(P.err, code);
@@ -800,12 +802,20 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
                 sph = ph0;
                 if (st >= NS) { st -= NS; sph ^= 1u; }
             };
-            auto store = [&](uint32_t st, uint32_t sph, uint32_t ready, const GemmOut<PRECISE>& v) -> bool {
+            auto store = [&](uint32_t st, uint32_t sph, uint32_t ready, GemmOut<PRECISE>& v) -> bool {
                 announce();
                 if (!__all_sync(0xFFFFFFFFu, ready) && (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[st]), sph))) { give_up(16); return false; }
                 tc_fence_after();
-                tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
-                if constexpr (PRECISE) tmem_st32(tmem_a + lane_addr + A_COLS * st + 32, v.lo);
+                if constexpr (PRECISE) {
+#pragma unroll
+                    for (uint32_t q = 0; q < 3; ++q) {
+                        uint32_t p[32];
+                        v.part(p);
+                        tmem_st32(tmem_a + lane_addr + A_COLS * st + 32 * q, p);
+                    }
+                } else {
+                    tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
+                }
                 pending = smem_u32(&bars->a_full[st]);
                 return true;
             };
@@ -853,16 +863,17 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
     announce();
 }
 
-// PRECISE: the weight operand keeps 16 significand bits, as bf16 hi and lo parts in two sets of tensor-memory columns,
-// and every activation box is multiplied by both (the lo half of f32 activations by the hi part only: what is left out
-// is below 2^-16 of a product).  It serves the shapes whose other kernel multiplies f32 weights.
+// PRECISE: the weight operand is the f32 weight, as three bf16 parts in three sets of tensor-memory columns, and f32
+// activations come as three parts as well (GemmOut; split_hi_lo_kernel).  It serves the shapes whose other kernel multiplies
+// f32 weights and activations: three products for bf16 activations, six for f32 ones, where the formats' own path takes one
+// and two.
 template <uint32_t SCHEME, bool PRECISE>
 __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
     constexpr uint32_t kGemmDecodeGroups = GemmRaw<SCHEME>::GROUPS;
     constexpr uint32_t RAW_BYTES = kGemmTileW * RAW_ROW;
     constexpr uint32_t RAW_STRIDE = (RAW_BYTES + 127) / 128 * 128;
-    constexpr uint32_t A_COLS = PRECISE ? 64 : 32;                    // tensor-memory columns of a weight stage
+    constexpr uint32_t A_COLS = PRECISE ? 96 : 32;                    // tensor-memory columns of a weight stage
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t NS = P.nstages, NR = P.nraw, B_BYTES = P.b_bytes;
@@ -900,9 +911,10 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
-    const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + 256;
-    // up to 128 activation rows there are two accumulators: a tile's epilogue runs under the next tile's MMAs
-    const uint32_t nacc = P.tx <= 128 ? 2u : 1u;
+    const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + (PRECISE ? 128 : 256);
+    // up to 128 activation rows there are two accumulators: a tile's epilogue runs under the next tile's MMAs (PRECISE, whose
+    // weight stages take 384 columns: one accumulator of 128)
+    const uint32_t nacc = !PRECISE && P.tx <= 128 ? 2u : 1u;
     auto give_up = [&](int code) {
         atomicExch(P.err, code);
         *abort_flag = 1u;
@@ -929,7 +941,8 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                     const uint32_t full = smem_u32(&bars->b_full[s]), dst = smem_u32(b_stage + s * B_BYTES);
                     mbar_arrive_expect_tx(full, B_BYTES);
                     tma_load_2d(dst, &P.xmap, (int32_t)(kb * kGemmBK), (int32_t)tr.xrow0, full);
-                    if (P.lo_row) tma_load_2d(dst + P.tx * 128u, &P.xmap, (int32_t)(kb * kGemmBK), (int32_t)(P.lo_row + tr.xrow0), full);
+                    for (uint32_t q = 1; q < P.xparts; ++q)
+                        tma_load_2d(dst + q * P.tx * 128u, &P.xmap, (int32_t)(kb * kGemmBK), (int32_t)(q * P.lo_row + tr.xrow0), full);
                     if (++s == NS) { s = 0; ph ^= 1u; }
                 }
             }
@@ -982,14 +995,20 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
 #pragma unroll
                     for (uint32_t j = 0; j < kGemmBK / 16; ++j)
                         tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, (kb | j) ? 1u : 0u);
+                    // PRECISE: weight parts 0..2 by activation part 0, 0..1 by part 1, 0 by part 2; the three products left out
+                    // are below 2^-24 of the whole
                     if (PRECISE) {
 #pragma unroll
-                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 32 + 8 * j, bdesc + 2 * j, idesc, 1u);
+                        for (uint32_t j = 0; j < 2 * kGemmBK / 16; ++j) tc_mma_ts(acc, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, 1u);
                     }
-                    if (P.lo_row) {
-                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + P.tx * 128u));
+                    for (uint32_t q = 1; q < P.xparts; ++q) {
+                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
 #pragma unroll
                         for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
+                        if (PRECISE && q == 1) {
+#pragma unroll
+                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 32 + 8 * j, ldesc + 2 * j, idesc, 1u);
+                        }
                     }
                     tc_commit(smem_u32(&bars->stage_free[s]));     // frees the B stage and the A columns when the MMAs retire
                     s = sn;
@@ -1436,30 +1455,40 @@ uint64_t gemm_relaid_pitch(uint32_t scheme, uint32_t k) {
     return ((uint64_t)((k + 255) / 256) * (256 / g.elems) * g.bytes + 15) / 16 * 16;
 }
 
+// Parts of an activation value: bf16 ones are one, f32 ones hi and lo, or all 24 bits beside PRECISE weights.
+uint32_t gemm_x_parts(bool f32, bool precise) { return !f32 ? 1u : precise ? 3u : 2u; }
+// The most activation rows of a tile: four operand stages and two raw boxes have to fit in shared memory (three parts of 96
+// rows beside all but the 8-bit formats' boxes), accumulators and weight stages in tensor memory.
+uint32_t gemm_most_rows(uint32_t scheme, bool f32, bool precise) {
+    if (!precise) return f32 ? 128u : 256u;
+    return !f32 ? 128u : scheme == RLXQ_Q8_0 || scheme == RLXQ_Q8_K ? 64u : 96u;
+}
+
+constexpr uint32_t kGemmPreciseRun = 1024;
 struct GemmShape { uint32_t tx, xtiles, slices; bool streamk, pair; };
 
 // Activation rows per tile, work split and kernel for a shape, by estimated time in cycles.  A 64-wide k block of a tile
 // costs the larger of its MMAs (2 cycles per activation row and product plus the hand-over; `products`: bf16 activations
-// 1, f32 2, one more with PRECISE weights) and its decode, whatever part of the tile's rows is padding; so few rows get a
+// 1, f32 2, three times that with PRECISE weights) and its decode, whatever part of the tile's rows is padding; so few rows get a
 // narrow tile, and rows are split evenly over the fewest tiles that leave no SM idle.  The constants are fits to 45 shapes
 // (five formats, 16 to 1526 rows, k 2048 to 14336), each timed at every tile width, split and kernel: the choice made here
 // takes 1 % longer than the best one in the geometric mean, up to 10 % at worst.
 static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t products, bool precise, bool pair) {
     const bool heavy = scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K;
     if (pair) return heavy && products == 1 ? 925 : 750 * products;        // 256 activation rows, both CTAs at once
-    uint32_t mma = 2 * tx * products + 265 + (products > 1 ? 65 : 0);
+    uint32_t mma = (precise && tx < 112 ? 228 : 2 * tx) * products + 265 + (products > 1 ? 65 : 0);   // an MMA takes 57 cycles at least
     if (products == 2 && tx >= 96 && mma < 800) mma = 800;
     if (heavy) mma += 90;
     uint32_t dec = scheme == RLXQ_Q3_K ? 1130 : heavy ? 740 : scheme == RLXQ_Q8_0 || scheme == RLXQ_Q4_0 || scheme == RLXQ_Q4_K ? 570 : 620;
-    if (precise) dec += 350;
+    if (precise) dec += 500;
     return mma > dec ? mma : dec;
 }
 // Two CTAs per MMA; PRECISE weights are not built in that form.
 static bool gemm_pair_fits(uint32_t n, bool precise) { return n % 256 == 0 && !precise; }
 static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise, bool can_split) {
     const uint64_t sms = (uint64_t)sm_count(), wt = (n + kGemmTileW - 1) / kGemmTileW, groups = (k + 255) / 256, blocks = 4 * groups;
-    const uint32_t products = 1 + (f32 ? 1 : 0) + (precise ? 1 : 0);
-    const uint32_t most = f32 ? 128 : 256;               // a stage holds 256 box rows
+    const uint32_t products = (precise ? 3 : 1) * (f32 ? 2 : 1);
+    const uint32_t most = gemm_most_rows(scheme, f32, precise);
     const int64_t fx = options().gemm_tile_x.load(), fs = can_split ? options().gemm_streamk.load() : 1, fp = options().gemm_pair.load();
     const GemmShape pair{256, (m + 255) / 256, 1, false, true};
     if (fp == 2 && gemm_pair_fits(n, precise)) return pair;
@@ -1470,6 +1499,10 @@ static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
         const uint64_t ptiles = (uint64_t)(n / 256) * pair.xtiles, pairs = sms / 2;
         take((ptiles + pairs - 1) / pairs * blocks * gemm_block_cycles(scheme, 256, products, precise, true) + 24 * 256, pair);
     }
+    // The tensor core truncates where f32 arithmetic rounds, every time it adds to an accumulator: over the 4000 additions of
+    // k = 11008 and six products that is 4e-5 of a result.  PRECISE tiles therefore never run further than kGemmPreciseRun
+    // columns; the kernel behind adds the slices, rounding.
+    const uint64_t runs = precise && can_split ? (groups + kGemmPreciseRun / 256 - 1) / (kGemmPreciseRun / 256) : 1;
     const uint32_t least_tiles = (m + most - 1) / most;
     for (uint32_t xt = least_tiles; xt <= least_tiles + 8; ++xt) {
         uint32_t tx = ((m + xt - 1) / xt + 31) / 32 * 32;
@@ -1478,6 +1511,12 @@ static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
         if (tiles_x != xt && !fx) continue;              // the same width as one tile fewer
         const uint64_t ntiles = wt * tiles_x, cyc = gemm_block_cycles(scheme, tx, products, precise, false);
         const uint64_t epi = 24 * tx;                    // the last tile's epilogue, and with one accumulator every tile's
+        if (runs > 1) {
+            const uint64_t fit = sms / ntiles, sl = std::max(runs, std::min(groups, fit));
+            take((ntiles * sl + sms - 1) / sms * (((groups + sl - 1) / sl * 4) * cyc + epi) + 3200 + sl * m * n / 600, GemmShape{tx, tiles_x, (uint32_t)sl, false, false});
+            if (fx) break;
+            continue;
+        }
         if (fs != 2) take((ntiles + sms - 1) / sms * (blocks * cyc + (tx > 128 ? epi : 0)) + epi, GemmShape{tx, tiles_x, 1, false, false});
         // k split over the SMs (stream-K): every SM gets the same blocks, and exchanges up to two parts of 128 x tx values
         if (fs != 1 && (fs == 2 || ntiles % sms))
@@ -1523,7 +1562,8 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     GemmParams P{};
     P.tx = sh.tx;
     P.lo_row = c.f32 ? c.x_rows : 0u;
-    int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * (c.f32 ? 2 : 1), c.k, P.tx);
+    P.xparts = gemm_x_parts(c.f32, PRECISE);
+    int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * P.xparts, c.k, P.tx);
     if (rc) return rc;
     rc = encode_weight_map(&P.wmap, c.w, (uint64_t)c.n * c.num_slabs, c.w_pitch ? c.w_pitch : (uint64_t)c.k / g.elems * g.bytes,
                            RAW_ROW / 8, kGemmTileW);
@@ -1544,10 +1584,11 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     P.err = device_error_word();
     if (!P.err) return fail(RLXQ_E_CUDA, "device error word unavailable");
     // as many operand stages as tensor memory and shared memory hold beside two raw boxes, then raw boxes
-    P.b_bytes = P.tx * kGemmBK * 2 * (c.f32 ? 2 : 1);
+    P.b_bytes = P.tx * kGemmBK * 2 * P.xparts;
     const uint32_t smem = 227 * 1024;   // all of it: one CTA per SM, so that none waits for another's tensor memory
     const uint32_t budget = smem - (1024 + sizeof(GemmBars) + 64 + kGemmEpiStage);
     P.nstages = std::min<uint32_t>(PRECISE ? 4 : kGemmMaxStages, (budget - kGemmRawStages * RAW_STRIDE) / P.b_bytes);
+    if (P.nstages < 4) return fail(RLXQ_E_LIMIT, "GEMM tile of %u activation rows too large", P.tx);   // a weight group is four
     P.nraw = std::min<uint32_t>(kGemmMaxRaw, (budget - P.nstages * P.b_bytes) / RAW_STRIDE);
     static std::atomic<uint32_t> attr_set[64];
     int dev = 0;

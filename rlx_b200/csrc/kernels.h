@@ -24,7 +24,9 @@ int launch_gemv_int(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
                     bool ybf, uint32_t m, uint32_t k, uint32_t n, void* ws, size_t ws_bytes);
 
 // tcgen05 / tensor-memory GEMV (m <= 8): weights decoded to fp16 in tensor memory, activations as bf16 high / low rows.
-int launch_split_hi_lo(cudaStream_t stream, const float* x, void* out, uint64_t rows, uint64_t k);
+int launch_split_hi_lo(cudaStream_t stream, const float* x, void* out, uint64_t rows, uint64_t k, uint32_t parts);
+uint32_t gemm_x_parts(bool f32, bool precise);
+uint32_t gemm_most_rows(uint32_t scheme, bool f32, bool precise);
 int launch_add_slices(cudaStream_t stream, const float* part, uint32_t slices, uint64_t stride, void* y, bool ybf, uint64_t total);
 int launch_swiglu_pair(cudaStream_t stream, const float* gu, void* h, uint32_t m, uint32_t f);
 // A chain of dependent batch-1/2 GEMVs in one cooperative launch (gemv_int.cu, gemv_chain_kernel).
@@ -50,7 +52,7 @@ struct GemmCall {
     bool f32;
     const uint8_t* w;
     uint64_t w_pitch;          // bytes between weight rows that a kernel in front has re-laid (0: packed, and constant)
-    bool precise;              // weights as bf16 hi + lo instead of rounded to bf16
+    bool precise;              // f32 weights and activations, in bf16 parts, instead of weights rounded to bf16
     void* y;
     bool ybf;
     uint32_t k, n;

@@ -23,7 +23,7 @@
 //   gemm_tcgen05_kernel every tile against its expert's slab of the stack (gemm_tcgen05.cu, GemmParams::groups), results
 //                       stored at the rows' original positions
 // The weight operand is bf16(d * q) there, as in the dense GEMM; for fewer than 32 rows, and rows of those other lengths,
-// it keeps 16 bits (hi + lo).
+// it is the f32 weight, in three bf16 parts.
 // All of them are launched as programmatic dependents.  1024 rows over 8 experts of 4096 -> 14336 Q4_K: 190 us; 331 us
 // with fixed 128-row tiles, an f32 result array and a scatter kernel behind the GEMM.
 //
@@ -198,13 +198,13 @@ constexpr uint32_t kMoeDecodeRows = 8;      // up to this many rows go row by ro
 // ---- the tensor-core GEMM in its grouped form ------------------------------------------------------------------
 
 constexpr uint32_t kMoeBf16Rows = 32;       // batches of this size and more multiply bf16-rounded weights (where TMA can
-                                            // tile them); smaller ones keep 16 bits of the weights (GemmCall::precise)
+                                            // tile them); smaller ones f32 ones (GemmCall::precise)
 
 // Activation rows per GEMM tile: what one expert's share of the rows needs, with room for an uneven routing (2.5 standard
 // deviations of an even one), so that a slab is hardly ever decoded twice; f32 activations take two boxes per tile.
-static uint32_t moe_tile_rows(uint32_t m, uint32_t E, bool xbf) {
+static uint32_t moe_tile_rows(uint32_t m, uint32_t E, uint32_t most) {
     const float share = (float)m / (float)E;
-    const uint32_t want = ((uint32_t)(share + 2.5f * sqrtf(share)) + 31u) / 32u * 32u, most = xbf ? 256u : 128u;
+    const uint32_t want = ((uint32_t)(share + 2.5f * sqrtf(share)) + 31u) / 32u * 32u;
     return want < 32u ? 32u : (want > most ? most : want);
 }
 
@@ -227,7 +227,7 @@ static bool moe_rows_stream(uint32_t m, uint32_t k, uint32_t n, uint32_t E) {
 template <bool XBF16>
 __global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict__ x, const uint32_t* __restrict__ perm,
                                                          const uint4* __restrict__ table, uint32_t m, uint32_t k,
-                                                         uint16_t* __restrict__ xg, uint8_t* __restrict__ y, uint64_t y_row_bytes) {
+                                                         uint32_t parts, uint16_t* __restrict__ xg, uint8_t* __restrict__ y, uint64_t y_row_bytes) {
     griddep_launch_dependents();
     griddep_wait();
     const uint32_t i = blockIdx.x, src = perm[i];
@@ -244,23 +244,26 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict_
         const float4* in = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + (size_t)src * k);
         uint2* hi = reinterpret_cast<uint2*>(xg + (size_t)i * k);
         uint2* lo = reinterpret_cast<uint2*>(xg + (size_t)(m + i) * k);
+        uint2* last = reinterpret_cast<uint2*>(xg + (size_t)(2 * m + i) * k);
         for (uint32_t c = threadIdx.x; c < k / 4; c += blockDim.x) {
             const float4 v = in[c];
             const float f[4] = {v.x, v.y, v.z, v.w};
-            uint32_t h[4], l[4];
+            uint32_t h[4], l[4], e[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 h[q] = f32_to_bf16_bits(f[q]) & 0xFFFFu;
-                const float rest = f[q] - __uint_as_float(h[q] << 16);
-                l[q] = f32_to_bf16_bits(isfinite(f[q]) ? rest : 0.f) & 0xFFFFu;
+                const float rest = isfinite(f[q]) ? f[q] - __uint_as_float(h[q] << 16) : 0.f;
+                l[q] = f32_to_bf16_bits(rest) & 0xFFFFu;
+                e[q] = f32_to_bf16_bits(rest - __uint_as_float(l[q] << 16)) & 0xFFFFu;
             }
             hi[c] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
             lo[c] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+            if (parts == 3) last[c] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
         }
     }
 }
 
-struct MoeTcPlan { bool ok, relaid; uint32_t tiles, tile_rows; uint64_t pitch; size_t off_table, off_xg, off_w, bytes; };
+struct MoeTcPlan { bool ok, relaid, precise; uint32_t tiles, tile_rows; uint64_t pitch; size_t off_table, off_xg, off_w, bytes; };
 
 // The scratch of the tensor-core path behind the sort's arrays (which end at `base`): tile table, gathered activations
 // and, for rows TMA cannot tile where they lie, the re-laid slabs.  Not taken (ok = false) for other formats or when it
@@ -272,12 +275,13 @@ static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
     p.relaid = !(w_aligned && gemm_tc_supported(scheme, m, k, n, aligned, aligned));
     if (p.relaid && !gemm_relaid_supported(scheme, m, k, n, aligned)) return p;
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-    p.tile_rows = moe_tile_rows(m, E, xbf);
+    p.precise = p.relaid || m < kMoeBf16Rows;
+    p.tile_rows = moe_tile_rows(m, E, gemm_most_rows(scheme, !xbf, p.precise));
     p.tiles = m / p.tile_rows + (E < m ? E : m);
     p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;
     p.off_table = up(base);
     p.off_xg = p.off_table + up((size_t)(p.tiles + 1) * 16);
-    p.off_w = p.off_xg + up((size_t)(xbf ? 1 : 2) * m * k * 2);
+    p.off_w = p.off_xg + up((size_t)gemm_x_parts(!xbf, p.precise) * m * k * 2);
     p.bytes = p.off_w + up((size_t)p.pitch * n * E);
     p.ok = p.bytes <= (4ull << 30) && (uint64_t)n * E <= 0x7FFFFFFFull;
     return p;
@@ -387,10 +391,10 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
             c.w = ws + tc.off_w;
         }
         rc = launch_pdl(xbf ? moe_gather_kernel<true> : moe_gather_kernel<false>, dim3(m), dim3(256), 0, s, x, (const uint32_t*)perm,
-                        (const uint4*)table, m, k, xg, (uint8_t*)y, (uint64_t)n * yes);
+                        (const uint4*)table, m, k, gemm_x_parts(!xbf, tc.precise), xg, (uint8_t*)y, (uint64_t)n * yes);
         if (rc) return rc;
         count_launch();
-        c.x = xg; c.x_rows = m; c.f32 = !xbf; c.w_pitch = tc.pitch; c.precise = tc.relaid || m < kMoeBf16Rows;
+        c.x = xg; c.x_rows = m; c.f32 = !xbf; c.w_pitch = tc.pitch; c.precise = tc.precise;
         c.y = y; c.ybf = ybf; c.k = k; c.n = n;
         c.num_slabs = num_experts; c.groups = table; c.group_tiles = tc.tiles; c.tile_rows = tc.tile_rows; c.row_map = perm;
         return launch_gemm(s, scheme, c, nullptr, 0);
