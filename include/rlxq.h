@@ -92,8 +92,9 @@ RLXQ_API int rlxq_packed_bytes(uint32_t scheme, uint64_t k, uint64_t n, uint64_t
  * (a few bytes per element of x), the partial output tiles of CTAs that share a row tile and
  * their counters: tens to hundreds of KiB (up to 4.9 MB while the option gemv_kernel is 4).  The tensor-core GEMM needs
  * none for most shapes; for few output tiles it asks for k slices of the result or two partial tiles per SM (tens of MB);
- * without them it runs whole tiles.  With f32 activations and m > 8 it needs their bf16 hi + lo parts (4 bytes a value), and
- * for rows that are no multiple of 16 bytes a copy of the weights on a padded pitch (256-byte aligned); without that
+ * without them it runs whole tiles.  With f32 activations and m > 8 it needs their bf16 hi + lo parts (4 bytes a value); for
+ * rows that are no multiple of 16 bytes a copy of the weights on a padded pitch, three parts of f32 activations and up to
+ * 192 MB of partial results (all 256-byte aligned); without that
  * workspace such a call runs the tiled generic kernel, some 40 times
  * slower.  The reference reserves k*n*4 bytes. */
 RLXQ_API int rlxq_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n,
