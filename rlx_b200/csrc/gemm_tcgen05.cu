@@ -137,6 +137,8 @@ template <bool PRECISE> struct GemmOut {
 };
 // An f32 weight is the sum of three bf16 values: the upper half of its bits, of what that leaves behind, and of what is
 // left then, all of it exact (one byte-permute per pair and part; a conversion instruction would pace the decoder).
+// Q4_0's weights (f16 scale times four bits: 15) are two such parts.
+constexpr uint32_t gemm_weight_parts(uint32_t scheme) { return scheme == RLXQ_Q4_0 ? 2u : 3u; }
 template <> struct GemmOut<true> {
     uint64_t f[32];
     __device__ __forceinline__ void put(int i, uint64_t pair) { f[i] = pair; }
@@ -808,7 +810,7 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
                 tc_fence_after();
                 if constexpr (PRECISE) {
 #pragma unroll
-                    for (uint32_t q = 0; q < 3; ++q) {
+                    for (uint32_t q = 0; q < gemm_weight_parts(SCHEME); ++q) {
                         uint32_t p[32];
                         v.part(p);
                         tmem_st32(tmem_a + lane_addr + A_COLS * st + 32 * q, p);
@@ -999,7 +1001,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                     // are below 2^-24 of the whole
                     if (PRECISE) {
 #pragma unroll
-                        for (uint32_t j = 0; j < 2 * kGemmBK / 16; ++j) tc_mma_ts(acc, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, 1u);
+                        for (uint32_t j = 0; j < (gemm_weight_parts(SCHEME) - 1) * (kGemmBK / 16); ++j) tc_mma_ts(acc, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, 1u);
                     }
                     for (uint32_t q = 1; q < P.xparts; ++q) {
                         const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
@@ -1487,7 +1489,7 @@ static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t product
 static bool gemm_pair_fits(uint32_t n, bool precise) { return n % 256 == 0 && !precise; }
 static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise, bool can_split) {
     const uint64_t sms = (uint64_t)sm_count(), wt = (n + kGemmTileW - 1) / kGemmTileW, groups = (k + 255) / 256, blocks = 4 * groups;
-    const uint32_t products = (precise ? 3 : 1) * (f32 ? 2 : 1);
+    const uint32_t products = !precise ? (f32 ? 2 : 1) : gemm_weight_parts(scheme) + (f32 ? 3 : 0);
     const uint32_t most = gemm_most_rows(scheme, f32, precise);
     const int64_t fx = options().gemm_tile_x.load(), fs = can_split ? options().gemm_streamk.load() : 1, fp = options().gemm_pair.load();
     const GemmShape pair{256, (m + 255) / 256, 1, false, true};
