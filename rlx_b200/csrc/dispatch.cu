@@ -31,11 +31,6 @@ static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_
         if (p.halves && chunk > 2048) chunk = 2048;
         if (chunk > m) chunk = m;
     }
-    // PRECISE: a slice of the result for each 1024 columns, 192 MiB of them at once (but no fewer than 192 rows)
-    if (p.relaid) {
-        const uint64_t rows = (192ull << 20) / (4ull * n * ((k + 1023) / 1024)) / 192 * 192;
-        if (chunk > rows) chunk = rows < 192 ? (m < 192 ? m : 192) : rows;
-    }
     p.chunk = (uint32_t)chunk;
     p.off_w = xbf ? 0 : al((size_t)gemm_x_parts(true, p.relaid) * chunk * k * 2);
     p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;

@@ -526,6 +526,7 @@ struct GemmParams {
     // rows behind them; a stage carries both boxes and both are multiplied by the same decoded weights into the same
     // accumulator, so a weight is decoded once for the two halves.
     uint32_t lo_row, xparts;
+    uint32_t main_run;     // PRECISE: k blocks the main accumulator takes at a time (gemm_precise_epilogue): 1, 2 or 4
     uint32_t nstages, nraw;               // depth of the operand ring (B in shared memory, A in tensor memory) and of the raw ring
     uint32_t b_bytes;                     // bytes of a B stage: tx * 128, twice that with lo_row
     uint32_t w_late;       // the weights are written by a kernel in front (re-laid rows): read them after the dependency wait
@@ -798,7 +799,7 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
             // off the free -> store -> MMA chain.
             const uint32_t s0 = s, ph0 = fph;
             s += 4;
-            if (s >= NS) { s -= NS; fph ^= 1u; }
+            while (s >= NS) { s -= NS; fph ^= 1u; }
             auto stage_of = [&](uint32_t sub, uint32_t& st, uint32_t& sph) {
                 st = s0 + sub;
                 sph = ph0;
@@ -869,6 +870,121 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
 // activations come as three parts as well (GemmOut; split_hi_lo_kernel).  It serves the shapes whose other kernel multiplies
 // f32 weights and activations: three products for bf16 activations, six for f32 ones, where the formats' own path takes one
 // and two.
+//
+// The tensor core truncates where f32 arithmetic rounds, every time it adds to an accumulator, so a long accumulation loses
+// a multiple of f32's error (6.8e-6 of a result after 1024 columns of six products in one accumulator, 5.7e-5 after 8192; the
+// general kernel, which multiplied these shapes before, 3.3e-7 over 11008).  Hence two accumulators of P.tx columns.  The main
+// one takes the leading parts' product of main_run k blocks; the epilogue warps add it, rounding, to sums in registers, while
+// the other products run.  Those are 2^-8 of the whole and smaller: they pile up in the second accumulator.  Every kGemmRun
+// blocks it joins the sums, and these move on to totals in shared memory, so that no chain of additions is long.  Error
+// against 64 bits, general kernel and this one: k = 256 8.0e-8 and 7.8e-8, 2816 1.8e-7 and 1.4e-7, 11008 3.3e-7 and 2.3e-7.
+// 300 x 11008 x 4096 Q6_K f32 4787 us (general kernel) and 226 us; with long accumulations 218 us.
+constexpr uint32_t kGemmRun = 16;
+// Activation rows of a PRECISE tile: what the epilogue threads have registers for (Q3_K's block is larger: 96 a thread) and
+// shared memory has room for totals beside three operand stages and two raw boxes (Q8_K's are the largest).
+constexpr uint32_t gemm_precise_rows(uint32_t scheme) { return scheme == RLXQ_Q3_K || scheme == RLXQ_Q8_K ? 64u : 96u; }
+
+// Blocks between two emptyings: a block costs 1.4e-8 of a result for each of its four truncated additions (5.6e-8, 1.1e-7 and
+// 2.2e-7 for runs of 1, 2 and 4), and f32 arithmetic in the general kernel, which is what the result is held against, 8e-8
+// at k = 256, 1.6e-7 at 2304, 2.9e-7 at 8192 and 3.3e-7 at 11008.
+static uint32_t gemm_main_run(uint32_t k) { return k >= 9216 ? 4u : k >= 2304 ? 2u : 1u; }
+
+// TX = P.tx: no branch between the additions of a block, which are on the chain from one block's product to the next.
+template <uint32_t SCHEME, uint32_t TX>
+__device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmBars* bars, float* total, uint32_t tmem_d,
+                                                      uint32_t xtiles, uint32_t warp, uint32_t lane) {
+    const uint32_t quarter = warp & 3u, row = quarter * 32 + lane, epi_tid = (warp - (4 + 4 * GemmRaw<SCHEME>::GROUPS)) * 32 + lane;
+    const uint32_t main_d = tmem_d + ((quarter * 32) << 16), cross_d = main_d + TX;
+    uint32_t mph = 0, cph = 0;
+    uint32_t cur, lim;
+    gemm_seg_init(P, xtiles, cur, lim);
+    GemmSeg sg;
+    while (gemm_seg_next(P, cur, lim, sg)) {
+        const GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
+        const uint32_t rows = tr.xlim - tr.xrow0, blocks = 4 * (sg.g1 - sg.g0);
+        auto wait_for = [&](uint32_t d, uint32_t& ph) -> bool {
+            if (!mbar_wait(smem_u32(&bars->d_full[d]), ph)) {
+                atomicExch(P.err, 17);
+                *reinterpret_cast<volatile uint32_t*>(&bars->abort_flag) = 1u;
+                return false;
+            }
+            ph ^= 1u;
+            tc_fence_after();
+            return true;
+        };
+        auto release = [&](uint32_t d) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->d_free[d]));
+        };
+        bool ok = true;
+#pragma unroll 1
+        for (uint32_t k0 = 0; ok && k0 < blocks; k0 += kGemmRun) {
+            uint64_t sum[TX / 2];                            // pairs of activation rows
+#pragma unroll
+            for (uint32_t j = 0; j < TX / 2; ++j) sum[j] = 0ull;
+            auto add_accumulator = [&](uint32_t acc) {
+#pragma unroll
+                for (uint32_t c = 0; c < TX / 16; ++c) {
+                    uint32_t v[16];
+                    tmem_ld16(acc + 16 * c, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j) sum[8 * c + j] = add_f32x2(sum[8 * c + j], f32x2(v[2 * j], v[2 * j + 1]));
+                }
+            };
+            const uint32_t k1 = min(blocks, k0 + kGemmRun);
+#pragma unroll 1
+            for (uint32_t kb = k0; kb < k1; kb += P.main_run) {
+                if (!(ok = wait_for(0, mph))) break;
+                add_accumulator(main_d);
+                release(0);
+            }
+            if (!ok || !(ok = wait_for(1, cph))) break;
+            add_accumulator(cross_d);
+            release(1);
+            // totals [activation row][weight row]: a thread's own column of them, sixteen loads before the first store
+#pragma unroll
+            for (uint32_t c = 0; c < TX / 16; ++c) {
+                float* t = total + 16 * c * kGemmTileW + row;
+                float old[16];
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j) old[j] = k0 ? t[j * kGemmTileW] : 0.f;
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    uint32_t lo, hi;
+                    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(sum[8 * c + j]));
+                    t[2 * j * kGemmTileW] = old[2 * j] + __uint_as_float(lo);
+                    t[(2 * j + 1) * kGemmTileW] = old[2 * j + 1] + __uint_as_float(hi);
+                }
+            }
+        }
+        // the four warps leave together: they share the barriers
+        if (epilogue_any(!ok || *reinterpret_cast<volatile uint32_t*>(&bars->abort_flag))) break;
+        uint8_t* const out = static_cast<uint8_t*>(P.y) + sg.slice * P.slice_elems * 4;
+        const uint32_t n0 = tr.wt * kGemmTileW;
+        const uint32_t ps = !P.y_vec ? 7u : P.y_bf16 ? 4u : 5u;      // a row of the tile is 2^ps pieces of 16 bytes, or values
+#pragma unroll 4
+        for (uint32_t p = epi_tid; p < rows << ps; p += 128) {
+            const uint32_t j = p >> ps, c = (p & ((1u << ps) - 1u)) << (7u - ps), ni = n0 + c, mi = tr.xrow0 + j;
+            if (ni >= P.n) continue;
+            const size_t o = (size_t)(P.row_map ? __ldg(&P.row_map[mi]) : mi) * P.n + ni;
+            const float* t = total + j * kGemmTileW + c;
+            if (!P.y_vec) {
+                if (P.y_bf16) reinterpret_cast<uint16_t*>(out)[o] = (uint16_t)bf16x2_of(f32x2(__float_as_uint(*t), 0u));
+                else reinterpret_cast<float*>(out)[o] = *t;
+            } else if (P.y_bf16) {
+                const uint4 a = *reinterpret_cast<const uint4*>(t), b = *reinterpret_cast<const uint4*>(t + 4);
+                *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(out) + o) =
+                    make_uint4(bf16x2_of(f32x2(a.x, a.y)), bf16x2_of(f32x2(a.z, a.w)), bf16x2_of(f32x2(b.x, b.y)), bf16x2_of(f32x2(b.z, b.w)));
+            } else {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + o) = *reinterpret_cast<const float4*>(t);
+            }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");       // the totals have been read: the next tile's may be written
+    }
+}
+
 template <uint32_t SCHEME, bool PRECISE>
 __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
@@ -905,7 +1021,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
         bars->abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {               // the whole warp allocates all 512 columns: 256 of accumulators, 256 of weight stages
+    if (warp == 1) {               // the whole warp allocates all 512 columns: 256 (PRECISE: 2 tx) of accumulators, then weight stages
         tmem_alloc(smem_u32(&bars->tmem_base), 512);
         tmem_relinquish();
     }
@@ -913,10 +1029,9 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
-    const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + (PRECISE ? 128 : 256);
-    // up to 128 activation rows there are two accumulators: a tile's epilogue runs under the next tile's MMAs (PRECISE, whose
-    // weight stages take 384 columns: one accumulator of 128)
-    const uint32_t nacc = !PRECISE && P.tx <= 128 ? 2u : 1u;
+    const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + (PRECISE ? 2 * P.tx : 256);
+    // up to 128 activation rows there are two accumulators: a tile's epilogue runs under the next tile's MMAs
+    const uint32_t nacc = P.tx <= 128 ? 2u : 1u;
     auto give_up = [&](int code) {
         atomicExch(P.err, code);
         *abort_flag = 1u;
@@ -974,17 +1089,20 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
         // ---------------- MMA issuer ----------------
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((P.tx >> 3) << 17) | ((kGemmTileW >> 4) << 24);
-            uint32_t s = 0, ph = 0, d = 0, dph = 1;   // dph: parity to wait for on d_free (1 passes the first time)
+            uint32_t s = 0, ph = 0, d = 0, dph = 1, cph = 1;   // dph, cph: parities to wait for on d_free (1 passes the first time)
             uint32_t cur, lim;
             gemm_seg_init(P, xtiles, cur, lim);
             GemmSeg sg;
             bool ok = true;
             while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
-                if (!mbar_wait(smem_u32(&bars->d_free[d]), dph)) { give_up(13); break; }
-                tc_fence_after();
-                const uint32_t acc = tmem_d + 128u * d;
+                const uint32_t blocks = 4 * (sg.g1 - sg.g0);
+                if (!PRECISE) {
+                    if (!mbar_wait(smem_u32(&bars->d_free[d]), dph)) { give_up(13); break; }
+                    tc_fence_after();
+                }
+                const uint32_t acc = tmem_d + (PRECISE ? 0u : 128u * d);
                 uint32_t rb = mbar_test(smem_u32(&bars->b_full[s]), ph), ra = mbar_test(smem_u32(&bars->a_full[s]), ph);
-                for (uint32_t kb = 0; kb < 4 * (sg.g1 - sg.g0); ++kb) {    // the first MMA of a segment overwrites the accumulator
+                for (uint32_t kb = 0; kb < blocks; ++kb) {    // the first MMA of a segment overwrites the accumulator
                     if ((!rb && (*abort_flag || !mbar_wait(smem_u32(&bars->b_full[s]), ph))) ||
                         (!ra && (*abort_flag || !mbar_wait(smem_u32(&bars->a_full[s]), ph)))) { give_up(14); ok = false; break; }
                     tc_fence_after();
@@ -994,22 +1112,46 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                     ra = mbar_test(smem_u32(&bars->a_full[sn]), phn);
                     const uint64_t bdesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES));
                     const uint32_t a = tmem_a + A_COLS * s;
+                    if constexpr (PRECISE) {
+                        // weight part 0 by activation part 0, main_run blocks of them in the main accumulator
+                        const uint32_t in_run = kb & (P.main_run - 1u);
+                        if (in_run == 0) {
+                            if (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[0]), dph)) { give_up(13); ok = false; break; }
+                            dph ^= 1u;
+                            tc_fence_after();
+                        }
 #pragma unroll
-                    for (uint32_t j = 0; j < kGemmBK / 16; ++j)
-                        tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, (kb | j) ? 1u : 0u);
-                    // PRECISE: weight parts 0..2 by activation part 0, 0..1 by part 1, 0 by part 2; the three products left out
-                    // are below 2^-24 of the whole
-                    if (PRECISE) {
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, in_run | j ? 1u : 0u);
+                        if (in_run == P.main_run - 1u || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[0]));
+                        // parts 1, 2 by part 0, 0..1 by part 1, 0 by part 2; the three products left out are below 2^-24 of the whole
+                        const uint32_t cross = acc + P.tx;
+                        const bool fresh = kb % kGemmRun == 0;
+                        if (fresh) {
+                            if (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[1]), cph)) { give_up(13); ok = false; break; }
+                            cph ^= 1u;
+                            tc_fence_after();
+                        }
 #pragma unroll
-                        for (uint32_t j = 0; j < (gemm_weight_parts(SCHEME) - 1) * (kGemmBK / 16); ++j) tc_mma_ts(acc, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, 1u);
-                    }
-                    for (uint32_t q = 1; q < P.xparts; ++q) {
-                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
+                        for (uint32_t j = 0; j < (gemm_weight_parts(SCHEME) - 1) * (kGemmBK / 16); ++j)
+                            tc_mma_ts(cross, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, fresh && j == 0 ? 0u : 1u);
+                        for (uint32_t q = 1; q < P.xparts; ++q) {
+                            const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
 #pragma unroll
-                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
-                        if (PRECISE && q == 1) {
+                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(cross, a + 8 * j, ldesc + 2 * j, idesc, 1u);
+                            if (q == 1) {
 #pragma unroll
-                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 32 + 8 * j, ldesc + 2 * j, idesc, 1u);
+                                for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(cross, a + 32 + 8 * j, ldesc + 2 * j, idesc, 1u);
+                            }
+                        }
+                        if (kb % kGemmRun == kGemmRun - 1 || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[1]));
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j)
+                            tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, (kb | j) ? 1u : 0u);
+                        for (uint32_t q = 1; q < P.xparts; ++q) {
+                            const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
+#pragma unroll
+                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
                         }
                     }
                     tc_commit(smem_u32(&bars->stage_free[s]));     // frees the B stage and the A columns when the MMAs retire
@@ -1017,8 +1159,10 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                     ph = phn;
                 }
                 if (!ok) break;
-                tc_commit(smem_u32(&bars->d_full[d]));
-                if (++d == nacc) { d = 0; dph ^= 1u; }
+                if (!PRECISE) {
+                    tc_commit(smem_u32(&bars->d_full[d]));
+                    if (++d == nacc) { d = 0; dph ^= 1u; }
+                }
             }
         }
     } else if (warp >= 4 && warp < 4 + 4 * kGemmDecodeGroups) {
@@ -1027,7 +1171,16 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
         if (ONE || warp < 8) gemm_decode_role<SCHEME, PRECISE, 0>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
         else gemm_decode_role<SCHEME, PRECISE, 1>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
         tmem_st_wait();                      // (after a timeout a store may still be on its way)
-    } else if (warp >= 4 + 4 * kGemmDecodeGroups) {
+    } else if (PRECISE && warp >= 4 + 4 * kGemmDecodeGroups) {
+        // ---------------- epilogue: accumulators -> sums in registers -> totals in shared memory -> y ----------------
+        griddep_wait();
+        if constexpr (PRECISE) {
+            float* total = reinterpret_cast<float*>(epi_stage);
+            if (P.tx == 32) gemm_precise_epilogue<SCHEME, 32>(P, bars, total, tmem_d, xtiles, warp, lane);
+            else if (P.tx == 64) gemm_precise_epilogue<SCHEME, 64>(P, bars, total, tmem_d, xtiles, warp, lane);
+            else if constexpr (gemm_precise_rows(SCHEME) == 96) gemm_precise_epilogue<SCHEME, 96>(P, bars, total, tmem_d, xtiles, warp, lane);
+        }
+    } else if (!PRECISE && warp >= 4 + 4 * kGemmDecodeGroups) {
         // ---------------- epilogue: accumulator -> y (or -> a partial tile, completed by the last contributor) ----------------
         const uint32_t quarter = warp & 3u;
         const uint32_t lane_addr = (quarter * 32) << 16;
@@ -1459,14 +1612,13 @@ uint64_t gemm_relaid_pitch(uint32_t scheme, uint32_t k) {
 
 // Parts of an activation value: bf16 ones are one, f32 ones hi and lo, or all 24 bits beside PRECISE weights.
 uint32_t gemm_x_parts(bool f32, bool precise) { return !f32 ? 1u : precise ? 3u : 2u; }
-// The most activation rows of a tile: four operand stages and two raw boxes have to fit in shared memory (three parts of 96
-// rows beside all but the 8-bit formats' boxes), accumulators and weight stages in tensor memory.
+// The most activation rows of a tile: four operand stages (PRECISE: three) and two raw boxes have to fit in shared memory,
+// accumulators and weight stages in tensor memory.
 uint32_t gemm_most_rows(uint32_t scheme, bool f32, bool precise) {
     if (!precise) return f32 ? 128u : 256u;
-    return !f32 ? 128u : scheme == RLXQ_Q8_0 || scheme == RLXQ_Q8_K ? 64u : 96u;
+    return gemm_precise_rows(scheme);
 }
 
-constexpr uint32_t kGemmPreciseRun = 1024;
 struct GemmShape { uint32_t tx, xtiles, slices; bool streamk, pair; };
 
 // Activation rows per tile, work split and kernel for a shape, by estimated time in cycles.  A 64-wide k block of a tile
@@ -1475,14 +1627,19 @@ struct GemmShape { uint32_t tx, xtiles, slices; bool streamk, pair; };
 // narrow tile, and rows are split evenly over the fewest tiles that leave no SM idle.  The constants are fits to 45 shapes
 // (five formats, 16 to 1526 rows, k 2048 to 14336), each timed at every tile width, split and kernel: the choice made here
 // takes 1 % longer than the best one in the geometric mean, up to 10 % at worst.
+// PRECISE: the decoders of three parts and the emptying of the accumulators, measured with one tile on every SM.
 static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t products, bool precise, bool pair) {
+    if (precise) {
+        const uint32_t base = scheme == RLXQ_Q4_0 ? 1150 : scheme == RLXQ_Q8_0 ? 1900 : scheme == RLXQ_Q3_K ? 3000 : scheme == RLXQ_Q6_K ? 1580 :
+                              scheme == RLXQ_Q4_K || scheme == RLXQ_Q5_K ? 1700 : 2750;
+        return base + (products > 3 ? 7 : 4) * tx;
+    }
     const bool heavy = scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K;
     if (pair) return heavy && products == 1 ? 925 : 750 * products;        // 256 activation rows, both CTAs at once
-    uint32_t mma = (precise && tx < 112 ? 228 : 2 * tx) * products + 265 + (products > 1 ? 65 : 0);   // an MMA takes 57 cycles at least
+    uint32_t mma = 2 * tx * products + 265 + (products > 1 ? 65 : 0);
     if (products == 2 && tx >= 96 && mma < 800) mma = 800;
     if (heavy) mma += 90;
     uint32_t dec = scheme == RLXQ_Q3_K ? 1130 : heavy ? 740 : scheme == RLXQ_Q8_0 || scheme == RLXQ_Q4_0 || scheme == RLXQ_Q4_K ? 570 : 620;
-    if (precise) dec += 500;
     return mma > dec ? mma : dec;
 }
 // Two CTAs per MMA; PRECISE weights are not built in that form.
@@ -1501,10 +1658,6 @@ static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
         const uint64_t ptiles = (uint64_t)(n / 256) * pair.xtiles, pairs = sms / 2;
         take((ptiles + pairs - 1) / pairs * blocks * gemm_block_cycles(scheme, 256, products, precise, true) + 24 * 256, pair);
     }
-    // The tensor core truncates where f32 arithmetic rounds, every time it adds to an accumulator: over the 4000 additions of
-    // k = 11008 and six products that is 4e-5 of a result.  PRECISE tiles therefore never run further than kGemmPreciseRun
-    // columns; the kernel behind adds the slices, rounding.
-    const uint64_t runs = precise && can_split ? (groups + kGemmPreciseRun / 256 - 1) / (kGemmPreciseRun / 256) : 1;
     const uint32_t least_tiles = (m + most - 1) / most;
     for (uint32_t xt = least_tiles; xt <= least_tiles + 8; ++xt) {
         uint32_t tx = ((m + xt - 1) / xt + 31) / 32 * 32;
@@ -1512,17 +1665,15 @@ static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
         const uint32_t tiles_x = (m + tx - 1) / tx;
         if (tiles_x != xt && !fx) continue;              // the same width as one tile fewer
         const uint64_t ntiles = wt * tiles_x, cyc = gemm_block_cycles(scheme, tx, products, precise, false);
-        const uint64_t epi = 24 * tx;                    // the last tile's epilogue, and with one accumulator every tile's
-        if (runs > 1) {
-            const uint64_t fit = sms / ntiles, sl = std::max(runs, std::min(groups, fit));
-            take((ntiles * sl + sms - 1) / sms * (((groups + sl - 1) / sl * 4) * cyc + epi) + 3200 + sl * m * n / 600, GemmShape{tx, tiles_x, (uint32_t)sl, false, false});
-            if (fx) break;
-            continue;
-        }
-        if (fs != 2) take((ntiles + sms - 1) / sms * (blocks * cyc + (tx > 128 ? epi : 0)) + epi, GemmShape{tx, tiles_x, 1, false, false});
+        const uint64_t epi = (precise ? 100 : 24) * tx;  // the last tile's epilogue, and with one accumulator every tile's
+        if (fs != 2 || precise) take((ntiles + sms - 1) / sms * (blocks * cyc + (tx > 128 || precise ? epi : 0)) + epi, GemmShape{tx, tiles_x, 1, false, false});
         // k split over the SMs (stream-K): every SM gets the same blocks, and exchanges up to two parts of 128 x tx values
-        if (fs != 1 && (fs == 2 || ntiles % sms))
+        // (PRECISE sums are in registers by then, with no code to exchange them: whole tiles and slices only)
+        if (!precise && fs != 1 && (fs == 2 || ntiles % sms))
             take((ntiles * blocks + sms - 1) / sms * cyc + epi + 6000 + 200 * tx, GemmShape{tx, tiles_x, 1, true, false});
+        // PRECISE: as many slices as make the last wave a full one
+        for (uint64_t sl = 2; precise && fs == 0 && sl <= 8 && 4 * sl <= groups; ++sl)
+            take((ntiles * sl + sms - 1) / sms * ((groups + sl - 1) / sl * 4 * cyc + epi) + 3200 + sl * m * n / 600, GemmShape{tx, tiles_x, (uint32_t)sl, false, false});
         // few tiles: every SM takes a slice of some tile's k, and a kernel behind this one adds the slices
         if (fs == 0 && 2 * ntiles <= sms) {
             const uint64_t fit = sms / ntiles, sl = groups < fit ? groups : fit;
@@ -1565,6 +1716,7 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     P.tx = sh.tx;
     P.lo_row = c.f32 ? c.x_rows : 0u;
     P.xparts = gemm_x_parts(c.f32, PRECISE);
+    P.main_run = gemm_main_run(c.k);
     int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * P.xparts, c.k, P.tx);
     if (rc) return rc;
     rc = encode_weight_map(&P.wmap, c.w, (uint64_t)c.n * c.num_slabs, c.w_pitch ? c.w_pitch : (uint64_t)c.k / g.elems * g.bytes,
@@ -1588,9 +1740,10 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     // as many operand stages as tensor memory and shared memory hold beside two raw boxes, then raw boxes
     P.b_bytes = P.tx * kGemmBK * 2 * P.xparts;
     const uint32_t smem = 227 * 1024;   // all of it: one CTA per SM, so that none waits for another's tensor memory
-    const uint32_t budget = smem - (1024 + sizeof(GemmBars) + 64 + kGemmEpiStage);
-    P.nstages = std::min<uint32_t>(PRECISE ? 4 : kGemmMaxStages, (budget - kGemmRawStages * RAW_STRIDE) / P.b_bytes);
-    if (P.nstages < 4) return fail(RLXQ_E_LIMIT, "GEMM tile of %u activation rows too large", P.tx);   // a weight group is four
+    const uint32_t budget = smem - (1024 + sizeof(GemmBars) + 64 + (PRECISE ? P.tx * kGemmTileW * 4 : kGemmEpiStage));
+    P.nstages = std::min<uint32_t>(PRECISE ? std::min(4u, (512u - 2u * P.tx) / 96u) : kGemmMaxStages, (budget - kGemmRawStages * RAW_STRIDE) / P.b_bytes);
+    // (a decode group's parts may lie up to three stages apart, gemm_decode_role: no ring below that)
+    if (P.nstages < (PRECISE ? 3u : 4u)) return fail(RLXQ_E_LIMIT, "GEMM tile of %u activation rows too large", P.tx);
     P.nraw = std::min<uint32_t>(kGemmMaxRaw, (budget - P.nstages * P.b_bytes) / RAW_STRIDE);
     static std::atomic<uint32_t> attr_set[64];
     int dev = 0;

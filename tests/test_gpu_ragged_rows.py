@@ -85,6 +85,55 @@ def test_gemm_on_relaid_rows(sch, m, k, n, x_bf16):
     assert_within_tolerance(y, ref, _bound(s, w, x, k, n), tol=2e-5, what=f"relaid {sch} {m}x{k}x{n}")
 
 
+def _error(y, ref):
+    return np.linalg.norm(y.astype(np.float64) - ref) / np.linalg.norm(ref)
+
+
+# every tile width, runs of 1, 2 and 4 blocks, one block, a ragged last run, slices, tiles of several kinds per SM
+@pytest.mark.parametrize("sch,m,k,n,x_bf16", [("q8_0", 9, 96, 130, False), ("q6_k", 33, 256, 200, True), ("q6_k", 96, 1280, 520, False),
+                                              ("q8_0", 65, 2336, 264, False), ("q4_0", 100, 4128, 300, True), ("q6_k", 300, 11008, 1024, False),
+                                              ("q6_k", 40, 16128, 128, True), ("q3_k", 70, 2304, 130, False), ("q8_k", 70, 768, 130, False),
+                                              ("q5_0", 200, 544, 4000, True), ("q2_k", 20, 9472, 136, False)])
+def test_gemm_on_relaid_rows_is_as_exact_as_the_general_kernel(sch, m, k, n, x_bf16):
+    """These shapes belonged to the general kernel, which multiplies f32 weights and activations in f32: measured against 64
+    bits, the tensor-core GEMM may be no further off (2 % for a result's own rounding, 6e-8 on both sides)."""
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, 900 + m)
+    wd = torch.from_numpy(w).cuda()
+    ref = x.astype(np.float64) @ O.dequant(s, w, k * n).reshape(n, k).astype(np.float64).T
+    y = R.matmul(xd, wd, s, n).cpu().numpy()
+    R.device_status()
+    R.set_option("gemm_kernel", 1)
+    try:
+        general = R.matmul(xd, wd, s, n).cpu().numpy()
+    finally:
+        R.set_option("gemm_kernel", 0)
+    assert not np.array_equal(y, general)                      # they are different kernels
+    assert _error(y, ref) <= 1.02 * _error(general, ref), (_error(y, ref), _error(general, ref))
+
+
+@pytest.mark.parametrize("sch,m,k,n,E,x_bf16", [("q6_k", 64, 7936, 256, 3, False), ("q5_0", 20, 4096, 300, 3, False), ("q3_k", 12, 2048, 136, 4, True),
+                                                ("q8_0", 400, 2080, 200, 2, True)])
+def test_expert_gemm_on_f32_weights_is_as_exact_as_the_general_kernel(sch, m, k, n, E, x_bf16):
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n * E, x_bf16, 950 + m)
+    idx = np.random.default_rng(m).integers(0, E, m)
+    args = (xd, torch.from_numpy(w).cuda(), torch.from_numpy(idx.astype(np.float32)).cuda(), s, n, E)
+    W = O.dequant(s, w, k * n * E).reshape(E, n, k).astype(np.float64)
+    ref = np.stack([W[e] @ x[i].astype(np.float64) for i, e in enumerate(idx)])
+    y = R.grouped_matmul(*args).cpu().numpy()
+    R.device_status()
+    R.set_option("gemm_kernel", 1)
+    try:
+        general = R.grouped_matmul(*args).cpu().numpy()
+    finally:
+        R.set_option("gemm_kernel", 0)
+    assert not np.array_equal(y, general)
+    assert _error(y, ref) <= 1.02 * _error(general, ref), (_error(y, ref), _error(general, ref))
+
+
 @pytest.mark.parametrize("sch", ["q4_0", "q8_0", "q4_k", "q5_k", "q6_k"])
 @pytest.mark.parametrize("m,n,x_bf16", [(32, 128, True), (33, 200, False), (97, 2000, True), (224, 136, True), (257, 264, False)])
 def test_gemm_tile_widths_and_slices(sch, m, n, x_bf16):
