@@ -258,5 +258,10 @@ __device__ __forceinline__ uint32_t f32_to_bf16_bits(float f) {
     x += 0x7FFFu + lsb;
     return x >> 16;
 }
+// The leading bf16 part of f: rounded, but finite where f is (a value past the largest bf16 is cut off there).
+__device__ __forceinline__ uint32_t bf16_hi_bits(float f) {
+    const uint32_t h = f32_to_bf16_bits(f) & 0xFFFFu;
+    return (h & 0x7FFFu) == 0x7F80u && isfinite(f) ? __float_as_uint(f) >> 16 : h;
+}
 
 }  // namespace rlxq

@@ -60,7 +60,8 @@ int launch_copy_bytes(cudaStream_t stream, void* dst, const void* src, uint64_t 
 // f32 activations for the tensor-core GEMM, whose operands are bf16: x = hi + lo with hi = bf16(x) and
 // lo = bf16(x - hi), which leaves 2^-17 of x behind, or (parts = 3) x = hi + mid + lo, which leaves nothing.  Rows [row0,
 // row0 + rows) of x become rows [0, rows) (hi), [rows, 2 rows) and, if asked for, [2 rows, 3 rows) of `out`; the GEMM multiplies both by the same decoded weights.  One pass of 8 bytes a
-// value, a few microseconds; the GEMM behind it is resident meanwhile and fetches its first weights.
+// value, a few microseconds; the GEMM behind it is resident meanwhile and fetches its first weights.  Infinities and NaN are
+// hi alone; finite values past the largest bf16 are cut off there and not rounded, which would make them infinite.
 __global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restrict__ x, uint16_t* __restrict__ out,
                                                           uint64_t rows, uint64_t k, uint32_t parts) {
     const uint64_t total = rows * k / 4, stride = (uint64_t)gridDim.x * blockDim.x;     // k % 4 == 0
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restric
         uint16_t h[4], l[4], e[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            h[j] = (uint16_t)f32_to_bf16_bits(f[j]);
+            h[j] = (uint16_t)bf16_hi_bits(f[j]);
             const float rest = isfinite(f[j]) ? f[j] - __uint_as_float((uint32_t)h[j] << 16) : 0.f;     // exact
             l[j] = (uint16_t)f32_to_bf16_bits(rest);
             e[j] = (uint16_t)f32_to_bf16_bits(rest - __uint_as_float((uint32_t)l[j] << 16));

@@ -923,12 +923,18 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
             uint64_t sum[TX / 2];                            // pairs of activation rows
 #pragma unroll
             for (uint32_t j = 0; j < TX / 2; ++j) sum[j] = 0ull;
-            auto add_accumulator = [&](uint32_t acc) {
+            auto add_accumulator = [&](uint32_t acc, bool cross) {
 #pragma unroll
                 for (uint32_t c = 0; c < TX / 16; ++c) {
                     uint32_t v[16];
                     tmem_ld16(acc + 16 * c, v);
                     tmem_ld_wait();
+                    // An infinite activation times a lower weight part that is zero is a NaN in there.  The main accumulator then
+                    // has the infinity (or the NaN) that the product is: its weight part is zero only where the weight is.
+                    if (cross) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 16; ++j) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), -3.402823466e38f));
+                    }
 #pragma unroll
                     for (uint32_t j = 0; j < 8; ++j) sum[8 * c + j] = add_f32x2(sum[8 * c + j], f32x2(v[2 * j], v[2 * j + 1]));
                 }
@@ -937,11 +943,11 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
 #pragma unroll 1
             for (uint32_t kb = k0; kb < k1; kb += P.main_run) {
                 if (!(ok = wait_for(0, mph))) break;
-                add_accumulator(main_d);
+                add_accumulator(main_d, false);
                 release(0);
             }
             if (!ok || !(ok = wait_for(1, cph))) break;
-            add_accumulator(cross_d);
+            add_accumulator(cross_d, true);
             release(1);
             // totals [activation row][weight row]: a thread's own column of them, sixteen loads before the first store
 #pragma unroll

@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict_
             uint32_t h[4], l[4], e[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                h[q] = f32_to_bf16_bits(f[q]) & 0xFFFFu;
+                h[q] = bf16_hi_bits(f[q]);
                 const float rest = isfinite(f[q]) ? f[q] - __uint_as_float(h[q] << 16) : 0.f;
                 l[q] = f32_to_bf16_bits(rest) & 0xFFFFu;
                 e[q] = f32_to_bf16_bits(rest - __uint_as_float(l[q] << 16)) & 0xFFFFu;

@@ -113,6 +113,38 @@ def test_gemm_on_relaid_rows_is_as_exact_as_the_general_kernel(sch, m, k, n, x_b
     assert _error(y, ref) <= 1.02 * _error(general, ref), (_error(y, ref), _error(general, ref))
 
 
+@pytest.mark.parametrize("sch,k", [("q4_0", 544), ("q8_0", 2336), ("q6_k", 1280)])
+@pytest.mark.parametrize("x_bf16", [False, True])
+def test_gemm_on_relaid_rows_with_values_that_are_not_finite(sch, k, x_bf16):
+    """One infinite activation gives infinities of its weights' signs (NaN where the weight is zero), two of opposite signs or
+    a NaN give NaN, and the largest finite f32 activation stays finite: what f32 arithmetic makes of them."""
+    import torch
+    import rlx_b200 as R
+    m, n = 40, 130
+    s, w, x, _ = _inputs(sch, m, k, n, x_bf16, 77)
+    x[1, 5], x[7, k - 1], x[8, 300], x[9, 301], x[9, 17], x[10, 40] = np.inf, -np.inf, np.inf, np.inf, -np.inf, np.nan
+    x[11], x[12] = 0, 0
+    x[11, 200], x[12, 33] = (3.38e38, -3.38e38) if x_bf16 else (3.4e38, -3.4028234e38)
+    xd = torch.from_numpy(x).cuda()
+    if x_bf16:
+        xd = xd.to(torch.bfloat16)
+        x = xd.float().cpu().numpy()
+    if sch == "q4_0":                                          # (row 8: infinity times a block of zeros)
+        w.reshape(n, k // 32, 18)[:, 300 // 32, :2] = 0
+    W = O.dequant(s, w, k * n).reshape(n, k)
+    with np.errstate(invalid="ignore", over="ignore"):
+        ref = np.stack([np.einsum("k,nk->n", xr.astype(np.float64), W.astype(np.float64)) for xr in x])
+        ref = np.where(np.abs(ref) > np.finfo(np.float32).max, np.sign(ref) * np.inf, ref)
+    y = R.matmul(xd, torch.from_numpy(w).cuda(), s, n).cpu().numpy()
+    R.device_status()
+    assert np.array_equal(np.isnan(y), np.isnan(ref))
+    assert np.array_equal(y[np.isinf(ref)], ref[np.isinf(ref)]) and np.isinf(ref).any()
+    fin = np.isfinite(ref)
+    assert np.isfinite(y[fin]).all() and fin[11].any() and fin[12].any()
+    for i in (11, 12):                                         # a single product: rounded weight parts leave nothing of 2^-20
+        assert np.allclose(y[i][fin[i]], ref[i][fin[i]], rtol=1e-6, atol=0)
+
+
 @pytest.mark.parametrize("sch,m,k,n,E,x_bf16", [("q6_k", 64, 7936, 256, 3, False), ("q5_0", 20, 4096, 300, 3, False), ("q3_k", 12, 2048, 136, 4, True),
                                                 ("q8_0", 400, 2080, 200, 2, True)])
 def test_expert_gemm_on_f32_weights_is_as_exact_as_the_general_kernel(sch, m, k, n, E, x_bf16):
