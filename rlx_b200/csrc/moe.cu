@@ -31,6 +31,7 @@
 // every row is one launch of the streaming integer GEMV over the whole stack seen as an
 // [experts * n, k] matrix, with the slab picked on the device from expert_idx[i] (gemv_int.cu,
 // expert-indirect mode), so a routed expert's weights come through the TMA ring at GEMV speed.
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -287,19 +288,41 @@ static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
     return p;
 }
 
-static size_t grouped_ws(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, bool w_aligned,
-                         size_t* off_cursor, size_t* off_perm, MoeTcPlan* tc) {
+// How a call is run.  Asked by the call with the real pointers and by the workspace query with aligned ones, so that nobody
+// is asked for scratch that no kernel touches (the re-laid slabs of a large stack are hundreds of megabytes).
+enum class MoeRoute {
+    Rows,        // one expert-indirect launch of the integer GEMV per row
+    Stream,      // one launch of the f32 streaming GEMV for all rows (an id out of range leaves zeros there, too)
+    Gemm,        // the grouped tensor-core GEMM
+    General      // moe_grouped_kernel
+};
+struct MoePlan { MoeRoute route; size_t off_cursor, off_perm, sort_bytes, bytes; MoeTcPlan tc; };
+static MoePlan plan_moe(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, const void* x, const void* w) {
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-    size_t off = up(((size_t)E + 1) * 4);
-    if (off_cursor) *off_cursor = off;
-    off += up(((size_t)E + 1) * 4);
-    if (off_perm) *off_perm = off;
-    off += up((size_t)m * 4);
-    const MoeTcPlan p = plan_moe_tc(scheme, m, k, n, E, xbf, w_aligned, off);
-    if (tc) *tc = p;
-    if (p.ok) off = p.bytes;
-    const size_t gemv = m <= kMoeDecodeRows ? up(int_workspace_bytes(scheme, 1, k, n)) : 0;   // the decode path's scratch
-    return off > gemv ? off : gemv;
+    MoePlan p{};
+    p.off_cursor = up(((size_t)E + 1) * 4);
+    p.off_perm = 2 * p.off_cursor;
+    p.sort_bytes = p.bytes = p.off_perm + up((size_t)m * 4);      // (every route asks for this much)
+    const int64_t gemv = options().gemv_kernel.load();
+    if (m <= kMoeDecodeRows && gemv != 1 && ((size_t)k * (xbf ? 2 : 4)) % 16 == 0 && (uint64_t)n * E <= 0x7FFFFFFFull &&
+        int_expert_supported(scheme, k, n, w, x)) {
+        p.route = MoeRoute::Rows;
+        const size_t need = up(int_workspace_bytes(scheme, 1, k, n));
+        if (need > p.bytes) p.bytes = need;
+        return p;
+    }
+    if (gemv == 0 && options().gemm_kernel.load() == 0 && gemv_f32_supported(scheme, 1, k, x) && moe_rows_stream(m, k, n, E)) {
+        p.route = MoeRoute::Stream;
+        return p;
+    }
+    p.route = MoeRoute::General;
+    if (m <= kMoeDecodeRows && gemv == 1) return p;
+    p.tc = plan_moe_tc(scheme, m, k, n, E, xbf, !((uintptr_t)w & 15u), p.sort_bytes);
+    if (p.tc.ok) {
+        p.route = MoeRoute::Gemm;
+        p.bytes = p.tc.bytes;
+    }
+    return p;
 }
 
 }  // namespace rlxq
@@ -313,10 +336,10 @@ extern "C" int rlxq_grouped_workspace_bytes(uint32_t scheme, uint32_t m, uint32_
     if (!geometry(scheme, &g)) return fail(RLXQ_E_SCHEME, "unknown scheme %u", scheme);
     if (k == 0 || k % g.elems) return fail(RLXQ_E_SHAPE, "k=%u is not a positive multiple of the block size %u", k, g.elems);
     if (num_experts == 0 || num_experts > 8192) return fail(RLXQ_E_LIMIT, "num_experts=%u must be in [1, 8192]", num_experts);
-    // f32 activations gather twice the rows, bf16 ones may need another tile table
-    *bytes = grouped_ws(scheme, m, k, n, num_experts, false, true, nullptr, nullptr, nullptr);
-    const size_t bf = grouped_ws(scheme, m, k, n, num_experts, true, true, nullptr, nullptr, nullptr);
-    if (bf > *bytes) *bytes = bf;
+    // f32 activations gather two or three times the rows, bf16 ones may need another tile table
+    const void* aligned = (const void*)256;
+    *bytes = std::max(plan_moe(scheme, m, k, n, num_experts, false, aligned, aligned).bytes,
+                      plan_moe(scheme, m, k, n, num_experts, true, aligned, aligned).bytes);
     return RLXQ_OK;
 }
 
@@ -334,34 +357,26 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     if (((uintptr_t)x & 15u) || ((uintptr_t)workspace & 15u)) return fail(RLXQ_E_ALIGN, "x and workspace must be 16-byte aligned");
     if ((uintptr_t)w_blocks & 1u) return fail(RLXQ_E_ALIGN, "w_blocks must be 2-byte aligned");
     if ((uintptr_t)y & (y_dtype == RLXQ_BF16 ? 1u : 3u)) return fail(RLXQ_E_ALIGN, "y must be aligned to its element size");
-    size_t off_cursor = 0, off_perm = 0;
     const bool xbf = x_dtype == RLXQ_BF16, ybf = y_dtype == RLXQ_BF16;
     const uint8_t* wst = (const uint8_t*)w_blocks;
     const size_t xes = xbf ? 2 : 4, yes = ybf ? 2 : 4;
-    MoeTcPlan tc{};
-    size_t need = grouped_ws(scheme, m, k, n, num_experts, xbf, !((uintptr_t)wst & 15u), &off_cursor, &off_perm, &tc);
+    MoePlan plan = plan_moe(scheme, m, k, n, num_experts, xbf, x, wst);
     // the tensor-core path is taken when the workspace holds its arrays; a smaller one still runs the general kernel
-    if (tc.ok && (workspace_bytes < tc.bytes || ((uintptr_t)workspace & 255u) || (m <= kMoeDecodeRows && options().gemv_kernel.load() == 1))) {
-        tc.ok = false;
-        need = off_perm + ((size_t)m * 4 + 255) / 256 * 256;
-    }
-    if (workspace_bytes < need) return fail(RLXQ_E_WORKSPACE, "grouped matmul needs %zu workspace bytes, got %zu", need, workspace_bytes);
+    if (plan.route == MoeRoute::Gemm && (workspace_bytes < plan.bytes || ((uintptr_t)workspace & 255u))) plan.route = MoeRoute::General;
+    if (workspace_bytes < plan.sort_bytes)
+        return fail(RLXQ_E_WORKSPACE, "grouped matmul needs %zu workspace bytes, got %zu", plan.sort_bytes, workspace_bytes);
+    const MoeTcPlan& tc = plan.tc;
     cudaStream_t s = (cudaStream_t)stream;
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     uint32_t* offsets = reinterpret_cast<uint32_t*>(ws);
-    uint32_t* cursor = reinterpret_cast<uint32_t*>(ws + off_cursor);
-    uint32_t* perm = reinterpret_cast<uint32_t*>(ws + off_perm);
-    const bool decode = m <= kMoeDecodeRows && options().gemv_kernel.load() != 1 && ((size_t)k * xes) % 16 == 0 &&
-                        (uint64_t)n * num_experts <= 0x7FFFFFFFull && int_expert_supported(scheme, k, n, wst, x);
-    // a few rows that the integer GEMV does not take: one launch of the f32 streaming GEMV for all of them (an id out of
-    // range leaves zeros there, too)
-    if (!decode && options().gemv_kernel.load() == 0 && options().gemm_kernel.load() == 0 && gemv_f32_supported(scheme, 1, k, x) &&
-        moe_rows_stream(m, k, n, num_experts))
+    uint32_t* cursor = reinterpret_cast<uint32_t*>(ws + plan.off_cursor);
+    uint32_t* perm = reinterpret_cast<uint32_t*>(ws + plan.off_perm);
+    if (plan.route == MoeRoute::Stream)
         return launch_gemv_f32(s, scheme, x, xbf, wst, y, ybf, m, k, n, expert_idx, num_experts);
     // rows with an id of num_experts or more are in no group: their outputs are zero (the gather kernel and the decode kernel
     // see to it)
-    if (!decode && !tc.ok) RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * yes, s));
-    if (decode) {
+    if (plan.route == MoeRoute::General) RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * yes, s));
+    if (plan.route == MoeRoute::Rows) {
         for (uint32_t i = 0; i < m; ++i) {
             int rc = launch_gemv_int_expert(s, scheme, (const uint8_t*)x + (size_t)i * k * xes, xbf, wst,
                                             (uint8_t*)y + (size_t)i * n * yes, ybf, k, n, num_experts, expert_idx + i,
@@ -377,7 +392,7 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     rc = launch_pdl(moe_place_kernel, dim3((m + 255) / 256), dim3(256), 0, s, expert_idx, m, num_experts, cursor, perm);
     if (rc) return rc;
     count_launch();
-    if (tc.ok) {
+    if (plan.route == MoeRoute::Gemm) {
         uint16_t* xg = reinterpret_cast<uint16_t*>(ws + tc.off_xg);
         uint4* table = reinterpret_cast<uint4*>(ws + tc.off_table);
         rc = launch_pdl(moe_tiles_kernel, dim3(1), dim3(kMoeScanThreads), 0, s, (const uint32_t*)offsets, num_experts, table, tc.tile_rows);

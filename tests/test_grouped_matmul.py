@@ -64,6 +64,23 @@ def test_oracle_grouped_equals_per_row_matmul():
         assert np.array_equal(y[i], ref.ravel())
 
 
+def test_workspace_of_few_rows_holds_no_copy_of_the_stack():
+    """Rows that the integer or the f32 streaming GEMV takes need neither a re-laid stack nor gathered activations: their
+    scratch is the sort's arrays or the integer GEMV's, a few hundred KB, whatever the stack's size."""
+    import ctypes as C
+    from rlx_b200._lib import lib
+
+    def need(sch, m, k, n, E):
+        b = C.c_size_t()
+        assert lib.rlxq_grouped_workspace_bytes(O.SCHEMES[sch], m, k, n, E, C.byref(b)) == 0
+        return b.value
+    for sch, m, k, n, E in [("q6_k", 1, 1792, 8320, 16), ("q6_k", 1, 11008, 4096, 8), ("q6_k", 2, 5632, 14336, 16), ("q8_0", 8, 288, 64, 8),
+                            ("q6_k", 10, 768, 40, 9), ("q4_k", 2, 4096, 14336, 8), ("q5_k", 8, 1024, 4096, 32)]:
+        assert need(sch, m, k, n, E) <= 1 << 20, (sch, m, k, n, E, need(sch, m, k, n, E))
+    # rows of this length for the GEMM: the stack on a padded pitch
+    assert need("q6_k", 64, 1792, 320, 4) >= 320 * 4 * 7 * 210
+
+
 # ------------------------------------------------------------------ GPU
 def _gpu(x, w, idx, s, n, E, x_bf16=False, y_bf16=False):
     import torch
