@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <chrono>
 
+#include "arrival.h"
 #include "common.cuh"
 #include "decode.cuh"
 #include "kernels.h"
@@ -535,8 +536,8 @@ struct GemmParams {
     // units_r CTAs one more), so every SM gets the same work however many tiles there are; a tile cut
     // by range boundaries is completed by the last of its contributors to arrive (partial tiles in
     // `partial`, one slot per CTA and end of its range).  Arrivals are counted in `counters` under the call's tag
-    // ((tag << 32) | count; any other upper half reads as zero), so the words need no zeroing before the call; the
-    // last arrival clears its word for a replay of the same launch.
+    // (arrival.h), so the words need no zeroing before the call; the last arrival clears its word for a replay of the
+    // same launch.
     // slices > 1 (never with streamk): unit (tile, slice) covers an equal part of the tile's k groups and stores its
     // sums to slice `slice` of an f32 array of y's shape (y points at it, slice_elems apart); a kernel behind this one
     // adds the slices in order.
@@ -544,7 +545,7 @@ struct GemmParams {
     size_t slice_elems;
     float* partial;
     unsigned long long* counters;
-    uint32_t tag;
+    unsigned long long tag;
     // Grouped mode (MoE expert stacks; null = one dense matrix): W is a stack of [n, k] slabs and activation
     // tile xt is described by groups[1 + xt] = {first row in x, rows, expert, -}: the tile multiplies those rows by slab
     // `expert`.  groups[0].x is the number of tiles.  The table is written on the device by the kernels in front.  Never
@@ -605,11 +606,11 @@ __device__ __forceinline__ bool gemm_seg_next(const GemmParams& P, uint32_t& cur
 }
 // Counts one contributor in and returns how many came before it.  Only the first arrival finds another call's (or
 // anybody's) bits in the word and has to install the tag.
-__device__ __forceinline__ uint32_t gemm_arrive(unsigned long long* word, uint32_t tag) {
+__device__ __forceinline__ uint32_t gemm_arrive(unsigned long long* word, unsigned long long tag) {
     unsigned long long old = *reinterpret_cast<volatile unsigned long long*>(word);
     for (;;) {
-        if ((uint32_t)(old >> 32) == tag) return (uint32_t)atomicAdd(word, 1ull);
-        const unsigned long long prev = atomicCAS(word, old, ((unsigned long long)tag << 32) | 1ull);
+        if (arrival_count(old, tag)) return arrival_count(atomicAdd(word, 1ull), tag);
+        const unsigned long long prev = atomicCAS(word, old, arrival_word(tag, 1u));
         if (prev == old) return 0u;
         old = prev;
     }
@@ -1222,7 +1223,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (epi_tid == 0) {
                         const unsigned long long word = *reinterpret_cast<volatile unsigned long long*>(&P.counters[sg.tile]);
-                        (&bars->epi_prev)[nseg & 1u] = word == (((unsigned long long)P.tag << 32) | 1ull) ? 1u : 0u;
+                        (&bars->epi_prev)[nseg & 1u] = arrival_count(word, P.tag);
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (reinterpret_cast<volatile uint32_t*>(&bars->epi_prev)[nseg & 1u] == 1u) {
@@ -1706,10 +1707,10 @@ size_t gemm_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t
     return gemm_shape_bytes(gemm_choose(scheme, m, k, n, f32, precise, true), m, n);
 }
 
-// Odd 32-bit tags, a different one for each of the calls that may be in flight together.
-static uint32_t next_gemm_tag() {
-    static std::atomic<uint32_t> epoch{(uint32_t)std::chrono::steady_clock::now().time_since_epoch().count() * 0x9E3779B9u};
-    return (epoch.fetch_add(1) << 1) | 1u;
+// A different tag for each of the calls that may be in flight together; where they start differs from process to process.
+static unsigned long long next_gemm_tag() {
+    static std::atomic<unsigned long long> calls{(unsigned long long)std::chrono::steady_clock::now().time_since_epoch().count() * 0x9E3779B97F4A7C15ull};
+    return arrival_tag(calls.fetch_add(1));
 }
 
 template <uint32_t SCHEME, bool PRECISE>

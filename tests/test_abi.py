@@ -122,3 +122,38 @@ def test_workspace_bytes_are_modest():
     for s, m, k, n in ((6, 1, 4096, 11008), (6, 1, 11008, 4096), (6, 8, 11008, 4096), (0, 1, 28672, 8192)):
         ws = R.workspace_bytes(s, m, k, n)
         assert ws % 16 == 0 and ws < k * n * 4 // 100
+
+
+def test_arrival_words_take_no_stray_value_for_a_count(tmp_path):
+    """The words in which the GEMM's split tiles count their contributors lie in scratch full of other calls' f32 sums: a
+    word counts only when 48 bits agree with the call's tag, so one equal f32 (32 bits) is not enough."""
+    import shutil
+    import subprocess
+    src = tmp_path / "arrival.cpp"
+    src.write_text(r'''
+#include <stdio.h>
+#include <initializer_list>
+#include "arrival.h"
+using namespace rlxq;
+int main() {
+    int bad = 0;
+    for (unsigned long long n : {0ull, 1ull, 0x9E3779B97F4A7C15ull, ~0ull, 0x3F800000ull << 15}) {
+        const unsigned long long tag = arrival_tag(n);
+        bad += tag == 0 || tag == arrival_tag(n + 1) || (tag & ~kArrivalTagMask) != 0;
+        for (unsigned c : {1u, 2u, 148u, 65535u}) bad += arrival_count(arrival_word(tag, c), tag) != c;
+        bad += arrival_count(arrival_word(tag, 1) + 1, tag) != 2 || arrival_count(arrival_word(arrival_tag(n + 1), 1), tag) != 0;
+        bad += arrival_count(0, tag) != 0;
+        // the f32 in the upper half equals the tag's upper 32 bits, whatever value lies beside it
+        for (unsigned lo = 0; lo < 1u << 20; ++lo) {
+            const unsigned long long word = (tag >> 16 << 32) | (lo * 2654435761u);
+            bad += arrival_count(word, tag) != 0 && word >> 16 != tag;
+        }
+        for (int bit = 16; bit < 64; ++bit) bad += arrival_count(arrival_word(tag, 1) ^ (1ull << bit), tag) != 0;
+    }
+    printf("%d\n", bad);
+    return bad != 0;
+}
+''')
+    exe = tmp_path / "arrival"
+    subprocess.run([shutil.which("g++") or "g++", "-std=c++17", "-I", os.path.join(ROOT, "rlx_b200", "csrc"), str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], capture_output=True, text=True).stdout == "0\n"

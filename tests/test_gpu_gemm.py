@@ -110,6 +110,21 @@ def test_stream_k_split_matches_oracle_and_is_deterministic(sch, m, k, n, y_bf16
         assert_within_tolerance(a[rows], c[rows], bnd, tol=2 * _tol(k, sch), what="stream-K vs whole tiles")
 
 
+@pytest.mark.parametrize("fill", [0xFF, 0x3F, 0x00])
+def test_stream_k_split_in_scratch_that_holds_anything(fill):
+    import torch
+    s, m, k, n = O.Q4_K, 200, 4096, 1100
+    w, xb, _ = _case(s, m, k, n, seed=123)
+    R.set_option("gemm_streamk", 2)
+    wd, xd = torch.from_numpy(w).cuda(), torch.from_numpy(xb.view(np.int16)).cuda().view(torch.bfloat16)
+    ws = torch.empty(R.workspace_bytes(s, m, k, n, 1, 0), dtype=torch.uint8, device="cuda")
+    want = R.matmul(xd, wd, s, n)
+    for part in (ws.numel(), 0, 4096):                            # all of it, none (the call before left its parts), the counters
+        ws[:part] = fill
+        assert torch.equal(R.matmul(xd, wd, s, n, workspace=ws), want)
+    R.device_status()
+
+
 PAIR_SHAPES = [("q8_0", 256, 256, 256, False), ("q4_0", 300, 512, 512, True), ("q4_k", 1000, 2048, 1024, False),
                ("q5_k", 777, 1024, 2560, True), ("q6_k", 512, 2048, 768, False), ("q8_0", 9, 768, 256, False),
                ("q4_k", 2048, 1024, 5120, True), ("q4_0", 129, 4096, 1280, False),
