@@ -1678,8 +1678,8 @@ static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
         // (PRECISE sums are in registers by then, with no code to exchange them: whole tiles and slices only)
         if (!precise && fs != 1 && (fs == 2 || ntiles % sms))
             take((ntiles * blocks + sms - 1) / sms * cyc + epi + 6000 + 200 * tx, GemmShape{tx, tiles_x, 1, true, false});
-        // PRECISE: as many slices as make the last wave a full one
-        for (uint64_t sl = 2; precise && fs == 0 && sl <= 8 && 4 * sl <= groups; ++sl)
+        // PRECISE: as many slices as make the last wave a full one, where they are no more than 192 MiB
+        for (uint64_t sl = 2; precise && fs == 0 && sl <= 8 && 4 * sl <= groups && sl * m * n <= (192ull << 20) / 4; ++sl)
             take((ntiles * sl + sms - 1) / sms * ((groups + sl - 1) / sl * 4 * cyc + epi) + 3200 + sl * m * n / 600, GemmShape{tx, tiles_x, (uint32_t)sl, false, false});
         // few tiles: every SM takes a slice of some tile's k, and a kernel behind this one adds the slices
         if (fs == 0 && 2 * ntiles <= sms) {

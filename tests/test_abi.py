@@ -157,3 +157,12 @@ int main() {
     exe = tmp_path / "arrival"
     subprocess.run([shutil.which("g++") or "g++", "-std=c++17", "-I", os.path.join(ROOT, "rlx_b200", "csrc"), str(src), "-o", str(exe)], check=True)
     assert subprocess.run([str(exe)], capture_output=True, text=True).stdout == "0\n"
+
+
+def test_workspace_of_long_prompts_on_relaid_rows_is_bounded():
+    """Rows that TMA cannot tile: the re-laid weights, three bf16 parts of at most 128 MiB of f32 activations and at most 192 MiB
+    of partial results, however many rows there are."""
+    for sch, m, k, n in [(9, 11588, 15904, 25587), (5, 4543, 16128, 15933), (9, 3828, 16192, 26910), (7, 9000, 16352, 6144), (6, 3000, 8224, 28672)]:
+        for xd in (0, 1):
+            weights = R.packed_bytes(sch, -(-k // 256) * 256, n) + 16 * n
+            assert R.workspace_bytes(sch, m, k, n, xd) <= weights + (192 + 192 + 1 << 20), (sch, m, k, n, xd)
