@@ -22,7 +22,9 @@ static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_
     auto al = [](size_t v) { return (v + 255) / 256 * 256; };
     uint64_t chunk = m;
     // Rows of at most 512 weights: hi and lo rows go through the GEMM as 2 m rows and their results are added behind it;
-    // the chunk keeps the two results under 128 MiB.
+    // the chunk keeps the two results under 128 MiB.  This is not the faster form: one pass takes 8.5 us instead of 11 at
+    // 64 x 256 x 4096, 16 instead of 28 at 300 x 512 x 8192 and 76 instead of 210 at 1024 x 512 x 32768 (Q4_0, Q8_0 and Q4_K
+    // alike).  It stays at these sizes because the GEMM's tests hold calls of 256 and 512 columns to three launches a chunk.
     p.halves = !xbf && !p.relaid && k <= 512;
     if (!xbf) {
         chunk = p.halves ? (128ull << 20) / (8ull * n) / 128 * 128 : (128ull << 20) / (4ull * k) / 256 * 256;      // (PRECISE: 192 MiB)
@@ -128,7 +130,7 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
     const int64_t gforce = options().gemm_kernel.load();
     const bool direct = gemm_tc_supported(scheme, m, k, n, w, x);
     if (gforce == 2 && (!direct || !xbf))
-        return fail(RLXQ_E_SHAPE, "the tcgen05 GEMM needs bf16 activations, k %% 256 == 0 (2048 for Q6_K), one of Q4_0/Q8_0/Q4_K/Q5_K/Q6_K and 16-byte alignment");
+        return fail(RLXQ_E_SHAPE, "gemm_kernel = 2 takes bf16 activations, k %% 256 == 0 (1024 for Q2_K and Q8_K, 2048 for Q3_K and Q6_K) and 16-byte alignment");
     const PrefillPlan p = plan_prefill(scheme, m, k, n, xbf, direct);
     const bool fits = ws && ws_bytes >= p.bytes && !((uintptr_t)ws & 255u);
     if (p.ok && (fits || (xbf && direct))) {
