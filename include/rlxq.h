@@ -96,7 +96,10 @@ RLXQ_API int rlxq_packed_bytes(uint32_t scheme, uint64_t k, uint64_t n, uint64_t
  * rows that are no multiple of 16 bytes a copy of the weights on a padded pitch, three parts of f32 activations and up to
  * 192 MB of partial results (all 256-byte aligned); without that
  * workspace such a call runs the tiled generic kernel, some 40 times
- * slower.  The reference reserves k*n*4 bytes. */
+ * slower.  w_blocks is taken to be 16-byte aligned: at m > 8, weights at another address run the tiled generic kernel with
+ * this size where the GEMM would read them in place, and the GEMM on a re-laid copy only with a workspace that has room for
+ * that copy too (n rows of k weights rounded up to 256, a multiple of 16 bytes each), a third part of f32 activations and the
+ * 192 MB.  The reference reserves k*n*4 bytes. */
 RLXQ_API int rlxq_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n,
                          uint32_t x_dtype, uint32_t y_dtype, size_t* bytes);
 

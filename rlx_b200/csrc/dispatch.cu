@@ -11,7 +11,9 @@ namespace rlxq {
 // rows of x at a time (the split rows are kept under 128 MiB), multiplied by the same decoded weights.  Rows that TMA
 // cannot tile where they lie (k not a whole number of 256 weights, or of the 16-byte groups of a format's super-blocks;
 // weights that are not 16-byte aligned) are first re-laid on a padded pitch in the workspace, and weights and activations
-// then keep all of their 24 bits (PRECISE), since those shapes were multiplied in f32 before they had this path.
+// then keep all of their 24 bits (PRECISE), since those shapes were multiplied in f32 before they had this path.  The
+// workspace query does not know the weights' address and plans for aligned ones: weights at another address are re-laid only
+// for a caller who brings more than it asks for, and run the general kernel for everybody else.
 struct PrefillPlan { bool ok, relaid, halves; uint32_t chunk; uint64_t pitch; size_t off_w, off_y2, off_gemm, bytes; };
 static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, bool direct) {
     PrefillPlan p{};

@@ -17,7 +17,9 @@
 // the workspace is too small for it (fewer than 32 rows of little work, moe_rows_stream, and eight or fewer of a shape the
 // integer GEMV does not take: one launch of the f32 streaming GEMV, gemv_f32.cu):
 //   moe_tiles_kernel    the table of activation tiles, one list per expert, from the sorted offsets
-//   relay_rows_kernel   (rows TMA cannot tile) the slabs of the experts in use on a padded pitch
+//   relay_rows_kernel   (rows TMA cannot tile) the slabs of the experts in use on a padded pitch.  (A stack that is not 16-byte
+//                       aligned only with a larger workspace than the query asks for, which plans for aligned ones; the
+//                       general kernel otherwise.)
 //   moe_gather_kernel   the rows of every expert, gathered next to each other as bf16 (f32 activations as
 //                       bf16 hi rows and, m rows further on, lo rows, so nothing of x is lost)
 //   gemm_tcgen05_kernel every tile against its expert's slab of the stack (gemm_tcgen05.cu, GemmParams::groups), results

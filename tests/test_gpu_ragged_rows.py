@@ -85,6 +85,33 @@ def test_gemm_on_relaid_rows(sch, m, k, n, x_bf16):
     assert_within_tolerance(y, ref, _bound(s, w, x, k, n), tol=2e-5, what=f"relaid {sch} {m}x{k}x{n}")
 
 
+@pytest.mark.parametrize("sch,x_bf16", [("q4_k", False), ("q8_0", True)])
+def test_prompt_on_weights_at_an_odd_address(sch, x_bf16):
+    """The workspace query plans for 16-byte aligned weights.  At another address a call with that much scratch runs the general
+    kernel, and one with room for a re-laid copy the GEMM on it."""
+    import torch
+    import rlx_b200 as R
+    from rlx_b200._lib import lib
+    m, k, n = 70, 1024, 264
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, 31)
+    buf = torch.zeros(w.size + 64, dtype=torch.uint8, device="cuda")
+    wd = buf[2:2 + w.size]
+    wd.copy_(torch.from_numpy(w))
+    ref = x.astype(np.float64) @ O.dequant(s, w, k * n).reshape(n, k).astype(np.float64).T
+    R.set_option("gemm_kernel", 1)
+    try:
+        general = R.matmul(xd, wd, s, n)
+    finally:
+        R.set_option("gemm_kernel", 0)
+    assert torch.equal(R.matmul(xd, wd, s, n), general)
+    ws, y = torch.empty(64 << 20, dtype=torch.uint8, device="cuda"), torch.empty((m, n), device="cuda")
+    assert lib.rlxq_matmul(torch.cuda.current_stream().cuda_stream, s, xd.data_ptr(), int(x_bf16), wd.data_ptr(), y.data_ptr(), 0, m, k, n,
+                           ws.data_ptr(), ws.numel()) == 0
+    R.device_status()
+    assert not torch.equal(y, general)
+    assert _error(y.cpu().numpy(), ref) <= 1.02 * _error(general.cpu().numpy(), ref)
+
+
 def _error(y, ref):
     return np.linalg.norm(y.astype(np.float64) - ref) / np.linalg.norm(ref)
 
