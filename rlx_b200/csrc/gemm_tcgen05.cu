@@ -23,14 +23,13 @@
 // Replaces the reference's dequantise-to-f32-scratch + cublasSgemm for m > 8
 // (rlx-cuda/src/gguf_gpu.rs:62-134), which also reads the scratch with the wrong leading
 // dimension for n > 1.
-#include <cuda_bf16.h>
-
 #include <algorithm>
 #include <chrono>
 
 #include "arrival.h"
 #include "common.cuh"
 #include "decode.cuh"
+#include "f32x2.cuh"
 #include "kernels.h"
 #include "staged_common.cuh"
 #include "tc_common.cuh"
@@ -43,11 +42,6 @@ constexpr uint32_t kGemmBK = 64;        // k per pipeline stage (one 128-byte sw
 constexpr uint32_t kGemmMaxStages = 8;  // B shared-memory stages == A tensor-memory stages (8 x 32 columns)
 constexpr uint32_t kGemmMaxRaw = 8;     // raw weight boxes (256 weights of 128 rows each): what shared memory is left for
 constexpr uint32_t kGemmRawStages = 2;  // the paired kernel's
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);       // .x (low half) = lo
-    return *reinterpret_cast<uint32_t*>(&v);
-}
 
 // ---- weight decode: 64 consecutive weights of one row -> 32 bf16 pairs ------------------------
 // The raw box holds 256 weights of 128 rows; RAW_ROW bytes per row (an odd number of 16-byte
@@ -95,37 +89,12 @@ __device__ __forceinline__ float u8_minus(uint32_t b) { return __uint_as_float(0
 // k block per 512 cycles), so they work on pairs: one byte-permute per weight builds the float 2^23 + byte
 // straight from the raw word, and the arithmetic uses the packed two-float instructions of this architecture.
 // Every step rounds exactly as the scalar f32 expression it replaces.
-__device__ __forceinline__ uint64_t f32x2(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t f32x2_splat(float f) { return f32x2(__float_as_uint(f), __float_as_uint(f)); }
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 // two floats -> bf16 pair, the first in the low half
 __device__ __forceinline__ uint32_t bf16x2_of(uint64_t v) {
     uint32_t lo, hi, d;
     asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
     return d;
-}
-// bytes 2 H and 2 H + 1 of u -> (2^23 + byte, 2^23 + byte)
-template <int H> __device__ __forceinline__ uint64_t magic_pair(uint32_t u) {
-    return f32x2(__byte_perm(u, 0x4B000000u, 0x7440 + 2 * H), __byte_perm(u, 0x4B000000u, 0x7441 + 2 * H));
 }
 // (byte - OFF) * scale for bytes 2 H, 2 H + 1 of u
 template <int H> __device__ __forceinline__ uint64_t scaled_pair(uint32_t u, uint64_t neg_off, uint64_t scale) {

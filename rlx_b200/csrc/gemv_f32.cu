@@ -18,6 +18,7 @@
 // (18 for 16) and half as many weights a lane did not help.
 #include "common.cuh"
 #include "decode.cuh"
+#include "f32x2.cuh"
 #include "kernels.h"
 #include "staged_common.cuh"
 
@@ -64,37 +65,17 @@ template <int N> __device__ __forceinline__ void s32_even(uint32_t a, uint32_t (
 }
 __device__ __forceinline__ uint32_t s16_even(uint32_t a) { return (s32(a & ~3u) >> ((a & 2u) * 8u)) & 0xFFFFu; }
 
-__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ float sum2(uint64_t v) {
-    uint32_t lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-    return __uint_as_float(lo) + __uint_as_float(hi);
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 // The four bytes of u, less OFF, times x pairs xi, xi + 1 of every batch row.
 template <int OFF, int MR, int NX>
 __device__ __forceinline__ void mul_word(uint32_t u, const uint64_t (&x)[MR][NX], int xi, uint64_t (&acc)[MR]) {
     const uint32_t o = __float_as_uint(-(8388608.0f + (float)OFF));
-    const uint64_t off = pack2(o, o);
-    const uint64_t a = add2(pack2(__byte_perm(u, 0x4B000000u, 0x7440), __byte_perm(u, 0x4B000000u, 0x7441)), off);
-    const uint64_t b = add2(pack2(__byte_perm(u, 0x4B000000u, 0x7442), __byte_perm(u, 0x4B000000u, 0x7443)), off);
+    const uint64_t off = f32x2(o, o);
+    const uint64_t a = add_f32x2(magic_pair<0>(u), off);
+    const uint64_t b = add_f32x2(magic_pair<1>(u), off);
 #pragma unroll
     for (int r = 0; r < MR; ++r) {
-        acc[r] = fma2(a, x[r][xi], acc[r]);
-        acc[r] = fma2(b, x[r][xi + 1], acc[r]);
+        acc[r] = fma_f32x2(a, x[r][xi], acc[r]);
+        acc[r] = fma_f32x2(b, x[r][xi + 1], acc[r]);
     }
 }
 
@@ -115,7 +96,7 @@ template <int MR, int LW> struct F32Lane<RLXQ_Q8_0, MR, LW> {
 #pragma unroll
         for (int i = 0; i < LW / 4; ++i) mul_word<128>(q[i] ^ 0x80808080u, x, 2 * i, acc);
 #pragma unroll
-        for (int r = 0; r < MR; ++r) sum[r] = d * sum2(acc[r]);
+        for (int r = 0; r < MR; ++r) sum[r] = d * sum_f32x2(acc[r]);
     }
 };
 
@@ -143,7 +124,7 @@ template <int MR, int LW> struct F32Lane<RLXQ_Q4_0, MR, LW> {
         }
         const float d = f16_bits_to_f32(s16_even(blk));
 #pragma unroll
-        for (int r = 0; r < MR; ++r) sum[r] = d * sum2(acc[r]);
+        for (int r = 0; r < MR; ++r) sum[r] = d * sum_f32x2(acc[r]);
     }
 };
 
@@ -173,7 +154,7 @@ template <int MR, int LW> struct F32Lane<RLXQ_Q6_K, MR, LW> {
                 mul_word<32>(((ql[i] >> nib) & 0x0F0F0F0Fu) | (((qh[i] >> hs) << 4) & 0x30303030u), x, 2 * i, acc);
             const float ds = d * (float)(int8_t)((sc >> (8 * s)) & 0xFFu);
 #pragma unroll
-            for (int r = 0; r < MR; ++r) sum[r] = fmaf(ds, sum2(acc[r]), sum[r]);
+            for (int r = 0; r < MR; ++r) sum[r] = fmaf(ds, sum_f32x2(acc[r]), sum[r]);
         }
     }
 };
@@ -205,7 +186,7 @@ template <uint32_t SCHEME, int MR, int LW> struct F32LaneK45 {
         }
         const float d = f16_bits_to_f32(h[0] & 0xFFFFu) * (float)sc, dm = f16_bits_to_f32(h[0] >> 16) * (float)mn;
 #pragma unroll
-        for (int r = 0; r < MR; ++r) sum[r] = fmaf(d, sum2(acc[r]), -dm * xs[r]);
+        for (int r = 0; r < MR; ++r) sum[r] = fmaf(d, sum_f32x2(acc[r]), -dm * xs[r]);
     }
 };
 template <int MR, int LW> struct F32Lane<RLXQ_Q4_K, MR, LW> : F32LaneK45<RLXQ_Q4_K, MR, LW> {};
@@ -324,15 +305,15 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
                             const uint4 v = have ? src[t] : make_uint4(0u, 0u, 0u, 0u);
                             const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) x[r][4 * t + q] = pack2(u[q] << 16, u[q] & 0xFFFF0000u);
+                            for (int q = 0; q < 4; ++q) x[r][4 * t + q] = f32x2(u[q] << 16, u[q] & 0xFFFF0000u);
                         }
                     } else {
                         const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(P.x) + (size_t)(m0 + r) * P.k + c0);
 #pragma unroll
                         for (int t = 0; t < LW / 4; ++t) {
                             const uint4 v = have ? src[t] : make_uint4(0u, 0u, 0u, 0u);
-                            x[r][2 * t] = pack2(v.x, v.y);
-                            x[r][2 * t + 1] = pack2(v.z, v.w);
+                            x[r][2 * t] = f32x2(v.x, v.y);
+                            x[r][2 * t + 1] = f32x2(v.z, v.w);
                         }
                     }
                 }
@@ -342,8 +323,8 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
                 for (int r = 0; r < MR; ++r) {
                     uint64_t t = 0ull;
 #pragma unroll
-                    for (int q = 0; q < LW / 2; ++q) t = add2(t, x[r][q]);
-                    xs[r] = sum2(t);
+                    for (int q = 0; q < LW / 2; ++q) t = add_f32x2(t, x[r][q]);
+                    xs[r] = sum_f32x2(t);
                 }
             }
             uint32_t at = (uint32_t)(uintptr_t)w + (r0 + b * kF32Batch) * (uint32_t)P.row_bytes + (pass * nwarps + warp) * PIECE;

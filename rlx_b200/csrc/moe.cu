@@ -44,8 +44,6 @@
 
 namespace rlxq {
 
-constexpr uint32_t kMoeInvalid = 0xFFFFFFFFu;
-
 constexpr uint32_t kMoeScanThreads = 1024;
 // Inclusive block-wide running sum over kMoeScanThreads threads.
 __device__ __forceinline__ uint32_t moe_block_scan(uint32_t v, uint32_t (&wsum)[32]) {
