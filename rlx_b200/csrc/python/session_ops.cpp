@@ -14,7 +14,11 @@ PyObject* g_as_f32 = nullptr;      // array -> contiguous f32 array
 
 struct Buffers {
     std::vector<Py_buffer> views;
-    ~Buffers() { for (Py_buffer& v : views) PyBuffer_Release(&v); }
+    std::vector<PyObject*> pairs;  // the names are theirs
+    ~Buffers() {
+        for (Py_buffer& v : views) PyBuffer_Release(&v);
+        for (PyObject* p : pairs) Py_DECREF(p);
+    }
     bool add(PyObject* o, int flags) {
         Py_buffer v;
         if (PyObject_GetBuffer(o, &v, flags)) return false;
@@ -53,14 +57,18 @@ PyObject* op_run(PyObject*, PyObject* const* a, Py_ssize_t na) {
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
     Buffers bufs;
     bufs.views.reserve(n + 1);
+    bufs.pairs.reserve(n);
     std::vector<const char*> names(n);
     std::vector<const float*> data(n);
     std::vector<uint64_t> elems(n);
     bool ok = true;
     for (Py_ssize_t i = 0; ok && i < n; ++i) {
-        PyObject* pair = PySequence_Fast_GET_ITEM(seq, i);
-        if (!PyTuple_Check(pair) || PyTuple_GET_SIZE(pair) != 2) {
-            PyErr_SetString(PyExc_TypeError, "inputs must be (name, array) pairs");
+        PyObject* pair = PySequence_Tuple(PySequence_Fast_GET_ITEM(seq, i));       // any two things in a row; owns both
+        ok = pair != nullptr;
+        if (!ok) break;
+        bufs.pairs.push_back(pair);
+        if (PyTuple_GET_SIZE(pair) != 2) {
+            PyErr_Format(PyExc_ValueError, "inputs must be (name, array) pairs, got %zd values", PyTuple_GET_SIZE(pair));
             ok = false;
             break;
         }

@@ -166,3 +166,17 @@ def test_workspace_of_long_prompts_on_relaid_rows_is_bounded():
         for xd in (0, 1):
             weights = R.packed_bytes(sch, -(-k // 256) * 256, n) + 16 * n
             assert R.workspace_bytes(sch, m, k, n, xd) <= weights + (192 + 192 + 1 << 20), (sch, m, k, n, xd)
+
+
+def test_run_takes_pairs_of_any_kind():
+    """CompiledGraph.run unpacks each input into a name and an array: tuples, lists, anything of two elements; the error is the
+    library's (there is no graph here) and not about the pair."""
+    import numpy as np
+    run, out = R.api._load_session_native().run, np.empty((1, 4), np.float32)
+    x = np.ones((1, 4), np.float32)
+    for inputs in ([("x", x)], [["x", x]], (["x", x],), {"x": x}.items(), [iter(("x", x))], [["x", [[1, 2, 3, 4]]]], []):
+        with pytest.raises(R.RlxqError):
+            run(None, inputs, out)
+    for inputs, error in (([("x",)], ValueError), ([["x", x, x]], ValueError), ([3], TypeError), (3, TypeError), ([(3, x)], TypeError)):
+        with pytest.raises(error):
+            run(None, inputs, out)
