@@ -4,12 +4,15 @@ native form of the Python calls on torch tensors, with the host compiler.
     python -m rlx_b200.build [--force] [--verbose]
 
 Only nvcc is needed (no GPU): the objects are cross-compiled.  Objects are cached under
-rlx_b200/csrc/build/ and rebuilt when a source or header is newer.
+rlx_b200/csrc/build/ and rebuilt when a source or header is newer, the extensions also when the interpreter or torch is
+another one than they were built for.  The extensions are left out where Python's headers or torch are missing.
 """
 from __future__ import annotations
 
 import concurrent.futures as cf
 import glob
+import importlib.metadata
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -60,20 +63,55 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
-def _build_ext(name: str, out: str, flags, force: bool) -> None:
+def _torch_root() -> str | None:
+    """Where torch is installed, without importing it; None where it is not."""
+    try:
+        spec = importlib.util.find_spec("torch")
+    except (ImportError, ValueError):
+        return None
+    root = os.path.dirname(spec.origin) if spec and spec.origin else None
+    return root if root and os.path.isdir(os.path.join(root, "include")) else None
+
+
+def _python_include() -> str | None:
+    inc = sysconfig.get_paths()["include"]
+    return inc if os.path.exists(os.path.join(inc, "Python.h")) else None
+
+
+def _built_for(torch_root: str | None) -> str:
+    """What an extension is built for: this interpreter and, with torch_root, this torch."""
+    ident = f"{sys.version} {sysconfig.get_config_var('SOABI')} {_python_include()}"
+    if torch_root:
+        try:
+            ident += f" torch {importlib.metadata.version('torch')} {torch_root}"
+        except importlib.metadata.PackageNotFoundError:
+            ident += f" torch {torch_root}"
+    return ident
+
+
+def _ext_is_current(out: str, sources, ident: str) -> bool:
+    """Whether `out` is newer than its sources and was built for `ident` (its note lies with the objects)."""
+    note = os.path.join(OBJ, os.path.basename(out) + ".for")
+    if not (os.path.exists(out) and os.path.exists(note)) or os.path.getmtime(out) < max(os.path.getmtime(p) for p in sources):
+        return False
+    with open(note) as f:
+        return f.read() == ident
+
+
+def _build_ext(name: str, out: str, flags, ident: str, force: bool) -> None:
     """csrc/python/<name> against this interpreter and librlxq.so beside it; flags() -> what else it needs."""
     src = os.path.join(CSRC, "python", name)
-    headers = glob.glob(os.path.join(PKG, "..", "include", "*.h"))
-    newest = max(os.path.getmtime(p) for p in [src, *headers])
-    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
+    if not force and _ext_is_current(out, [src, *glob.glob(os.path.join(PKG, "..", "include", "*.h"))], ident):
         return
     compile_flags, link_flags = flags()
     cmd = [os.environ.get("CXX") or shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           *compile_flags, "-isystem", sysconfig.get_paths()["include"], "-I", os.path.join(PKG, "..", "include"), src, "-o", out,
+           *compile_flags, "-isystem", _python_include(), "-I", os.path.join(PKG, "..", "include"), src, "-o", out,
            *link_flags, "-L", PKG, "-l:librlxq.so", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"{cmd[0]} failed for {src}:\n{r.stdout}\n{r.stderr}")
+    with open(os.path.join(OBJ, os.path.basename(out) + ".for"), "w") as f:
+        f.write(ident)
 
 
 def _torch_flags():
@@ -84,6 +122,20 @@ def _torch_flags():
              "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
              "-isystem", os.path.join(cuda, "include")],
             ["-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+
+
+def _build_python_face(force: bool) -> None:
+    """The two extensions.  A user of the C ABI alone needs neither: without Python's headers none is built, without torch only
+    CompiledGraph.run's.  The calls that need a missing one say so when they are made."""
+    if _python_include() is None:
+        sys.stderr.write("rlx_b200: no Python.h, librlxq.so is built without the Python extensions\n")
+        return
+    _build_ext("session_ops.cpp", SESSION_OPS, lambda: ([], []), _built_for(None), force)
+    root = _torch_root()
+    if root is None:
+        sys.stderr.write("rlx_b200: torch is not installed, librlxq.so is built without _torch_ops.so\n")
+        return
+    _build_ext("torch_ops.cpp", OPS, _torch_flags, _built_for(root), force)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -105,8 +157,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    _build_ext("torch_ops.cpp", OPS, _torch_flags, force)
-    _build_ext("session_ops.cpp", SESSION_OPS, lambda: ([], []), force)
+    _build_python_face(force)
     return LIB
 
 
