@@ -496,7 +496,7 @@ struct GemmParams {
     // rows behind them; a stage carries both boxes and both are multiplied by the same decoded weights into the same
     // accumulator, so a weight is decoded once for the two halves.
     uint32_t lo_row, xparts;
-    uint32_t main_run;     // PRECISE: k blocks the main accumulator takes at a time (gemm_precise_epilogue): 1, 2 or 4
+    uint32_t main_run, sum_run;    // PRECISE: k blocks the main accumulator takes at a time, and the sums; powers of two (gemm_main_run)
     uint32_t nstages, nraw;               // depth of the operand ring (B in shared memory, A in tensor memory) and of the raw ring
     uint32_t b_bytes;                     // bytes of a B stage: tx * 128, twice that with lo_row
     uint32_t w_late;       // the weights are written by a kernel in front (re-laid rows): read them after the dependency wait
@@ -845,19 +845,22 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
 // a multiple of f32's error (6.8e-6 of a result after 1024 columns of six products in one accumulator, 5.7e-5 after 8192; the
 // general kernel, which multiplied these shapes before, 3.3e-7 over 11008).  Hence two accumulators of P.tx columns.  The main
 // one takes the leading parts' product of main_run k blocks; the epilogue warps add it, rounding, to sums in registers, while
-// the other products run.  Those are 2^-8 of the whole and smaller: they pile up in the second accumulator.  Every kGemmRun
+// the other products run.  Those are 2^-8 of the whole and smaller: they pile up in the second accumulator.  Every sum_run
 // blocks it joins the sums, and these move on to totals in shared memory, so that no chain of additions is long.  Error
-// against 64 bits, general kernel and this one: k = 256 8.0e-8 and 7.8e-8, 2816 1.8e-7 and 1.4e-7, 11008 3.3e-7 and 2.3e-7.
-// 300 x 11008 x 4096 Q6_K f32 4787 us (general kernel) and 226 us; with long accumulations 218 us.
-constexpr uint32_t kGemmRun = 16;
+// against 64 bits, general kernel and this one, f32 activations: k = 256 8.1e-8 and 8.0e-8, 2304 1.6e-7 and 9.8e-8, 11008
+// 3.3e-7 and 1.4e-7, 16128 4.0e-7 and 1.5e-7.  300 x 11008 x 4096 Q6_K f32 4787 us (general kernel) and 240 us; with long
+// accumulations 218 us (L2 cold).
 // Activation rows of a PRECISE tile: what the epilogue threads have registers for (Q3_K's block is larger: 96 a thread) and
 // shared memory has room for totals beside three operand stages and two raw boxes (Q8_K's are the largest).
 constexpr uint32_t gemm_precise_rows(uint32_t scheme) { return scheme == RLXQ_Q3_K || scheme == RLXQ_Q8_K ? 64u : 96u; }
 
-// Blocks between two emptyings: a block costs 1.4e-8 of a result for each of its four truncated additions (5.6e-8, 1.1e-7 and
-// 2.2e-7 for runs of 1, 2 and 4), and f32 arithmetic in the general kernel, which is what the result is held against, 8e-8
-// at k = 256, 1.6e-7 at 2304, 2.9e-7 at 8192 and 3.3e-7 at 11008.
-static uint32_t gemm_main_run(uint32_t k) { return k >= 9216 ? 4u : k >= 2304 ? 2u : 1u; }
+// Blocks between two emptyings of the main accumulator, and of the sums.  A block costs 1.4e-8 of a result for each of its four
+// truncated additions (5.6e-8, 1.0e-7 and 1.9e-7 for runs of 1, 2 and 4), always towards zero, so that the layers of a SwiGLU
+// chain add up: held against the general kernel are chains, 2.24e-7 at widths 1024 -> 3328 (here 2.17e-7; 2.22e-7 with f32
+// activations), 3.0e-7 at 2304 -> 5888 (2.7e-7), 5.1e-7 at 6912 -> 22272 (4.4e-7).  Shorter runs cost time: 300 x 11040 x 4096 Q8_0
+// bf16 takes 220, 236 and 243 us with main runs of 4, 2 and 1, 236, 261 and 300 us with sums of 16, 8 and 4 blocks.
+static uint32_t gemm_main_run(uint32_t k) { return k >= 20480 ? 4u : k >= 5632 ? 2u : 1u; }
+static uint32_t gemm_sum_run(uint32_t k) { return k >= 5632 ? 16u : k >= 2048 ? 8u : 4u; }
 
 // TX = P.tx: no branch between the additions of a block, which are on the chain from one block's product to the next.
 template <uint32_t SCHEME, uint32_t TX>
@@ -889,7 +892,7 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
         };
         bool ok = true;
 #pragma unroll 1
-        for (uint32_t k0 = 0; ok && k0 < blocks; k0 += kGemmRun) {
+        for (uint32_t k0 = 0; ok && k0 < blocks; k0 += P.sum_run) {
             uint64_t sum[TX / 2];                            // pairs of activation rows
 #pragma unroll
             for (uint32_t j = 0; j < TX / 2; ++j) sum[j] = 0ull;
@@ -909,7 +912,7 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
                     for (uint32_t j = 0; j < 8; ++j) sum[8 * c + j] = add_f32x2(sum[8 * c + j], f32x2(v[2 * j], v[2 * j + 1]));
                 }
             };
-            const uint32_t k1 = min(blocks, k0 + kGemmRun);
+            const uint32_t k1 = min(blocks, k0 + P.sum_run);
 #pragma unroll 1
             for (uint32_t kb = k0; kb < k1; kb += P.main_run) {
                 if (!(ok = wait_for(0, mph))) break;
@@ -1101,7 +1104,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                         if (in_run == P.main_run - 1u || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[0]));
                         // parts 1, 2 by part 0, 0..1 by part 1, 0 by part 2; the three products left out are below 2^-24 of the whole
                         const uint32_t cross = acc + P.tx;
-                        const bool fresh = kb % kGemmRun == 0;
+                        const bool fresh = (kb & (P.sum_run - 1u)) == 0;
                         if (fresh) {
                             if (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[1]), cph)) { give_up(13); ok = false; break; }
                             cph ^= 1u;
@@ -1119,7 +1122,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                                 for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(cross, a + 32 + 8 * j, ldesc + 2 * j, idesc, 1u);
                             }
                         }
-                        if (kb % kGemmRun == kGemmRun - 1 || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[1]));
+                        if ((kb & (P.sum_run - 1u)) == P.sum_run - 1u || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[1]));
                     } else {
 #pragma unroll
                         for (uint32_t j = 0; j < kGemmBK / 16; ++j)
@@ -1693,6 +1696,7 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     P.lo_row = c.f32 ? c.x_rows : 0u;
     P.xparts = gemm_x_parts(c.f32, PRECISE);
     P.main_run = gemm_main_run(c.k);
+    P.sum_run = gemm_sum_run(c.k);
     int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * P.xparts, c.k, P.tx);
     if (rc) return rc;
     rc = encode_weight_map(&P.wmap, c.w, (uint64_t)c.n * c.num_slabs, c.w_pitch ? c.w_pitch : (uint64_t)c.k / g.elems * g.bytes,

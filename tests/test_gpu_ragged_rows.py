@@ -140,6 +140,31 @@ def test_gemm_on_relaid_rows_is_as_exact_as_the_general_kernel(sch, m, k, n, x_b
     assert _error(y, ref) <= 1.02 * _error(general, ref), (_error(y, ref), _error(general, ref))
 
 
+# (widths between which neither layer's rows can be tiled; 3e-2 for what the truncation of three matrices leaves at the smallest)
+@pytest.mark.parametrize("m,d,f,x_bf16", [(30, 1024, 2816, True), (40, 1280, 4352, False), (9, 1792, 4864, False), (20, 2304, 5888, True)])
+def test_swiglu_chain_on_relaid_rows_is_as_exact_as_the_general_kernel(m, d, f, x_bf16):
+    """The truncation of the tensor core has a direction, so the errors of a chain's layers add up instead of averaging out."""
+    import torch
+    import rlx_b200 as R
+    s, gu, x, xd = _inputs("q6_k", m, d, 2 * f, x_bf16, 40 + m)
+    dn = O.fill_weights(s, 41 + m, f, d)
+    layers = [(torch.from_numpy(gu).cuda(), 2 * f), (torch.from_numpy(dn).cuda(), d, True)]
+    h = x.astype(np.float64) @ O.dequant(s, gu, d * 2 * f).reshape(2 * f, d).astype(np.float64).T
+    gate, up = h[:, :f], h[:, f:]
+    with np.errstate(over="ignore"):
+        ref = (up * gate / (1 + np.exp(-gate))) @ O.dequant(s, dn, f * d).reshape(d, f).astype(np.float64).T
+    y = R.matmul_chain(xd, layers, s).cpu().numpy()
+    R.device_status()
+    R.set_option("gemm_kernel", 1)
+    try:
+        general = R.matmul_chain(xd, layers, s).cpu().numpy()
+    finally:
+        R.set_option("gemm_kernel", 0)
+    assert not np.array_equal(y, general)
+    assert _error(general, ref) < 1e-6                          # (gate first, then up)
+    assert _error(y, ref) <= 1.03 * _error(general, ref), (_error(y, ref), _error(general, ref))
+
+
 @pytest.mark.parametrize("sch,k", [("q4_0", 544), ("q8_0", 2336), ("q6_k", 1280)])
 @pytest.mark.parametrize("x_bf16", [False, True])
 def test_gemm_on_relaid_rows_with_values_that_are_not_finite(sch, k, x_bf16):
