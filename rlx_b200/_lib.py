@@ -13,7 +13,7 @@ LIB_PATH = os.path.join(_HERE, "librlxq.so")
 
 if not os.path.exists(LIB_PATH):
     raise ImportError(
-        f"{LIB_PATH} is missing: build it with `python -m rlx_b200.build` (needs nvcc). "
+        f"{LIB_PATH} is missing: build it with `python rlx_b200/build.py` (needs nvcc). "
         "rlx_b200 has no fallback path.")
 
 lib = C.CDLL(LIB_PATH, mode=C.RTLD_GLOBAL)

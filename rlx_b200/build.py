@@ -1,7 +1,7 @@
 """Builds rlx_b200/librlxq.so (the C-ABI library) with nvcc for sm_100a, in-tree, and rlx_b200/_torch_ops.so, the
 native form of the Python calls on torch tensors, with the host compiler.
 
-    python -m rlx_b200.build [--force] [--verbose]
+    python rlx_b200/build.py [--force] [--verbose]
 
 Only nvcc is needed (no GPU): the objects are cross-compiled.  Objects are cached under
 rlx_b200/csrc/build/ and rebuilt when a source or header is newer, the extensions also when the interpreter or torch is

@@ -47,3 +47,17 @@ def test_extensions_are_built_again_for_another_torch_or_interpreter(monkeypatch
     assert B._built_for(root) != before
     monkeypatch.setattr(B.sys, "version", "another")
     assert B._built_for(None) != ident["session_ops.cpp"]
+
+
+def test_the_build_runs_before_there_is_a_library(tmp_path):
+    """The command that the import error names does not itself import the package, which needs the library."""
+    import shutil
+    import subprocess
+    import sys
+    pkg = tmp_path / "rlx_b200"
+    shutil.copytree(B.PKG, pkg, ignore=shutil.ignore_patterns("*.so", "csrc", "__pycache__"))
+    r = subprocess.run([sys.executable, "-c", "import rlx_b200"], cwd=tmp_path, capture_output=True, text=True)
+    command = r.stderr.split("build it with `")[1].split("`")[0].split()
+    assert r.returncode and command[0] == "python"
+    r = subprocess.run([sys.executable, *command[1:]], cwd=tmp_path, capture_output=True, text=True, env={**os.environ, "NVCC": "", "PATH": ""})
+    assert "ImportError" not in r.stderr and "missing: build it" not in r.stderr, r.stderr
