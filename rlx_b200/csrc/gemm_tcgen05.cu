@@ -859,8 +859,10 @@ constexpr uint32_t gemm_precise_rows(uint32_t scheme) { return scheme == RLXQ_Q3
 // chain add up: held against the general kernel are chains, 2.24e-7 at widths 1024 -> 3328 (here 2.17e-7; 2.22e-7 with f32
 // activations), 3.0e-7 at 2304 -> 5888 (2.7e-7), 5.1e-7 at 6912 -> 22272 (4.4e-7).  Shorter runs cost time: 300 x 11040 x 4096 Q8_0
 // bf16 takes 220, 236 and 243 us with main runs of 4, 2 and 1, 236, 261 and 300 us with sums of 16, 8 and 4 blocks.
-static uint32_t gemm_main_run(uint32_t k) { return k >= 20480 ? 4u : k >= 5632 ? 2u : 1u; }
-static uint32_t gemm_sum_run(uint32_t k) { return k >= 5632 ? 16u : k >= 2048 ? 8u : 4u; }
+// A result that is stored as bf16 has the error of that rounding, 1.655e-3, the same to six digits with the general kernel and
+// with runs of 16 blocks (9e-7 before it is rounded); 300 x 11040 x 4096 Q8_0 bf16 204 us.
+static uint32_t gemm_main_run(uint32_t k, bool ybf) { return ybf ? 16u : k >= 20480 ? 4u : k >= 5632 ? 2u : 1u; }
+static uint32_t gemm_sum_run(uint32_t k, bool ybf) { return ybf || k >= 5632 ? 16u : k >= 2048 ? 8u : 4u; }
 
 // TX = P.tx: no branch between the additions of a block, which are on the chain from one block's product to the next.
 template <uint32_t SCHEME, uint32_t TX>
@@ -1695,8 +1697,8 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     P.tx = sh.tx;
     P.lo_row = c.f32 ? c.x_rows : 0u;
     P.xparts = gemm_x_parts(c.f32, PRECISE);
-    P.main_run = gemm_main_run(c.k);
-    P.sum_run = gemm_sum_run(c.k);
+    P.main_run = gemm_main_run(c.k, c.ybf);
+    P.sum_run = gemm_sum_run(c.k, c.ybf);
     int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * P.xparts, c.k, P.tx);
     if (rc) return rc;
     rc = encode_weight_map(&P.wmap, c.w, (uint64_t)c.n * c.num_slabs, c.w_pitch ? c.w_pitch : (uint64_t)c.k / g.elems * g.bytes,
