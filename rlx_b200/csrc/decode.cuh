@@ -258,10 +258,33 @@ __device__ __forceinline__ uint32_t f32_to_bf16_bits(float f) {
     x += 0x7FFFu + lsb;
     return x >> 16;
 }
-// The leading bf16 part of f: rounded, but finite where f is (a value past the largest bf16 is cut off there).
-__device__ __forceinline__ uint32_t bf16_hi_bits(float f) {
-    const uint32_t h = f32_to_bf16_bits(f) & 0xFFFFu;
-    return (h & 0x7FFFu) == 0x7F80u && isfinite(f) ? __float_as_uint(f) >> 16 : h;
+// f = hi + mid + lo in three bf16 values (exactly, for finite f): each the rounding of what is left.  Infinities and NaN are hi
+// alone, and a finite value past the largest bf16 is cut off there, since rounding would make it infinite.  Four at a time, with
+// one test for values of that kind.
+__device__ __forceinline__ void split_bf16x4(const float (&f)[4], uint32_t (&hi)[4], uint32_t (&mid)[4], uint32_t (&lo)[4]) {
+    constexpr uint32_t kPast = 0x7F7F8000u;                  // the first magnitude that rounds past the largest bf16
+    uint32_t most = 0u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) most = max(most, __float_as_uint(f[q]) & 0x7FFFFFFFu);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t x = __float_as_uint(f[q]);
+        hi[q] = (x + 0x7FFFu + ((x >> 16) & 1u)) >> 16;
+    }
+    if (most >= kPast) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t x = __float_as_uint(f[q]), m = x & 0x7FFFFFFFu;
+            if (m >= kPast) hi[q] = m > 0x7F800000u ? (x >> 16) | 0x40u : x >> 16;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float rest = f[q] - __uint_as_float(hi[q] << 16);    // exact
+        if (most > 0x7F7FFFFFu && !isfinite(f[q])) rest = 0.f;
+        mid[q] = f32_to_bf16_bits(rest) & 0xFFFFu;
+        lo[q] = f32_to_bf16_bits(rest - __uint_as_float(mid[q] << 16)) & 0xFFFFu;
+    }
 }
 
 }  // namespace rlxq

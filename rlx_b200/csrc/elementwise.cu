@@ -57,11 +57,10 @@ int launch_copy_bytes(cudaStream_t stream, void* dst, const void* src, uint64_t 
     return check_launch("copy_bytes_kernel");
 }
 
-// f32 activations for the tensor-core GEMM, whose operands are bf16: x = hi + lo with hi = bf16(x) and
-// lo = bf16(x - hi), which leaves 2^-17 of x behind, or (parts = 3) x = hi + mid + lo, which leaves nothing.  Rows [row0,
-// row0 + rows) of x become rows [0, rows) (hi), [rows, 2 rows) and, if asked for, [2 rows, 3 rows) of `out`; the GEMM multiplies both by the same decoded weights.  One pass of 8 bytes a
-// value, a few microseconds; the GEMM behind it is resident meanwhile and fetches its first weights.  Infinities and NaN are
-// hi alone; finite values past the largest bf16 are cut off there and not rounded, which would make them infinite.
+// f32 activations for the tensor-core GEMM, whose operands are bf16 (split_bf16x4): x = hi + lo, which leaves 2^-17 of x behind,
+// or (parts = 3) x = hi + mid + lo, which leaves nothing.  Rows [0, rows) of x become rows [0, rows) (hi), [rows, 2 rows) and, if
+// asked for, [2 rows, 3 rows) of `out`; the GEMM multiplies all of them by the same decoded weights.  One pass of 8 bytes a
+// value, a few microseconds; the GEMM behind it is resident meanwhile and fetches its first weights.
 __global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restrict__ x, uint16_t* __restrict__ out,
                                                           uint64_t rows, uint64_t k, uint32_t parts) {
     const uint64_t total = rows * k / 4, stride = (uint64_t)gridDim.x * blockDim.x;     // k % 4 == 0
@@ -70,17 +69,11 @@ __global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restric
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const float4 v = reinterpret_cast<const float4*>(x)[i];
         const float f[4] = {v.x, v.y, v.z, v.w};
-        uint16_t h[4], l[4], e[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            h[j] = (uint16_t)bf16_hi_bits(f[j]);
-            const float rest = isfinite(f[j]) ? f[j] - __uint_as_float((uint32_t)h[j] << 16) : 0.f;     // exact
-            l[j] = (uint16_t)f32_to_bf16_bits(rest);
-            e[j] = (uint16_t)f32_to_bf16_bits(rest - __uint_as_float((uint32_t)l[j] << 16));
-        }
-        reinterpret_cast<uint2*>(out)[i] = make_uint2(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16));
-        reinterpret_cast<uint2*>(out + rows * k)[i] = make_uint2(l[0] | ((uint32_t)l[1] << 16), l[2] | ((uint32_t)l[3] << 16));
-        if (parts == 3) reinterpret_cast<uint2*>(out + 2 * rows * k)[i] = make_uint2(e[0] | ((uint32_t)e[1] << 16), e[2] | ((uint32_t)e[3] << 16));
+        uint32_t h[4], l[4], e[4];
+        split_bf16x4(f, h, l, e);
+        reinterpret_cast<uint2*>(out)[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+        reinterpret_cast<uint2*>(out + rows * k)[i] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+        if (parts == 3) reinterpret_cast<uint2*>(out + 2 * rows * k)[i] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
     }
 }
 

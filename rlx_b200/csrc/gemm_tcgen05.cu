@@ -769,7 +769,8 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
             // off the free -> store -> MMA chain.
             const uint32_t s0 = s, ph0 = fph;
             s += 4;
-            while (s >= NS) { s -= NS; fph ^= 1u; }
+            if (s >= NS) { s -= NS; fph ^= 1u; }
+            if (PRECISE && s >= NS) { s -= NS; fph ^= 1u; }          // (three stages)
             auto stage_of = [&](uint32_t sub, uint32_t& st, uint32_t& sph) {
                 st = s0 + sub;
                 sph = ph0;

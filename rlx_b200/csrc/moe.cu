@@ -250,13 +250,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict_
             const float4 v = in[c];
             const float f[4] = {v.x, v.y, v.z, v.w};
             uint32_t h[4], l[4], e[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                h[q] = bf16_hi_bits(f[q]);
-                const float rest = isfinite(f[q]) ? f[q] - __uint_as_float(h[q] << 16) : 0.f;
-                l[q] = f32_to_bf16_bits(rest) & 0xFFFFu;
-                e[q] = f32_to_bf16_bits(rest - __uint_as_float(l[q] << 16)) & 0xFFFFu;
-            }
+            split_bf16x4(f, h, l, e);
             hi[c] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
             lo[c] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
             if (parts == 3) last[c] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
