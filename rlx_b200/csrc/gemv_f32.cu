@@ -366,6 +366,26 @@ __global__ void __launch_bounds__(kF32MaxWarps * 32, 1) gemv_f32_kernel(const __
             float v = 0.f;
             for (uint32_t c = 0; c < nwarps; ++c) v += rb[(i * nwarps + c) * MR + r];
             if (m0 + r < P.m) {
+                if constexpr (F32Lane<SCHEME, MR, LW>::NEEDS_SUM) {
+                    // An infinite activation makes infinities of the products and of the minima, and NaN of their difference.
+                    // Weight by weight it is the infinity of its weight's sign: once more, out of the way of the main loop.
+                    if (v != v && !none) {
+                        v = 0.f;
+                        const uint8_t* row = w + (uint64_t)(r0 + b * kF32Batch + i) * P.row_bytes;
+                        constexpr uint32_t E = SchemeTraits<SCHEME>::kElems, B = SchemeTraits<SCHEME>::kBytes;
+#pragma unroll 1
+                        for (uint32_t el = 0; el < P.k; el += 4) {
+                            const float4 wv = decode4_exact<SCHEME>(row + (uint64_t)(el / E) * B, el % E);
+                            const float wf[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+                            for (uint32_t q = 0; q < 4; ++q) {
+                                const size_t xi = (size_t)(m0 + r) * P.k + el + q;
+                                v = fmaf(wf[q], P.x_bf16 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(P.x)[xi])
+                                                         : reinterpret_cast<const float*>(P.x)[xi], v);
+                            }
+                        }
+                    }
+                }
                 const size_t out = (size_t)(m0 + r) * P.n + r0 + b * kF32Batch + i;
                 if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[out] = (uint16_t)f32_to_bf16_bits(v);
                 else reinterpret_cast<float*>(P.y)[out] = v;

@@ -71,6 +71,25 @@ def test_expert_rows_of_odd_lengths_in_one_launch(sch, m, k, n, E):
     assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("sch,m,k,n,E", [("q4_k", 10, 3072, 96, 4), ("q5_k", 12, 1792, 70, 3), ("q6_k", 10, 1280, 96, 4), ("q8_0", 5, 2080, 50, 2),
+                                         ("q4_0", 9, 544, 50, 2)])
+def test_expert_rows_with_values_that_are_not_finite(sch, m, k, n, E):
+    import torch
+    import rlx_b200 as R
+    s, w, x, _ = _inputs(sch, m, k, n * E, False, 170 + m)
+    x[0, 3], x[1, k - 1], x[2, 40], x[2, 300], x[3, 77] = np.inf, -np.inf, np.inf, -np.inf, np.nan
+    idx = (np.arange(m) % E).astype(np.float32)
+    before = R.launch_count()
+    y = R.grouped_matmul(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), torch.from_numpy(idx).cuda(), s, n, E).cpu().numpy()
+    assert R.launch_count() - before == 1                      # the streaming GEMV took them
+    with np.errstate(invalid="ignore"):
+        ref = O.grouped_matmul_bt(x, w, idx, m, k, n, E, s)
+    assert np.array_equal(np.isnan(y), np.isnan(ref)) and np.isinf(ref).any()
+    assert np.array_equal(y[np.isinf(ref)], ref[np.isinf(ref)])
+    fin = np.isfinite(ref)
+    assert np.abs(y[fin] - ref[fin]).max() <= 1e-5 * np.abs(ref[fin]).max()
+
+
 @pytest.mark.parametrize("sch,m,k,n,x_bf16", [("q6_k", 9, 256, 130, False), ("q6_k", 300, 2304, 128, True), ("q8_0", 33, 288, 77, True),
                                               ("q4_0", 40, 4128, 257, False), ("q8_0", 130, 1056, 64, False), ("q5_0", 20, 96, 40, True),
                                               ("q2_k", 17, 768, 40, False), ("q3_k", 12, 512, 136, True)])
