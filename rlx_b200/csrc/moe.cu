@@ -26,7 +26,7 @@
 //                       stored at the rows' original positions
 // The weight operand is bf16(d * q) there, as in the dense GEMM; for fewer than 32 rows, and rows of those other lengths,
 // it is the f32 weight, in three bf16 parts.
-// All of them are launched as programmatic dependents.  1024 rows over 8 experts of 4096 -> 14336 Q4_K: 190 us; 331 us
+// All of them are launched as programmatic dependents.  1024 rows over 8 experts of 4096 -> 14336 Q4_K: 196 us; 331 us
 // with fixed 128-row tiles, an f32 result array and a scatter kernel behind the GEMM.
 //
 // Decode (m <= 8 rows, Q4_0 / Q8_0 / Q4_K / Q5_K / Q6_K, k a multiple of 256 up to 12288) skips both kernels:
@@ -209,18 +209,28 @@ static uint32_t moe_tile_rows(uint32_t m, uint32_t E, uint32_t most) {
     return want < 32u ? 32u : (want > most ? most : want);
 }
 
-// Whether m rows are cheaper row by row (the f32 GEMV: every row reads its expert's slab, about 0.25 us per million weights,
-// and nothing goes in front of it) than as a GEMM (sort, gather and PRECISE weights: 14 us, and 0.5 us for each 64 columns of
-// each wave of 128-row weight tiles of the experts in use).  GEMV and GEMM measured: 4 x 7424 x 640 Q5_K E16 11 and 73 us,
-// 12 x 1792 x 8320 Q5_K E16 63 and 76 us, 10 x 3072 x 576 Q4_K E16 8 and 34 us, 20 x 2816 x 6720 Q8_0 E16 96 and 118 us.
+// Whether m rows are cheaper row by row (the f32 GEMV: every row reads its expert's slab, so many us per million weights, and
+// nothing goes in front of it) than as a GEMM on f32 weights (sort, gather: 14 us, so many us for each 64 columns of each wave
+// of 128-row weight tiles of the experts in use, and a copy of their slabs where TMA cannot tile the rows).  The constants are
+// fits to 56 shapes, 9 to 31 rows, both ways timed: the choice takes 0.4 % longer than the better one in the geometric mean, 20 %
+// at worst.  GEMV and GEMM: 10 x 3072 x 576 Q4_K E16 8 and 34 us, 12 x 7168 x 11840 Q8_0 E4 244 and 346 us, 24 x 4352 x 5632 Q4_0 E16
+// 146 and 222 us, 27 x 2560 x 5440 Q4_0 E4 88 and 69 us, 22 x 4352 x 3200 Q5_K E4 124 and 70 us.
 // Batches that the GEMM multiplies in bf16 (kMoeBf16Rows and more) stay with it.
-static bool moe_rows_stream(uint32_t m, uint32_t k, uint32_t n, uint32_t E) {
+static bool moe_rows_stream(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool relaid) {
     if (m <= kMoeDecodeRows) return true;
     if (m >= kMoeBf16Rows) return false;
-    const float stream_us = 4.0f + 0.25e-6f * (float)m * (float)k * (float)n;
+    float row = 0.32f, block = 1.0f;                    // Q6_K; a block is paced by the decoder, which makes three bf16 parts
+    if (scheme == RLXQ_Q4_0) { row = 0.215f; block = 0.65f; }          // (two)
+    else if (scheme == RLXQ_Q8_0) row = 0.22f;
+    else if (scheme == RLXQ_Q4_K) { row = 0.265f; block = 0.78f; }
+    else if (scheme == RLXQ_Q5_K) { row = 0.31f; block = 0.8f; }
+    const float stream_us = 4.0f + row * 1e-6f * (float)m * (float)k * (float)n;
     const float used = (float)E * (1.0f - powf(1.0f - 1.0f / (float)E, (float)m));
     const float waves = ceilf(ceilf((float)n / 128.0f) * used / (float)sm_count());
-    return stream_us < 14.0f + waves * (float)(k / 64) * 0.5f;
+    Geometry g;
+    geometry(scheme, &g);
+    const float copy_us = relaid ? used * (float)n * (float)(k / g.elems * g.bytes) * 2.0f / 4.5e6f : 0.0f;
+    return stream_us < 14.0f + waves * (float)(k / 64) * block + copy_us;
 }
 
 // One CTA per sorted position i: row perm[i] of x becomes row i of xg, as bf16 hi and, for f32 activations, lo part (m
@@ -305,7 +315,8 @@ static MoePlan plan_moe(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uin
         if (need > p.bytes) p.bytes = need;
         return p;
     }
-    if (gemv == 0 && options().gemm_kernel.load() == 0 && gemv_f32_supported(scheme, 1, k, x) && moe_rows_stream(m, k, n, E)) {
+    if (gemv == 0 && options().gemm_kernel.load() == 0 && gemv_f32_supported(scheme, 1, k, x) &&
+        moe_rows_stream(scheme, m, k, n, E, !gemm_tc_supported(scheme, m, k, n, w, x))) {
         p.route = MoeRoute::Stream;
         return p;
     }
