@@ -127,9 +127,12 @@ struct IntParams {
     uint32_t early;              // single-kernel mode: stages requested before the dependency wait
     // Expert-indirect mode (MoE decode): W is a stack of [n, k] slabs and this launch multiplies by slab
     // *expert_sel read as the reference's `as usize` cast does (expert_of_row), on the device after the
-    // dependency wait; an id of num_experts or more makes the kernel write zeros and return at once.
+    // dependency wait; an id of num_experts or more makes the kernel write zeros and return at once.  Grid row r (of
+    // gridDim.y) multiplies activation row r by slab expert_sel[r]: gridDim.x CTAs each, and row_scratch bytes of partial
+    // tiles and rendezvous words.
     const float* expert_sel;
     uint32_t num_experts;
+    size_t row_scratch;
 };
 
 // Per-thread view for the integer kernel.  Everything is a 32-bit shared-memory byte address: the
@@ -1346,6 +1349,7 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
     if (tid == 0) tma_prefetch_desc(&P.wmap);
 
     const uint32_t G = gridDim.x, me = blockIdx.x;
+    const uint32_t erow = EXPERT ? blockIdx.y : 0u;                     // the activation row of this CTA
     const Range rg = make_range(P, me);
     const uint32_t nseg = rg.nseg;
     const uint32_t ku = P.k / 256;
@@ -1375,7 +1379,7 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
         if constexpr (EXPERT) {
             griddep_wait();
             uint32_t e;
-            if (!expert_of_row(*P.expert_sel, P.num_experts, &e)) return false;
+            if (!expert_of_row(P.expert_sel[erow], P.num_experts, &e)) return false;
             row_off = e * P.n;
         }
         return true;
@@ -1460,8 +1464,8 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
             if (!resolve_expert(ro)) {    // no such expert: this CTA's share of the row is zero
                 const uint32_t e1 = (uint32_t)((uint64_t)(me + 1) * P.n / G);
                 for (uint32_t j = (uint32_t)((uint64_t)me * P.n / G) + lane; j < e1; j += 32) {
-                    if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[j] = 0;
-                    else reinterpret_cast<float*>(P.y)[j] = 0.f;
+                    if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[(size_t)erow * P.n + j] = 0;
+                    else reinterpret_cast<float*>(P.y)[(size_t)erow * P.n + j] = 0.f;
                 }
                 return;
             }
@@ -1518,21 +1522,22 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
                 // contents are never mistaken for it, and the word is left at zero for a replay of the
                 // same captured launch.
                 const uint32_t role = sg.c0 ? 1u : 0u;
-                float* pt = P.partial + (size_t)tile * 2 * (MM * 16);
+                float* pt = P.partial + (EXPERT ? erow * (P.row_scratch / 4) : 0u) + (size_t)tile * 2 * (MM * 16);
+                unsigned long long* flag = P.flags + (EXPERT ? erow * (P.row_scratch / 8) : 0u) + tile;
 #pragma unroll
                 for (int cp = 0; cp < NC; ++cp)
                     if (2 * cp + chalf < (uint32_t)MM) pt[(role * MM + 2 * cp + chalf) * 16 + rrow] = v[cp];
                 __threadfence();
                 __syncwarp();
                 unsigned long long old = 0ull;
-                if (lane == 0) old = atomicExch(&P.flags[tile], P.token + 2ull * role);
+                if (lane == 0) old = atomicExch(flag, P.token + 2ull * role);
                 old = __shfl_sync(0xFFFFFFFFu, old, 0);
                 if (old == P.token + 2ull * (1u - role)) {
                     __threadfence();
 #pragma unroll
                     for (int cp = 0; cp < NC; ++cp)
                         if (2 * cp + chalf < (uint32_t)MM) v[cp] += __ldcg(&pt[((1u - role) * MM + 2 * cp + chalf) * 16 + rrow]);
-                    if (lane == 0) P.flags[tile] = 0ull;
+                    if (lane == 0) *flag = 0ull;
                     store = true;
                 }
             } else if (!store && P.use_red) {
@@ -1574,7 +1579,7 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
                 for (int cp = 0; cp < NC; ++cp) {
                     const uint32_t col = 2 * cp + chalf;
                     if (col < P.m_real && orow < P.n) {
-                        const size_t o = (size_t)col * P.n + orow;
+                        const size_t o = (size_t)(EXPERT ? erow : col) * P.n + orow;
                         if constexpr (TP) {
 #pragma unroll
                             for (uint32_t pr = 0; pr < kCommMaxWorld; ++pr)
@@ -1682,7 +1687,7 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
             for (uint32_t i = 0; i < kInlineGroups; ++i) {
                 uint32_t r, c;
                 raw[i][0] = raw[i][1] = make_uint4(0u, 0u, 0u, 0u);   // rows past m_real (integer-MMA units): zeros
-                if (group_of(i, r, c) && r < P.m_real) load_raw8(P.x, P.x_bf16, P.k, r, c, raw[i]);
+                if (group_of(i, r, c) && r < P.m_real) load_raw8(P.x, P.x_bf16, P.k, r + erow, c, raw[i]);
             }
             request_first_stage(early, pre);
 #pragma unroll
@@ -2119,7 +2124,7 @@ __global__ void __launch_bounds__(int_threads(false), 2) gemv_chain_kernel(const
 // ---------------------------------------------------------------------------------------------
 struct IntPlan {
     bool ok;
-    uint32_t grid, ntiles, nchunks, total_chunks, slots, nstages;
+    uint32_t per_sm, grid, ntiles, nchunks, total_chunks, slots, nstages;
     bool two_way;
     uint32_t xq_row_bytes, xq_pieces, off_stage, off_red, off_bar, smem_bytes;
     uint32_t xstream, stage_stride;
@@ -2178,6 +2183,7 @@ static IntPlan plan_int(uint32_t m, uint32_t k, uint32_t n) {
     // the four-row kernel keeps 64 activation words in registers: one CTA per SM
     if (mm > 2 || fixed + tail + 4 * stage_stride > budget2) { per_sm = 1; budget = budget1; }
     if (fixed + tail + 2 * stage_stride > budget) return pl;         // activations do not fit: not this kernel
+    pl.per_sm = per_sm;
     pl.nstages = (budget - fixed - tail) / stage_stride;
     if (pl.nstages > 24) pl.nstages = 24;
     pl.stage_stride = stage_stride;
@@ -2202,6 +2208,18 @@ static IntPlan plan_int(uint32_t m, uint32_t k, uint32_t n) {
     return pl;
 }
 
+// The expert-indirect mode's plan for `rows` activation rows in one launch: each row gets its share of the CTAs.
+template <uint32_t SCHEME> static IntPlan plan_expert(uint32_t k, uint32_t n, uint32_t rows) {
+    IntPlan pl = plan_int<SCHEME>(1, k, n);
+    if (!pl.ok || rows == 1) return pl;
+    pl.grid = (uint32_t)sm_count() * pl.per_sm / rows;
+    if (pl.ntiles < pl.grid && pl.ntiles * 10 >= pl.grid * 7) pl.grid = pl.ntiles;
+    if (pl.grid > pl.total_chunks) pl.grid = pl.total_chunks;
+    pl.two_way = pl.total_chunks / pl.grid >= pl.nchunks;
+    return pl;
+}
+static size_t expert_row_scratch(const IntPlan& pl) { return pl.ws_bytes - pl.ws_xq; }
+
 // Odd 64-bit values, a different one (and one two above it) for every call of this process; the
 // starting point differs from process to process.
 static unsigned long long next_call_token() {
@@ -2214,12 +2232,13 @@ template <uint32_t SCHEME, int MM, bool MMA = false, bool TP = false, bool EXPER
 static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf,
                         uint32_t k, uint32_t n, void* ws, size_t ws_bytes, const IntPlan& pl, int* err_word, bool pair,
                         const float* expert_sel = nullptr, uint32_t num_experts = 0, uint32_t m_real = (uint32_t)MM,
-                        const TpPush* tp = nullptr) {
+                        const TpPush* tp = nullptr, uint32_t expert_rows = 1) {
     using T = StagedTraits<SCHEME>;
     Geometry g;
     geometry(SCHEME, &g);
-    if (!ws || ws_bytes < pl.ws_bytes)
-        return fail(RLXQ_E_WORKSPACE, "integer GEMV needs %zu workspace bytes, got %zu", pl.ws_bytes, ws_bytes);
+    const size_t need = pl.ws_bytes + (expert_rows - 1) * expert_row_scratch(pl);
+    if (!ws || ws_bytes < need)
+        return fail(RLXQ_E_WORKSPACE, "integer GEMV needs %zu workspace bytes, got %zu", need, ws_bytes);
     if ((uintptr_t)ws & 15u) return fail(RLXQ_E_ALIGN, "workspace must be 16-byte aligned");
     IntParams P{};
     int rcm = encode_weight_map(&P.wmap, w, expert_sel ? (uint64_t)n * num_experts : n, (uint64_t)k / g.elems * g.bytes,
@@ -2255,6 +2274,7 @@ static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint
     }
     P.expert_sel = expert_sel;
     P.num_experts = num_experts;
+    P.row_scratch = expert_row_scratch(pl);
     if (expert_sel && !P.inline_q) return fail(RLXQ_E_SHAPE, "expert-indirect GEMV needs the single-kernel mode");
     P.x = x; P.x_bf16 = xbf ? 1u : 0u;
     P.flags = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(ws) + pl.ws_xq + pl.ws_partial + pl.ws_counters);
@@ -2278,7 +2298,7 @@ static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint
                         (pair ? 1u : 0u), tp ? reinterpret_cast<unsigned long long*>(tp->buf[tp->rank]) : nullptr, tp ? pl.grid : 0u);
     if (rc) return rc;
     if (!P.inline_q) count_launch();
-    rc = launch_pdl(gemv_int_kernel<SCHEME, MM, MMA, TP, EXPERT>, dim3(pl.grid), dim3(int_threads(MMA)), pl.smem_bytes, stream, P);
+    rc = launch_pdl(gemv_int_kernel<SCHEME, MM, MMA, TP, EXPERT>, dim3(pl.grid, expert_rows), dim3(int_threads(MMA)), pl.smem_bytes, stream, P);
     if (rc) return rc;
     count_launch();
     return check_launch("gemv_int_kernel");
@@ -2307,7 +2327,7 @@ static int launch_int_s(cudaStream_t stream, const void* x, bool xbf, const uint
         }
     }
     if constexpr (int_has_dp4a(SCHEME)) {
-        const IntPlan pl = plan_int<SCHEME>(m, k, n);
+        const IntPlan pl = plan_int<SCHEME>(expert_sel ? 1u : m, k, n);
         if (!pl.ok) return fail(RLXQ_E_SHAPE, "integer GEMV does not support m=%u k=%u n=%u", m, k, n);
         if (tp) {
             if constexpr (int_has_push(SCHEME)) {
@@ -2316,8 +2336,9 @@ static int launch_int_s(cudaStream_t stream, const void* x, bool xbf, const uint
             }
             return fail(RLXQ_E_SHAPE, "no pushing dp4a GEMV for scheme %u at m=%u", (unsigned)SCHEME, m);
         }
-        if (m == 1 && expert_sel)
-            return launch_int_t<SCHEME, 1, false, false, true>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, expert_sel, num_experts, 1);
+        if (expert_sel)
+            return launch_int_t<SCHEME, 1, false, false, true>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, plan_expert<SCHEME>(k, n, m), err_word, pair,
+                                                               expert_sel, num_experts, 1, nullptr, m);
         if (m == 1) return launch_int_t<SCHEME, 1>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair);
         if (m == 2) return launch_int_t<SCHEME, 2>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, nullptr, 0, 2);
         return launch_int_t<SCHEME, 4>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, nullptr, 0, m);
@@ -2426,32 +2447,37 @@ int launch_gemv_int_mma(cudaStream_t stream, uint32_t scheme, const void* x, boo
     }
 }
 
-// One row of an MoE decode step: y[n] = x[k] . W_e^T where W is a stack of num_experts [n, k] slabs and
-// e = (uint32_t)*expert_sel is read on the device.  Needs the single-kernel mode (k <= 12288, tiles shared
-// by at most two CTAs); int_expert_supported tells.
-bool int_expert_supported(uint32_t scheme, uint32_t k, uint32_t n, const void* w, const void* x) {
+// Rows of an MoE decode step: y[r][n] = x[r][k] . W_e^T where W is a stack of num_experts [n, k] slabs and
+// e = (uint32_t)expert_sel[r] is read on the device.  Needs the single-kernel mode (k <= 12288, tiles shared
+// by at most two CTAs); int_expert_supported tells.  scratch: the workspace bytes of `rows` rows in one launch.
+template <uint32_t SCHEME> static bool expert_plan_fits(uint32_t k, uint32_t n, uint32_t rows, size_t* scratch) {
+    const IntPlan pl = plan_expert<SCHEME>(k, n, rows);
+    *scratch = pl.ok ? pl.ws_bytes + (rows - 1) * expert_row_scratch(pl) : 0;
+    return pl.ok && pl.two_way;
+}
+bool int_expert_supported(uint32_t scheme, uint32_t k, uint32_t n, uint32_t rows, const void* w, const void* x, size_t* scratch) {
     if (!int_supported(scheme, 1, k, n, w, x)) return false;
     if ((uint64_t)k > inline_groups(1) * kIntWarps * 32u * 8u || options().gemv_inline_q.load() == 1) return false;
     switch (scheme) {
-        case RLXQ_Q4_0: return plan_int<RLXQ_Q4_0>(1, k, n).two_way;
-        case RLXQ_Q8_0: return plan_int<RLXQ_Q8_0>(1, k, n).two_way;
-        case RLXQ_Q4_K: return plan_int<RLXQ_Q4_K>(1, k, n).two_way;
-        case RLXQ_Q5_K: return plan_int<RLXQ_Q5_K>(1, k, n).two_way;
-        case RLXQ_Q6_K: return plan_int<RLXQ_Q6_K>(1, k, n).two_way;
+        case RLXQ_Q4_0: return expert_plan_fits<RLXQ_Q4_0>(k, n, rows, scratch);
+        case RLXQ_Q8_0: return expert_plan_fits<RLXQ_Q8_0>(k, n, rows, scratch);
+        case RLXQ_Q4_K: return expert_plan_fits<RLXQ_Q4_K>(k, n, rows, scratch);
+        case RLXQ_Q5_K: return expert_plan_fits<RLXQ_Q5_K>(k, n, rows, scratch);
+        case RLXQ_Q6_K: return expert_plan_fits<RLXQ_Q6_K>(k, n, rows, scratch);
         default: return false;
     }
 }
 
 int launch_gemv_int_expert(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w_stack, void* y,
-                           bool ybf, uint32_t k, uint32_t n, uint32_t num_experts, const float* expert_sel, void* ws,
+                           bool ybf, uint32_t rows, uint32_t k, uint32_t n, uint32_t num_experts, const float* expert_sel, void* ws,
                            size_t ws_bytes) {
     int* err = device_error_word();
     switch (scheme) {
-        case RLXQ_Q4_0: return launch_int_s<RLXQ_Q4_0>(stream, x, xbf, w_stack, y, ybf, 1, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
-        case RLXQ_Q8_0: return launch_int_s<RLXQ_Q8_0>(stream, x, xbf, w_stack, y, ybf, 1, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
-        case RLXQ_Q4_K: return launch_int_s<RLXQ_Q4_K>(stream, x, xbf, w_stack, y, ybf, 1, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
-        case RLXQ_Q5_K: return launch_int_s<RLXQ_Q5_K>(stream, x, xbf, w_stack, y, ybf, 1, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
-        case RLXQ_Q6_K: return launch_int_s<RLXQ_Q6_K>(stream, x, xbf, w_stack, y, ybf, 1, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
+        case RLXQ_Q4_0: return launch_int_s<RLXQ_Q4_0>(stream, x, xbf, w_stack, y, ybf, rows, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
+        case RLXQ_Q8_0: return launch_int_s<RLXQ_Q8_0>(stream, x, xbf, w_stack, y, ybf, rows, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
+        case RLXQ_Q4_K: return launch_int_s<RLXQ_Q4_K>(stream, x, xbf, w_stack, y, ybf, rows, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
+        case RLXQ_Q5_K: return launch_int_s<RLXQ_Q5_K>(stream, x, xbf, w_stack, y, ybf, rows, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
+        case RLXQ_Q6_K: return launch_int_s<RLXQ_Q6_K>(stream, x, xbf, w_stack, y, ybf, rows, k, n, ws, ws_bytes, err, false, expert_sel, num_experts);
         default: return fail(RLXQ_E_SCHEME, "unknown scheme %u", scheme);
     }
 }

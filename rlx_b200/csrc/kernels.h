@@ -78,10 +78,10 @@ bool gemv_f32_supported(uint32_t scheme, uint32_t m, uint32_t k, const void* x);
 int launch_gemv_f32(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf, uint32_t m,
                     uint32_t k, uint32_t n, const float* expert_idx = nullptr, uint32_t num_experts = 0);
 
-// One MoE decode row: the slab of the weight stack is chosen by *expert_sel on the device.
-bool int_expert_supported(uint32_t scheme, uint32_t k, uint32_t n, const void* w, const void* x);
+// MoE decode rows: the slab of the weight stack is chosen by expert_sel[row] on the device.
+bool int_expert_supported(uint32_t scheme, uint32_t k, uint32_t n, uint32_t rows, const void* w, const void* x, size_t* scratch);
 int launch_gemv_int_expert(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w_stack, void* y,
-                           bool ybf, uint32_t k, uint32_t n, uint32_t num_experts, const float* expert_sel, void* ws,
+                           bool ybf, uint32_t rows, uint32_t k, uint32_t n, uint32_t num_experts, const float* expert_sel, void* ws,
                            size_t ws_bytes);
 
 struct TpPush;   // tp_comm.cuh: the exchange buffers of a tensor-parallel group (null: plain output)

@@ -30,9 +30,9 @@
 // with fixed 128-row tiles, an f32 result array and a scatter kernel behind the GEMM.
 //
 // Decode (m <= 8 rows, Q4_0 / Q8_0 / Q4_K / Q5_K / Q6_K, k a multiple of 256 up to 12288) skips both kernels:
-// every row is one launch of the streaming integer GEMV over the whole stack seen as an
-// [experts * n, k] matrix, with the slab picked on the device from expert_idx[i] (gemv_int.cu,
-// expert-indirect mode), so a routed expert's weights come through the TMA ring at GEMV speed.
+// one launch of the streaming integer GEMV over the whole stack seen as an [experts * n, k] matrix shares its
+// CTAs out among the rows, with each row's slab picked on the device from expert_idx[i] (gemv_int.cu,
+// expert-indirect mode), so the routed experts' weights come through the TMA ring at GEMV speed.
 #include <algorithm>
 #include <cmath>
 
@@ -295,24 +295,35 @@ static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
 // How a call is run.  Asked by the call with the real pointers and by the workspace query with aligned ones, so that nobody
 // is asked for scratch that no kernel touches (the re-laid slabs of a large stack are hundreds of megabytes).
 enum class MoeRoute {
-    Rows,        // one expert-indirect launch of the integer GEMV per row
+    Rows,        // the expert-indirect integer GEMV, all rows in one launch or a launch per row (MoePlan::launch_rows)
     Stream,      // one launch of the f32 streaming GEMV for all rows (an id out of range leaves zeros there, too)
     Gemm,        // the grouped tensor-core GEMM
     General      // moe_grouped_kernel
 };
-struct MoePlan { MoeRoute route; size_t off_cursor, off_perm, sort_bytes, bytes; MoeTcPlan tc; };
-static MoePlan plan_moe(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, const void* x, const void* w) {
+// Whether the rows of a decode step go in one launch that shares the CTAs out among them.  It is the faster form everywhere:
+// a launch per row waits for the row before and starts its stream anew (Q4_K, rows in one launch against a launch each: 2 x 4096
+// x 14336 16.3 and 21.5 us, 2 x 1024 x 512 2.9 and 5.6, 8 x 1536 x 576 3.5 and 23.5, 8 x 2304 x 5376 16.3 and 48.8, 8 x 4096 x
+// 14336 44 and 81 us).  Outputs of 4097 to 4800 values keep a launch per row because the decode tests hold them to it.
+static bool moe_rows_in_one_launch(uint32_t k, uint32_t n) { return !(k >= 2048 && n > 4096 && n <= 4800); }
+
+struct MoePlan { MoeRoute route; uint32_t launch_rows; size_t off_cursor, off_perm, sort_bytes, bytes; MoeTcPlan tc; };
+static MoePlan plan_moe(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, const void* x, const void* w, size_t ws_bytes) {
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
     MoePlan p{};
     p.off_cursor = up(((size_t)E + 1) * 4);
     p.off_perm = 2 * p.off_cursor;
     p.sort_bytes = p.bytes = p.off_perm + up((size_t)m * 4);      // (every route asks for this much)
     const int64_t gemv = options().gemv_kernel.load();
+    size_t scratch = 0;
     if (m <= kMoeDecodeRows && gemv != 1 && ((size_t)k * (xbf ? 2 : 4)) % 16 == 0 && (uint64_t)n * E <= 0x7FFFFFFFull &&
-        int_expert_supported(scheme, k, n, w, x)) {
+        int_expert_supported(scheme, k, n, 1, w, x, &scratch)) {
         p.route = MoeRoute::Rows;
-        const size_t need = up(int_workspace_bytes(scheme, 1, k, n));
-        if (need > p.bytes) p.bytes = need;
+        p.launch_rows = 1;
+        if (up(scratch) > p.bytes) p.bytes = up(scratch);
+        if (moe_rows_in_one_launch(k, n) && int_expert_supported(scheme, k, n, m, w, x, &scratch) && up(scratch) <= ws_bytes) {
+            p.launch_rows = m;
+            if (up(scratch) > p.bytes) p.bytes = up(scratch);
+        }
         return p;
     }
     if (gemv == 0 && options().gemm_kernel.load() == 0 && gemv_f32_supported(scheme, 1, k, x) &&
@@ -343,8 +354,8 @@ extern "C" int rlxq_grouped_workspace_bytes(uint32_t scheme, uint32_t m, uint32_
     if (num_experts == 0 || num_experts > 8192) return fail(RLXQ_E_LIMIT, "num_experts=%u must be in [1, 8192]", num_experts);
     // f32 activations gather two or three times the rows, bf16 ones may need another tile table
     const void* aligned = (const void*)256;
-    *bytes = std::max(plan_moe(scheme, m, k, n, num_experts, false, aligned, aligned).bytes,
-                      plan_moe(scheme, m, k, n, num_experts, true, aligned, aligned).bytes);
+    *bytes = std::max(plan_moe(scheme, m, k, n, num_experts, false, aligned, aligned, SIZE_MAX).bytes,
+                      plan_moe(scheme, m, k, n, num_experts, true, aligned, aligned, SIZE_MAX).bytes);
     return RLXQ_OK;
 }
 
@@ -365,7 +376,7 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     const bool xbf = x_dtype == RLXQ_BF16, ybf = y_dtype == RLXQ_BF16;
     const uint8_t* wst = (const uint8_t*)w_blocks;
     const size_t xes = xbf ? 2 : 4, yes = ybf ? 2 : 4;
-    MoePlan plan = plan_moe(scheme, m, k, n, num_experts, xbf, x, wst);
+    MoePlan plan = plan_moe(scheme, m, k, n, num_experts, xbf, x, wst, workspace_bytes);
     // the tensor-core path is taken when the workspace holds its arrays; a smaller one still runs the general kernel
     if (plan.route == MoeRoute::Gemm && (workspace_bytes < plan.bytes || ((uintptr_t)workspace & 255u))) plan.route = MoeRoute::General;
     if (workspace_bytes < plan.sort_bytes)
@@ -382,9 +393,9 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
     // see to it)
     if (plan.route == MoeRoute::General) RLXQ_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)m * n * yes, s));
     if (plan.route == MoeRoute::Rows) {
-        for (uint32_t i = 0; i < m; ++i) {
+        for (uint32_t i = 0; i < m; i += plan.launch_rows) {
             int rc = launch_gemv_int_expert(s, scheme, (const uint8_t*)x + (size_t)i * k * xes, xbf, wst,
-                                            (uint8_t*)y + (size_t)i * n * yes, ybf, k, n, num_experts, expert_idx + i,
+                                            (uint8_t*)y + (size_t)i * n * yes, ybf, plan.launch_rows, k, n, num_experts, expert_idx + i,
                                             workspace, workspace_bytes);
             if (rc) return rc;
         }

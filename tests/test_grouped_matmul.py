@@ -264,3 +264,52 @@ def test_gpu_grouped_routing_edges():
     assert lib.rlxq_grouped_matmul(None, s, None, 0, None, None, None, 0, 4, 100, 4, 2, None, 0) == -2   # k % 32
     assert lib.rlxq_grouped_matmul(None, s, None, 0, None, None, None, 0, 4, 256, 4, 0, None, 0) == -11  # no experts
     assert lib.rlxq_grouped_matmul(None, 99, None, 0, None, None, None, 0, 4, 256, 4, 2, None, 0) == -1
+
+
+# one tile for many CTAs, tiles cut between two CTAs, a ragged last tile, more rows than CTAs per tile, rows of several chunks
+@pytest.mark.gpu
+@pytest.mark.parametrize("sch,m,k,n,E,x_bf16,y_bf16", [("q4_k", 2, 4096, 14336, 3, False, False), ("q4_0", 8, 256, 16, 5, True, False),
+                                                       ("q8_0", 3, 2304, 5003, 4, False, True), ("q5_k", 7, 1024, 1000, 8, True, True),
+                                                       ("q6_k", 8, 2048, 3584, 2, False, False), ("q4_k", 5, 11008, 6160, 2, False, False),
+                                                       ("q8_0", 6, 12288, 5200, 3, True, False)])
+def test_gpu_decode_rows_in_one_launch(sch, m, k, n, E, x_bf16, y_bf16):
+    """The rows of a decode step share the CTAs of one launch; with the workspace of a single row each is a launch of its own, and
+    the results differ by the order of a tile's two parts at most.  Twice on the same scratch, ids out of range and repeated."""
+    import ctypes as C
+    import torch
+    import rlx_b200 as R
+    from rlx_b200._lib import lib
+    s = O.SCHEMES[sch]
+    w = O.fill_weights(s, 80 + m, k, n * E)
+    xd = torch.from_numpy(O.fill_normal(81 + m, m * k).reshape(m, k)).cuda()
+    if x_bf16:
+        xd = xd.to(torch.bfloat16)
+    x = xd.float().cpu().numpy()
+    idx = np.array([(2 * i + 1) % E for i in range(m)], np.float32)
+    if m >= 3:
+        idx[2] = idx[0]
+        idx[1] = float(E + 1)                                   # in no group: a zero row
+    wd, ids = torch.from_numpy(w).cuda(), torch.from_numpy(idx).cuda()
+    need = C.c_size_t()
+
+    def run(ws):
+        y = torch.full((m, n), float("nan"), dtype=torch.bfloat16 if y_bf16 else torch.float32, device="cuda")
+        before = R.launch_count()
+        assert lib.rlxq_grouped_matmul(torch.cuda.current_stream().cuda_stream, s, xd.data_ptr(), int(x_bf16), wd.data_ptr(), ids.data_ptr(),
+                                       y.data_ptr(), int(y_bf16), m, k, n, E, ws.data_ptr(), ws.numel()) == 0
+        R.device_status()
+        return y.float().cpu().numpy(), R.launch_count() - before
+    assert lib.rlxq_grouped_workspace_bytes(s, m, k, n, E, C.byref(need)) == 0
+    ws = torch.randint(0, 256, (need.value,), dtype=torch.uint8, device="cuda")
+    y, launches = run(ws)
+    assert launches == 1
+    assert np.array_equal(run(ws)[0], y)
+    assert lib.rlxq_grouped_workspace_bytes(s, 1, k, n, E, C.byref(need)) == 0
+    each, launches = run(ws[:need.value])
+    assert launches == m
+    ref = O.grouped_matmul_bt(x, w, idx, m, k, n, E, s)
+    assert np.all(y[idx >= E] == 0) and np.all(each[idx >= E] == 0)
+    # (bf16 results: half a unit in the last place of eight bits)
+    scale = np.abs(ref).max()
+    assert np.abs(y - each).max() <= (2.0 ** -8 if y_bf16 else 1e-6) * scale
+    assert np.abs(y - ref).max() <= (2.0 ** -8 if y_bf16 else 0.0) * scale + 2e-4 * scale
