@@ -38,7 +38,7 @@ static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_
     p.chunk = (uint32_t)chunk;
     p.off_w = xbf ? 0 : al((size_t)gemm_x_parts(true, p.relaid) * chunk * k * 2);
     p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;
-    p.off_y2 = p.off_w + al((size_t)(p.pitch * n));
+    p.off_y2 = p.off_w + (p.relaid ? al((size_t)gemm_relaid_bytes(scheme, k, n)) : 0);
     p.off_gemm = p.off_y2 + (p.halves ? al((size_t)2 * chunk * n * 4) : 0);
     p.bytes = p.off_gemm;
     if (!p.halves) {
@@ -140,9 +140,7 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
         GemmCall c{};
         c.w = w; c.w_pitch = p.pitch; c.precise = p.relaid; c.k = k; c.n = n;
         if (p.relaid) {
-            Geometry g;
-            geometry(scheme, &g);
-            int rc = launch_relay_rows(stream, w, (uint64_t)k / g.elems * g.bytes, n, base + p.off_w, p.pitch);
+            int rc = launch_relay(stream, scheme, w, k, n, base + p.off_w);
             if (rc) return rc;
             c.w = base + p.off_w;
         }

@@ -215,4 +215,93 @@ int launch_relay_rows(cudaStream_t stream, const uint8_t* w, uint64_t row_bytes,
     return check_launch("relay_rows_kernel");
 }
 
+// Q6_K rows for the GEMM on f32 weights: a super-block (ql[128] | qh[64] | sc[16] | d, 210 bytes that start on any even byte)
+// becomes 272 bytes, its quants 0 .. 63 one a byte in the order of the weights, then its scale bytes, and 2^12 d goes to
+// d_out[group][row].  The decoders, which read a row once per tile of activations, then find whole aligned words.  A warp takes
+// four super-blocks at a time, which lie one after the other whatever rows they belong to, in 16-byte loads, and picks them
+// apart in shared memory, eight weights a lane; HBM-bound like the copy above.
+__global__ void __launch_bounds__(256) widen_q6_kernel(const uint8_t* __restrict__ w, uint32_t groups, uint64_t n, uint8_t* __restrict__ out,
+                                                       float* __restrict__ d_out, const uint32_t* __restrict__ used, uint32_t slab_rows) {
+    constexpr uint32_t kAtOnce = 4, kChunks = (kAtOnce * 210 + 14 + 15) / 16;
+    __shared__ __align__(16) uint8_t buf[8][kChunks * 16 + 16];       // (a word past the last d)
+    griddep_launch_dependents();
+    griddep_wait();
+    const uint32_t lane = threadIdx.x & 31u;
+    uint8_t* const mine = buf[threadIdx.x >> 5];
+    const uint64_t items = groups * n, step = (uint64_t)gridDim.x * (blockDim.x >> 5) * kAtOnce;
+    const uintptr_t base = reinterpret_cast<uintptr_t>(w), end = base + items * 210u;
+    // lane: weights 8 lane .. of the super-block = half h, group g of 32, bytes l .. l + 7 of it
+    const uint32_t h = lane >> 4, g = (lane >> 2) & 3u, l = 8 * (lane & 3u);
+    const uint32_t ql = 64 * h + 32 * (g & 1u) + l, qh = 128 + 32 * h + l, nib = 4 * (g >> 1);
+    auto skip = [&](uint64_t it, uint32_t count) {             // nobody is routed to the slab (or to either of two)
+        return used && used[(uint32_t)((it + count - 1) / groups / slab_rows) + 1] == used[(uint32_t)(it / groups / slab_rows)];
+    };
+    auto fetch = [&](uint64_t it, uint4 (&v)[2]) {             // a lane's two chunks of the super-blocks from `it` on
+        if (it >= items) return;
+        const uint32_t count = (uint32_t)min((uint64_t)kAtOnce, items - it);
+        if (skip(it, count)) return;
+        const uintptr_t src = base + it * 210u, a0 = src & ~(uintptr_t)15;
+        const uint32_t chunks = ((uint32_t)(src - a0) + count * 210u + 15u) / 16u;
+#pragma unroll
+        for (uint32_t t = 0; t < 2; ++t) {
+            const uintptr_t a = a0 + 16 * (lane + 32 * t);
+            if (lane + 32 * t >= chunks) continue;
+            if (a >= base && a + 16 <= end) {
+                v[t] = __ldg(reinterpret_cast<const uint4*>(a));
+            } else {                                           // the ends of the weights: what lies inside
+                uint32_t q[8];
+                for (uint32_t i = 0; i < 8; ++i) q[i] = a + 2 * i >= base && a + 2 * i + 2 <= end ? __ldg(reinterpret_cast<const uint16_t*>(a + 2 * i)) : 0u;
+                v[t] = make_uint4(q[0] | (q[1] << 16), q[2] | (q[3] << 16), q[4] | (q[5] << 16), q[6] | (q[7] << 16));
+            }
+        }
+    };
+    uint64_t it = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kAtOnce;
+    uint4 ahead[2] = {};
+    fetch(it, ahead);
+    for (; it < items; it += step) {
+        const uint32_t count = (uint32_t)min((uint64_t)kAtOnce, items - it), lead = (uint32_t)((base + it * 210u) & 15u);
+        __syncwarp();
+#pragma unroll
+        for (uint32_t t = 0; t < 2; ++t)
+            if (lane + 32 * t < kChunks) *reinterpret_cast<uint4*>(mine + 16 * (lane + 32 * t)) = ahead[t];
+        __syncwarp();
+        fetch(it + step, ahead);                               // on its way while these are picked apart
+        if (skip(it, count)) continue;
+        uint64_t r = items <= 0xFFFFFFFFull ? (uint32_t)it / groups : it / groups;
+        uint32_t gi = (uint32_t)(it - r * groups);
+#pragma unroll
+        for (uint32_t i = 0; i < kAtOnce; ++i) {
+            if (i >= count) break;
+            // (every offset below is a multiple of four: one shift for the whole super-block)
+            const uint32_t at = lead + 210u * i, sh = (at & 2u) * 8u;
+            const uint32_t* p = reinterpret_cast<const uint32_t*>(mine + (at & ~3u));
+            const uint32_t a0 = p[ql / 4], a1 = p[ql / 4 + 1], a2 = p[ql / 4 + 2], b0 = p[qh / 4], b1 = p[qh / 4 + 1], b2 = p[qh / 4 + 2];
+            const uint32_t v0 = ((__funnelshift_r(a0, a1, sh) >> nib) & 0x0F0F0F0Fu) | (((__funnelshift_r(b0, b1, sh) >> (2 * g)) & 0x03030303u) << 4);
+            const uint32_t v1 = ((__funnelshift_r(a1, a2, sh) >> nib) & 0x0F0F0F0Fu) | (((__funnelshift_r(b1, b2, sh) >> (2 * g)) & 0x03030303u) << 4);
+            uint8_t* dst = out + (it + i) * 272u;
+            reinterpret_cast<uint2*>(dst)[lane] = make_uint2(v0, v1);
+            if (lane < 5) {                                    // four words of scales, d
+                const uint32_t u = __funnelshift_r(p[48 + lane], p[49 + lane], sh);
+                if (lane < 4) reinterpret_cast<uint32_t*>(dst + 256)[lane] = u;
+                else d_out[(uint64_t)gi * n + r] = f16_bits_to_f32(u & 0xFFFFu) * 0x1p12f;
+            }
+            if (++gi == groups) { gi = 0; ++r; }
+        }
+    }
+}
+
+int launch_widen_q6(cudaStream_t stream, const uint8_t* w, uint32_t k, uint64_t n, uint8_t* out, const uint32_t* used, uint32_t slab_rows) {
+    if (n == 0 || k == 0) return RLXQ_OK;
+    if (((uintptr_t)w & 1u) || ((uintptr_t)out & 15u) || k % 256) return fail(RLXQ_E_ALIGN, "widen_q6: bad alignment");
+    const uint32_t groups = k / 256;
+    uint64_t blocks = (groups * n + 31) / 32;
+    const uint64_t cap = (uint64_t)sm_count() * 8;
+    if (blocks > cap) blocks = cap;
+    int rc = launch_pdl(widen_q6_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, w, groups, n, out,
+                        reinterpret_cast<float*>(out + (uint64_t)groups * 272u * n), used, slab_rows);
+    if (rc) return rc;
+    count_launch();
+    return check_launch("widen_q6_kernel");
+}
+
 }  // namespace rlxq

@@ -42,6 +42,8 @@ constexpr uint32_t kGemmBK = 64;        // k per pipeline stage (one 128-byte sw
 constexpr uint32_t kGemmMaxStages = 8;  // B shared-memory stages == A tensor-memory stages (8 x 32 columns)
 constexpr uint32_t kGemmMaxRaw = 8;     // raw weight boxes (256 weights of 128 rows each): what shared memory is left for
 constexpr uint32_t kGemmRawStages = 2;  // the paired kernel's
+// Q6_K rows as widen_q6_kernel re-lays them: 256 bytes of quants in order, 16 scale bytes; the super-blocks' d apart.
+constexpr uint32_t kQ6Wide = 0x100u + RLXQ_Q6_K;
 
 // ---- weight decode: 64 consecutive weights of one row -> 32 bf16 pairs ------------------------
 // The raw box holds 256 weights of 128 rows; RAW_ROW bytes per row (an odd number of 16-byte
@@ -69,6 +71,7 @@ template <> struct GemmRaw<RLXQ_Q5_1> { static constexpr uint32_t ROW = 208, GRO
 // boundary, a 304-byte box (19 chunks) covers 12 + 292.
 template <> struct GemmRaw<RLXQ_Q8_K> { static constexpr uint32_t ROW = 304, GROUPS = 2; };
 template <> struct GemmRaw<RLXQ_Q3_K> { static constexpr uint32_t ROW = 144, GROUPS = 3; };
+template <> struct GemmRaw<kQ6Wide> { static constexpr uint32_t ROW = 272, GROUPS = 2; };
 template <uint32_t SCHEME> __device__ __forceinline__ uint32_t gemm_raw_x(uint32_t g) {   // box start, 8-byte elements
     if (SCHEME == RLXQ_Q6_K) return ((210u * g) & ~15u) / 8u;
     if (SCHEME == RLXQ_Q2_K) return ((84u * g) & ~15u) / 8u;
@@ -107,8 +110,10 @@ template <bool PRECISE> struct GemmOut {
 };
 // An f32 weight is the sum of three bf16 values: the upper half of its bits, of what that leaves behind, and of what is
 // left then, all of it exact (one byte-permute per pair and part; a conversion instruction would pace the decoder).
-// Q4_0's weights (f16 scale times four bits: 15) are two such parts.
-constexpr uint32_t gemm_weight_parts(uint32_t scheme) { return scheme == RLXQ_Q4_0 ? 2u : 3u; }
+// Q4_0's weights (f16 scale times four bits: 15) are two such parts, and so are re-laid Q6_K's without the
+// super-block's scale (sub-block scale times six bits: 13), which is left to the epilogue (gemm_late_scale).
+constexpr bool gemm_late_scale(uint32_t scheme) { return scheme == kQ6Wide; }
+constexpr uint32_t gemm_weight_parts(uint32_t scheme) { return scheme == RLXQ_Q4_0 || gemm_late_scale(scheme) ? 2u : 3u; }
 template <> struct GemmOut<true> {
     uint64_t f[32];
     __device__ __forceinline__ void put(int i, uint64_t pair) { f[i] = pair; }
@@ -123,6 +128,23 @@ template <> struct GemmOut<true> {
     }
 };
 
+// Weights without a scale of their group, as two bf16 parts that the decoder forms itself, 32 at a time.
+struct GemmOutTwo { uint32_t hi[16], lo[16]; };
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
 template <uint32_t SCHEME, int S> struct Decode64;
 
 // Words of a row buffer at compile-time byte offsets: loads the 16-byte chunks covering [B0, B0 + LEN)
@@ -394,7 +416,7 @@ __device__ __forceinline__ void decode64(const uint8_t* row, uint32_t g, Out& v)
 // formats, whose odd parts start one word later): four unrolled copies of 250 instructions left a quarter of the decode
 // warps' time to instruction fetch.  The other formats keep unrolled copies (Decode64).
 constexpr bool gemm_part_loop(uint32_t scheme) {
-    return scheme == RLXQ_Q4_0 || scheme == RLXQ_Q8_0 || scheme == RLXQ_Q4_K || scheme == RLXQ_Q5_K || scheme == RLXQ_Q6_K;
+    return scheme == RLXQ_Q4_0 || scheme == RLXQ_Q8_0 || scheme == RLXQ_Q4_K || scheme == RLXQ_Q5_K || scheme == RLXQ_Q6_K || scheme == kQ6Wide;
 }
 // Words [0, N) from word GRP + 2 * high on of the chunks at p.
 template <int N, uint32_t GRP> __device__ __forceinline__ void words_from(const uint8_t* p, bool high, uint32_t (&q)[N]) {
@@ -476,10 +498,35 @@ __device__ __forceinline__ void decode_k45(const uint8_t* row, uint32_t S, Out& 
     }
 }
 
+// Half H of part S of a widened Q6_K row, without d and times 2^-12: sub-block scale (8 bits) times quant (6 bits), rounded to
+// bf16, and what the rounding left (4 bits): a product, and a fused multiply-add that takes the rounded one off again, both
+// exact.  2^-12 keeps a product within the activation's range.
+__device__ __forceinline__ void decode_q6_wide(const uint8_t* row, uint32_t S, int H, GemmOutTwo& v) {
+    const uint32_t scw = *reinterpret_cast<const uint16_t*>(row + 256 + 4 * S + 2 * H) ^ 0x8080u;  // int8 -> s + 128
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {                            // sixteen weights of one scale
+        const float f = u8_minus<128>((scw >> (8 * i)) & 0xFFu) * 0x1p-12f;
+        const uint32_t s2 = __byte_perm(__float_as_uint(f), 0u, 0x3232);
+        const uint4 t = *reinterpret_cast<const uint4*>(row + 64 * S + 32 * H + 16 * i);
+        const uint32_t q[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            // 0x43 over a byte below 128 is the bf16 128 + byte; less 160
+            const uint32_t w = sub_bf16x2(__byte_perm(q[j / 2], 0x43434343u, j & 1 ? 0x4342 : 0x4140), 0x43204320u);
+            const uint32_t r = mul_bf16x2(s2, w);
+            v.hi[8 * i + j] = r;
+            v.lo[8 * i + j] = fma_bf16x2(s2, w, r ^ 0x80008000u);
+        }
+    }
+}
+
 // ---- kernel -----------------------------------------------------------------------------------
 // B TMA, MMA, raw TMA, spare | decode | epilogue.  The block's real size goes into the launch bounds: with two decode
 // groups a thread may then use 128 registers, and the decoders keep a row's loads and 32 (PRECISE: 64) results in flight.
-constexpr uint32_t gemm_threads(uint32_t groups) { return (4 + 4 * groups + 4) * 32; }
+constexpr uint32_t gemm_threads(uint32_t groups, uint32_t epilogue = 4) { return (4 + 4 * groups + epilogue) * 32; }
+// Epilogue warps: two for each quarter of the rows, half of the tile's columns each, where every fourth block's products have to
+// be scaled and added (gemm_late_scale); their decoder fits the 96 registers a thread that leaves.
+constexpr uint32_t gemm_epilogue_warps(uint32_t scheme, bool precise) { return precise && gemm_late_scale(scheme) ? 8u : 4u; }
 // warp roles: 0 = activation (B) TMA producer, 1 = MMA issuer and tensor-memory owner,
 // 2 = raw weight TMA producer, 3 = idle, then GROUPS x 4 decode warps (tensor-memory lane quarter =
 // warp % 4), then 4 epilogue warps (lane quarter = warp % 4).
@@ -496,7 +543,11 @@ struct GemmParams {
     // rows behind them; a stage carries both boxes and both are multiplied by the same decoded weights into the same
     // accumulator, so a weight is decoded once for the two halves.
     uint32_t lo_row, xparts;
-    uint32_t main_run, sum_run;    // PRECISE: k blocks the main accumulator takes at a time, and the sums; powers of two (gemm_main_run)
+    // PRECISE: k blocks a main accumulator takes at a time, the accumulator of the lower products, and the sums; powers of two
+    // (gemm_main_run).  nmain, ncross: accumulators of either kind, used in turn.
+    uint32_t main_run, cross_run, sum_run, nmain, ncross;
+    const float* late;      // gemm_late_scale: 2^12 d of the groups of the stack's rows, [k group][row], late_rows rows
+    size_t late_rows;
     uint32_t nstages, nraw;               // depth of the operand ring (B in shared memory, A in tensor memory) and of the raw ring
     uint32_t b_bytes;                     // bytes of a B stage: tx * 128, twice that with lo_row
     uint32_t w_late;       // the weights are written by a kernel in front (re-laid rows): read them after the dependency wait
@@ -584,11 +635,11 @@ __device__ __forceinline__ uint32_t gemm_arrive(unsigned long long* word, unsign
         old = prev;
     }
 }
-// Barrier of the four epilogue warps that tells all of them whether any thread passed true.
-__device__ __forceinline__ bool epilogue_any(bool v) {
+// Barrier of the epilogue warps that tells all of them whether any thread passed true.
+template <uint32_t THREADS = 128> __device__ __forceinline__ bool epilogue_any(bool v) {
     uint32_t r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                 : "=r"(r) : "r"((uint32_t)v) : "memory");
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)v), "n"(THREADS) : "memory");
     return r != 0u;
 }
 
@@ -718,10 +769,14 @@ __device__ __noinline__ void gemm_reduce_parts(const GemmParams& P, uint32_t til
     }
 }
 
+// tensor-memory columns of a weight stage
+constexpr uint32_t gemm_a_cols(uint32_t scheme, bool precise) { return precise ? 32u * gemm_weight_parts(scheme) : 32u; }
+
 struct GemmBars {
-    uint64_t b_full[kGemmMaxStages], a_full[kGemmMaxStages], stage_free[kGemmMaxStages];
+    // full: a stage's activations (their bytes) and its weights (four decode warps) are there: one barrier to look at for both
+    uint64_t full[kGemmMaxStages], stage_free[kGemmMaxStages];
     uint64_t raw_full[kGemmMaxRaw], raw_empty[kGemmMaxRaw];
-    uint64_t d_full[2], d_free[2];
+    uint64_t d_full[4], d_free[4];        // two accumulators (PRECISE: two for the leading product, two for the others)
     uint32_t tmem_base, abort_flag, epi_prev, epi_prev1;   // epi_prev, epi_prev1: arrival counts of alternate segments
 };
 
@@ -732,7 +787,8 @@ template <uint32_t SCHEME, bool PRECISE, uint32_t GRP>
 __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* bars, const uint8_t* raw_stage, uint32_t tmem_a,
                                                  uint32_t xtiles, uint32_t warp, uint32_t lane) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW, GROUPS = GemmRaw<SCHEME>::GROUPS;
-    constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128, A_COLS = PRECISE ? 96 : 32;
+    constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128, A_COLS = gemm_a_cols(SCHEME, PRECISE);
+    constexpr bool LATE = PRECISE && gemm_late_scale(SCHEME);
     volatile uint32_t* abort_flag = &bars->abort_flag;
     auto give_up = [&](int code) {
         atomicExch(P.err, code);
@@ -776,11 +832,18 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
                 sph = ph0;
                 if (st >= NS) { st -= NS; sph ^= 1u; }
             };
-            auto store = [&](uint32_t st, uint32_t sph, uint32_t ready, GemmOut<PRECISE>& v) -> bool {
+            using Out = std::conditional_t<LATE, GemmOutTwo[2], GemmOut<PRECISE>>;
+            auto store = [&](uint32_t st, uint32_t sph, uint32_t ready, Out& v) -> bool {
                 announce();
                 if (!__all_sync(0xFFFFFFFFu, ready) && (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[st]), sph))) { give_up(16); return false; }
                 tc_fence_after();
-                if constexpr (PRECISE) {
+                if constexpr (LATE) {
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        tmem_st16(tmem_a + lane_addr + A_COLS * st + 16 * h, v[h].hi);
+                        tmem_st16(tmem_a + lane_addr + A_COLS * st + 32 + 16 * h, v[h].lo);
+                    }
+                } else if constexpr (PRECISE) {
 #pragma unroll
                     for (uint32_t q = 0; q < gemm_weight_parts(SCHEME); ++q) {
                         uint32_t p[32];
@@ -790,7 +853,7 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
                 } else {
                     tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
                 }
-                pending = smem_u32(&bars->a_full[st]);
+                pending = smem_u32(&bars->full[st]);
                 return true;
             };
             uint32_t st, sph;
@@ -802,8 +865,9 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
                     const uint32_t sub = SCHEME == RLXQ_Q6_K ? 2 * grp + p : grp + 2 * p;
                     stage_of(sub, st, sph);
                     const uint32_t ready = mbar_test(smem_u32(&bars->stage_free[st]), sph);    // answered while decoding
-                    GemmOut<PRECISE> v;
-                    if constexpr (SCHEME == RLXQ_Q6_K) hf.decode(p, v);
+                    Out v;
+                    if constexpr (LATE) { decode_q6_wide(rp, sub, 0, v[0]); decode_q6_wide(rp, sub, 1, v[1]); }
+                    else if constexpr (SCHEME == RLXQ_Q6_K) hf.decode(p, v);
                     else if constexpr (SCHEME == RLXQ_Q4_K || SCHEME == RLXQ_Q5_K) decode_k45<SCHEME>(rp, sub, v);
                     else decode_blocks32<SCHEME, GRP>(rp, p, v);
                     if (!store(st, sph, ready, v)) return;
@@ -849,8 +913,15 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
 // the other products run.  Those are 2^-8 of the whole and smaller: they pile up in the second accumulator.  Every sum_run
 // blocks it joins the sums, and these move on to totals in shared memory, so that no chain of additions is long.  Error
 // against 64 bits, general kernel and this one, f32 activations: k = 256 8.1e-8 and 8.0e-8, 2304 1.6e-7 and 9.8e-8, 11008
-// 3.3e-7 and 1.4e-7, 16128 4.0e-7 and 1.5e-7.  300 x 11008 x 4096 Q6_K f32 4787 us (general kernel) and 240 us; with long
-// accumulations 218 us (L2 cold).
+// 3.3e-7 and 1.4e-7, 16128 4.0e-7 and 1.5e-7.
+// Re-laid Q6_K rows (gemm_late_scale) are multiplied without their super-blocks' scale, as two parts instead of three: five
+// products for f32 activations and two for bf16 ones, a decoder of four packed instructions a pair of weights on aligned words,
+// and the scale applied by the epilogue warps, eight of them, as they add a super-block's sums.  Two threads issue MMAs, for the
+// leading product and for the others: beside the products a round of hand-overs takes one thread 0.4 us, whatever else is left
+// out (loads, decoding, adding).  Second accumulators of either kind are worth 5 to 9 %.  300 x 11008 x 4096 f32 222 us with three
+// parts, 172 with two, 187 with aligned rows from a slow first pass, 173 with barriers looked at before a round's last MMAs, 148 with two
+// issuers and a faster first pass; bf16 184 and 107; 587 x 1280 x 5568 bf16 68 and 38 us, 31 x 13056 x 17990 f32 272 and 208 us.
+// Error against 64 bits at k = 11008 1.5e-7 and 1.2e-7.
 // Activation rows of a PRECISE tile: what the epilogue threads have registers for (Q3_K's block is larger: 96 a thread) and
 // shared memory has room for totals beside three operand stages and two raw boxes (Q8_K's are the largest).
 constexpr uint32_t gemm_precise_rows(uint32_t scheme) { return scheme == RLXQ_Q3_K || scheme == RLXQ_Q8_K ? 64u : 96u; }
@@ -862,29 +933,33 @@ constexpr uint32_t gemm_precise_rows(uint32_t scheme) { return scheme == RLXQ_Q3
 // bf16 takes 220, 236 and 243 us with main runs of 4, 2 and 1, 236, 261 and 300 us with sums of 16, 8 and 4 blocks.
 // A result that is stored as bf16 has the error of that rounding, 1.655e-3, the same to six digits with the general kernel and
 // with runs of 16 blocks (9e-7 before it is rounded); 300 x 11040 x 4096 Q8_0 bf16 204 us.
-static uint32_t gemm_main_run(uint32_t k, bool ybf) { return ybf ? 16u : k >= 20480 ? 4u : k >= 5632 ? 2u : 1u; }
+static uint32_t gemm_main_run(uint32_t scheme, uint32_t k, bool ybf) {
+    const uint32_t most = gemm_late_scale(scheme) ? 4u : 16u;           // (a group's blocks share a scale)
+    return std::min(most, ybf ? 16u : k >= 20480 ? 4u : k >= 5632 ? 2u : 1u);
+}
 static uint32_t gemm_sum_run(uint32_t k, bool ybf) { return ybf || k >= 5632 ? 16u : k >= 2048 ? 8u : 4u; }
 
 // TX = P.tx: no branch between the additions of a block, which are on the chain from one block's product to the next.
 template <uint32_t SCHEME, uint32_t TX>
 __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmBars* bars, float* total, uint32_t tmem_d,
                                                       uint32_t xtiles, uint32_t warp, uint32_t lane) {
+    constexpr bool LATE = gemm_late_scale(SCHEME);
+    constexpr uint32_t EW = gemm_epilogue_warps(SCHEME, true), CHUNKS = (TX / 16 + EW / 4 - 1) / (EW / 4);    // chunks of 16 columns of a warp
     const uint32_t quarter = warp & 3u, row = quarter * 32 + lane, epi_tid = (warp - (4 + 4 * GemmRaw<SCHEME>::GROUPS)) * 32 + lane;
-    const uint32_t main_d = tmem_d + ((quarter * 32) << 16), cross_d = main_d + TX;
-    uint32_t mph = 0, cph = 0;
+    const uint32_t main_d = tmem_d + ((quarter * 32) << 16), cross_d = main_d + TX * (LATE ? P.nmain : 1u), chunk0 = EW == 8 && epi_tid >= 128 ? CHUNKS : 0u;
+    uint32_t mph = 0, cph = 0, mb = 0, cb = 0;
     uint32_t cur, lim;
     gemm_seg_init(P, xtiles, cur, lim);
     GemmSeg sg;
     while (gemm_seg_next(P, cur, lim, sg)) {
         const GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
         const uint32_t rows = tr.xlim - tr.xrow0, blocks = 4 * (sg.g1 - sg.g0);
-        auto wait_for = [&](uint32_t d, uint32_t& ph) -> bool {
+        auto wait_for = [&](uint32_t d, uint32_t ph) -> bool {
             if (!mbar_wait(smem_u32(&bars->d_full[d]), ph)) {
                 atomicExch(P.err, 17);
                 *reinterpret_cast<volatile uint32_t*>(&bars->abort_flag) = 1u;
                 return false;
             }
-            ph ^= 1u;
             tc_fence_after();
             return true;
         };
@@ -896,39 +971,64 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
         bool ok = true;
 #pragma unroll 1
         for (uint32_t k0 = 0; ok && k0 < blocks; k0 += P.sum_run) {
-            uint64_t sum[TX / 2];                            // pairs of activation rows
+            uint64_t sum[8 * CHUNKS];                        // pairs of activation rows
 #pragma unroll
-            for (uint32_t j = 0; j < TX / 2; ++j) sum[j] = 0ull;
+            for (uint32_t j = 0; j < 8 * CHUNKS; ++j) sum[j] = 0ull;
+            uint64_t scale = 0ull;                           // LATE: of the group (2^12 d), twice
             auto add_accumulator = [&](uint32_t acc, bool cross) {
 #pragma unroll
-                for (uint32_t c = 0; c < TX / 16; ++c) {
+                for (uint32_t c = 0; c < CHUNKS; ++c) {
+                    if (CHUNKS * (EW / 4) > TX / 16 && chunk0 + c >= TX / 16) break;
                     uint32_t v[16];
-                    tmem_ld16(acc + 16 * c, v);
+                    tmem_ld16(acc + 16 * (chunk0 + c), v);
                     tmem_ld_wait();
                     // An infinite activation times a lower weight part that is zero is a NaN in there.  The main accumulator then
                     // has the infinity (or the NaN) that the product is: its weight part is zero only where the weight is.
+                    if (LATE && cross) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j) {
+                            const uint64_t p = mul_f32x2(f32x2(v[2 * j], v[2 * j + 1]), scale);
+                            asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(p));
+                        }
+                    }
                     if (cross) {
 #pragma unroll
-                        for (uint32_t j = 0; j < 16; ++j) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), -3.402823466e38f));
+                        for (uint32_t j = 0; j < 16; ++j) {
+                            float f = fmaxf(__uint_as_float(v[j]), -3.402823466e38f);
+                            if (LATE) f = fminf(f, 3.402823466e38f);             // (a rounded weight's second part may have the other sign)
+                            v[j] = __float_as_uint(f);
+                        }
                     }
 #pragma unroll
-                    for (uint32_t j = 0; j < 8; ++j) sum[8 * c + j] = add_f32x2(sum[8 * c + j], f32x2(v[2 * j], v[2 * j + 1]));
+                    for (uint32_t j = 0; j < 8; ++j) {
+                        if (LATE && !cross) sum[8 * c + j] = fma_f32x2(f32x2(v[2 * j], v[2 * j + 1]), scale, sum[8 * c + j]);
+                        else sum[8 * c + j] = add_f32x2(sum[8 * c + j], f32x2(v[2 * j], v[2 * j + 1]));
+                    }
                 }
             };
             const uint32_t k1 = min(blocks, k0 + P.sum_run);
 #pragma unroll 1
-            for (uint32_t kb = k0; kb < k1; kb += P.main_run) {
-                if (!(ok = wait_for(0, mph))) break;
-                add_accumulator(main_d, false);
-                release(0);
+            for (uint32_t kc = k0; ok && kc < k1; kc += LATE ? P.cross_run : k1 - k0) {
+                const uint32_t k2 = LATE ? min(k1, kc + P.cross_run) : k1;
+                if (LATE) scale = f32x2_splat(tr.wt * kGemmTileW + row < P.n ? __ldcg(P.late + (size_t)(sg.g0 + kc / 4) * P.late_rows + tr.wrow0 + row) : 0.f);
+#pragma unroll 1
+                for (uint32_t kb = kc; kb < k2; kb += P.main_run) {
+                    if (!(ok = wait_for(mb, mph))) break;
+                    add_accumulator(main_d + mb * TX, false);
+                    release(mb);
+                    if (!LATE || ++mb == P.nmain) { mb = 0; mph ^= 1u; }
+                }
+                if (!ok || !(ok = wait_for(2 + cb, cph))) break;
+                add_accumulator(cross_d + cb * TX, true);
+                release(2 + cb);
+                if (!LATE || ++cb == P.ncross) { cb = 0; cph ^= 1u; }
             }
-            if (!ok || !(ok = wait_for(1, cph))) break;
-            add_accumulator(cross_d, true);
-            release(1);
+            if (!ok) break;
             // totals [activation row][weight row]: a thread's own column of them, sixteen loads before the first store
 #pragma unroll
-            for (uint32_t c = 0; c < TX / 16; ++c) {
-                float* t = total + 16 * c * kGemmTileW + row;
+            for (uint32_t c = 0; c < CHUNKS; ++c) {
+                if (CHUNKS * (EW / 4) > TX / 16 && chunk0 + c >= TX / 16) break;
+                float* t = total + 16 * (chunk0 + c) * kGemmTileW + row;
                 float old[16];
 #pragma unroll
                 for (uint32_t j = 0; j < 16; ++j) old[j] = k0 ? t[j * kGemmTileW] : 0.f;
@@ -941,13 +1041,13 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
                 }
             }
         }
-        // the four warps leave together: they share the barriers
-        if (epilogue_any(!ok || *reinterpret_cast<volatile uint32_t*>(&bars->abort_flag))) break;
+        // the warps leave together: they share the barriers
+        if (epilogue_any<32 * EW>(!ok || *reinterpret_cast<volatile uint32_t*>(&bars->abort_flag))) break;
         uint8_t* const out = static_cast<uint8_t*>(P.y) + sg.slice * P.slice_elems * 4;
         const uint32_t n0 = tr.wt * kGemmTileW;
         const uint32_t ps = !P.y_vec ? 7u : P.y_bf16 ? 4u : 5u;      // a row of the tile is 2^ps pieces of 16 bytes, or values
 #pragma unroll 4
-        for (uint32_t p = epi_tid; p < rows << ps; p += 128) {
+        for (uint32_t p = epi_tid; p < rows << ps; p += 32 * EW) {
             const uint32_t j = p >> ps, c = (p & ((1u << ps) - 1u)) << (7u - ps), ni = n0 + c, mi = tr.xrow0 + j;
             if (ni >= P.n) continue;
             const size_t o = (size_t)(P.row_map ? __ldg(&P.row_map[mi]) : mi) * P.n + ni;
@@ -963,17 +1063,17 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
                 *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + o) = *reinterpret_cast<const float4*>(t);
             }
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");       // the totals have been read: the next tile's may be written
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");       // the totals have been read: the next tile's may be written
     }
 }
 
 template <uint32_t SCHEME, bool PRECISE>
-__global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P) {
+__global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS, gemm_epilogue_warps(SCHEME, PRECISE)), 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P) {
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
     constexpr uint32_t kGemmDecodeGroups = GemmRaw<SCHEME>::GROUPS;
     constexpr uint32_t RAW_BYTES = kGemmTileW * RAW_ROW;
     constexpr uint32_t RAW_STRIDE = (RAW_BYTES + 127) / 128 * 128;
-    constexpr uint32_t A_COLS = PRECISE ? 96 : 32;                    // tensor-memory columns of a weight stage
+    constexpr uint32_t A_COLS = gemm_a_cols(SCHEME, PRECISE);         // tensor-memory columns of a weight stage
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t NS = P.nstages, NR = P.nraw, B_BYTES = P.b_bytes;
@@ -988,22 +1088,21 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
 
     if (tid == 0) {
         for (uint32_t s = 0; s < NS; ++s) {
-            mbar_init(smem_u32(&bars->b_full[s]), 1);
-            mbar_init(smem_u32(&bars->a_full[s]), 4);
-            mbar_init(smem_u32(&bars->stage_free[s]), 1);
+            mbar_init(smem_u32(&bars->full[s]), 1 + 4);
+            mbar_init(smem_u32(&bars->stage_free[s]), PRECISE ? 2 : 1);
         }
         for (uint32_t r = 0; r < NR; ++r) {
             mbar_init(smem_u32(&bars->raw_full[r]), 1);
             mbar_init(smem_u32(&bars->raw_empty[r]), 4 * kGemmDecodeGroups);
         }
-        for (uint32_t b = 0; b < 2; ++b) {
+        for (uint32_t b = 0; b < 4; ++b) {
             mbar_init(smem_u32(&bars->d_full[b]), 1);
-            mbar_init(smem_u32(&bars->d_free[b]), 4);
+            mbar_init(smem_u32(&bars->d_free[b]), gemm_epilogue_warps(SCHEME, PRECISE));
         }
         bars->abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {               // the whole warp allocates all 512 columns: 256 (PRECISE: 2 tx) of accumulators, then weight stages
+    if (warp == 1) {               // the whole warp allocates all 512 columns: 256 (PRECISE: nmain + ncross of tx) of accumulators, then weight stages
         tmem_alloc(smem_u32(&bars->tmem_base), 512);
         tmem_relinquish();
     }
@@ -1011,7 +1110,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
-    const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + (PRECISE ? 2 * P.tx : 256);
+    const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + (PRECISE ? (P.nmain + P.ncross) * P.tx : 256);
     // up to 128 activation rows there are two accumulators: a tile's epilogue runs under the next tile's MMAs
     const uint32_t nacc = P.tx <= 128 ? 2u : 1u;
     auto give_up = [&](int code) {
@@ -1021,7 +1120,9 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
     // The weights may be requested while the kernel in front still runs; all else that is read from global memory
     // (or written) comes after the dependency wait.  In grouped mode the tile table does, too.
     if (P.groups) griddep_wait();
-    const uint32_t xtiles = P.groups ? __ldg(&P.groups[0]).x : P.xtiles;
+    // (A plain load: one through the read-only path may be moved up in front of the wait, and read the table before the kernel in
+    // front had written it.  The others' addresses depend on this one.)
+    const uint32_t xtiles = P.groups ? P.groups[0].x : P.xtiles;
 
     if (warp == 0) {
         // ---------------- activation tiles (B operand) ----------------
@@ -1037,7 +1138,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                 const GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
                 for (uint32_t kb = 4 * sg.g0; kb < 4 * sg.g1; ++kb) {
                     if (*abort_flag || !mbar_wait(smem_u32(&bars->stage_free[s]), ph)) { give_up(11); ok = false; break; }
-                    const uint32_t full = smem_u32(&bars->b_full[s]), dst = smem_u32(b_stage + s * B_BYTES);
+                    const uint32_t full = smem_u32(&bars->full[s]), dst = smem_u32(b_stage + s * B_BYTES);
                     mbar_arrive_expect_tx(full, B_BYTES);
                     tma_load_2d(dst, &P.xmap, (int32_t)(kb * kGemmBK), (int32_t)tr.xrow0, full);
                     for (uint32_t q = 1; q < P.xparts; ++q)
@@ -1067,89 +1168,112 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
                 }
             }
         }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
+    } else if (PRECISE && (warp == 1 || warp == 3)) {
+        // ---------------- MMA issuers: the leading product, and the others ----------------
+        // Two threads, because issue is what the rounds are made of: beside the products a round takes 0.4 us of one, whatever
+        // else is left out.  They use different accumulators, so neither waits for the other.
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((P.tx >> 3) << 17) | ((kGemmTileW >> 4) << 24);
-            uint32_t s = 0, ph = 0, d = 0, dph = 1, cph = 1;   // dph, cph: parities to wait for on d_free (1 passes the first time)
+            const bool lead = warp == 1;
+            const uint32_t run = lead ? P.main_run : P.cross_run, count = lead ? P.nmain : P.ncross, bar0 = lead ? 0u : 2u;
+            const uint32_t acc0 = tmem_d + (lead ? 0u : P.nmain * P.tx);
+            uint32_t s = 0, ph = 0, d = 0, dph = 1, acc = acc0;        // dph: parity to wait for on d_free (1 passes the first time)
             uint32_t cur, lim;
             gemm_seg_init(P, xtiles, cur, lim);
             GemmSeg sg;
             bool ok = true;
             while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
                 const uint32_t blocks = 4 * (sg.g1 - sg.g0);
-                if (!PRECISE) {
-                    if (!mbar_wait(smem_u32(&bars->d_free[d]), dph)) { give_up(13); break; }
+                // what a round waits for is looked at before the last MMAs of the round in front: an answer takes 118 cycles
+                uint32_t ready = mbar_test(smem_u32(&bars->full[s]), ph), free = mbar_test(smem_u32(&bars->d_free[bar0 + d]), dph);
+                for (uint32_t kb = 0; kb < blocks; ++kb) {    // the first MMA of a run overwrites the accumulator
+                    if (!ready && (*abort_flag || !mbar_wait(smem_u32(&bars->full[s]), ph))) { give_up(14); ok = false; break; }
+                    const uint32_t in_run = kb & (run - 1u);
+                    if (in_run == 0) {
+                        if (!free && (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[bar0 + d]), dph))) { give_up(13); ok = false; break; }
+                        acc = acc0 + d * P.tx;
+                    }
                     tc_fence_after();
-                }
-                const uint32_t acc = tmem_d + (PRECISE ? 0u : 128u * d);
-                uint32_t rb = mbar_test(smem_u32(&bars->b_full[s]), ph), ra = mbar_test(smem_u32(&bars->a_full[s]), ph);
-                for (uint32_t kb = 0; kb < blocks; ++kb) {    // the first MMA of a segment overwrites the accumulator
-                    if ((!rb && (*abort_flag || !mbar_wait(smem_u32(&bars->b_full[s]), ph))) ||
-                        (!ra && (*abort_flag || !mbar_wait(smem_u32(&bars->a_full[s]), ph)))) { give_up(14); ok = false; break; }
-                    tc_fence_after();
-                    // look at the next stage now: the answer arrives while this stage's MMAs are issued
                     const uint32_t sn = s + 1 == NS ? 0u : s + 1, phn = s + 1 == NS ? ph ^ 1u : ph;
-                    rb = mbar_test(smem_u32(&bars->b_full[sn]), phn);
-                    ra = mbar_test(smem_u32(&bars->a_full[sn]), phn);
+                    const bool last = in_run == run - 1u || kb == blocks - 1;
+                    const uint32_t dn = !last ? d : d + 1 == count ? 0u : d + 1, dphn = last && d + 1 == count ? dph ^ 1u : dph;
                     const uint64_t bdesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES));
                     const uint32_t a = tmem_a + A_COLS * s;
-                    if constexpr (PRECISE) {
-                        // weight part 0 by activation part 0, main_run blocks of them in the main accumulator
-                        const uint32_t in_run = kb & (P.main_run - 1u);
-                        if (in_run == 0) {
-                            if (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[0]), dph)) { give_up(13); ok = false; break; }
-                            dph ^= 1u;
-                            tc_fence_after();
-                        }
+                    auto look_ahead = [&] {
+                        ready = mbar_test(smem_u32(&bars->full[sn]), phn);
+                        if (last) free = mbar_test(smem_u32(&bars->d_free[bar0 + dn]), dphn);
+                    };
+                    if (lead) {          // weight part 0 by activation part 0
+                        look_ahead();
 #pragma unroll
                         for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, in_run | j ? 1u : 0u);
-                        if (in_run == P.main_run - 1u || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[0]));
-                        // parts 1, 2 by part 0, 0..1 by part 1, 0 by part 2; the three products left out are below 2^-24 of the whole
-                        const uint32_t cross = acc + P.tx;
-                        const bool fresh = (kb & (P.sum_run - 1u)) == 0;
-                        if (fresh) {
-                            if (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[1]), cph)) { give_up(13); ok = false; break; }
-                            cph ^= 1u;
-                            tc_fence_after();
-                        }
-#pragma unroll
-                        for (uint32_t j = 0; j < (gemm_weight_parts(SCHEME) - 1) * (kGemmBK / 16); ++j)
-                            tc_mma_ts(cross, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, fresh && j == 0 ? 0u : 1u);
+                    } else {             // parts 1, 2 by part 0, 0..1 by part 1, 0 by part 2; the products left out are below 2^-24 of the whole
                         for (uint32_t q = 1; q < P.xparts; ++q) {
                             const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
 #pragma unroll
-                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(cross, a + 8 * j, ldesc + 2 * j, idesc, 1u);
+                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, in_run | (q - 1u) | j ? 1u : 0u);
                             if (q == 1) {
 #pragma unroll
-                                for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(cross, a + 32 + 8 * j, ldesc + 2 * j, idesc, 1u);
+                                for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 32 + 8 * j, ldesc + 2 * j, idesc, 1u);
                             }
                         }
-                        if ((kb & (P.sum_run - 1u)) == P.sum_run - 1u || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[1]));
-                    } else {
+                        look_ahead();
 #pragma unroll
-                        for (uint32_t j = 0; j < kGemmBK / 16; ++j)
-                            tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, (kb | j) ? 1u : 0u);
-                        for (uint32_t q = 1; q < P.xparts; ++q) {
-                            const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
-#pragma unroll
-                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
-                        }
+                        for (uint32_t j = 0; j < (gemm_weight_parts(SCHEME) - 1) * (kGemmBK / 16); ++j)
+                            tc_mma_ts(acc, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, in_run | (P.xparts - 1u) | j ? 1u : 0u);
                     }
+                    if (last) tc_commit(smem_u32(&bars->d_full[bar0 + d]));
+                    tc_commit(smem_u32(&bars->stage_free[s]));     // frees the B stage and the A columns when both issuers' MMAs retire
+                    d = dn;
+                    dph = dphn;
+                    s = sn;
+                    ph = phn;
+                }
+            }
+        }
+    } else if (!PRECISE && warp == 1) {
+        // ---------------- MMA issuer ----------------
+        if (elect_one()) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((P.tx >> 3) << 17) | ((kGemmTileW >> 4) << 24);
+            uint32_t s = 0, ph = 0, d = 0, dph = 1;            // dph: parity to wait for on d_free (1 passes the first time)
+            uint32_t cur, lim;
+            gemm_seg_init(P, xtiles, cur, lim);
+            GemmSeg sg;
+            bool ok = true;
+            while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
+                const uint32_t blocks = 4 * (sg.g1 - sg.g0);
+                if (!mbar_wait(smem_u32(&bars->d_free[d]), dph)) { give_up(13); break; }
+                tc_fence_after();
+                const uint32_t acc = tmem_d + 128u * d;
+                uint32_t ready = mbar_test(smem_u32(&bars->full[s]), ph);
+                for (uint32_t kb = 0; kb < blocks; ++kb) {    // the first MMA of a segment overwrites the accumulator
+                    if (!ready && (*abort_flag || !mbar_wait(smem_u32(&bars->full[s]), ph))) { give_up(14); ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t sn = s + 1 == NS ? 0u : s + 1, phn = s + 1 == NS ? ph ^ 1u : ph;
+                    const uint64_t bdesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES));
+                    const uint32_t a = tmem_a + A_COLS * s;
+                    for (uint32_t q = 1; q < P.xparts; ++q) {
+                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
+#pragma unroll
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, (kb | j) ? 1u : 0u);
+                    }
+                    // The next stage is looked at before the round's last MMAs are issued: the answer takes 118 cycles, and arrives meanwhile.
+                    ready = mbar_test(smem_u32(&bars->full[sn]), phn);
+#pragma unroll
+                    for (uint32_t j = 0; j < kGemmBK / 16; ++j)
+                        tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, kb || j || P.xparts > 1u ? 1u : 0u);
                     tc_commit(smem_u32(&bars->stage_free[s]));     // frees the B stage and the A columns when the MMAs retire
                     s = sn;
                     ph = phn;
                 }
                 if (!ok) break;
-                if (!PRECISE) {
-                    tc_commit(smem_u32(&bars->d_full[d]));
-                    if (++d == nacc) { d = 0; dph ^= 1u; }
-                }
+                tc_commit(smem_u32(&bars->d_full[d]));
+                if (++d == nacc) { d = 0; dph ^= 1u; }
             }
         }
     } else if (warp >= 4 && warp < 4 + 4 * kGemmDecodeGroups) {
         // ---------------- decode ----------------
-        constexpr bool ONE = kGemmDecodeGroups != 2 || SCHEME == RLXQ_Q4_K || SCHEME == RLXQ_Q5_K || SCHEME == RLXQ_Q6_K;
+        constexpr bool ONE = kGemmDecodeGroups != 2 || SCHEME == RLXQ_Q4_K || SCHEME == RLXQ_Q5_K || SCHEME == RLXQ_Q6_K || SCHEME == kQ6Wide;
         if (ONE || warp < 8) gemm_decode_role<SCHEME, PRECISE, 0>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
         else gemm_decode_role<SCHEME, PRECISE, 1>(P, bars, raw_stage, tmem_a, xtiles, warp, lane);
         tmem_st_wait();                      // (after a timeout a store may still be on its way)
@@ -1160,7 +1284,10 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS), 1) gemm
             float* total = reinterpret_cast<float*>(epi_stage);
             if (P.tx == 32) gemm_precise_epilogue<SCHEME, 32>(P, bars, total, tmem_d, xtiles, warp, lane);
             else if (P.tx == 64) gemm_precise_epilogue<SCHEME, 64>(P, bars, total, tmem_d, xtiles, warp, lane);
-            else if constexpr (gemm_precise_rows(SCHEME) == 96) gemm_precise_epilogue<SCHEME, 96>(P, bars, total, tmem_d, xtiles, warp, lane);
+            else if constexpr (gemm_precise_rows(SCHEME) == 96) {
+                if (gemm_late_scale(SCHEME) && P.tx == 80) gemm_precise_epilogue<SCHEME, 80>(P, bars, total, tmem_d, xtiles, warp, lane);
+                else gemm_precise_epilogue<SCHEME, 96>(P, bars, total, tmem_d, xtiles, warp, lane);
+            }
         }
     } else if (!PRECISE && warp >= 4 + 4 * kGemmDecodeGroups) {
         // ---------------- epilogue: accumulator -> y (or -> a partial tile, completed by the last contributor) ----------------
@@ -1585,11 +1712,25 @@ bool gemm_tc_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, cons
 bool gemm_relaid_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* x) {
     return m != 0 && n != 0 && k != 0 && k % 32 == 0 && gemm_tc_format(scheme) && !((uintptr_t)x & 15u);
 }
-// Bytes from one re-laid row to the next: whole 256-weight groups (zero blocks past k), a multiple of 16.
+// Bytes from one re-laid row to the next: whole 256-weight groups (zero blocks past k), a multiple of 16; and bytes of `rows`
+// re-laid rows, with the scales that widened ones keep behind them.
 uint64_t gemm_relaid_pitch(uint32_t scheme, uint32_t k) {
+    if (scheme == RLXQ_Q6_K) return (uint64_t)(k / 256) * GemmRaw<kQ6Wide>::ROW;
     Geometry g;
     geometry(scheme, &g);
     return ((uint64_t)((k + 255) / 256) * (256 / g.elems) * g.bytes + 15) / 16 * 16;
+}
+
+uint64_t gemm_relaid_bytes(uint32_t scheme, uint32_t k, uint64_t rows) {
+    return gemm_relaid_pitch(scheme, k) * rows + (scheme == RLXQ_Q6_K ? (uint64_t)(k / 256) * rows * 4 : 0);
+}
+
+int launch_relay(cudaStream_t stream, uint32_t scheme, const uint8_t* w, uint32_t k, uint64_t n, uint8_t* out, const uint32_t* used,
+                 uint32_t slab_rows) {
+    if (scheme == RLXQ_Q6_K) return launch_widen_q6(stream, w, k, n, out, used, slab_rows);
+    Geometry g;
+    geometry(scheme, &g);
+    return launch_relay_rows(stream, w, (uint64_t)k / g.elems * g.bytes, n, out, gemm_relaid_pitch(scheme, k), used, slab_rows);
 }
 
 // Parts of an activation value: bf16 ones are one, f32 ones hi and lo, or all 24 bits beside PRECISE weights.
@@ -1609,12 +1750,15 @@ struct GemmShape { uint32_t tx, xtiles, slices; bool streamk, pair; };
 // narrow tile, and rows are split evenly over the fewest tiles that leave no SM idle.  The constants are fits to 45 shapes
 // (five formats, 16 to 1526 rows, k 2048 to 14336), each timed at every tile width, split and kernel: the choice made here
 // takes 1 % longer than the best one in the geometric mean, up to 10 % at worst.
-// PRECISE: the decoders of three parts and the emptying of the accumulators, measured with one tile on every SM.
+// PRECISE: the decoders of three parts and the emptying of the accumulators, measured with one tile on every SM; re-laid Q6_K is
+// bound by MMA issue and, above 64 rows of f32 activations, by its three stages (cycles a block at 32, 64, 80, 96 rows: f32 960,
+// 1365, 1463, 1800, bf16 850, 885, 900, 920).
 static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t products, bool precise, bool pair) {
+    if (gemm_late_scale(scheme)) return products > 3 ? (tx <= 64 ? 560 + 12 * tx : 20 * tx - 140) : 820 + tx;
     if (precise) {
         const uint32_t base = scheme == RLXQ_Q4_0 ? 1150 : scheme == RLXQ_Q8_0 ? 1900 : scheme == RLXQ_Q3_K ? 3000 : scheme == RLXQ_Q6_K ? 1580 :
                               scheme == RLXQ_Q4_K || scheme == RLXQ_Q5_K ? 1700 : 2750;
-        return base + (products > 3 ? 7 : 4) * tx;
+        return base + base / 12 + (products > 3 ? 5 : 3) * tx;
     }
     const bool heavy = scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K;
     if (pair) return heavy && products == 1 ? 925 : 750 * products;        // 256 activation rows, both CTAs at once
@@ -1643,6 +1787,7 @@ static GemmShape gemm_choose(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
     const uint32_t least_tiles = (m + most - 1) / most;
     for (uint32_t xt = least_tiles; xt <= least_tiles + 8; ++xt) {
         uint32_t tx = ((m + xt - 1) / xt + 31) / 32 * 32;
+        if (gemm_late_scale(scheme) && tx == 96 && (m + xt - 1) / xt <= 80) tx = 80;
         if (fx) tx = (uint32_t)fx < most ? (uint32_t)fx : most;
         const uint32_t tiles_x = (m + tx - 1) / tx;
         if (tiles_x != xt && !fx) continue;              // the same width as one tile fewer
@@ -1679,7 +1824,8 @@ static size_t gemm_shape_bytes(const GemmShape& sh, uint32_t m, uint32_t n) {
 // Scratch the GEMM would use for this shape (0 when whole tiles fill the SMs well enough).
 size_t gemm_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise) {
     if (m == 0 || k == 0 || n == 0) return 0;
-    return gemm_shape_bytes(gemm_choose(scheme, m, k, n, f32, precise, true), m, n);
+    // (a dense call multiplies f32 weights where it has re-laid them)
+    return gemm_shape_bytes(gemm_choose(precise && scheme == RLXQ_Q6_K ? kQ6Wide : scheme, m, k, n, f32, precise, true), m, n);
 }
 
 // A different tag for each of the calls that may be in flight together; where they start differs from process to process.
@@ -1693,13 +1839,16 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     constexpr uint32_t RAW_ROW = GemmRaw<SCHEME>::ROW;
     constexpr uint32_t RAW_STRIDE = (kGemmTileW * RAW_ROW + 127) / 128 * 128;
     Geometry g;
-    geometry(SCHEME, &g);
+    geometry(SCHEME & 0xFFu, &g);
     GemmParams P{};
     P.tx = sh.tx;
     P.lo_row = c.f32 ? c.x_rows : 0u;
     P.xparts = gemm_x_parts(c.f32, PRECISE);
-    P.main_run = gemm_main_run(c.k, c.ybf);
+    P.main_run = gemm_main_run(SCHEME, c.k, c.ybf);
     P.sum_run = gemm_sum_run(c.k, c.ybf);
+    P.cross_run = gemm_late_scale(SCHEME) ? 4u : P.sum_run;
+    P.late_rows = (size_t)c.n * c.num_slabs;
+    P.late = reinterpret_cast<const float*>(c.w + c.w_pitch * P.late_rows);
     int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * P.xparts, c.k, P.tx);
     if (rc) return rc;
     rc = encode_weight_map(&P.wmap, c.w, (uint64_t)c.n * c.num_slabs, c.w_pitch ? c.w_pitch : (uint64_t)c.k / g.elems * g.bytes,
@@ -1724,7 +1873,15 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     P.b_bytes = P.tx * kGemmBK * 2 * P.xparts;
     const uint32_t smem = 227 * 1024;   // all of it: one CTA per SM, so that none waits for another's tensor memory
     const uint32_t budget = smem - (1024 + sizeof(GemmBars) + 64 + (PRECISE ? P.tx * kGemmTileW * 4 : kGemmEpiStage));
-    P.nstages = std::min<uint32_t>(PRECISE ? std::min(4u, (512u - 2u * P.tx) / 96u) : kGemmMaxStages, (budget - kGemmRawStages * RAW_STRIDE) / P.b_bytes);
+    P.nstages = std::min<uint32_t>(PRECISE ? 4u : kGemmMaxStages, (budget - kGemmRawStages * RAW_STRIDE) / P.b_bytes);
+    if (PRECISE) {
+        // tensor memory: weight stages first, then a second accumulator of either kind
+        constexpr uint32_t A_COLS = gemm_a_cols(SCHEME, true);
+        P.nstages = std::min(P.nstages, (512u - 2u * P.tx) / A_COLS);
+        const uint32_t spare = gemm_late_scale(SCHEME) ? (512u - 2u * P.tx - P.nstages * A_COLS) / P.tx : 0u;
+        P.nmain = spare >= 1 ? 2u : 1u;
+        P.ncross = spare >= 2 ? 2u : 1u;
+    }
     // (a decode group's parts may lie up to three stages apart, gemm_decode_role: no ring below that)
     if (P.nstages < (PRECISE ? 3u : 4u)) return fail(RLXQ_E_LIMIT, "GEMM tile of %u activation rows too large", P.tx);
     P.nraw = std::min<uint32_t>(kGemmMaxRaw, (budget - P.nstages * P.b_bytes) / RAW_STRIDE);
@@ -1752,7 +1909,8 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     } else if (grid > ntiles && !c.groups) {
         grid = (uint32_t)ntiles;
     }
-    rc = launch_pdl(gemm_tcgen05_kernel<SCHEME, PRECISE>, dim3(grid), dim3(gemm_threads(GemmRaw<SCHEME>::GROUPS)), smem, stream, P);
+    rc = launch_pdl(gemm_tcgen05_kernel<SCHEME, PRECISE>, dim3(grid), dim3(gemm_threads(GemmRaw<SCHEME>::GROUPS, gemm_epilogue_warps(SCHEME, PRECISE))), smem,
+                    stream, P);
     if (rc) return rc;
     count_launch();
     if (P.slices > 1) return launch_add_slices(stream, static_cast<const float*>(ws), P.slices, P.slice_elems, c.y, c.ybf, (uint64_t)c.x_rows * c.n);
@@ -1760,7 +1918,8 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
 }
 template <uint32_t SCHEME>
 static int launch_gemm_t_any(cudaStream_t stream, const GemmCall& c, const GemmShape& sh, void* ws) {
-    return c.precise ? launch_gemm_t<SCHEME, true>(stream, c, sh, ws) : launch_gemm_t<SCHEME, false>(stream, c, sh, ws);
+    if constexpr (SCHEME == kQ6Wide) return launch_gemm_t<SCHEME, true>(stream, c, sh, ws);
+    else return c.precise ? launch_gemm_t<SCHEME, true>(stream, c, sh, ws) : launch_gemm_t<SCHEME, false>(stream, c, sh, ws);
 }
 
 // The two-CTA form: whole 256 x 256 tile pairs dealt round-robin to as many clusters as are resident at once.
@@ -1826,7 +1985,8 @@ static int launch_gemm_s(cudaStream_t stream, const GemmCall& c, void* ws, size_
     GemmShape sh = gemm_choose(SCHEME, c.x_rows, c.k, c.n, c.f32, c.precise, true);
     if ((sh.streamk || sh.slices > 1) && (!ws || ((uintptr_t)ws & 15u) || ws_bytes < gemm_shape_bytes(sh, c.x_rows, c.n)))
         sh = gemm_choose(SCHEME, c.x_rows, c.k, c.n, c.f32, c.precise, false);
-    if (sh.pair) return launch_gemm_pair_t<SCHEME>(stream, c);
+    if constexpr (SCHEME != kQ6Wide)
+        if (sh.pair) return launch_gemm_pair_t<SCHEME>(stream, c);
     return launch_gemm_t_any<SCHEME>(stream, c, sh, ws);
 }
 
@@ -1843,7 +2003,7 @@ int launch_gemm(cudaStream_t stream, uint32_t scheme, const GemmCall& c, void* w
         case RLXQ_Q5_0: return launch_gemm_s<RLXQ_Q5_0>(stream, c, ws, ws_bytes);
         case RLXQ_Q5_1: return launch_gemm_s<RLXQ_Q5_1>(stream, c, ws, ws_bytes);
         case RLXQ_Q3_K: return launch_gemm_s<RLXQ_Q3_K>(stream, c, ws, ws_bytes);
-        case RLXQ_Q6_K: return launch_gemm_s<RLXQ_Q6_K>(stream, c, ws, ws_bytes);
+        case RLXQ_Q6_K: return c.w_pitch ? launch_gemm_s<kQ6Wide>(stream, c, ws, ws_bytes) : launch_gemm_s<RLXQ_Q6_K>(stream, c, ws, ws_bytes);
         default: return fail(RLXQ_E_SCHEME, "unknown scheme");
     }
 }

@@ -287,7 +287,7 @@ static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
     p.off_table = up(base);
     p.off_xg = p.off_table + up((size_t)(p.tiles + 1) * 16);
     p.off_w = p.off_xg + up((size_t)gemm_x_parts(!xbf, p.precise) * m * k * 2);
-    p.bytes = p.off_w + up((size_t)p.pitch * n * E);
+    p.bytes = p.off_w + (p.relaid ? up((size_t)gemm_relaid_bytes(scheme, k, (uint64_t)n * E)) : 0);
     p.ok = p.bytes <= (4ull << 30) && (uint64_t)n * E <= 0x7FFFFFFFull;
     return p;
 }
@@ -417,7 +417,7 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
         GemmCall c{};
         c.w = wst;
         if (tc.relaid) {
-            rc = launch_relay_rows(s, wst, (uint64_t)k / g.elems * g.bytes, (uint64_t)n * num_experts, ws + tc.off_w, tc.pitch, offsets, n);
+            rc = launch_relay(s, scheme, wst, k, (uint64_t)n * num_experts, ws + tc.off_w, offsets, n);
             if (rc) return rc;
             c.w = ws + tc.off_w;
         }

@@ -184,6 +184,38 @@ def test_swiglu_chain_on_relaid_rows_is_as_exact_as_the_general_kernel(m, d, f, 
     assert _error(y, ref) <= 1.03 * _error(general, ref), (_error(y, ref), _error(general, ref))
 
 
+# one super-block, tiles of 80 rows, more super-blocks than the copy takes at a time and a ragged end, weights off 16 bytes
+@pytest.mark.parametrize("m,k,n,x_bf16,shift", [(9, 256, 1, False, 0), (75, 1792, 264, False, 0), (150, 768, 131, True, 0), (80, 2048, 129, False, 2),
+                                                (64, 1280, 257, True, 14), (96, 4864, 300, False, 6)])
+def test_gemm_on_widened_q6_k_rows(m, k, n, x_bf16, shift):
+    """Two bf16 parts of every weight without its super-block's scale, which the sums get: no further from 64 bits than the general
+    kernel (2 %, as above)."""
+    import torch
+    import rlx_b200 as R
+    from rlx_b200._lib import lib
+    s, w, x, xd = _inputs("q6_k", m, k, n, x_bf16, 1200 + m)
+    buf = torch.zeros(w.size + 16, dtype=torch.uint8, device="cuda")
+    wd = buf[shift:shift + w.size]
+    wd.copy_(torch.from_numpy(w))
+    ref = x.astype(np.float64) @ O.dequant(s, w, k * n).reshape(n, k).astype(np.float64).T
+    ws, y = torch.empty(64 << 20, dtype=torch.uint8, device="cuda"), torch.empty((m, n), device="cuda")
+
+    def run():
+        assert lib.rlxq_matmul(torch.cuda.current_stream().cuda_stream, s, xd.data_ptr(), int(x_bf16), wd.data_ptr(), y.data_ptr(), 0, m, k, n,
+                               ws.data_ptr(), ws.numel()) == 0
+        R.device_status()
+        return y.cpu().numpy()
+    got = run()
+    assert np.array_equal(got, run())
+    R.set_option("gemm_kernel", 1)
+    try:
+        general = run()
+    finally:
+        R.set_option("gemm_kernel", 0)
+    assert not np.array_equal(got, general)
+    assert _error(got, ref) <= 1.02 * _error(general, ref), (_error(got, ref), _error(general, ref))
+
+
 @pytest.mark.parametrize("sch,k", [("q4_0", 544), ("q8_0", 2336), ("q6_k", 1280)])
 @pytest.mark.parametrize("x_bf16", [False, True])
 def test_gemm_on_relaid_rows_with_values_that_are_not_finite(sch, k, x_bf16):
