@@ -125,6 +125,7 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
             }
         }
         // rows that TMA cannot tile: f32 arithmetic like the general kernel's, at streaming speed
+        if (force == 0 && gemv_parts_pays(scheme, m, k, n, xbf, x)) return launch_gemv_parts(stream, scheme, x, xbf, w, y, ybf, m, k, n);
         if (force == 0 && gemv_f32_supported(scheme, m, k, x)) return launch_gemv_f32(stream, scheme, x, xbf, w, y, ybf, m, k, n);
         return launch_matmul_generic(stream, scheme, x, xbf, w, y, ybf, m, k, n);
     }

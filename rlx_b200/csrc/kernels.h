@@ -84,6 +84,11 @@ bool gemv_f32_supported(uint32_t scheme, uint32_t m, uint32_t k, const void* x);
 int launch_gemv_f32(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf, uint32_t m,
                     uint32_t k, uint32_t n, const float* expert_idx = nullptr, uint32_t num_experts = 0);
 
+// The same accuracy on the matrix instruction, for five to eight rows of the 32-weight formats and Q6_K: whether it is the faster one.
+bool gemv_parts_pays(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, const void* x);
+int launch_gemv_parts(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf, uint32_t m,
+                      uint32_t k, uint32_t n);
+
 // MoE decode rows: the slab of the weight stack is chosen by expert_sel[row] on the device.
 bool int_expert_supported(uint32_t scheme, uint32_t k, uint32_t n, uint32_t rows, const void* w, const void* x, size_t* scratch);
 int launch_gemv_int_expert(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w_stack, void* y,

@@ -43,6 +43,39 @@ def test_streaming_f32_gemv(sch, k, m, n, x_bf16):
     assert torch.equal(yb, y.to(torch.bfloat16))
 
 
+# one warp and fifteen streams, rows on and off whole words, a ragged last piece and tile, two and three column passes, more tiles a
+# CTA than keep their totals between passes
+@pytest.mark.parametrize("sch,m,k,n,x_bf16,shift", [("q6_k", 5, 256, 40000, False, 0), ("q6_k", 8, 768, 14529, True, 2), ("q8_0", 7, 2080, 5003, False, 0),
+                                                    ("q8_0", 6, 1056, 2500, True, 6), ("q4_0", 8, 544, 8000, False, 0), ("q4_0", 5, 4128, 3001, True, 0),
+                                                    ("q6_k", 6, 4352, 3011, False, 0), ("q4_0", 8, 2080, 153001, False, 4), ("q8_0", 5, 1024, 2300, False, 14)])
+def test_gemv_in_parts(sch, m, k, n, x_bf16, shift):
+    """Five to eight rows on the matrix instruction: against the f32 kernel, which takes rows four at a time, with one row of
+    infinities and NaN, and (small ones) the oracle."""
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, 60 + m)
+    buf = torch.zeros(w.size + 16, dtype=torch.uint8, device="cuda")
+    wd = buf[shift:shift + w.size]
+    wd.copy_(torch.from_numpy(w))
+
+    def by_four():
+        return torch.cat([R.matmul(xd[i:i + 4].contiguous(), wd, s, n) for i in range(0, m, 4)])
+    before = R.launch_count()
+    y = R.matmul(xd, wd, s, n)
+    yb = R.matmul(xd, wd, s, n, out_dtype=torch.bfloat16)
+    assert R.launch_count() - before == 2
+    f32 = by_four()
+    assert not torch.equal(y, f32)                              # they are different kernels
+    # each is off by 2^-24 of its partial sums at most, in 32 roundings a scale and one a scale and a warp
+    assert float((y - f32).abs().max()) <= 4e-6 * float(f32.square().mean().sqrt())
+    assert torch.equal(yb, y.to(torch.bfloat16))
+    if k * n < 10_000_000:
+        assert_within_tolerance(y.cpu().numpy(), O.matmul_bt_mt(x, w, m, k, n, s), _bound(s, w, x, k, n), tol=2e-6, what=f"parts {sch} {m}x{k}x{n}")
+    xd[1, 5], xd[m - 1, k - 1], xd[2, 40], xd[2, 41], xd[3, 7] = np.inf, -np.inf, np.inf, -np.inf, np.nan
+    y, f32 = R.matmul(xd, wd, s, n), by_four()
+    assert torch.equal(y.isnan(), f32.isnan()) and torch.equal(y[y.isinf()], f32[f32.isinf()]) and y[1].isinf().any() and not y[0].isnan().any()
+
+
 def test_streaming_f32_gemv_on_weights_at_an_odd_address():
     import torch
     import rlx_b200 as R
