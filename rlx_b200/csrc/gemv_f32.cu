@@ -1,7 +1,8 @@
 // Streaming decode GEMV for weight rows of any length (batch 1-8; Q4_0, Q8_0, Q4_K, Q5_K, Q6_K): the rows that TMA cannot
 // tile, because they are no multiple of 16 bytes (Q6_K with k not a multiple of 2048, the 32-weight formats with k not a
 // multiple of 256) or the weights do not start on a 16-byte boundary; and, in one launch, the rows of an expert batch that
-// has too few of them for the GEMM (moe.cu).
+// has too few of them for the GEMM (moe.cu).  (Five to eight rows of three of the formats, where there is enough work:
+// gemv_parts.cu.)
 //
 // Activations stay f32, in registers.  A CTA's warps stand side by side over the columns: warp c owns columns
 // [c * 32 * LW, (c + 1) * 32 * LW), a lane LW of them, and keeps its activations of MR batch rows for the whole kernel, while
