@@ -34,7 +34,7 @@ int launch_swiglu_mul(cudaStream_t stream, const float* gate, const float* up, f
 // Launched with programmatic stream serialization: the kernel behind an input copy becomes resident and
 // requests its first weights while the input crosses PCIe, and an output copy is resident, waiting, when
 // the kernel in front of it completes.
-__global__ void __launch_bounds__(256) copy_bytes_kernel(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src,
+__global__ void __launch_bounds__(256) copy_bytes_kernel(uint8_t* __restrict__ dst, const uint8_t* src,
                                                          uint64_t bytes) {
     griddep_launch_dependents();
     griddep_wait();                // every thread: whoever waits for this kernel has then waited for its predecessors
@@ -61,7 +61,7 @@ int launch_copy_bytes(cudaStream_t stream, void* dst, const void* src, uint64_t 
 // or (parts = 3) x = hi + mid + lo, which leaves nothing.  Rows [0, rows) of x become rows [0, rows) (hi), [rows, 2 rows) and, if
 // asked for, [2 rows, 3 rows) of `out`; the GEMM multiplies all of them by the same decoded weights.  One pass of 8 bytes a
 // value, a few microseconds; the GEMM behind it is resident meanwhile and fetches its first weights.
-__global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* __restrict__ x, uint16_t* __restrict__ out,
+__global__ void __launch_bounds__(256) split_hi_lo_kernel(const float* x, uint16_t* __restrict__ out,
                                                           uint64_t rows, uint64_t k, uint32_t parts) {
     const uint64_t total = rows * k / 4, stride = (uint64_t)gridDim.x * blockDim.x;     // k % 4 == 0
     griddep_launch_dependents();
@@ -91,7 +91,7 @@ int launch_split_hi_lo(cudaStream_t stream, const float* x, void* out, uint64_t 
 // y[i] = the sum over s, in order, of part[s * stride + i]: the k slices of a GEMM with few tiles, or (two "slices") the
 // hi and lo results of f32 activations.  Every slice's value is loaded before the first is added; out of L2.
 template <bool VEC>
-__global__ void __launch_bounds__(256) add_slices_kernel(const float* __restrict__ part, uint32_t slices, uint64_t stride,
+__global__ void __launch_bounds__(256) add_slices_kernel(const float* part, uint32_t slices, uint64_t stride,
                                                          void* __restrict__ y, uint32_t y_bf16, uint64_t total) {
     constexpr uint32_t W = VEC ? 4 : 1, kAtOnce = 8;
     griddep_launch_dependents();
@@ -154,7 +154,7 @@ int launch_add_slices(cudaStream_t stream, const float* part, uint32_t slices, u
 // used (expert stacks; may be null): slab s of slab_rows rows is skipped when used[s + 1] == used[s].
 __global__ void __launch_bounds__(256) relay_rows_kernel(const uint8_t* __restrict__ w, uint64_t row_bytes, uint64_t n,
                                                          uint8_t* __restrict__ out, uint64_t pitch,
-                                                         const uint32_t* __restrict__ used, uint32_t slab_rows) {
+                                                         const uint32_t* used, uint32_t slab_rows) {
     constexpr uint32_t kSeg = 1024;
     griddep_launch_dependents();
     griddep_wait();
@@ -221,7 +221,7 @@ int launch_relay_rows(cudaStream_t stream, const uint8_t* w, uint64_t row_bytes,
 // four super-blocks at a time, which lie one after the other whatever rows they belong to, in 16-byte loads, and picks them
 // apart in shared memory, eight weights a lane; HBM-bound like the copy above.
 __global__ void __launch_bounds__(256) widen_q6_kernel(const uint8_t* __restrict__ w, uint32_t groups, uint64_t n, uint8_t* __restrict__ out,
-                                                       float* __restrict__ d_out, const uint32_t* __restrict__ used, uint32_t slab_rows) {
+                                                       float* __restrict__ d_out, const uint32_t* used, uint32_t slab_rows) {
     constexpr uint32_t kAtOnce = 4, kChunks = (kAtOnce * 210 + 14 + 15) / 16;
     __shared__ __align__(16) uint8_t buf[8][kChunks * 16 + 16];       // (a word past the last d)
     griddep_launch_dependents();

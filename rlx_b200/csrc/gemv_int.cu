@@ -1197,7 +1197,7 @@ __device__ __forceinline__ void quantise_store8_frag(const float (&f)[8], uint32
 }
 
 template <uint32_t SUB, int MMG = 0, bool FSUM = false>
-__global__ void __launch_bounds__(256) quantise_x_kernel(const void* __restrict__ x, uint32_t x_bf16, uint32_t m,
+__global__ void __launch_bounds__(256) quantise_x_kernel(const void* x, uint32_t x_bf16, uint32_t m,
                                                          uint32_t k, int bias, uint8_t* __restrict__ xq,
                                                          uint32_t xq_row_bytes, uint32_t* __restrict__ counters,
                                                          uint32_t ntiles, float* __restrict__ y_zero, uint32_t y_count,

@@ -251,7 +251,7 @@ template <> struct Unit<RLXQ_Q6_K> {
 // row: its maximum, then the exact power-of-two rescale, the fp16 conversion and the sums per
 // SUB-weight block.  Also clears the split-k tile counters of the main kernel.
 template <uint32_t SUB>
-__global__ void __launch_bounds__(1024) convert_x_f16_kernel(const void* __restrict__ x, uint32_t x_bf16, uint32_t m,
+__global__ void __launch_bounds__(1024) convert_x_f16_kernel(const void* x, uint32_t x_bf16, uint32_t m,
                                                              uint32_t mp, uint32_t k, float bias, __half* __restrict__ xh,
                                                              float* __restrict__ sxb, float* __restrict__ inv,
                                                              uint32_t* __restrict__ counters, uint32_t ncounters) {
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kThreads) gemv_staged_kernel(const __grid_cons
 #pragma unroll
         for (uint32_t wv = 0; wv < kConsumerWarps; ++wv) v += rbuf[wv * 128 + rrow * 8 + col];
         const bool live = col < P.m && orow < P.n;
-        v *= __ldg(P.inv_ws + col);
+        v *= P.inv_ws[col];
         if (P.ksl == 1) {
             if (live) {
                 const size_t o = (size_t)col * P.n + orow;

@@ -48,7 +48,7 @@ __device__ __forceinline__ uint64_t lm_key(float v, uint32_t id) {
     return ord ? (uint64_t)ord << 32 | (uint32_t)~id : 0ull;
 }
 
-__global__ void __launch_bounds__(kLmThreads) lm_peaks_kernel(const float* __restrict__ logits, uint32_t n, uint32_t slice,
+__global__ void __launch_bounds__(kLmThreads) lm_peaks_kernel(const float* logits, uint32_t n, uint32_t slice,
                                                               uint32_t nslices, uint64_t* __restrict__ peaks,
                                                               uint32_t* __restrict__ done) {
     const uint32_t s = (blockIdx.x * kLmThreads + threadIdx.x) / 32, lane = threadIdx.x & 31u;

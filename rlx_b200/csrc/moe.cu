@@ -63,7 +63,7 @@ __device__ __forceinline__ uint32_t moe_block_scan(uint32_t v, uint32_t (&wsum)[
 
 // One CTA: offsets[0..E] = exclusive scan of the rows per expert, cursor[0..E] the same (where the next row of an expert
 // goes; [E]: the rows no expert takes, behind all others).
-__global__ void __launch_bounds__(kMoeScanThreads) moe_count_kernel(const float* __restrict__ expert_idx, uint32_t m, uint32_t E,
+__global__ void __launch_bounds__(kMoeScanThreads) moe_count_kernel(const float* expert_idx, uint32_t m, uint32_t E,
                                                                     uint32_t* __restrict__ offsets, uint32_t* __restrict__ cursor) {
     extern __shared__ uint32_t cnt[];          // [E]
     __shared__ uint32_t wsum[32], total;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kMoeScanThreads) moe_count_kernel(const float*
 }
 
 // perm[sorted position] = original row.
-__global__ void __launch_bounds__(256) moe_place_kernel(const float* __restrict__ expert_idx, uint32_t m, uint32_t E,
+__global__ void __launch_bounds__(256) moe_place_kernel(const float* expert_idx, uint32_t m, uint32_t E,
                                                         uint32_t* __restrict__ cursor, uint32_t* __restrict__ perm) {
     griddep_launch_dependents();
     griddep_wait();
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) moe_place_kernel(const float* __restrict_
 
 // The GEMM's tile table: table[0] = {tiles, routed rows}, table[1 + t] = {first sorted position, rows, expert, 0}, tiles of
 // tile_rows rows, expert by expert.
-__global__ void __launch_bounds__(kMoeScanThreads) moe_tiles_kernel(const uint32_t* __restrict__ offsets, uint32_t E,
+__global__ void __launch_bounds__(kMoeScanThreads) moe_tiles_kernel(const uint32_t* offsets, uint32_t E,
                                                                     uint4* __restrict__ table, uint32_t tile_rows) {
     __shared__ uint32_t wsum[32], total;
     griddep_launch_dependents();
@@ -236,8 +236,8 @@ static bool moe_rows_stream(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n,
 // One CTA per sorted position i: row perm[i] of x becomes row i of xg, as bf16 hi and, for f32 activations, lo part (m
 // rows further on).  The rows no expert takes come last; their outputs are set to zero here.
 template <bool XBF16>
-__global__ void __launch_bounds__(256) moe_gather_kernel(const void* __restrict__ x, const uint32_t* __restrict__ perm,
-                                                         const uint4* __restrict__ table, uint32_t m, uint32_t k,
+__global__ void __launch_bounds__(256) moe_gather_kernel(const void* x, const uint32_t* perm,
+                                                         const uint4* table, uint32_t m, uint32_t k,
                                                          uint32_t parts, uint16_t* __restrict__ xg, uint8_t* __restrict__ y, uint64_t y_row_bytes) {
     griddep_launch_dependents();
     griddep_wait();

@@ -189,6 +189,9 @@ __device__ __forceinline__ uint32_t lds_u32(const uint8_t* p) {
 }
 
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// What the kernels in front write is read behind griddep_wait(), and through pointers that are not `const __restrict__`: of a
+// parameter that is, the compiler may take the memory as unchanging for the whole kernel and read it before the wait.  Weights,
+// which no kernel of a chain writes, are requested ahead of it on purpose.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Launch with programmatic stream serialization (unless the "pdl" option is 0): the kernel may become

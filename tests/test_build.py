@@ -61,3 +61,20 @@ def test_the_build_runs_before_there_is_a_library(tmp_path):
     assert r.returncode and command[0] == "python"
     r = subprocess.run([sys.executable, *command[1:]], cwd=tmp_path, capture_output=True, text=True, env={**os.environ, "NVCC": "", "PATH": ""})
     assert "ImportError" not in r.stderr and "missing: build it" not in r.stderr, r.stderr
+
+
+def test_dependent_kernels_read_no_invariant_parameters():
+    """A kernel that is launched as a programmatic dependent starts while the one in front still writes its inputs.  Memory behind a
+    `const __restrict__` parameter may be read ahead of griddep_wait(): only the weights may be one."""
+    import glob
+    import re
+    kernels = 0
+    for path in sorted(glob.glob(os.path.join(B.PKG, "csrc", "**", "*.cu"), recursive=True)):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\)\s*)?(\w+)\(([^{]*)\)\s*\{(.*?)\n\}", text, re.S):
+            if "griddep_wait()" not in m[3]:
+                continue
+            kernels += 1
+            invariant = set(re.findall(r"const\s+[\w ]+\*\s*__restrict__\s+(\w+)", m[2])) - {"w"}
+            assert not invariant, (os.path.basename(path), m[1], invariant)
+    assert kernels >= 15
