@@ -2,10 +2,12 @@
 // rows of any length (Q4_0, Q8_0, Q6_K; gemv_f32.cu has the same rows' batches of one to four).
 //
 // Quants are small integers, exact in bf16, and an f32 activation is the exact sum of three bf16 parts.  So the products of
-// mma.m16n8k16 (sixteen weight rows, eight columns of activations) are exact, and what f32 arithmetic would round per weight is
-// only rounded when a scale's 16 or 32 columns have been added: their sums are multiplied by the scale and added to the row's
-// total in f32.  A weight is decoded once for all eight rows, one instruction a 16 x 16 tile of weights for bf16 activations,
-// three for f32 ones.
+// mma.m16n8k16 (sixteen weight rows, eight columns of activations) are exact.  What is rounded are the sums that each of a
+// scale's one to six instructions leaves behind, small parts first, and then, in f32, the sum times the scale and the row's
+// total: two or four totals a step and four over the warps, added pairwise, because one chain through all scales was up to 1.26
+// times as far from 64 bits as the f32 kernel (Q6_K, bf16 activations).  600 calls of batch 5 to 8, k 256 to 16416: error 0.77
+// to 0.97 of the f32 kernel's, 0.86 in the mean; the additional sums cost 1 % in the mean, 5 % for long Q6_K rows in bf16.  A weight is
+// decoded once for all eight rows, one instruction a 16 x 16 tile of weights for bf16 activations, three for f32 ones.
 //
 // A CTA's warps form streams: the warps of a stream stand side by side over the columns, 256 each, and take tiles of sixteen
 // weight rows, every stream its own.  The activations lie in shared memory in the instruction's operand order, for all
@@ -133,6 +135,17 @@ __device__ __forceinline__ void parts_scale(float (&tot)[4], const float (&acc)[
     tot[0] = fmaf(acc[0], sa, tot[0]); tot[1] = fmaf(acc[1], sa, tot[1]);
     tot[2] = fmaf(acc[2], sb, tot[2]); tot[3] = fmaf(acc[3], sb, tot[3]);
 }
+// A step's scales are added in N totals, which are then added pairwise: one chain through all of them left a fifth more error.
+template <int N> __device__ __forceinline__ void parts_join(float (&tot)[4], float (&sum)[N][4]) {
+#pragma unroll
+    for (int d = N / 2; d >= 1; d /= 2)
+#pragma unroll
+        for (int i = 0; i < d; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[i][j] += sum[i + d][j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tot[j] += sum[0][j];
+}
 
 // One step of a warp: rows lane / 4 (ra) and lane / 4 + 8 (rb) of the tile; `blocks` of its 32-column blocks exist.
 template <uint32_t SCHEME, int NP, bool W4> struct PartsStep;
@@ -140,6 +153,7 @@ template <uint32_t SCHEME, int NP, bool W4> struct PartsStep;
 template <int NP, bool W4> struct PartsStep<RLXQ_Q4_0, NP, W4> {
     __device__ static __forceinline__ void run(PartsRow ra, PartsRow rb, uint32_t lane, const PartsX& X, uint32_t, uint32_t blocks, float (&tot)[4]) {
         const uint32_t t4 = 4 * (lane & 3u);
+        float sum[2][4] = {};
 #pragma unroll 2
         for (uint32_t b0 = 0; b0 < blocks; b0 += 2) {
 #pragma unroll
@@ -158,11 +172,12 @@ template <int NP, bool W4> struct PartsStep<RLXQ_Q4_0, NP, W4> {
                 const float da = f16_bits_to_f32(parts_lds16(ra.at + 18 * b)), db = f16_bits_to_f32(parts_lds16(rb.at + 18 * b));
                 float acc[4];
                 parts_multiply<NP>(x, a, acc);
-                parts_scale(tot, acc, da, db);
+                parts_scale(sum[b], acc, da, db);
             }
             ra.move(36);
             rb.move(36);
         }
+        parts_join<2>(tot, sum);
     }
 };
 
@@ -173,6 +188,7 @@ template <int NP, bool W4> struct PartsStep<RLXQ_Q8_0, NP, W4> {
     }
     __device__ static __forceinline__ void run(PartsRow ra, PartsRow rb, uint32_t lane, const PartsX& X, uint32_t part, uint32_t blocks, float (&tot)[4]) {
         const uint32_t t8 = 8 * (lane & 3u), lim = min(blocks, 4 * part + 4);
+        float sum[2][4] = {};
 #pragma unroll 2
         for (uint32_t b0 = 4 * part; b0 < lim; b0 += 2) {
 #pragma unroll
@@ -203,11 +219,12 @@ template <int NP, bool W4> struct PartsStep<RLXQ_Q8_0, NP, W4> {
                 const float da = f16_bits_to_f32(parts_lds16(ra.at + 34 * b)), db = f16_bits_to_f32(parts_lds16(rb.at + 34 * b));
                 float acc[4];
                 parts_multiply<NP>(x, a, acc);
-                parts_scale(tot, acc, da, db);
+                parts_scale(sum[b], acc, da, db);
             }
             ra.move(68);
             rb.move(68);
         }
+        parts_join<2>(tot, sum);
     }
 };
 
@@ -229,6 +246,7 @@ template <int NP, bool W4> struct PartsStep<RLXQ_Q6_K, NP, W4> {
         PartsRow ha = ra, hb = rb;        // (qh advances by half the bytes)
         ha.move(128);
         hb.move(128);
+        float sum[4][4] = {};
 #pragma unroll 1
         for (uint32_t h = 0; h < 2; ++h) {
             uint32_t qh[2][2], ql[2][2][2];
@@ -259,12 +277,13 @@ template <int NP, bool W4> struct PartsStep<RLXQ_Q6_K, NP, W4> {
                     float acc[4];
                     if (i) parts_multiply1<NP, 1>(x, a, acc);
                     else parts_multiply1<NP, 0>(x, a, acc);
-                    parts_scale(tot, acc, __shfl_sync(0xFFFFFFFFu, sa[s & 3u], from), __shfl_sync(0xFFFFFFFFu, sb[s & 3u], from));
+                    parts_scale(sum[s & 3u], acc, __shfl_sync(0xFFFFFFFFu, sa[s & 3u], from), __shfl_sync(0xFFFFFFFFu, sb[s & 3u], from));
                 }
             }
             ra.move(64); rb.move(64);
             ha.move(32); hb.move(32);
         }
+        parts_join<4>(tot, sum);
     }
 };
 
@@ -437,9 +456,12 @@ __global__ void __launch_bounds__(kPartsMaxWarps * 32, 1) gemv_parts_kernel(cons
                 for (uint32_t i0 = 4 * cw; i0 < kPartsTile; i0 += 4 * nw) {
                     const uint32_t i = i0 + (lane >> 3), c = lane & 7u;
                     const float* src = red + turn * nw * 128u + i * 8u + c;
-                    float v = 0.f;
-#pragma unroll 4
-                    for (uint32_t q = 0; q < nw; ++q) v += src[q * 128u];
+                    float part[4] = {0.f, 0.f, 0.f, 0.f};
+                    for (uint32_t q = 0; q < nw; q += 4)
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; ++j)
+                            if (q + j < nw) part[j] += src[(q + j) * 128u];
+                    float v = (part[0] + part[2]) + (part[1] + part[3]);
                     if (c >= P.m) continue;
                     if (P.passes > 1) {
                         float* sum = total + ((tile - c0) * kPartsTile + i) * 8u + c;
