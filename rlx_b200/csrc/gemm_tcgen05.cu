@@ -1252,16 +1252,17 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS, gemm_epi
                     const uint32_t sn = s + 1 == NS ? 0u : s + 1, phn = s + 1 == NS ? ph ^ 1u : ph;
                     const uint64_t bdesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES));
                     const uint32_t a = tmem_a + A_COLS * s;
-                    for (uint32_t q = 1; q < P.xparts; ++q) {
-                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
+                    // Upper part of the activations first, as in the paired kernel.  The next stage is looked at before the round's last MMAs
+                    // are issued: the answer takes 118 cycles, and arrives meanwhile.
+                    if (P.xparts == 1u) ready = mbar_test(smem_u32(&bars->full[sn]), phn);
 #pragma unroll
-                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, (kb | j) ? 1u : 0u);
+                    for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, kb | j ? 1u : 0u);
+                    if (P.xparts == 2u) {
+                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + P.tx * 128u));
+                        ready = mbar_test(smem_u32(&bars->full[sn]), phn);
+#pragma unroll
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
                     }
-                    // The next stage is looked at before the round's last MMAs are issued: the answer takes 118 cycles, and arrives meanwhile.
-                    ready = mbar_test(smem_u32(&bars->full[sn]), phn);
-#pragma unroll
-                    for (uint32_t j = 0; j < kGemmBK / 16; ++j)
-                        tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, kb || j || P.xparts > 1u ? 1u : 0u);
                     tc_commit(smem_u32(&bars->stage_free[s]));     // frees the B stage and the A columns when the MMAs retire
                     s = sn;
                     ph = phn;

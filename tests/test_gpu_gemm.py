@@ -163,6 +163,23 @@ def test_two_cta_gemm_matches_oracle_and_the_single_cta_kernel(sch, m, k, n, y_b
         assert_within_tolerance(pair[rows], ref, bnd, tol=_tol(k, sch), what=f"paired gemm {sch} {m}x{k}x{n}")
 
 
+@pytest.mark.parametrize("sch,m,k,n", [("q8_0", 300, 1024, 256), ("q4_0", 130, 2048, 512), ("q4_k", 520, 4096, 256), ("q6_k", 70, 2048, 256)])
+def test_two_cta_gemm_on_f32_activations_has_the_single_cta_kernels_bits(sch, m, k, n):
+    """The upper and the lower part of every 64 columns of activations are added in the same order by both."""
+    import torch
+    s = O.SCHEMES[sch]
+    w = torch.from_numpy(O.fill_weights(s, 340 + m, k, n)).cuda()
+    x = torch.from_numpy(O.fill_normal(341 + m, m * k).reshape(m, k)).cuda()
+    R.set_option("gemm_streamk", 1)
+    R.set_option("gemm_pair", 1)
+    single = R.matmul(x, w, s, n)
+    R.set_option("gemm_pair", 2)
+    pair = R.matmul(x, w, s, n)
+    R.device_status()
+    assert R.get_option("gemm_pair_clusters") >= 1
+    assert torch.equal(pair, single)
+
+
 def test_two_cta_gemm_is_chosen_by_itself_and_refused_where_it_cannot_run():
     """Automatic choice: at least one tile pair per cluster and not Q6_K; n not a multiple of 256 always runs the
     single-CTA kernel, also when the pair is forced."""
