@@ -528,8 +528,8 @@ constexpr uint32_t gemm_threads(uint32_t groups, uint32_t epilogue = 4) { return
 // be scaled and added (gemm_late_scale); their decoder fits the 96 registers a thread that leaves.
 constexpr uint32_t gemm_epilogue_warps(uint32_t scheme, bool precise) { return precise && gemm_late_scale(scheme) ? 8u : 4u; }
 // warp roles: 0 = activation (B) TMA producer, 1 = MMA issuer and tensor-memory owner,
-// 2 = raw weight TMA producer, 3 = idle, then GROUPS x 4 decode warps (tensor-memory lane quarter =
-// warp % 4), then 4 epilogue warps (lane quarter = warp % 4).
+// 2 = raw weight TMA producer, 3 = the second MMA issuer (gemm_late_scale; idle otherwise), then GROUPS x 4 decode warps
+// (tensor-memory lane quarter = warp % 4), then 4 (gemm_late_scale: 8) epilogue warps (lane quarter = warp % 4).
 
 struct GemmParams {
     CUtensorMap xmap;      // x[rows, k] bf16, box tx rows x 64 columns, 128-byte swizzle
@@ -773,8 +773,10 @@ __device__ __noinline__ void gemm_reduce_parts(const GemmParams& P, uint32_t til
 constexpr uint32_t gemm_a_cols(uint32_t scheme, bool precise) { return precise ? 32u * gemm_weight_parts(scheme) : 32u; }
 
 struct GemmBars {
-    // full: a stage's activations (their bytes) and its weights (four decode warps) are there: one barrier to look at for both
-    uint64_t full[kGemmMaxStages], stage_free[kGemmMaxStages];
+    // full: a stage's activations (their bytes) and its weights (four decode warps) are there: one barrier to look at for both.
+    // (f32 weights in three parts, and Q4_0's in two, have a_full for the weights: with one barrier Q4_0 300 x 11040 x 14336
+    // bf16 took 489 us instead of 463, f32 in the mean 3 % less.)
+    uint64_t full[kGemmMaxStages], a_full[kGemmMaxStages], stage_free[kGemmMaxStages];
     uint64_t raw_full[kGemmMaxRaw], raw_empty[kGemmMaxRaw];
     uint64_t d_full[4], d_free[4];        // two accumulators (PRECISE: two for the leading product, two for the others)
     uint32_t tmem_base, abort_flag, epi_prev, epi_prev1;   // epi_prev, epi_prev1: arrival counts of alternate segments
@@ -853,7 +855,7 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
                 } else {
                     tmem_st32(tmem_a + lane_addr + A_COLS * st, v.hi);
                 }
-                pending = smem_u32(&bars->full[st]);
+                pending = smem_u32(PRECISE && !LATE ? &bars->a_full[st] : &bars->full[st]);
                 return true;
             };
             uint32_t st, sph;
@@ -1007,21 +1009,37 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
                 }
             };
             const uint32_t k1 = min(blocks, k0 + P.sum_run);
+            // the leading product's runs, then what the other products piled up meanwhile
+            // (LATE or not apart: one loop for both kept values alive that cost the others as many spills again)
+            if constexpr (LATE) {
 #pragma unroll 1
-            for (uint32_t kc = k0; ok && kc < k1; kc += LATE ? P.cross_run : k1 - k0) {
-                const uint32_t k2 = LATE ? min(k1, kc + P.cross_run) : k1;
-                if (LATE) scale = f32x2_splat(tr.wt * kGemmTileW + row < P.n ? __ldcg(P.late + (size_t)(sg.g0 + kc / 4) * P.late_rows + tr.wrow0 + row) : 0.f);
+                for (uint32_t kc = k0; ok && kc < k1; kc += P.cross_run) {
+                    const uint32_t k2 = min(k1, kc + P.cross_run);
+                    scale = f32x2_splat(tr.wt * kGemmTileW + row < P.n ? __ldcg(P.late + (size_t)(sg.g0 + kc / 4) * P.late_rows + tr.wrow0 + row) : 0.f);
 #pragma unroll 1
-                for (uint32_t kb = kc; kb < k2; kb += P.main_run) {
-                    if (!(ok = wait_for(mb, mph))) break;
-                    add_accumulator(main_d + mb * TX, false);
-                    release(mb);
-                    if (!LATE || ++mb == P.nmain) { mb = 0; mph ^= 1u; }
+                    for (uint32_t kb = kc; kb < k2; kb += P.main_run) {
+                        if (!(ok = wait_for(mb, mph))) break;
+                        add_accumulator(main_d + mb * TX, false);
+                        release(mb);
+                        if (++mb == P.nmain) { mb = 0; mph ^= 1u; }
+                    }
+                    if (!ok || !(ok = wait_for(2 + cb, cph))) break;
+                    add_accumulator(cross_d + cb * TX, true);
+                    release(2 + cb);
+                    if (++cb == P.ncross) { cb = 0; cph ^= 1u; }
                 }
-                if (!ok || !(ok = wait_for(2 + cb, cph))) break;
-                add_accumulator(cross_d + cb * TX, true);
-                release(2 + cb);
-                if (!LATE || ++cb == P.ncross) { cb = 0; cph ^= 1u; }
+            } else {
+#pragma unroll 1
+                for (uint32_t kb = k0; kb < k1; kb += P.main_run) {
+                    if (!(ok = wait_for(0, mph))) break;
+                    mph ^= 1u;
+                    add_accumulator(main_d, false);
+                    release(0);
+                }
+                if (!ok || !(ok = wait_for(2, cph))) break;
+                cph ^= 1u;
+                add_accumulator(cross_d, true);
+                release(2);
             }
             if (!ok) break;
             // totals [activation row][weight row]: a thread's own column of them, sixteen loads before the first store
@@ -1074,6 +1092,7 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS, gemm_epi
     constexpr uint32_t RAW_BYTES = kGemmTileW * RAW_ROW;
     constexpr uint32_t RAW_STRIDE = (RAW_BYTES + 127) / 128 * 128;
     constexpr uint32_t A_COLS = gemm_a_cols(SCHEME, PRECISE);         // tensor-memory columns of a weight stage
+    constexpr bool LATE = PRECISE && gemm_late_scale(SCHEME);         // two MMA issuers
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t NS = P.nstages, NR = P.nraw, B_BYTES = P.b_bytes;
@@ -1088,8 +1107,9 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS, gemm_epi
 
     if (tid == 0) {
         for (uint32_t s = 0; s < NS; ++s) {
-            mbar_init(smem_u32(&bars->full[s]), 1 + 4);
-            mbar_init(smem_u32(&bars->stage_free[s]), PRECISE ? 2 : 1);
+            mbar_init(smem_u32(&bars->full[s]), PRECISE && !LATE ? 1 : 1 + 4);
+            mbar_init(smem_u32(&bars->a_full[s]), 4);
+            mbar_init(smem_u32(&bars->stage_free[s]), LATE ? 2 : 1);
         }
         for (uint32_t r = 0; r < NR; ++r) {
             mbar_init(smem_u32(&bars->raw_full[r]), 1);
@@ -1168,10 +1188,11 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS, gemm_epi
                 }
             }
         }
-    } else if (PRECISE && (warp == 1 || warp == 3)) {
+    } else if (LATE && (warp == 1 || warp == 3)) {
         // ---------------- MMA issuers: the leading product, and the others ----------------
         // Two threads, because issue is what the rounds are made of: beside the products a round takes 0.4 us of one, whatever
-        // else is left out.  They use different accumulators, so neither waits for the other.
+        // else is left out.  They use different accumulators, so neither waits for the other.  (Where a decoder paces the rounds one
+        // issuer is faster: with two, Q4_0 300 x 544 x 4096 bf16 takes 33.8 us instead of 28, Q8_0 587 x 2080 x 1024 bf16 48 instead of 42.)
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((P.tx >> 3) << 17) | ((kGemmTileW >> 4) << 24);
             const bool lead = warp == 1;
@@ -1231,45 +1252,86 @@ __global__ void __launch_bounds__(gemm_threads(GemmRaw<SCHEME>::GROUPS, gemm_epi
                 }
             }
         }
-    } else if (!PRECISE && warp == 1) {
+    } else if (!LATE && warp == 1) {
         // ---------------- MMA issuer ----------------
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((P.tx >> 3) << 17) | ((kGemmTileW >> 4) << 24);
-            uint32_t s = 0, ph = 0, d = 0, dph = 1;            // dph: parity to wait for on d_free (1 passes the first time)
+            uint32_t s = 0, ph = 0, d = 0, dph = 1, cph = 1;   // dph, cph: parities to wait for on d_free (1 passes the first time)
             uint32_t cur, lim;
             gemm_seg_init(P, xtiles, cur, lim);
             GemmSeg sg;
             bool ok = true;
             while (ok && !*abort_flag && gemm_seg_next(P, cur, lim, sg)) {
                 const uint32_t blocks = 4 * (sg.g1 - sg.g0);
-                if (!mbar_wait(smem_u32(&bars->d_free[d]), dph)) { give_up(13); break; }
-                tc_fence_after();
-                const uint32_t acc = tmem_d + 128u * d;
-                uint32_t ready = mbar_test(smem_u32(&bars->full[s]), ph);
+                if (!PRECISE) {
+                    if (!mbar_wait(smem_u32(&bars->d_free[d]), dph)) { give_up(13); break; }
+                    tc_fence_after();
+                }
+                const uint32_t acc = tmem_d + (PRECISE ? 0u : 128u * d);
+                uint32_t ready = mbar_test(smem_u32(&bars->full[s]), ph), ra = PRECISE ? mbar_test(smem_u32(&bars->a_full[s]), ph) : 1u;
                 for (uint32_t kb = 0; kb < blocks; ++kb) {    // the first MMA of a segment overwrites the accumulator
-                    if (!ready && (*abort_flag || !mbar_wait(smem_u32(&bars->full[s]), ph))) { give_up(14); ok = false; break; }
+                    if ((!ready && (*abort_flag || !mbar_wait(smem_u32(&bars->full[s]), ph))) || (PRECISE && !ra && (*abort_flag || !mbar_wait(smem_u32(&bars->a_full[s]), ph)))) { give_up(14); ok = false; break; }
                     tc_fence_after();
                     const uint32_t sn = s + 1 == NS ? 0u : s + 1, phn = s + 1 == NS ? ph ^ 1u : ph;
                     const uint64_t bdesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES));
                     const uint32_t a = tmem_a + A_COLS * s;
-                    // Upper part of the activations first, as in the paired kernel.  The next stage is looked at before the round's last MMAs
-                    // are issued: the answer takes 118 cycles, and arrives meanwhile.
-                    if (P.xparts == 1u) ready = mbar_test(smem_u32(&bars->full[sn]), phn);
-#pragma unroll
-                    for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, kb | j ? 1u : 0u);
-                    if (P.xparts == 2u) {
-                        const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + P.tx * 128u));
+                    if constexpr (PRECISE) {
+                        // look at the next stage now: the answer arrives while this stage's MMAs are issued
                         ready = mbar_test(smem_u32(&bars->full[sn]), phn);
+                        ra = mbar_test(smem_u32(&bars->a_full[sn]), phn);
+                        // weight part 0 by activation part 0, main_run blocks of them in the main accumulator
+                        const uint32_t in_run = kb & (P.main_run - 1u);
+                        if (in_run == 0) {
+                            if (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[0]), dph)) { give_up(13); ok = false; break; }
+                            dph ^= 1u;
+                            tc_fence_after();
+                        }
 #pragma unroll
-                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, in_run | j ? 1u : 0u);
+                        if (in_run == P.main_run - 1u || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[0]));
+                        // parts 1, 2 by part 0, 0..1 by part 1, 0 by part 2; the products left out are below 2^-24 of the whole
+                        const uint32_t cross = acc + P.tx;
+                        const bool fresh = (kb & (P.sum_run - 1u)) == 0;
+                        if (fresh) {
+                            if (*abort_flag || !mbar_wait(smem_u32(&bars->d_free[2]), cph)) { give_up(13); ok = false; break; }
+                            cph ^= 1u;
+                            tc_fence_after();
+                        }
+#pragma unroll
+                        for (uint32_t j = 0; j < (gemm_weight_parts(SCHEME) - 1) * (kGemmBK / 16); ++j)
+                            tc_mma_ts(cross, a + 32 + 8 * j, bdesc + 2 * (j & 3u), idesc, fresh && j == 0 ? 0u : 1u);
+                        for (uint32_t q = 1; q < P.xparts; ++q) {
+                            const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + q * P.tx * 128u));
+#pragma unroll
+                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(cross, a + 8 * j, ldesc + 2 * j, idesc, 1u);
+                            if (q == 1) {
+#pragma unroll
+                                for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(cross, a + 32 + 8 * j, ldesc + 2 * j, idesc, 1u);
+                            }
+                        }
+                        if ((kb & (P.sum_run - 1u)) == P.sum_run - 1u || kb == blocks - 1) tc_commit(smem_u32(&bars->d_full[2]));
+                    } else {
+                        // Upper part of the activations first, as in the paired kernel.  The next stage is looked at before the round's last MMAs
+                        // are issued: the answer takes 118 cycles, and arrives meanwhile.
+                        if (P.xparts == 1u) ready = mbar_test(smem_u32(&bars->full[sn]), phn);
+#pragma unroll
+                        for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, bdesc + 2 * j, idesc, kb | j ? 1u : 0u);
+                        if (P.xparts == 2u) {
+                            const uint64_t ldesc = kmajor_sw128_desc(smem_u32(b_stage + s * B_BYTES + P.tx * 128u));
+                            ready = mbar_test(smem_u32(&bars->full[sn]), phn);
+#pragma unroll
+                            for (uint32_t j = 0; j < kGemmBK / 16; ++j) tc_mma_ts(acc, a + 8 * j, ldesc + 2 * j, idesc, 1u);
+                        }
                     }
                     tc_commit(smem_u32(&bars->stage_free[s]));     // frees the B stage and the A columns when the MMAs retire
                     s = sn;
                     ph = phn;
                 }
                 if (!ok) break;
-                tc_commit(smem_u32(&bars->d_full[d]));
-                if (++d == nacc) { d = 0; dph ^= 1u; }
+                if (!PRECISE) {
+                    tc_commit(smem_u32(&bars->d_full[d]));
+                    if (++d == nacc) { d = 0; dph ^= 1u; }
+                }
             }
         }
     } else if (warp >= 4 && warp < 4 + 4 * kGemmDecodeGroups) {
@@ -1759,7 +1821,7 @@ static uint32_t gemm_block_cycles(uint32_t scheme, uint32_t tx, uint32_t product
     if (precise) {
         const uint32_t base = scheme == RLXQ_Q4_0 ? 1150 : scheme == RLXQ_Q8_0 ? 1900 : scheme == RLXQ_Q3_K ? 3000 : scheme == RLXQ_Q6_K ? 1580 :
                               scheme == RLXQ_Q4_K || scheme == RLXQ_Q5_K ? 1700 : 2750;
-        return base + base / 12 + (products > 3 ? 5 : 3) * tx;
+        return base + (products > 3 ? 7 : 4) * tx;
     }
     const bool heavy = scheme == RLXQ_Q6_K || scheme == RLXQ_Q3_K;
     if (pair) return heavy && products == 1 ? 925 : 750 * products;        // 256 activation rows, both CTAs at once
