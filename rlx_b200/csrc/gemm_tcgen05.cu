@@ -548,6 +548,8 @@ struct GemmParams {
     uint32_t main_run, cross_run, sum_run, nmain, ncross;
     const float* late;      // gemm_late_scale: 2^12 d of the groups of the stack's rows, [k group][row], late_rows rows
     size_t late_rows;
+    const uint16_t* x;      // gemm_late_scale: what xmap and wmap describe, for gemm_late_infinite
+    const uint8_t* w;
     uint32_t nstages, nraw;               // depth of the operand ring (B in shared memory, A in tensor memory) and of the raw ring
     uint32_t b_bytes;                     // bytes of a B stage: tx * 128, twice that with lo_row
     uint32_t w_late;       // the weights are written by a kernel in front (re-laid rows): read them after the dependency wait
@@ -941,6 +943,35 @@ static uint32_t gemm_main_run(uint32_t scheme, uint32_t k, bool ybf) {
 }
 static uint32_t gemm_sum_run(uint32_t k, bool ybf) { return ybf || k >= 5632 ? 16u : k >= 2048 ? 8u : 4u; }
 
+// A super-block whose scale is infinite makes infinities of its weights, and NaN of those that are zero.  A sum of weights without
+// the scale knows neither the zeros nor the signs, so such a row is multiplied once more, weight by weight: `count` activation rows
+// from mi on by row wrow of the stack over the k groups [g0, g1), in f32.  Out of the way of the main loop.
+__device__ __noinline__ void gemm_late_infinite(const GemmParams& P, float* total, uint32_t mi, uint32_t rows, uint32_t wrow, uint32_t g0, uint32_t blocks) {
+    const uint32_t g1 = g0 + blocks / 4;
+    bool infinite = false;
+#pragma unroll 1
+    for (uint32_t g = g0; g < g1; ++g) infinite |= isinf(P.late[g * P.late_rows + wrow]);
+    if (!infinite) return;
+#pragma unroll 1
+    for (uint32_t i = 0; i < rows; ++i) {
+        float sum = 0.f;
+#pragma unroll 1
+        for (uint32_t g = g0; g < g1; ++g) {
+            const float d = P.late[g * P.late_rows + wrow];
+            const uint8_t* row = P.w + ((size_t)wrow * P.kgroups + g) * GemmRaw<kQ6Wide>::ROW;
+#pragma unroll 1
+            for (uint32_t j = 0; j < 256; ++j) {
+                const float w = d * (float)(int8_t)row[256 + j / 16] * (float)((int)row[j] - 32) * 0x1p-12f;
+                float x = 0.f;                               // the parts' sum: exact
+#pragma unroll 1
+                for (uint32_t q = 0; q < P.xparts; ++q) x += bf16_bits_to_f32(P.x[((size_t)q * P.lo_row + mi + i) * P.kgroups * 256 + g * 256 + j]);
+                sum = fmaf(w, x, sum);
+            }
+        }
+        total[i * kGemmTileW] = sum;
+    }
+}
+
 // TX = P.tx: no branch between the additions of a block, which are on the chain from one block's product to the next.
 template <uint32_t SCHEME, uint32_t TX>
 __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmBars* bars, float* total, uint32_t tmem_d,
@@ -954,8 +985,9 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
     gemm_seg_init(P, xtiles, cur, lim);
     GemmSeg sg;
     while (gemm_seg_next(P, cur, lim, sg)) {
-        const GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
-        const uint32_t rows = tr.xlim - tr.xrow0, blocks = 4 * (sg.g1 - sg.g0);
+        GemmTileRows tr = gemm_tile_rows(P, xtiles, sg.tile);
+        uint32_t rows = tr.xlim - tr.xrow0;
+        const uint32_t blocks = 4 * (sg.g1 - sg.g0);
         auto wait_for = [&](uint32_t d, uint32_t ph) -> bool {
             if (!mbar_wait(smem_u32(&bars->d_full[d]), ph)) {
                 atomicExch(P.err, 17);
@@ -1058,6 +1090,16 @@ __device__ __forceinline__ void gemm_precise_epilogue(const GemmParams& P, GemmB
                     t[(2 * j + 1) * kGemmTileW] = old[2 * j + 1] + __uint_as_float(hi);
                 }
             }
+        }
+        if constexpr (LATE) {                                // worked out again, so that they need no registers up to here
+            uint32_t tile = sg.tile;
+            asm volatile("" : "+r"(tile));
+            tr = gemm_tile_rows(P, xtiles, tile);
+            rows = tr.xlim - tr.xrow0;
+            // an infinite scale leaves nothing finite in its row
+            float* t = total + 16 * chunk0 * kGemmTileW + row;
+            if (ok && tr.wt * kGemmTileW + row < P.n && 16 * chunk0 < rows && __builtin_expect(!isfinite(*t), 0))
+                gemm_late_infinite(P, t, tr.xrow0 + 16 * chunk0, min(rows - 16 * chunk0, 16 * CHUNKS), tr.wrow0 + row, sg.g0, blocks);
         }
         // the warps leave together: they share the barriers
         if (epilogue_any<32 * EW>(!ok || *reinterpret_cast<volatile uint32_t*>(&bars->abort_flag))) break;
@@ -1912,6 +1954,8 @@ static int launch_gemm_t(cudaStream_t stream, const GemmCall& c, const GemmShape
     P.cross_run = gemm_late_scale(SCHEME) ? 4u : P.sum_run;
     P.late_rows = (size_t)c.n * c.num_slabs;
     P.late = reinterpret_cast<const float*>(c.w + c.w_pitch * P.late_rows);
+    P.x = static_cast<const uint16_t*>(c.x);
+    P.w = c.w;
     int rc = encode_bf16_kmajor_map(&P.xmap, c.x, (uint64_t)c.x_rows * P.xparts, c.k, P.tx);
     if (rc) return rc;
     rc = encode_weight_map(&P.wmap, c.w, (uint64_t)c.n * c.num_slabs, c.w_pitch ? c.w_pitch : (uint64_t)c.k / g.elems * g.bytes,

@@ -268,6 +268,40 @@ def test_gemm_on_widened_q6_k_rows(m, k, n, x_bf16, shift):
     assert _error(got, ref) <= 1.02 * _error(general, ref), (_error(got, ref), _error(general, ref))
 
 
+# narrow tiles and tiles of 80 and 96 rows, slices (few tiles, long rows), the last group of a row
+@pytest.mark.parametrize("m,k,n,x_bf16", [(20, 768, 130, False), (75, 1280, 200, True), (96, 5888, 128, False), (300, 2304, 140, True)])
+def test_gemm_on_widened_q6_k_rows_with_infinite_scales(m, k, n, x_bf16):
+    """A super-block's scale that is not finite: NaN of its zero weights and of infinities of both signs, an infinity where all
+    products have one sign, as in f32 arithmetic; the other rows are as they would be without it."""
+    import torch
+    import rlx_b200 as R
+    s, w, x, _ = _inputs("q6_k", m, k, n, x_bf16, 1500 + m)
+    blocks = w.reshape(n, k // 256, 210)
+    last = k // 256 - 1
+    x[0] = np.abs(x[0]) + 0.1                                    # one sign, no zeros
+    x[1] = -x[0]
+    for row, g, d in ((1, 0, 0x7C00), (2, last, 0xFC00), (3, 1, 0x7C00), (5, 0, 0x7E00), (n - 1, last, 0x7C00)):
+        blocks[row, g, 208:] = np.frombuffer(np.uint16(d).tobytes(), np.uint8)
+    for row, g in ((2, last), (3, 1)):
+        blocks[row, g, :128] |= 0x11                             # odd quants: none is 32, which stands for zero
+        blocks[row, g, 128:192] = 0xFF if row == 2 else 0xAA     # 49 and more: positive weights
+        blocks[row, g, 192:208] = np.abs(blocks[row, g, 192:208].view(np.int8).astype(np.int32)).clip(1, 127).astype(np.uint8)
+    blocks[3, 1, 192] = 0x85                                     # a scale of the other sign
+    xd = torch.from_numpy(x).cuda()
+    if x_bf16:
+        xd = xd.to(torch.bfloat16)
+        x = xd.float().cpu().numpy()
+    with np.errstate(invalid="ignore"):
+        W = O.dequant(s, w, k * n).reshape(n, k).astype(np.float64)
+        ref = np.stack([np.einsum("k,nk->n", xr.astype(np.float64), W) for xr in x])
+    assert np.isinf(ref[0, 2]) and np.isinf(ref[1, 2]) and np.isnan(ref[:, [1, 3, 5, n - 1]]).all()
+    y = R.matmul(xd, torch.from_numpy(w).cuda(), s, n).cpu().numpy()
+    R.device_status()
+    assert np.array_equal(np.isnan(y), np.isnan(ref)) and np.array_equal(y[np.isinf(ref)], ref[np.isinf(ref)])
+    fin = np.isfinite(ref)
+    assert np.isfinite(y[fin]).all() and np.abs(y[fin] - ref[fin]).max() <= 1e-5 * np.abs(ref[fin]).max()
+
+
 @pytest.mark.parametrize("sch,k", [("q4_0", 544), ("q8_0", 2336), ("q6_k", 1280)])
 @pytest.mark.parametrize("x_bf16", [False, True])
 def test_gemm_on_relaid_rows_with_values_that_are_not_finite(sch, k, x_bf16):
