@@ -13,9 +13,11 @@ namespace rlxq {
 // weights that are not 16-byte aligned) are first re-laid on a padded pitch in the workspace, and weights and activations
 // then keep all of their 24 bits (PRECISE), since those shapes were multiplied in f32 before they had this path.  The
 // workspace query does not know the weights' address and plans for aligned ones: weights at another address are re-laid only
-// for a caller who brings more than it asks for, and run the general kernel for everybody else.
-struct PrefillPlan { bool ok, relaid, halves; uint32_t chunk; uint64_t pitch; size_t off_w, off_y2, off_gemm, bytes; };
-static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, bool direct) {
+// for a caller who brings more than it asks for, and run the general kernel for everybody else.  Q6_K rows are widened, which
+// takes a third more scratch than the rows have bytes; a caller who brings less than that, but room for the rows, has them copied
+// as they are (300 x 11008 x 4096 f32: 170 us widened, 240 copied, 4.8 ms through the general kernel).
+struct PrefillPlan { bool ok, relaid, halves; uint32_t layout, chunk; uint64_t pitch; size_t off_w, off_y2, off_gemm, bytes; };
+static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, bool direct, bool widen = true) {
     PrefillPlan p{};
     const void* aligned = (const void*)256;              // dispatch checks the real pointers
     if (m <= 8 || options().gemm_kernel.load() == 1) return p;
@@ -36,15 +38,16 @@ static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_
         if (chunk > m) chunk = m;
     }
     p.chunk = (uint32_t)chunk;
+    p.layout = p.relaid && widen && scheme == RLXQ_Q6_K ? kQ6Wide : scheme;
     p.off_w = xbf ? 0 : al((size_t)gemm_x_parts(true, p.relaid) * chunk * k * 2);
-    p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;
-    p.off_y2 = p.off_w + (p.relaid ? al((size_t)gemm_relaid_bytes(scheme, k, n)) : 0);
+    p.pitch = p.relaid ? gemm_relaid_pitch(p.layout, k) : 0;
+    p.off_y2 = p.off_w + (p.relaid ? al((size_t)gemm_relaid_bytes(p.layout, k, n)) : 0);
     p.off_gemm = p.off_y2 + (p.halves ? al((size_t)2 * chunk * n * 4) : 0);
     p.bytes = p.off_gemm;
     if (!p.halves) {
-        size_t g = gemm_tc_workspace_bytes(scheme, (uint32_t)chunk, k, n, !xbf, p.relaid);
+        size_t g = gemm_tc_workspace_bytes(p.layout, (uint32_t)chunk, k, n, !xbf, p.relaid);
         if (m % chunk) {                                 // the last, shorter chunk may be split over the SMs differently
-            const size_t g2 = gemm_tc_workspace_bytes(scheme, (uint32_t)(m % chunk), k, n, !xbf, p.relaid);
+            const size_t g2 = gemm_tc_workspace_bytes(p.layout, (uint32_t)(m % chunk), k, n, !xbf, p.relaid);
             g = g2 > g ? g2 : g;
         }
         p.bytes += al(g);
@@ -134,14 +137,15 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
     const bool direct = gemm_tc_supported(scheme, m, k, n, w, x);
     if (gforce == 2 && (!direct || !xbf))
         return fail(RLXQ_E_SHAPE, "gemm_kernel = 2 takes bf16 activations, k %% 256 == 0 (1024 for Q2_K and Q8_K, 2048 for Q3_K and Q6_K) and 16-byte alignment");
-    const PrefillPlan p = plan_prefill(scheme, m, k, n, xbf, direct);
+    PrefillPlan p = plan_prefill(scheme, m, k, n, xbf, direct);
+    if (p.ok && p.layout != scheme && ws_bytes < p.bytes) p = plan_prefill(scheme, m, k, n, xbf, direct, false);
     const bool fits = ws && ws_bytes >= p.bytes && !((uintptr_t)ws & 255u);
     if (p.ok && (fits || (xbf && direct))) {
         uint8_t* base = static_cast<uint8_t*>(ws);
         GemmCall c{};
         c.w = w; c.w_pitch = p.pitch; c.precise = p.relaid; c.k = k; c.n = n;
         if (p.relaid) {
-            int rc = launch_relay(stream, scheme, w, k, n, base + p.off_w);
+            int rc = launch_relay(stream, p.layout, w, k, n, base + p.off_w);
             if (rc) return rc;
             c.w = base + p.off_w;
         }
@@ -158,12 +162,12 @@ int dispatch_matmul(cudaStream_t stream, uint32_t scheme, const void* x, bool xb
             if (p.halves) {
                 float* y2 = reinterpret_cast<float*>(base + p.off_y2);
                 c.x_rows = 2 * rows; c.y = y2;
-                rc = launch_gemm(stream, scheme, c, nullptr, 0);
+                rc = launch_gemm(stream, p.layout, c, nullptr, 0);
                 if (!rc) rc = launch_add_slices(stream, y2, 2, (uint64_t)rows * n, out, ybf, (uint64_t)rows * n);
             } else {
                 c.x_rows = rows; c.f32 = !xbf; c.y = out; c.ybf = ybf;
                 // (bf16 activations: a workspace too small for the k split runs whole tiles)
-                rc = launch_gemm(stream, scheme, c, fits ? base + p.off_gemm : nullptr, fits ? ws_bytes - p.off_gemm : 0);
+                rc = launch_gemm(stream, p.layout, c, fits ? base + p.off_gemm : nullptr, fits ? ws_bytes - p.off_gemm : 0);
             }
             if (rc) return rc;
         }

@@ -42,8 +42,6 @@ constexpr uint32_t kGemmBK = 64;        // k per pipeline stage (one 128-byte sw
 constexpr uint32_t kGemmMaxStages = 8;  // B shared-memory stages == A tensor-memory stages (8 x 32 columns)
 constexpr uint32_t kGemmMaxRaw = 8;     // raw weight boxes (256 weights of 128 rows each): what shared memory is left for
 constexpr uint32_t kGemmRawStages = 2;  // the paired kernel's
-// Q6_K rows as widen_q6_kernel re-lays them: 256 bytes of quants in order, 16 scale bytes; the super-blocks' d apart.
-constexpr uint32_t kQ6Wide = 0x100u + RLXQ_Q6_K;
 
 // ---- weight decode: 64 consecutive weights of one row -> 32 bf16 pairs ------------------------
 // The raw box holds 256 weights of 128 rows; RAW_ROW bytes per row (an odd number of 16-byte
@@ -1819,23 +1817,23 @@ bool gemm_relaid_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, 
 }
 // Bytes from one re-laid row to the next: whole 256-weight groups (zero blocks past k), a multiple of 16; and bytes of `rows`
 // re-laid rows, with the scales that widened ones keep behind them.
-uint64_t gemm_relaid_pitch(uint32_t scheme, uint32_t k) {
-    if (scheme == RLXQ_Q6_K) return (uint64_t)(k / 256) * GemmRaw<kQ6Wide>::ROW;
+uint64_t gemm_relaid_pitch(uint32_t layout, uint32_t k) {
+    if (layout == kQ6Wide) return (uint64_t)(k / 256) * GemmRaw<kQ6Wide>::ROW;
     Geometry g;
-    geometry(scheme, &g);
+    geometry(layout, &g);
     return ((uint64_t)((k + 255) / 256) * (256 / g.elems) * g.bytes + 15) / 16 * 16;
 }
 
-uint64_t gemm_relaid_bytes(uint32_t scheme, uint32_t k, uint64_t rows) {
-    return gemm_relaid_pitch(scheme, k) * rows + (scheme == RLXQ_Q6_K ? (uint64_t)(k / 256) * rows * 4 : 0);
+uint64_t gemm_relaid_bytes(uint32_t layout, uint32_t k, uint64_t rows) {
+    return gemm_relaid_pitch(layout, k) * rows + (layout == kQ6Wide ? (uint64_t)(k / 256) * rows * 4 : 0);
 }
 
-int launch_relay(cudaStream_t stream, uint32_t scheme, const uint8_t* w, uint32_t k, uint64_t n, uint8_t* out, const uint32_t* used,
+int launch_relay(cudaStream_t stream, uint32_t layout, const uint8_t* w, uint32_t k, uint64_t n, uint8_t* out, const uint32_t* used,
                  uint32_t slab_rows) {
-    if (scheme == RLXQ_Q6_K) return launch_widen_q6(stream, w, k, n, out, used, slab_rows);
+    if (layout == kQ6Wide) return launch_widen_q6(stream, w, k, n, out, used, slab_rows);
     Geometry g;
-    geometry(scheme, &g);
-    return launch_relay_rows(stream, w, (uint64_t)k / g.elems * g.bytes, n, out, gemm_relaid_pitch(scheme, k), used, slab_rows);
+    geometry(layout, &g);
+    return launch_relay_rows(stream, w, (uint64_t)k / g.elems * g.bytes, n, out, gemm_relaid_pitch(layout, k), used, slab_rows);
 }
 
 // Parts of an activation value: bf16 ones are one, f32 ones hi and lo, or all 24 bits beside PRECISE weights.
@@ -1927,10 +1925,9 @@ static size_t gemm_shape_bytes(const GemmShape& sh, uint32_t m, uint32_t n) {
 }
 
 // Scratch the GEMM would use for this shape (0 when whole tiles fill the SMs well enough).
-size_t gemm_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise) {
+size_t gemm_tc_workspace_bytes(uint32_t layout, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise) {
     if (m == 0 || k == 0 || n == 0) return 0;
-    // (a dense call multiplies f32 weights where it has re-laid them)
-    return gemm_shape_bytes(gemm_choose(precise && scheme == RLXQ_Q6_K ? kQ6Wide : scheme, m, k, n, f32, precise, true), m, n);
+    return gemm_shape_bytes(gemm_choose(layout, m, k, n, f32, precise, true), m, n);
 }
 
 // A different tag for each of the calls that may be in flight together; where they start differs from process to process.
@@ -2097,9 +2094,9 @@ static int launch_gemm_s(cudaStream_t stream, const GemmCall& c, void* ws, size_
     return launch_gemm_t_any<SCHEME>(stream, c, sh, ws);
 }
 
-int launch_gemm(cudaStream_t stream, uint32_t scheme, const GemmCall& c, void* ws, size_t ws_bytes) {
+int launch_gemm(cudaStream_t stream, uint32_t layout, const GemmCall& c, void* ws, size_t ws_bytes) {
     if ((uint64_t)c.n * c.num_slabs > 0x7FFFFFFFull) return fail(RLXQ_E_LIMIT, "weights too tall for a tensor map");
-    switch (scheme) {
+    switch (layout) {
         case RLXQ_Q4_0: return launch_gemm_s<RLXQ_Q4_0>(stream, c, ws, ws_bytes);
         case RLXQ_Q8_0: return launch_gemm_s<RLXQ_Q8_0>(stream, c, ws, ws_bytes);
         case RLXQ_Q4_K: return launch_gemm_s<RLXQ_Q4_K>(stream, c, ws, ws_bytes);
@@ -2110,7 +2107,8 @@ int launch_gemm(cudaStream_t stream, uint32_t scheme, const GemmCall& c, void* w
         case RLXQ_Q5_0: return launch_gemm_s<RLXQ_Q5_0>(stream, c, ws, ws_bytes);
         case RLXQ_Q5_1: return launch_gemm_s<RLXQ_Q5_1>(stream, c, ws, ws_bytes);
         case RLXQ_Q3_K: return launch_gemm_s<RLXQ_Q3_K>(stream, c, ws, ws_bytes);
-        case RLXQ_Q6_K: return c.w_pitch ? launch_gemm_s<kQ6Wide>(stream, c, ws, ws_bytes) : launch_gemm_s<RLXQ_Q6_K>(stream, c, ws, ws_bytes);
+        case RLXQ_Q6_K: return launch_gemm_s<RLXQ_Q6_K>(stream, c, ws, ws_bytes);
+        case kQ6Wide: return launch_gemm_s<kQ6Wide>(stream, c, ws, ws_bytes);
         default: return fail(RLXQ_E_SCHEME, "unknown scheme");
     }
 }

@@ -45,7 +45,9 @@ size_t gemv_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t
 int launch_gemv_tc(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf,
                    uint32_t m, uint32_t k, uint32_t n, void* ws, size_t ws_bytes);
 
-// tcgen05 / tensor-memory GEMM (m > 8).
+// tcgen05 / tensor-memory GEMM (m > 8).  What it reads its weights from (`layout`) is a format's own id, or Q6_K rows as
+// widen_q6_kernel re-lays them: 256 bytes of quants in order, 16 scale bytes; the super-blocks' d apart.  These are PRECISE weights.
+constexpr uint32_t kQ6Wide = 0x100u + RLXQ_Q6_K;
 struct GemmCall {
     const void* x;             // bf16 [x_rows, k]; with f32 set, bf16(x) followed by bf16(x - bf16(x)), x_rows rows each
     uint32_t x_rows;
@@ -65,18 +67,18 @@ struct GemmCall {
 };
 bool gemm_tc_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* w, const void* x);
 bool gemm_relaid_supported(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, const void* x);
-uint64_t gemm_relaid_pitch(uint32_t scheme, uint32_t k);
-uint64_t gemm_relaid_bytes(uint32_t scheme, uint32_t k, uint64_t rows);
-size_t gemm_tc_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise);
-int launch_gemm(cudaStream_t stream, uint32_t scheme, const GemmCall& c, void* ws, size_t ws_bytes);
+uint64_t gemm_relaid_pitch(uint32_t layout, uint32_t k);
+uint64_t gemm_relaid_bytes(uint32_t layout, uint32_t k, uint64_t rows);
+size_t gemm_tc_workspace_bytes(uint32_t layout, uint32_t m, uint32_t k, uint32_t n, bool f32, bool precise);
+int launch_gemm(cudaStream_t stream, uint32_t layout, const GemmCall& c, void* ws, size_t ws_bytes);
 // n rows of row_bytes bytes -> rows of pitch bytes (a multiple of 16), zero behind the row.  With `used` (the exclusive
 // scan of an expert stack's row counts) slabs of slab_rows rows that nobody is routed to are left out.
 int launch_relay_rows(cudaStream_t stream, const uint8_t* w, uint64_t row_bytes, uint64_t n, uint8_t* out, uint64_t pitch,
                       const uint32_t* used = nullptr, uint32_t slab_rows = 1);
 int launch_widen_q6(cudaStream_t stream, const uint8_t* w, uint32_t k, uint64_t n, uint8_t* out, const uint32_t* used = nullptr,
                     uint32_t slab_rows = 1);
-// Whichever of the two the GEMM reads `scheme` from: gemm_relaid_bytes(scheme, k, n) bytes at out.
-int launch_relay(cudaStream_t stream, uint32_t scheme, const uint8_t* w, uint32_t k, uint64_t n, uint8_t* out, const uint32_t* used = nullptr,
+// Whichever of the two makes `layout`: gemm_relaid_bytes(layout, k, n) bytes at out.
+int launch_relay(cudaStream_t stream, uint32_t layout, const uint8_t* w, uint32_t k, uint64_t n, uint8_t* out, const uint32_t* used = nullptr,
                  uint32_t slab_rows = 1);
 
 // f32 streaming GEMV (m <= 8) for rows of any length; with expert_idx, row i of x by the slab it names, all rows in one launch.

@@ -268,12 +268,12 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const void* x, const ui
     }
 }
 
-struct MoeTcPlan { bool ok, relaid, precise; uint32_t tiles, tile_rows; uint64_t pitch; size_t off_table, off_xg, off_w, bytes; };
+struct MoeTcPlan { bool ok, relaid, precise; uint32_t layout, tiles, tile_rows; uint64_t pitch; size_t off_table, off_xg, off_w, bytes; };
 
 // The scratch of the tensor-core path behind the sort's arrays (which end at `base`): tile table, gathered activations
 // and, for rows TMA cannot tile where they lie, the re-laid slabs.  Not taken (ok = false) for other formats or when it
-// would need more than 4 GiB.
-static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, bool w_aligned, size_t base) {
+// would need more than 4 GiB.  Q6_K's slabs are widened (276 bytes a super-block) or, with less room, copied as they are (210).
+static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool xbf, bool w_aligned, size_t base, bool widen = true) {
     MoeTcPlan p{};
     const void* aligned = (const void*)256;
     if (options().gemm_kernel.load() == 1) return p;
@@ -283,11 +283,12 @@ static MoeTcPlan plan_moe_tc(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n
     p.precise = p.relaid || m < kMoeBf16Rows;
     p.tile_rows = moe_tile_rows(m, E, gemm_most_rows(scheme, !xbf, p.precise));
     p.tiles = m / p.tile_rows + (E < m ? E : m);
-    p.pitch = p.relaid ? gemm_relaid_pitch(scheme, k) : 0;
+    p.layout = p.relaid && widen && scheme == RLXQ_Q6_K ? kQ6Wide : scheme;
+    p.pitch = p.relaid ? gemm_relaid_pitch(p.layout, k) : 0;
     p.off_table = up(base);
     p.off_xg = p.off_table + up((size_t)(p.tiles + 1) * 16);
     p.off_w = p.off_xg + up((size_t)gemm_x_parts(!xbf, p.precise) * m * k * 2);
-    p.bytes = p.off_w + (p.relaid ? up((size_t)gemm_relaid_bytes(scheme, k, (uint64_t)n * E)) : 0);
+    p.bytes = p.off_w + (p.relaid ? up((size_t)gemm_relaid_bytes(p.layout, k, (uint64_t)n * E)) : 0);
     p.ok = p.bytes <= (4ull << 30) && (uint64_t)n * E <= 0x7FFFFFFFull;
     return p;
 }
@@ -334,6 +335,7 @@ static MoePlan plan_moe(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uin
     p.route = MoeRoute::General;
     if (m <= kMoeDecodeRows && gemv == 1) return p;
     p.tc = plan_moe_tc(scheme, m, k, n, E, xbf, !((uintptr_t)w & 15u), p.sort_bytes);
+    if (p.tc.layout == kQ6Wide && (!p.tc.ok || p.tc.bytes > ws_bytes)) p.tc = plan_moe_tc(scheme, m, k, n, E, xbf, !((uintptr_t)w & 15u), p.sort_bytes, false);
     if (p.tc.ok) {
         p.route = MoeRoute::Gemm;
         p.bytes = p.tc.bytes;
@@ -417,7 +419,7 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
         GemmCall c{};
         c.w = wst;
         if (tc.relaid) {
-            rc = launch_relay(s, scheme, wst, k, (uint64_t)n * num_experts, ws + tc.off_w, offsets, n);
+            rc = launch_relay(s, tc.layout, wst, k, (uint64_t)n * num_experts, ws + tc.off_w, offsets, n);
             if (rc) return rc;
             c.w = ws + tc.off_w;
         }
@@ -428,7 +430,7 @@ extern "C" int rlxq_grouped_matmul(rlxq_stream_t stream, uint32_t scheme, const 
         c.x = xg; c.x_rows = m; c.f32 = !xbf; c.w_pitch = tc.pitch; c.precise = tc.precise;
         c.y = y; c.ybf = ybf; c.k = k; c.n = n;
         c.num_slabs = num_experts; c.groups = table; c.group_tiles = tc.tiles; c.tile_rows = tc.tile_rows; c.row_map = perm;
-        return launch_gemm(s, scheme, c, nullptr, 0);
+        return launch_gemm(s, tc.layout, c, nullptr, 0);
     }
     const uint32_t wpc = 8;
     unsigned gx = (n + wpc - 1) / wpc;

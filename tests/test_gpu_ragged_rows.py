@@ -268,6 +268,39 @@ def test_gemm_on_widened_q6_k_rows(m, k, n, x_bf16, shift):
     assert _error(got, ref) <= 1.02 * _error(general, ref), (_error(got, ref), _error(general, ref))
 
 
+@pytest.mark.parametrize("m,k,n,x_bf16,shift,slices", [(96, 768, 18944, False, 0, 0), (64, 1280, 19000, True, 0, 0), (33, 2048, 18945, False, 2, 2)])
+def test_q6_k_prompt_with_room_for_the_rows_alone(m, k, n, x_bf16, shift, slices):
+    """Widened rows take 276 bytes a super-block.  A caller with scratch for 210, all that such a call once needed, has the rows copied
+    as they are, and with less than that the general kernel."""
+    import torch
+    import rlx_b200 as R
+    from rlx_b200._lib import lib
+    s, w, x, xd = _inputs("q6_k", m, k, n, x_bf16, 1600 + m)
+    buf = torch.zeros(w.size + 16, dtype=torch.uint8, device="cuda")
+    wd = buf[shift:shift + w.size]
+    wd.copy_(torch.from_numpy(w))
+
+    def up(v):
+        return (v + 255) // 256 * 256
+    # activations in three parts, rows on a multiple of 16 bytes; 149 tiles of eight k groups on 148 SMs in two slices
+    need = up(0 if x_bf16 else 6 * m * k) + up(n * ((k // 256 * 210 + 15) // 16 * 16)) + up(slices * (m * n + 3) // 4 * 16)
+    ws, y = torch.empty(need + 256, dtype=torch.uint8, device="cuda"), torch.empty((m, n), device="cuda")
+
+    def run(bytes):
+        before = R.launch_count()
+        assert lib.rlxq_matmul(torch.cuda.current_stream().cuda_stream, s, xd.data_ptr(), int(x_bf16), wd.data_ptr(), y.data_ptr(), 0, m, k, n,
+                               ws.data_ptr(), bytes) == 0
+        R.device_status()
+        return y.cpu().numpy(), R.launch_count() - before
+    (got, launches), (general, rounds) = run(need), run(need - 256)
+    assert launches == (2 if x_bf16 else 3) + (slices > 0) and rounds == (m + 7) // 8      # (split,) copy, GEMM(, sum of slices)
+    cols = np.arange(0, n, 37)
+    rb = k // 256 * 210
+    W = np.stack([O.dequant(s, w[c * rb:(c + 1) * rb], k) for c in cols]).astype(np.float64)
+    ref = x.astype(np.float64) @ W.T
+    assert _error(got[:, cols], ref) <= 1.02 * _error(general[:, cols], ref), (_error(got[:, cols], ref), _error(general[:, cols], ref))
+
+
 # narrow tiles and tiles of 80 and 96 rows, slices (few tiles, long rows), the last group of a row
 @pytest.mark.parametrize("m,k,n,x_bf16", [(20, 768, 130, False), (75, 1280, 200, True), (96, 5888, 128, False), (300, 2304, 140, True)])
 def test_gemm_on_widened_q6_k_rows_with_infinite_scales(m, k, n, x_bf16):

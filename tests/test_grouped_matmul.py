@@ -81,6 +81,19 @@ def test_workspace_of_few_rows_holds_no_copy_of_the_stack():
     assert need("q6_k", 64, 1792, 320, 4) >= 320 * 4 * 7 * 210
 
 
+def test_workspace_of_a_stack_that_has_no_room_to_be_widened():
+    """A stack of Q6_K rows that TMA cannot tile, 3.6 GB as they are copied and 4.7 as they are widened: over the 4 GiB that a call
+    asks for at most, so the GEMM gets them copied, and its scratch is asked for."""
+    import ctypes as C
+    from rlx_b200._lib import lib
+    b = C.c_size_t()
+    k, n, E = 11008, 50000, 8
+    assert lib.rlxq_grouped_workspace_bytes(O.Q6_K, 512, k, n, E, C.byref(b)) == 0
+    assert n * E * (k // 256) * 210 <= b.value <= 4 << 30
+    assert lib.rlxq_grouped_workspace_bytes(O.Q6_K, 512, k, n // 2, E, C.byref(b)) == 0
+    assert n // 2 * E * (k // 256) * 276 <= b.value <= 4 << 30
+
+
 # ------------------------------------------------------------------ GPU
 def _gpu(x, w, idx, s, n, E, x_bf16=False, y_bf16=False):
     import torch
@@ -313,3 +326,49 @@ def test_gpu_decode_rows_in_one_launch(sch, m, k, n, E, x_bf16, y_bf16):
     scale = np.abs(ref).max()
     assert np.abs(y - each).max() <= (2.0 ** -8 if y_bf16 else 1e-6) * scale
     assert np.abs(y - ref).max() <= (2.0 ** -8 if y_bf16 else 0.0) * scale + 2e-4 * scale
+
+
+# slabs in use and not, four super-blocks (what a warp takes at a time) over the end of one: 129 and 3 rows of one or three
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,k,n,E,used,x_bf16", [(40, 768, 129, 9, (1, 4, 8), False), (64, 256, 3, 40, (0, 2, 5, 6, 39), True),
+                                                 (33, 256, 129, 5, (3,), False), (48, 1280, 3, 12, (11, 0), True)])
+def test_gpu_grouped_gemm_on_re_laid_q6_k_slabs(m, k, n, E, used, x_bf16):
+    """Rows that TMA cannot tile, with slabs that nobody is routed to: widened with the scratch that is asked for, copied as they are
+    with less, and no further from 64 bits than the general kernel (2 %) either way."""
+    import ctypes as C
+    import torch
+    import rlx_b200 as R
+    from rlx_b200._lib import lib
+    s = O.Q6_K
+    w = O.fill_weights(s, 90 + m, k, n * E)
+    xd = torch.from_numpy(O.fill_normal(91 + m, m * k).reshape(m, k)).cuda()
+    if x_bf16:
+        xd = xd.to(torch.bfloat16)
+    x = xd.float().cpu().numpy()
+    idx = np.array([used[i % len(used)] for i in range(m)], np.float32)
+    idx[7] = E
+    wd, ids = torch.from_numpy(w).cuda(), torch.from_numpy(idx).cuda()
+    W = O.dequant(s, w, k * n * E).reshape(E, n, k).astype(np.float64)
+    ref = np.stack([x[i].astype(np.float64) @ W[int(e)].T if e < E else np.zeros(n) for i, e in enumerate(idx)])
+    need = C.c_size_t()
+    assert lib.rlxq_grouped_workspace_bytes(s, m, k, n, E, C.byref(need)) == 0
+
+    def run(bytes):
+        ws = torch.full((bytes + 256,), 0xFF, dtype=torch.uint8, device="cuda")      # (every value is NaN)
+        y = torch.full((m, n), float("nan"), device="cuda")
+        before = R.launch_count()
+        assert lib.rlxq_grouped_matmul(torch.cuda.current_stream().cuda_stream, s, xd.data_ptr(), int(x_bf16), wd.data_ptr(), ids.data_ptr(),
+                                       y.data_ptr(), 0, m, k, n, E, ws.data_ptr(), bytes) == 0
+        R.device_status()
+        y = y.cpu().numpy()
+        assert np.all(y[7] == 0)
+        return np.linalg.norm(y - ref) / np.linalg.norm(ref), R.launch_count() - before
+    copied = need.value - n * E * (k // 256 * 276 - (k // 256 * 210 + 15) // 16 * 16) + 256      # (arrays start on multiples of 256)
+    (wide, launches), (narrow, launches2) = run(need.value), run(copied)
+    R.set_option("gemm_kernel", 1)
+    try:
+        general, launches3 = run(need.value)
+    finally:
+        R.set_option("gemm_kernel", 0)
+    assert launches == launches2 == 6 and launches3 == 3      # sort, tiles, copy, gather, GEMM; sort, the general kernel
+    assert wide <= 1.02 * general and narrow <= 1.02 * general, (wide, narrow, general)
