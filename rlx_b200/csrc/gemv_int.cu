@@ -87,6 +87,9 @@ template <uint32_t SCHEME, bool MMA = false> struct IntBox {
     static constexpr uint32_t STAGE_BYTES = NB * BOX_BYTES;
 };
 
+constexpr uint32_t kExpertRows = 8;
+struct ExpertSplit { uint32_t ctas, chunks_q; };   // CTAs of a row, and the chunks that each takes at least
+
 struct IntParams {
     CUtensorMap wmap;      // W as [n rows][row_bytes / 8] eight-byte elements, box = 16 rows x IntBox::ROW
     const uint8_t* w;
@@ -127,11 +130,12 @@ struct IntParams {
     uint32_t early;              // single-kernel mode: stages requested before the dependency wait
     // Expert-indirect mode (MoE decode): W is a stack of [n, k] slabs and this launch multiplies by slab
     // *expert_sel read as the reference's `as usize` cast does (expert_of_row), on the device after the
-    // dependency wait; an id of num_experts or more makes the kernel write zeros and return at once.  Grid row r (of
-    // gridDim.y) multiplies activation row r by slab expert_sel[r]: gridDim.x CTAs each, and row_scratch bytes of partial
-    // tiles and rendezvous words.
+    // dependency wait; an id of num_experts or more makes the row zero.  Grid row r (of gridDim.y) multiplies activation row
+    // r by slab expert_sel[r], with row_scratch bytes of partial tiles and rendezvous words: gridDim.x CTAs each, or, where
+    // some rows are zero, split[rows left - 1].
     const float* expert_sel;
     uint32_t num_experts;
+    ExpertSplit split[kExpertRows];
     size_t row_scratch;
 };
 
@@ -1236,12 +1240,11 @@ struct Segment { uint32_t tile, c0, c1; };
 // tail tile (chunks 0 .. tail_c1 of tile tail_tile) if has_tail, and nwhole whole tiles from first_whole.
 struct Range { uint32_t len, has_head, has_tail, head_tile, head_c0, head_c1, tail_tile, tail_c1, first_whole, nseg, nshared; };
 
-__device__ __forceinline__ Range make_range(const IntParams& P, uint32_t me) {
-    // CTA i takes chunks [i*q + min(i, r), ...): the first r CTAs one chunk more (q, r from the host)
+// CTA i takes chunks [i*q + min(i, r), ...): the first r CTAs one chunk more; nc chunks are a tile
+__device__ __forceinline__ Range make_range(uint32_t nc, uint32_t q, uint32_t r, uint32_t me) {
     Range rg;
-    const uint32_t nc = P.nchunks;
-    const uint32_t beg = me * P.chunks_q + min(me, P.chunks_r);
-    const uint32_t end = beg + P.chunks_q + (me < P.chunks_r ? 1u : 0u);
+    const uint32_t beg = me * q + min(me, r);
+    const uint32_t end = beg + q + (me < r ? 1u : 0u);
     rg.len = end - beg;
     const uint32_t bt = beg / nc, et = end / nc;
     const uint32_t bc = beg - bt * nc, ec = end - et * nc;
@@ -1261,6 +1264,7 @@ __device__ __forceinline__ Range make_range(const IntParams& P, uint32_t me) {
     rg.nseg = rg.nshared + nwhole;
     return rg;
 }
+__device__ __forceinline__ Range make_range(const IntParams& P, uint32_t me) { return make_range(P.nchunks, P.chunks_q, P.chunks_r, me); }
 // The CTA whose range holds chunk g (the inverse of the split in make_range).
 __device__ __forceinline__ uint32_t owner_of(const IntParams& P, uint32_t g) {
     const uint32_t big = P.chunks_r * (P.chunks_q + 1);
@@ -1348,10 +1352,10 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
     griddep_launch_dependents();
     if (tid == 0) tma_prefetch_desc(&P.wmap);
 
-    const uint32_t G = gridDim.x, me = blockIdx.x;
-    const uint32_t erow = EXPERT ? blockIdx.y : 0u;                     // the activation row of this CTA
-    const Range rg = make_range(P, me);
-    const uint32_t nseg = rg.nseg;
+    const uint32_t G = gridDim.x;
+    uint32_t me = blockIdx.x;
+    uint32_t erow = 0u, row_off = 0u;                                   // EXPERT: the activation row of this CTA, its slab's first row
+    Range rg = make_range(P, me);
     const uint32_t ku = P.k / 256;
 
     if (tid == 0) {
@@ -1368,27 +1372,52 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if constexpr (EXPERT) {
+        // every warp learns the slabs after the dependency wait (nothing is requested before it)
+        griddep_wait();
+        const uint32_t rows = gridDim.y;
+        erow = blockIdx.y;
+        float id = P.expert_sel[erow];
+        const float all = P.expert_sel[min(lane, rows - 1u)];
+        const uint32_t there = __ballot_sync(0xFFFFFFFFu, !(all >= (float)P.num_experts));       // (as expert_of_row has it)
+        if (__builtin_expect(there != 0xFFFFFFFFu, 0)) {       // (the lanes past the rows repeat the last one)
+            // Rows of no expert are zero, a share of them from every CTA, and their CTAs join the other rows': one row in eight of
+            // Q6_K 4096 x 14336, as it is routed where the experts lie on several GPUs, took 84 us on its own CTAs alone (26 us as
+            // a launch per row), 18 us now.
+            uint32_t left = there & ((1u << rows) - 1u);
+            const uint32_t ctas = G * rows, cta = blockIdx.y * G + me, count = __popc(left);
+            if (warp == CW + 1) {
+                const uint32_t j0 = (uint32_t)((uint64_t)cta * P.n / ctas), j1 = (uint32_t)((uint64_t)(cta + 1) * P.n / ctas);
+#pragma unroll 1
+                for (uint32_t row = 0; row < rows; ++row) {
+                    if ((left >> row) & 1u) continue;
+#pragma unroll 1
+                    for (uint32_t j = j0 + lane; j < j1; j += 32) {
+                        if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[(size_t)row * P.n + j] = 0;
+                        else reinterpret_cast<float*>(P.y)[(size_t)row * P.n + j] = 0.f;
+                    }
+                }
+            }
+            if (count == 0) return;
+            const ExpertSplit sp = P.split[count - 1u];
+#pragma unroll 1
+            for (me = cta; me >= sp.ctas; me -= sp.ctas) left &= left - 1u;
+            if (left == 0u) return;
+            erow = (uint32_t)__ffs((int)left) - 1u;
+            id = P.expert_sel[erow];
+            rg = make_range(P.nchunks, sp.chunks_q, P.total_chunks - sp.ctas * sp.chunks_q, me);
+        }
+        uint32_t e = 0u;
+        expert_of_row(id, P.num_experts, &e);
+        row_off = e * P.n;
+    }
+    const uint32_t nseg = rg.nseg;
     // The first fill of the ring is spread over the warps, one stage each: a TMA request occupies its
     // issuing thread for a few hundred cycles, and one thread issuing them all delays the stream's start.
     const uint32_t pre = P.xstream ? 0u : min(min(NS, CW), rg.len);
 
-    // expert-indirect mode: every role learns the slab after the dependency wait (nothing is requested
-    // before it) and leaves at once when the id is out of range
-    auto resolve_expert = [&](uint32_t& row_off) -> bool {
-        row_off = 0u;
-        if constexpr (EXPERT) {
-            griddep_wait();
-            uint32_t e;
-            if (!expert_of_row(P.expert_sel[erow], P.num_experts, &e)) return false;
-            row_off = e * P.n;
-        }
-        return true;
-    };
-
     if (warp == CW) {
         // ---------------- producer warp ----------------
-        uint32_t row_off;
-        if (!resolve_expert(row_off)) return;
         auto produce = [&](uint32_t tile, uint32_t chunk, uint32_t s) {
             // rows past n and bytes past the row end arrive as zeros (d = 0: they add nothing)
             const uint32_t full = smem_u32(&bars[s]);
@@ -1459,17 +1488,6 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
 
     if (warp == CW + 1) {
         // ---------------- finisher warp ----------------
-        {
-            uint32_t ro;
-            if (!resolve_expert(ro)) {    // no such expert: this CTA's share of the row is zero
-                const uint32_t e1 = (uint32_t)((uint64_t)(me + 1) * P.n / G);
-                for (uint32_t j = (uint32_t)((uint64_t)me * P.n / G) + lane; j < e1; j += 32) {
-                    if (P.y_bf16) reinterpret_cast<uint16_t*>(P.y)[(size_t)erow * P.n + j] = 0;
-                    else reinterpret_cast<float*>(P.y)[(size_t)erow * P.n + j] = 0.f;
-                }
-                return;
-            }
-        }
         // Adds the 16 partials of every output (2 halves x 8 warps, fixed order) and writes the tile,
         // or, for a tile shared with other CTAs, runs the publish / count / re-read sequence.  That
         // sequence is a chain of three global round trips; here it delays nobody, because the
@@ -1620,8 +1638,6 @@ __global__ void __launch_bounds__(int_threads(MMA), (MMA || MM > 2) ? 1 : 2) gem
     }
 
     // ---------------- consumer warps: lane = (tile row, half of the unit) ----------------
-    uint32_t row_off;
-    if (!resolve_expert(row_off)) return;
     auto request_first_stage = [&](uint32_t w0, uint32_t w1) {
         if (warp >= w0 && warp < min(w1, pre) && lane == 0) {
             uint32_t i = warp, si = 0;
@@ -2208,13 +2224,17 @@ static IntPlan plan_int(uint32_t m, uint32_t k, uint32_t n) {
     return pl;
 }
 
-// The expert-indirect mode's plan for `rows` activation rows in one launch: each row gets its share of the CTAs.
+// The expert-indirect mode's plan for `rows` activation rows in one launch: each row gets its share of the CTAs, `share` as far as
+// it has work for them (whole tiles, as in plan_int) and a tile is cut once (`most`, the CTAs of a single row's plan).
+static uint32_t expert_row_ctas(const IntPlan& pl, uint32_t share, uint32_t most) {
+    uint32_t ctas = std::min(share, most);
+    if (pl.ntiles < ctas && pl.ntiles * 10 >= ctas * 7) ctas = pl.ntiles;
+    return std::min(ctas, pl.total_chunks);
+}
 template <uint32_t SCHEME> static IntPlan plan_expert(uint32_t k, uint32_t n, uint32_t rows) {
     IntPlan pl = plan_int<SCHEME>(1, k, n);
     if (!pl.ok || rows == 1) return pl;
-    pl.grid = (uint32_t)sm_count() * pl.per_sm / rows;
-    if (pl.ntiles < pl.grid && pl.ntiles * 10 >= pl.grid * 7) pl.grid = pl.ntiles;
-    if (pl.grid > pl.total_chunks) pl.grid = pl.total_chunks;
+    pl.grid = expert_row_ctas(pl, (uint32_t)sm_count() * pl.per_sm / rows, ~0u);
     pl.two_way = pl.total_chunks / pl.grid >= pl.nchunks;
     return pl;
 }
@@ -2232,7 +2252,7 @@ template <uint32_t SCHEME, int MM, bool MMA = false, bool TP = false, bool EXPER
 static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf,
                         uint32_t k, uint32_t n, void* ws, size_t ws_bytes, const IntPlan& pl, int* err_word, bool pair,
                         const float* expert_sel = nullptr, uint32_t num_experts = 0, uint32_t m_real = (uint32_t)MM,
-                        const TpPush* tp = nullptr, uint32_t expert_rows = 1) {
+                        const TpPush* tp = nullptr, uint32_t expert_rows = 1, uint32_t most_ctas = 0) {
     using T = StagedTraits<SCHEME>;
     Geometry g;
     geometry(SCHEME, &g);
@@ -2274,6 +2294,10 @@ static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint
     }
     P.expert_sel = expert_sel;
     P.num_experts = num_experts;
+    for (uint32_t left = 1; expert_sel && left <= expert_rows; ++left) {
+        const uint32_t ctas = expert_row_ctas(pl, pl.grid * expert_rows / left, most_ctas);
+        P.split[left - 1] = ExpertSplit{ctas, pl.total_chunks / ctas};
+    }
     P.row_scratch = expert_row_scratch(pl);
     if (expert_sel && !P.inline_q) return fail(RLXQ_E_SHAPE, "expert-indirect GEMV needs the single-kernel mode");
     P.x = x; P.x_bf16 = xbf ? 1u : 0u;
@@ -2338,7 +2362,7 @@ static int launch_int_s(cudaStream_t stream, const void* x, bool xbf, const uint
         }
         if (expert_sel)
             return launch_int_t<SCHEME, 1, false, false, true>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, plan_expert<SCHEME>(k, n, m), err_word, pair,
-                                                               expert_sel, num_experts, 1, nullptr, m);
+                                                               expert_sel, num_experts, 1, nullptr, m, pl.grid);
         if (m == 1) return launch_int_t<SCHEME, 1>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair);
         if (m == 2) return launch_int_t<SCHEME, 2>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, nullptr, 0, 2);
         return launch_int_t<SCHEME, 4>(stream, x, xbf, w, y, ybf, k, n, ws, ws_bytes, pl, err_word, pair, nullptr, 0, m);

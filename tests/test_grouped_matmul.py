@@ -328,6 +328,49 @@ def test_gpu_decode_rows_in_one_launch(sch, m, k, n, E, x_bf16, y_bf16):
     assert np.abs(y - ref).max() <= (2.0 ** -8 if y_bf16 else 0.0) * scale + 2e-4 * scale
 
 
+# cut tiles, whole tiles, fewer tiles than CTAs; one, some, all but one and none of the rows routed
+@pytest.mark.gpu
+@pytest.mark.parametrize("sch,m,k,n,x_bf16,y_bf16", [("q4_k", 8, 4096, 14336, False, False), ("q8_0", 4, 2304, 5003, True, False), ("q5_k", 2, 4096, 3600, False, True),
+                                                     ("q4_0", 7, 11008, 8000, True, True), ("q6_k", 3, 2048, 3584, False, False), ("q4_k", 5, 256, 16, False, False)])
+def test_gpu_decode_rows_of_no_expert_leave_their_ctas_to_the_others(sch, m, k, n, x_bf16, y_bf16):
+    """Rows with an id out of range are zero, and the others are multiplied as by a launch with no such rows: a single one, where the
+    CTAs of a step divide evenly, has the bits of a launch of its own, and any differ by the order of a tile's two parts at most."""
+    import ctypes as C
+    import torch
+    from rlx_b200._lib import lib
+    import rlx_b200 as R
+    E = 3
+    s = O.SCHEMES[sch]
+    wd = torch.from_numpy(O.fill_weights(s, 70 + m, k, n * E)).cuda()
+    xd = torch.from_numpy(O.fill_normal(71 + m, m * k).reshape(m, k)).cuda()
+    if x_bf16:
+        xd = xd.to(torch.bfloat16)
+
+    def scratch(rows):
+        need = C.c_size_t()
+        assert lib.rlxq_grouped_workspace_bytes(s, rows, k, n, E, C.byref(need)) == 0
+        return torch.randint(0, 256, (need.value,), dtype=torch.uint8, device="cuda")
+
+    def run(idx, ws):
+        y = torch.full((m, n), float("nan"), dtype=torch.bfloat16 if y_bf16 else torch.float32, device="cuda")
+        before = R.launch_count()
+        assert lib.rlxq_grouped_matmul(torch.cuda.current_stream().cuda_stream, s, xd.data_ptr(), int(x_bf16), wd.data_ptr(),
+                                       torch.from_numpy(idx).cuda().data_ptr(), y.data_ptr(), int(y_bf16), m, k, n, E, ws.data_ptr(), ws.numel()) == 0
+        R.device_status()
+        return y.float().cpu().numpy(), R.launch_count() - before
+    ws, ws1 = scratch(m), scratch(1)
+    for routed in ({m - 1}, {0, m // 2}, set(range(m)) - {1}, set()):
+        idx = np.array([(2 * i + 1) % E if i in routed else E + i for i in range(m)], np.float32)
+        (y, launches), (each, launches1) = run(idx, ws), run(idx, ws1)
+        assert (launches, launches1) == (1, m)
+        assert np.array_equal(run(idx, ws)[0], y)
+        out = [i for i in range(m) if i not in routed]
+        assert np.all(y[out] == 0) and np.all(each[out] == 0) and np.isfinite(y).all()
+        assert np.abs(y - each).max() <= (2.0 ** -8 if y_bf16 else 1e-6) * max(np.abs(each).max(), 1e-30)
+        if len(routed) == 1 and 296 % m == 0:
+            assert np.array_equal(y, each)
+
+
 # slabs in use and not, four super-blocks (what a warp takes at a time) over the end of one: 129 and 3 rows of one or three
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,k,n,E,used,x_bf16", [(40, 768, 129, 9, (1, 4, 8), False), (64, 256, 3, 40, (0, 2, 5, 6, 39), True),
