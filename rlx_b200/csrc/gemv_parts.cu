@@ -479,31 +479,32 @@ __global__ void __launch_bounds__(kPartsMaxWarps * 32, 1) gemv_parts_kernel(cons
     }
 }
 
-template <uint32_t SCHEME, int NP, bool W4>
-static int launch_parts_t(cudaStream_t stream, PartsParams P) {
-    using G = PartsGeom<SCHEME>;
+// The split of k x n weights: sets P's work split and shared-memory layout, returns the bytes of shared memory.  As few passes as
+// leave every warp a ring of two steps at least, with as many streams as sixteen warps make.
+template <uint32_t SCHEME> static uint32_t plan_parts(PartsParams& P, uint32_t np) {
     const uint32_t pieces = (P.k + kPartsCols - 1) / kPartsCols;
     P.tiles = (P.n + kPartsTile - 1) / kPartsTile;
     const uint32_t sms = (uint32_t)sm_count();                // one CTA per SM
     P.ctas = sms < P.tiles ? sms : P.tiles;
     const uint32_t most = (P.tiles + P.ctas - 1) / P.ctas;    // tiles of a CTA
-    uint32_t smem = 0;
-    // as few passes as leave every warp a ring of two steps at least
     for (P.passes = (pieces + kPartsMaxWarps - 1) / kPartsMaxWarps;; ++P.passes) {
         P.nw = (pieces + P.passes - 1) / P.passes;
         P.streams = std::min({kPartsMaxWarps / P.nw, most, 15u});      // (a named barrier each, of fifteen)
-        const uint32_t warps = P.nw * P.streams, step = warps * kPartsTile * G::SLOT;
-        P.off_ring = NP * P.nw * (8u * 512u);
+        const uint32_t warps = P.nw * P.streams, step = warps * kPartsTile * PartsGeom<SCHEME>::SLOT;
+        P.off_ring = np * P.nw * (8u * 512u);
         const uint32_t red = warps * (2u * 512u), totals = P.passes > 1 ? std::min(most, kPartsTotals) * kPartsTile * 8u * 4u : 0u;
         if (P.off_ring + red + totals + 2 * step <= 227u * 1024u) {
             P.depth = std::min(4u, (227u * 1024u - P.off_ring - red - totals) / step);
             P.off_red = P.off_ring + P.depth * step;
             P.off_total = P.off_red + red;
-            smem = P.off_total + totals;
-            break;
+            return P.off_total + totals;
         }
     }
-    const uint32_t warps = P.nw * P.streams;
+}
+
+template <uint32_t SCHEME, int NP, bool W4>
+static int launch_parts_t(cudaStream_t stream, PartsParams P) {
+    const uint32_t smem = plan_parts<SCHEME>(P, NP), warps = P.nw * P.streams;
     static std::atomic<uint32_t> attr_set[64];
     int dev = 0;
     RLXQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -523,13 +524,42 @@ static int launch_parts_s(cudaStream_t stream, const PartsParams& P, bool xbf) {
     return xbf ? launch_parts_t<SCHEME, 1, false>(stream, P) : launch_parts_t<SCHEME, 3, false>(stream, P);
 }
 
-// Five to eight rows where this kernel is the faster one: the f32 kernel takes 3 us and 1.15 us a million weights, this one 4 us,
-// 0.55 us a million, and 2.4 us for every column pass, of 2048 columns (f32 activations) or 4096 (bf16).
+// Microseconds, this kernel (a call, a column pass, a pass of one stream, a tile of a stream and pass, and for each of a CTA's warps)
+// and the f32 kernel (a call, a row of a CTA and pass, and for sixteen warps of them): fits to 1900 calls of batch 5 to 8, both timed.
+struct PartsCost { float call, pass, alone, tile, warp, f32_call, f32_row, f32_warps; };
+template <uint32_t SCHEME> static bool parts_is_faster(uint32_t k, uint32_t n, bool xbf) {
+    const PartsCost c = SCHEME == RLXQ_Q4_0   ? (xbf ? PartsCost{0.46f, 1.20f, -0.06f, 1.13f, 0.11f, 1.74f, 0.18f, 0.31f} : PartsCost{0.62f, 0.66f, 2.52f, 0.35f, 0.19f, 2.51f, 0.18f, 0.33f})
+                        : SCHEME == RLXQ_Q8_0 ? (xbf ? PartsCost{-0.26f, 2.20f, -0.61f, 1.49f, 0.16f, 1.64f, 0.18f, 0.35f} : PartsCost{0.72f, 0.34f, 2.80f, 0.30f, 0.29f, 2.34f, 0.17f, 0.37f})
+                                              : (xbf ? PartsCost{-0.03f, 2.30f, -0.52f, 0.98f, 0.18f, 1.66f, 0.23f, 0.37f} : PartsCost{0.90f, 1.04f, 2.22f, 0.34f, 0.25f, 2.51f, 0.20f, 0.42f});
+    PartsParams P{};
+    P.k = k; P.n = n;
+    plan_parts<SCHEME>(P, xbf ? 1 : 3);
+    const uint32_t most = (P.tiles + P.ctas - 1) / P.ctas;
+    const float passes = (float)P.passes, rounds = passes * (float)((most + P.streams - 1) / P.streams);
+    const float parts = c.call + passes * (c.pass + c.alone / (float)P.streams) + rounds * (c.tile + c.warp * (float)(P.nw * P.streams));
+    // gemv_f32.cu with four activation rows: 512 columns a warp, sixteen warps an SM, half of the CTAs for either four rows, two
+    // weight rows a step
+    const uint32_t pieces = (k + 511) / 512, f32_passes = (pieces + 15) / 16, warps = (pieces + f32_passes - 1) / f32_passes;
+    const uint32_t per_sm = 16 / warps, tiles = std::max(1u, (uint32_t)sm_count() * per_sm / 2), rows = ((n + tiles - 1) / tiles + 1) / 2 * 2;
+    const float f32 = c.f32_call + (float)f32_passes * (float)rows * (c.f32_row + c.f32_warps * (float)(warps * per_sm) / 16.0f);
+    return parts < f32;
+}
+
+// Five to eight rows where this kernel is the faster one.  Rows of up to 1024 weights: from 2 M weights on, where the two are level
+// (2.3 M: Q8_0 1.04 to 1.11 of the f32 kernel's time with f32 activations; 2.9 M: 0.74 to 0.91).  Longer rows: by the estimate,
+// because what a column pass or a second tile of a few CTAs costs depends on the split; with the weight count alone one call in
+// 27 was slower than the f32 kernel, up to 1.30 times (Q6_K 3840 x 2410 f32, 13.2 and 16.4 us), now one in 160, 1.11 at worst, of 2934.
 bool gemv_parts_pays(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, const void* x) {
     const bool known = scheme == RLXQ_Q4_0 || scheme == RLXQ_Q8_0 || scheme == RLXQ_Q6_K;
     if (!known || m < 5 || m > 8 || ((uintptr_t)x & 15u) || k % 32 || k == 0) return false;
     const uint64_t cols = xbf ? 4096 : 2048, passes = (k + cols - 1) / cols;
-    return (uint64_t)k * n > 2000000ull + 5500000ull * (passes - 1);
+    if ((uint64_t)k * n <= 2000000ull + 5500000ull * (passes - 1)) return false;      // (too few to be asked about)
+    if (k <= 1024) return true;
+    switch (scheme) {
+        case RLXQ_Q4_0: return parts_is_faster<RLXQ_Q4_0>(k, n, xbf);
+        case RLXQ_Q8_0: return parts_is_faster<RLXQ_Q8_0>(k, n, xbf);
+        default: return parts_is_faster<RLXQ_Q6_K>(k, n, xbf);
+    }
 }
 
 int launch_gemv_parts(cudaStream_t stream, uint32_t scheme, const void* x, bool xbf, const uint8_t* w, void* y, bool ybf, uint32_t m,

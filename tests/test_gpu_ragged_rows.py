@@ -76,6 +76,25 @@ def test_gemv_in_parts(sch, m, k, n, x_bf16, shift):
     assert torch.equal(y.isnan(), f32.isnan()) and torch.equal(y[y.isinf()], f32[f32.isinf()]) and y[1].isinf().any() and not y[0].isnan().any()
 
 
+# more tiles a CTA than keep their totals between two column passes, three passes, four
+@pytest.mark.parametrize("sch,m,k,n,x_bf16", [("q4_0", 5, 3360, 153001, False), ("q6_k", 8, 3840, 4503, False), ("q8_0", 6, 8224, 3001, False),
+                                              ("q6_k", 7, 5888, 2304, False), ("q6_k", 5, 16640, 2403, True)])
+def test_gemv_in_parts_over_several_passes(sch, m, k, n, x_bf16):
+    """Against the f32 kernel as above and, the smaller ones, against 64 bits as below."""
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, 1700 + m)
+    wd = torch.from_numpy(w).cuda()
+    y = R.matmul(xd, wd, s, n)
+    f32 = torch.cat([R.matmul(xd[i:i + 4].contiguous(), wd, s, n) for i in range(0, m, 4)])
+    R.device_status()
+    assert not torch.equal(y, f32)                              # they are different kernels
+    assert float((y - f32).abs().max()) <= 4e-6 * float(f32.square().mean().sqrt())
+    if n < 10000:
+        ref = x.astype(np.float64) @ O.dequant(s, w, k * n).reshape(n, k).astype(np.float64).T
+        assert _error(y.cpu().numpy(), ref) <= 1.03 * _error(f32.cpu().numpy(), ref), (_error(y.cpu().numpy(), ref), _error(f32.cpu().numpy(), ref))
+
+
 # one super-block, one warp and many side by side, both activation types, one and several column passes; 12000 to 40000 results each
 @pytest.mark.parametrize("sch,m,k,n,x_bf16", [("q6_k", 8, 256, 8000, True), ("q6_k", 5, 768, 5003, True), ("q6_k", 8, 3840, 2304, True),
                                               ("q6_k", 6, 2304, 2304, False), ("q6_k", 5, 11008, 2304, True), ("q8_0", 8, 2080, 2304, True),
@@ -93,6 +112,19 @@ def test_gemv_in_parts_is_as_exact_as_the_f32_kernel(sch, m, k, n, x_bf16):
     R.device_status()
     assert not torch.equal(y, f32)                              # they are different kernels
     assert _error(y.cpu().numpy(), ref) <= 1.03 * _error(f32.cpu().numpy(), ref), (_error(y.cpu().numpy(), ref), _error(f32.cpu().numpy(), ref))
+
+
+# a second tile in a few CTAs, three passes for a second stream, one pass of fifteen warps for 34 tiles
+@pytest.mark.parametrize("sch,m,k,n,x_bf16", [("q6_k", 8, 3840, 2410, False), ("q8_0", 8, 14368, 2908, False), ("q8_0", 5, 6176, 3093, False),
+                                              ("q6_k", 6, 5888, 2631, False), ("q6_k", 7, 3840, 541, True)])
+def test_gemv_in_parts_leaves_calls_to_the_f32_kernel_where_that_is_faster(sch, m, k, n, x_bf16):
+    """Calls that the matrix instruction took 1.14 to 1.25 times as long for: the f32 kernel's bits."""
+    import torch
+    import rlx_b200 as R
+    s, w, x, xd = _inputs(sch, m, k, n, x_bf16, 1800 + m)
+    wd = torch.from_numpy(w).cuda()
+    last = torch.cat([xd[4:], torch.zeros_like(xd[:8 - m])])       # (one and two rows have a kernel of their own)
+    assert torch.equal(R.matmul(xd, wd, s, n), torch.cat([R.matmul(xd[:4].contiguous(), wd, s, n), R.matmul(last, wd, s, n)[:m - 4]]))
 
 
 def test_streaming_f32_gemv_on_weights_at_an_odd_address():
