@@ -15,7 +15,7 @@ namespace rlxq {
 // workspace query does not know the weights' address and plans for aligned ones: weights at another address are re-laid only
 // for a caller who brings more than it asks for, and run the general kernel for everybody else.  Q6_K rows are widened, which
 // takes a third more scratch than the rows have bytes; a caller who brings less than that, but room for the rows, has them copied
-// as they are (300 x 11008 x 4096 f32: 170 us widened, 240 copied, 4.8 ms through the general kernel).
+// as they are (300 x 11008 x 4096 f32: 151 us widened, 224 copied, 4.8 ms through the general kernel).
 struct PrefillPlan { bool ok, relaid, halves; uint32_t layout, chunk; uint64_t pitch; size_t off_w, off_y2, off_gemm, bytes; };
 static PrefillPlan plan_prefill(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, bool xbf, bool direct, bool widen = true) {
     PrefillPlan p{};

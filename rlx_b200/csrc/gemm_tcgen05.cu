@@ -920,9 +920,10 @@ __device__ __forceinline__ void gemm_decode_role(const GemmParams& P, GemmBars* 
 // products for f32 activations and two for bf16 ones, a decoder of four packed instructions a pair of weights on aligned words,
 // and the scale applied by the epilogue warps, eight of them, as they add a super-block's sums.  Two threads issue MMAs, for the
 // leading product and for the others: beside the products a round of hand-overs takes one thread 0.4 us, whatever else is left
-// out (loads, decoding, adding).  Second accumulators of either kind are worth 5 to 9 %.  300 x 11008 x 4096 f32 222 us with three
-// parts, 172 with two, 187 with aligned rows from a slow first pass, 173 with barriers looked at before a round's last MMAs, 148 with two
-// issuers and a faster first pass; bf16 184 and 107; 587 x 1280 x 5568 bf16 68 and 38 us, 31 x 13056 x 17990 f32 272 and 208 us.
+// out (loads, decoding, adding).  Second accumulators of either kind are worth 5 to 9 %.  300 x 11008 x 4096 f32, calls in a graph,
+// copy and split included: 223 us with three parts, 172 with two, 187 with aligned rows from a slow first pass, 173 with barriers looked
+// at before a round's last MMAs, 148 with two issuers and a faster first pass (167 us a call by itself, its rows in no cache); bf16
+// activations and f32 results 188 and 116; 587 x 1280 x 5568 bf16 82 and 50 us, 31 x 13056 x 17990 f32 273 and 210 us.
 // Error against 64 bits at k = 11008 1.5e-7 and 1.2e-7.
 // Activation rows of a PRECISE tile: what the epilogue threads have registers for (Q3_K's block is larger: 96 a thread) and
 // shared memory has room for totals beside three operand stages and two raw boxes (Q8_K's are the largest).

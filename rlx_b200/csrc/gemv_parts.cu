@@ -17,10 +17,12 @@
 // after the other.  The loops are rolled: a call lasts microseconds, and straight-line code for 256 columns cost three of
 // them to fetch.
 //
-// Bound: instruction issue (5 to 7 lane instructions a weight, a third of them copies, scales and the meeting of the warps) at
-// sixteen warps an SM.  Batch 8, f32 activations, the f32 kernel (four rows a pass, so twice) and this one: Q6_K 2304 x 6000 19.2
-// and 13.1 us, 5888 x 14336 93 and 54, 12544 x 14400 220 and 111; Q8_0 1056 x 16000 25.1 and 12.6, 9280 x 3328 40.9 and 37.2;
-// Q4_0 544 x 8000 8.9 and 5.0; bf16 activations, Q6_K 5888 x 14336 92 and 44.  At batch 3 and 4 the f32 kernel is level or ahead.
+// Bound: latency at twelve to sixteen warps an SM.  Q6_K 5888 x 14336, batch 8, f32 activations: issue slots 42 % used (8.2 lane
+// instructions a weight, a third of them copies, scales and the meeting of the warps), 7.2 cycles from a warp's instruction to its
+// next (fixed latencies 1.3, loads 1.1, the meeting 1.0, shared memory 0.8), DRAM 14 %.  Batch 8, f32 activations, the f32 kernel (four
+// rows a pass, so twice) and this one: Q6_K 2304 x 6000 19.2 and 13.3 us, 5888 x 14336 95 and 58, 12544 x 14400 224 and 119;
+// Q8_0 1056 x 16000 25.4 and 12.8, 9280 x 3328 41.6 and 36.7; Q4_0 544 x 8000 8.8 and 4.7; bf16 activations, Q6_K 5888 x 14336 94
+// and 45.  At batch 3 and 4 the f32 kernel is level or ahead.
 #include <algorithm>
 
 #include "common.cuh"

@@ -215,6 +215,8 @@ static uint32_t moe_tile_rows(uint32_t m, uint32_t E, uint32_t most) {
 // fits to 56 shapes, 9 to 31 rows, both ways timed: the choice takes 0.4 % longer than the better one in the geometric mean, 20 %
 // at worst.  GEMV and GEMM: 10 x 3072 x 576 Q4_K E16 8 and 34 us, 12 x 7168 x 11840 Q8_0 E4 244 and 346 us, 24 x 4352 x 5632 Q4_0 E16
 // 146 and 222 us, 27 x 2560 x 5440 Q4_0 E4 88 and 69 us, 22 x 4352 x 3200 Q5_K E4 124 and 70 us.
+// Re-laid Q6_K has a faster GEMM since, on widened rows: over 70 batches of them the choice takes 0.6 % longer than the better way, and
+// one is wrong, 29 x 4352 x 2176 E4, 107 us for 72.
 // Batches that the GEMM multiplies in bf16 (kMoeBf16Rows and more) stay with it.
 static bool moe_rows_stream(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t E, bool relaid) {
     if (m <= kMoeDecodeRows) return true;
