@@ -99,7 +99,8 @@ RLXQ_API int rlxq_packed_bytes(uint32_t scheme, uint64_t k, uint64_t n, uint64_t
  * slower.  w_blocks is taken to be 16-byte aligned: at m > 8, weights at another address run the tiled generic kernel with
  * this size where the GEMM would read them in place, and the GEMM on a re-laid copy only with a workspace that has room for
  * that copy too (n rows of k weights rounded up to 256, a multiple of 16 bytes each), a third part of f32 activations and the
- * 192 MB.  The reference reserves k*n*4 bytes. */
+ * 192 MB.  The copy of Q6_K rows that is asked for is widened, 276 bytes for a super-block's 210; with less than that, but room
+ * for the rows as they are, the GEMM takes half as long again.  The reference reserves k*n*4 bytes. */
 RLXQ_API int rlxq_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n,
                          uint32_t x_dtype, uint32_t y_dtype, size_t* bytes);
 

@@ -9,7 +9,7 @@
  * host, counting-sorts the rows there, runs dequantise + sgemm per expert and copies back; here the
  * counting sort (grouped_moe_sort_plan, gguf_matmul.rs:178-205) runs on the device and one kernel
  * walks every expert's rows, so nothing crosses PCIe and nothing synchronises.  Up to 8 rows (decode)
- * go row by row through the streaming GEMV, the expert picked on the device, and so do up to 31 where that is less work.
+ * go through the streaming GEMV, the expert of each picked on the device, and so do up to 31 where that is less work.
  * Above that every expert's rows are gathered next to each other as bf16 (f32 activations in two or three parts) and one
  * launch of the tensor-core GEMM in its grouped form multiplies each tile of 32 to 256 rows by its expert's slab.  From 32
  * rows on, where k is a multiple of 256 (1024 for Q2_K and Q8_K, 2048 for Q3_K and Q6_K) and the stack 16-byte aligned, the
@@ -27,7 +27,8 @@ extern "C" {
 /* Scratch for rlxq_grouped_matmul, for what this many rows are run by: expert offsets, the row permutation and
  * per-expert cursors; for the integer GEMV (decode sizes) its own scratch; for the tensor-core path also the tile
  * table, the gathered activations (m rows of k bf16, two or three times as many for f32 ones) and, for rows of no whole
- * number of 16-byte groups, the slabs on a padded pitch.  256-byte aligned.  A call given less than that (but enough
+ * number of 16-byte groups, the slabs on a padded pitch (Q6_K widened, 276 bytes for 210, where all of it stays within 4 GiB; a
+ * call with room for the 210 alone has them copied as they are).  256-byte aligned.  A call given less than that (but enough
  * for the sort) runs the general kernel instead.  Weights are taken to be 16-byte aligned. */
 RLXQ_API int rlxq_grouped_workspace_bytes(uint32_t scheme, uint32_t m, uint32_t k, uint32_t n, uint32_t num_experts,
                                           size_t* bytes);
