@@ -2294,6 +2294,7 @@ static int launch_int_t(cudaStream_t stream, const void* x, bool xbf, const uint
     }
     P.expert_sel = expert_sel;
     P.num_experts = num_experts;
+    if (expert_rows > kExpertRows) return fail(RLXQ_E_LIMIT, "expert-indirect GEMV: at most %u rows", kExpertRows);
     for (uint32_t left = 1; expert_sel && left <= expert_rows; ++left) {
         const uint32_t ctas = expert_row_ctas(pl, pl.grid * expert_rows / left, most_ctas);
         P.split[left - 1] = ExpertSplit{ctas, pl.total_chunks / ctas};
